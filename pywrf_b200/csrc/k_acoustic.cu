@@ -147,22 +147,28 @@ __global__ void k_p_rho0(Grid g, S s) {
   s[WF_PM1][p] = pnew;
 }
 
-// calc_coef_w: a block owns 16 adjacent mass columns of one row and 16 level
-// groups; the per-level coefficients a, b, c are formed in parallel into
-// shared memory, one thread per column runs the recurrence alpha = 1 / (b - a
-// gamma), gamma = c alpha in the reference's order, and the levels are stored
-// in parallel again.
-constexpr int kCwTX = 16, kCwKT = 16;
+// calc_coef_w: a block owns 32 adjacent mass columns of one row (a warp's
+// lanes) and 8 level groups (its warps).  The per-level coefficients a, b, c
+// are formed over levels in parallel, every operand of a thread's levels in
+// flight at once; one warp then runs the recurrence alpha = 1 / (b - a
+// gamma), gamma = c alpha from shared memory in the reference's order, and
+// the levels are stored in parallel again.  Five field passes: the earlier
+// one-thread-per-column form waited on a memory round trip every few levels
+// and, below about 20 000 columns, left most of the chip idle.  Divisions by
+// mut^2 and the reciprocals are in their correctly rounded forms.
+constexpr int kCwTX = 32, kCwKT = 8;
 
-__global__ void __launch_bounds__(kCwTX * kCwKT) k_coef_w(Grid g, S s, float dts) {
-  __shared__ float sa[kMaxNz][kCwTX], sb[kMaxNz][kCwTX], sc[kMaxNz][kCwTX];
-  __shared__ float stop[2][kCwTX];  // atop, alpha at the top
-  const int tx = threadIdx.x % kCwTX, tk = threadIdx.x / kCwTX;
-  const int i = g.ids + blockIdx.x * kCwTX + tx, j = g.jds + blockIdx.y;
-  const bool col = i < g.ide - 1;
+__global__ void __launch_bounds__(kCwTX* kCwKT) k_coef_w(Grid g, S s, float dts, int i0) {
+  extern __shared__ float cw_smem[];
   const int nz = g.nz;
+  const int tx = threadIdx.x % kCwTX, tk = threadIdx.x / kCwTX;
+  float* const sa = cw_smem + tx;                  // [nz][32]: a
+  float* const sb = sa + nz * kCwTX;               // b, then alpha
+  float* const sc = sb + nz * kCwTX;               // c, then gamma
+  const int i = i0 + blockIdx.x * kCwTX + tx, j = g.jds + blockIdx.y;
+  const bool col = i >= g.ids && i < g.ide - 1;
   const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
-  const size_t lev = (size_t)g.ny * g.nx;
+  const int lev = g.ny * g.nx;
   const double cofd = (0.5 * (double)dts * G * (1.0 + (double)g.epssm)) * (0.5 * (double)dts * G * (1.0 + (double)g.epssm));
   const float cof = (float)cofd, cofm2 = (float)(-2.0 * cofd), cof2 = (float)(2.0 * cofd);
   const float* cqw = s[WF_CQW];
@@ -172,99 +178,55 @@ __global__ void __launch_bounds__(kCwTX * kCwKT) k_coef_w(Grid g, S s, float dts
   float* a = s[WF_A];
   float* alpha = s[WF_ALPHA];
   float* gamma = s[WF_GAMMA];
-  const float mut = col ? s[WF_MUT][c] : 1.f;
-  const float mm = mut * mut;
-  if (col) {
-    for (int k = 1 + tk; k < nz - 1; k += kCwKT) {
-      const size_t p = k * lev + c;
-      const float cw = __ldg(&cqw[p]), c2k = __ldg(&c2a[p]), c2m = __ldg(&c2a[p - lev]);
-      sa[k][tx] = k >= 2 ? -cw * cof * rdn[k] * rdnw[k - 1] * c2m / mm : 0.f;
-      sb[k][tx] = 1.0f + cw * cof * rdn[k] * (rdnw[k] * c2k / mm + rdnw[k - 1] * c2m / mm);
-      sc[k][tx] = -cw * cof * rdn[k] * rdnw[k] * c2k / mm;
-    }
+  const float mut = __ldg(&s[WF_MUT][c]);
+  const float c2t = __ldg(&c2a[(nz - 2) * lev + c]);
+  const float mm = mut * mut, r_mm = __frcp_rn(mm);
+#pragma unroll 4
+  for (int k = 1 + tk; k < nz - 1; k += kCwKT) {
+    const int p = k * lev + c;
+    const float cw = __ldg(&cqw[p]), c2k = __ldg(&c2a[p]), c2m = __ldg(&c2a[p - lev]);
+    const float rk = __ldg(&rdn[k]), rwk = __ldg(&rdnw[k]), rwm = __ldg(&rdnw[k - 1]);
+    sa[k * kCwTX] = k >= 2 ? divc(-cw * cof * rk * rwm * c2m, mm, r_mm) : 0.f;
+    sb[k * kCwTX] = 1.0f + cw * cof * rk * (divc(rwk * c2k, mm, r_mm) + divc(rwm * c2m, mm, r_mm));
+    sc[k * kCwTX] = divc(-cw * cof * rk * rwk * c2k, mm, r_mm);
   }
   __syncthreads();
-  if (col && tk == 0) {
+  if (tk == 0) {
     const float lid = g.top_lid ? 0.f : 1.f;
-    const float c2t = __ldg(&c2a[(nz - 2) * lev + c]);
-    const float atop = cofm2 * (rdnw[nz - 2] * rdnw[nz - 2]) * c2t * lid / mm;
+    const float rwt = __ldg(&rdnw[nz - 2]);
+    const float atop = divc(cofm2 * (rwt * rwt) * c2t * lid, mm, r_mm);
     float gm = 0.f;
+#pragma unroll 8
     for (int k = 1; k < nz - 1; ++k) {
-      const float al = 1.0f / (sb[k][tx] - sa[k][tx] * gm);
-      sb[k][tx] = al;  // alpha(k)
-      gm = sc[k][tx] * al;
-      sc[k][tx] = gm;  // gamma(k)
+      const float al = __frcp_rn(sb[k * kCwTX] - sa[k * kCwTX] * gm);
+      sb[k * kCwTX] = al;
+      gm = sc[k * kCwTX] * al;
+      sc[k * kCwTX] = gm;
     }
-    const float btop = 1.0f + cof2 * (rdnw[nz - 2] * rdnw[nz - 2]) * c2t / mm;
-    stop[0][tx] = atop;
-    stop[1][tx] = 1.0f / (btop - atop * gm);
+    const float btop = 1.0f + divc(cof2 * (rwt * rwt) * c2t, mm, r_mm);
+    sa[(nz - 1) * kCwTX] = atop;
+    sb[(nz - 1) * kCwTX] = __frcp_rn(btop - atop * gm);
+    sc[(nz - 1) * kCwTX] = 0.f;
+    sc[0] = 0.f;
   }
   __syncthreads();
   if (!col) return;
+#pragma unroll 4
   for (int k = tk; k < nz; k += kCwKT) {
-    const size_t p = k * lev + c;
-    if (k == 0) {
-      gamma[p] = 0.f;
-    } else if (k < nz - 1) {
-      a[p] = k >= 2 ? sa[k][tx] : 0.f;
-      alpha[p] = sb[k][tx];
-      gamma[p] = sc[k][tx];
-    } else {
-      a[p] = stop[0][tx];
-      alpha[p] = stop[1][tx];
-      gamma[p] = 0.f;
+    const int p = k * lev + c;
+    if (k > 0) {
+      a[p] = sa[k * kCwTX];
+      alpha[p] = sb[k * kCwTX];
     }
+    gamma[p] = sc[k * kCwTX];
   }
 }
 
-// calc_coef_w with one thread per mass column (32 x 4 columns per block): the
-// coefficients of level k are formed as the recurrence reaches it, so nothing
-// waits on a block barrier and every level's loads and stores are coalesced
-// across the warp.  The same operations as k_coef_w, in the same order (the
-// divisions by mut^2 and the reciprocals in their correctly rounded forms).
-__global__ void __launch_bounds__(128) k_coef_w_col(Grid g, S s, float dts) {
-  const int i = g.ids + blockIdx.x * 32 + threadIdx.x, j = g.jds + blockIdx.y * 4 + threadIdx.y;
-  if (i >= g.ide - 1 || j >= g.jde - 1) return;
-  const int nz = g.nz;
-  const int c = g.i2(j, i);
-  const size_t lev = (size_t)g.ny * g.nx;
-  const double cofd = (0.5 * (double)dts * G * (1.0 + (double)g.epssm)) * (0.5 * (double)dts * G * (1.0 + (double)g.epssm));
-  const float cof = (float)cofd, cofm2 = (float)(-2.0 * cofd), cof2 = (float)(2.0 * cofd);
-  const float* cqw = s[WF_CQW];
-  const float* c2a = s[WF_C2A];
-  const float* rdn = s[WF_RDN];
-  const float* rdnw = s[WF_RDNW];
-  float* a = s[WF_A];
-  float* alpha = s[WF_ALPHA];
-  float* gamma = s[WF_GAMMA];
-  const float mut = s[WF_MUT][c];
-  const float mm = mut * mut, r_mm = __frcp_rn(mm);
-  gamma[c] = 0.f;
-  float gm = 0.f;
-  float c2m = __ldg(&c2a[c]);
-#pragma unroll 4
-  for (int k = 1; k < nz - 1; ++k) {
-    const size_t p = k * lev + c;
-    const float cw = __ldg(&cqw[p]), c2k = __ldg(&c2a[p]);
-    const float rk = __ldg(&rdn[k]), rwk = __ldg(&rdnw[k]), rwm = __ldg(&rdnw[k - 1]);
-    const float ak = k >= 2 ? divc(-cw * cof * rk * rwm * c2m, mm, r_mm) : 0.f;
-    const float bk = 1.0f + cw * cof * rk * (divc(rwk * c2k, mm, r_mm) + divc(rwm * c2m, mm, r_mm));
-    const float ck = divc(-cw * cof * rk * rwk * c2k, mm, r_mm);
-    const float al = __frcp_rn(bk - ak * gm);
-    gm = ck * al;
-    a[p] = ak;
-    alpha[p] = al;
-    gamma[p] = gm;
-    c2m = c2k;
-  }
-  const float lid = g.top_lid ? 0.f : 1.f;
-  const float rwt = __ldg(&rdnw[nz - 2]);
-  const float atop = divc(cofm2 * (rwt * rwt) * c2m * lid, mm, r_mm);
-  const float btop = 1.0f + divc(cof2 * (rwt * rwt) * c2m, mm, r_mm);
-  const size_t pt = (size_t)(nz - 1) * lev + c;
-  a[pt] = atop;
-  alpha[pt] = __frcp_rn(btop - atop * gm);
-  gamma[pt] = 0.f;
+// columns of a 32-wide block start on a 32-byte sector when the rows do
+static void run_coef_w(const Grid& g, const S& s, float dts, cudaStream_t st) {
+  const int i0 = g.nx % 8 == 0 ? g.ids / 8 * 8 : g.ids;
+  k_coef_w<<<dim3((g.ide - 1 - i0 + kCwTX - 1) / kCwTX, g.jde - 1 - g.jds), kCwTX * kCwKT,
+             3 * g.nz * kCwTX * sizeof(float), st>>>(g, s, dts, i0);
 }
 
 __global__ void k_advance_uv(Grid g, S s, float dts) {
@@ -1124,12 +1086,7 @@ int launch_small_step_prep(const Grid& g, const S& s, int rk_step, float dts, cu
   k_ssp2d<<<col_grid(g, b2), b2, 0, st>>>(g, s, rk_step);
   k_ssp3d<<<point_grid(g, b3), b3, 0, st>>>(g, s, rk_step);
   k_p_rho0<<<point_grid(g, b3), b3, 0, st>>>(g, s);
-  if (kernel_form() == WRF_FORM_FAST) {
-    const dim3 bc(32, 4);
-    k_coef_w_col<<<dim3((g.ide - 1 - g.ids + 31) / 32, (g.jde - 1 - g.jds + 3) / 4), bc, 0, st>>>(g, s, dts);
-  } else {
-    k_coef_w<<<dim3((g.ide - 1 - g.ids + kCwTX - 1) / kCwTX, g.jde - 1 - g.jds), kCwTX * kCwKT, 0, st>>>(g, s, dts);
-  }
+  run_coef_w(g, s, dts, st);
   return 4;
 }
 
@@ -1152,7 +1109,7 @@ int launch_coef_w(const Grid& g, const float* mut, const float* cqw, const float
   s.f[WF_A] = a;
   s.f[WF_ALPHA] = alpha;
   s.f[WF_GAMMA] = gamma;
-  k_coef_w<<<dim3((g.ide - 1 - g.ids + kCwTX - 1) / kCwTX, g.jde - 1 - g.jds), kCwTX * kCwKT, 0, st>>>(g, s, dts);
+  run_coef_w(g, s, dts, st);
   return 1;
 }
 

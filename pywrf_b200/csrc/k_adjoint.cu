@@ -1546,168 +1546,304 @@ int launch_relax_field_adj(const Grid& g, const float* tbar, float* fbar, char v
   return 1;
 }
 
-__global__ void k_vsolve_w(int ncol, int nz, const float* x, const float* a, const float* alpha, const float* gamma,
-                           float* w) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncol) return;
+// The implicit solve and its reverse: a block owns 32 adjacent columns (a
+// warp's lanes) and 8 level groups (its warps).  All operands of the block's
+// columns are brought into shared memory in one memory round trip, single
+// warps run the sweeps from there, and the levels are stored in parallel.
+// One thread per column instead (57 600 at 240x240, 41 levels) waited on
+// memory once per level and kept its intermediates in local arrays: 43 us
+// forward and 121 us reverse, against five and thirteen field passes of
+// 9.45 MB.
+constexpr int kVsTX = 32, kVsKT = 8;
+
+__global__ void __launch_bounds__(kVsTX* kVsKT) k_vsolve_w(int ncol, int nz, const float* x, const float* a,
+                                                           const float* alpha, const float* gamma, float* w) {
+  extern __shared__ float vs_smem[];
+  const int tx = threadIdx.x % kVsTX, tk = threadIdx.x / kVsTX;
+  const int c = blockIdx.x * kVsTX + tx;
+  const bool col = c < ncol;
+  float* const sx = vs_smem + tx;  // x, then y, then w
+  float* const sa = sx + nz * kVsTX;
+  float* const sl = sa + nz * kVsTX;
+  float* const sg = sl + nz * kVsTX;
   const size_t lev = (size_t)ncol;
   const int kend = nz - 1;
-  float prev = x[c];
-  w[c] = prev;
-  for (int k = 1; k <= kend; ++k) {
-    const size_t p = k * lev + c;
-    prev = (x[p] - a[p] * prev) * alpha[p];
-    w[p] = prev;
+  if (col) {
+#pragma unroll 4
+    for (int k = tk; k <= kend; k += kVsKT) {
+      const size_t p = k * lev + c;
+      sx[k * kVsTX] = __ldg(&x[p]);
+      if (k == 0) continue;
+      sa[k * kVsTX] = __ldg(&a[p]);
+      sl[k * kVsTX] = __ldg(&alpha[p]);
+      sg[k * kVsTX] = __ldg(&gamma[p]);
+    }
   }
-  for (int k = kend - 1; k >= 1; --k) {
-    const size_t p = k * lev + c;
-    prev = w[p] - gamma[p] * prev;
-    w[p] = prev;
+  __syncthreads();
+  if (col && tk == 0) {
+    float prev = sx[0];
+#pragma unroll 8
+    for (int k = 1; k <= kend; ++k) {
+      prev = (sx[k * kVsTX] - sa[k * kVsTX] * prev) * sl[k * kVsTX];
+      sx[k * kVsTX] = prev;
+    }
+#pragma unroll 8
+    for (int k = kend - 1; k >= 1; --k) {
+      prev = sx[k * kVsTX] - sg[k * kVsTX] * prev;
+      sx[k * kVsTX] = prev;
+    }
   }
+  __syncthreads();
+  if (!col) return;
+#pragma unroll 4
+  for (int k = tk; k <= kend; k += kVsKT) w[k * lev + c] = sx[k * kVsTX];
 }
 
-__global__ void k_vsolve_w_adj(int ncol, int nz, const float* x, const float* a, const float* alpha,
-                               const float* gamma, const float* wbar, float* xbar, float* abar, float* alphabar,
-                               float* gammabar) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncol) return;
+// Warp 0 recomputes the forward (y up, z down) while warp 1 runs the two
+// reversed sweeps, which read the coefficients but not y or z; the products
+// of each level follow in parallel.
+__global__ void __launch_bounds__(kVsTX* kVsKT) k_vsolve_w_adj(int ncol, int nz, const float* x, const float* a,
+                                                               const float* alpha, const float* gamma,
+                                                               const float* wbar, float* xbar, float* abar,
+                                                               float* alphabar, float* gammabar) {
+  extern __shared__ float vs_smem[];
+  const int tx = threadIdx.x % kVsTX, tk = threadIdx.x / kVsTX;
+  const int c = blockIdx.x * kVsTX + tx;
+  const bool col = c < ncol;
+  const int n = nz * kVsTX;
+  float* const sx = vs_smem + tx;
+  float *const sa = sx + n, *const sl = sx + 2 * n, *const sg = sx + 3 * n, *const szb = sx + 4 * n;
+  float *const sy = sx + 5 * n, *const sz = sx + 6 * n, *const syb = sx + 7 * n;
   const size_t lev = (size_t)ncol;
   const int kend = nz - 1;
-  float y[kMaxNz], z[kMaxNz], zb[kMaxNz], yb[kMaxNz];
-  // forward recomputation
-  y[0] = x[c];
-  for (int k = 1; k <= kend; ++k) {
+  if (col) {
+#pragma unroll 4
+    for (int k = tk; k <= kend; k += kVsKT) {
+      const size_t p = k * lev + c;
+      sx[k * kVsTX] = __ldg(&x[p]);
+      szb[k * kVsTX] = __ldg(&wbar[p]);
+      if (k == 0) continue;
+      sa[k * kVsTX] = __ldg(&a[p]);
+      sl[k * kVsTX] = __ldg(&alpha[p]);
+      sg[k * kVsTX] = __ldg(&gamma[p]);
+    }
+  }
+  __syncthreads();
+  if (col && tk == 0) {
+    float prev = sx[0];
+    sy[0] = prev;
+#pragma unroll 8
+    for (int k = 1; k <= kend; ++k) {
+      prev = (sx[k * kVsTX] - sa[k * kVsTX] * prev) * sl[k * kVsTX];
+      sy[k * kVsTX] = prev;
+    }
+    sz[kend * kVsTX] = prev;
+#pragma unroll 8
+    for (int k = kend - 1; k >= 1; --k) {
+      prev = sy[k * kVsTX] - sg[k * kVsTX] * prev;
+      sz[k * kVsTX] = prev;
+    }
+  } else if (col && tk == 1) {
+    // back-substitution in reverse (it computed k = kend-1 down to 1)
+    float zb = szb[kVsTX];
+#pragma unroll 8
+    for (int k = 1; k <= kend - 1; ++k) {
+      zb = szb[(k + 1) * kVsTX] + -sg[k * kVsTX] * zb;
+      szb[(k + 1) * kVsTX] = zb;
+    }
+    // forward sweep in reverse (it computed k = 1 up to kend)
+    float yb = zb;
+    syb[kend * kVsTX] = yb;
+#pragma unroll 8
+    for (int k = kend; k >= 1; --k) {
+      yb = szb[(k - 1) * kVsTX] + -sa[k * kVsTX] * sl[k * kVsTX] * yb;
+      syb[(k - 1) * kVsTX] = yb;
+    }
+  }
+  __syncthreads();
+  if (!col) return;
+  float xo[kMaxNz / kVsKT], ao[kMaxNz / kVsKT], lo[kMaxNz / kVsKT], go[kMaxNz / kVsKT];
+#pragma unroll
+  for (int q = 0; q < kMaxNz / kVsKT; ++q) {
+    const int k = tk + q * kVsKT;
+    if (k > kend) continue;
     const size_t p = k * lev + c;
-    y[k] = (x[p] - a[p] * y[k - 1]) * alpha[p];
+    xo[q] = xbar[p];
+    if (k == 0) continue;
+    ao[q] = abar[p];
+    lo[q] = alphabar[p];
+    if (k < kend) go[q] = gammabar[p];
   }
-  z[kend] = y[kend];
-  for (int k = kend - 1; k >= 1; --k) z[k] = y[k] - gamma[k * lev + c] * z[k + 1];
-  z[0] = y[0];
-  for (int k = 0; k <= kend; ++k) {
-    zb[k] = wbar[k * lev + c];
-    yb[k] = 0.f;
-  }
-  // back-substitution in reverse (it computed k = kend-1 down to 1)
-  for (int k = 1; k <= kend - 1; ++k) {
+#pragma unroll
+  for (int q = 0; q < kMaxNz / kVsKT; ++q) {
+    const int k = tk + q * kVsKT;
+    if (k > kend) continue;
     const size_t p = k * lev + c;
-    yb[k] += zb[k];
-    gammabar[p] += -z[k + 1] * zb[k];
-    zb[k + 1] += -gamma[p] * zb[k];
+    const float yb = syb[k * kVsTX];
+    if (k == 0) {
+      xbar[p] = xo[q] + yb;
+      continue;
+    }
+    const float al = sl[k * kVsTX], ym = sy[(k - 1) * kVsTX];
+    xbar[p] = xo[q] + al * yb;
+    abar[p] = ao[q] + -ym * al * yb;
+    alphabar[p] = lo[q] + (sx[k * kVsTX] - sa[k * kVsTX] * ym) * yb;
+    if (k < kend) gammabar[p] = go[q] + -sz[(k + 1) * kVsTX] * szb[k * kVsTX];
   }
-  yb[kend] += zb[kend];
-  yb[0] += zb[0];
-  // forward sweep in reverse (it computed k = 1 up to kend)
-  for (int k = kend; k >= 1; --k) {
-    const size_t p = k * lev + c;
-    const float al = alpha[p], ak = a[p];
-    xbar[p] += al * yb[k];
-    abar[p] += -y[k - 1] * al * yb[k];
-    alphabar[p] += (x[p] - ak * y[k - 1]) * yb[k];
-    yb[k - 1] += -ak * al * yb[k];
-  }
-  xbar[c] += yb[0];
 }
 
 int launch_vsolve_w(int ncol, int nz, const float* x, const float* a, const float* alpha, const float* gamma, float* w,
                     cudaStream_t st) {
-  k_vsolve_w<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, nz, x, a, alpha, gamma, w);
+  k_vsolve_w<<<(ncol + kVsTX - 1) / kVsTX, kVsTX * kVsKT, 4 * nz * kVsTX * sizeof(float), st>>>(ncol, nz, x, a, alpha,
+                                                                                                gamma, w);
   return 1;
+}
+
+// a kernel whose dynamic shared memory can pass 48 KB has its limit raised
+// once per device
+template <typename K>
+static void allow_smem(K kernel, size_t bytes) {
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 int launch_vsolve_w_adj(int ncol, int nz, const float* x, const float* a, const float* alpha, const float* gamma,
                         const float* wbar, float* xbar, float* abar, float* alphabar, float* gammabar,
                         cudaStream_t st) {
-  k_vsolve_w_adj<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, nz, x, a, alpha, gamma, wbar, xbar, abar, alphabar,
-                                                      gammabar);
+  const size_t smem = 8 * (size_t)nz * kVsTX * sizeof(float);
+  allow_smem(k_vsolve_w_adj, smem);
+  k_vsolve_w_adj<<<(ncol + kVsTX - 1) / kVsTX, kVsTX * kVsKT, smem, st>>>(ncol, nz, x, a, alpha, gamma, wbar, xbar,
+                                                                          abar, alphabar, gammabar);
   return 1;
 }
 
-// one column of calc_coef_w's adjoint; the forward is k_coef_w (k_acoustic.cu)
-// (the cotangent arrays are the caller's own buffers, distinct from the
-// operands: __restrict__ lets the level loops' loads run ahead of their
-// stores)
-__global__ void k_coef_w_adj(Grid g, const float* __restrict__ mut_, const float* __restrict__ cqw,
-                             const float* __restrict__ c2a, const float* __restrict__ rdn,
-                             const float* __restrict__ rdnw, float dts, const float* __restrict__ abar,
-                             const float* __restrict__ alphabar, const float* __restrict__ gammabar,
-                             float* __restrict__ mutbar, float* __restrict__ cqwbar, float* __restrict__ c2abar) {
-  WRF_COLUMN_INDEX(g, j, i);
-  if (j < g.jds || j >= g.jde - 1 || i < g.ids || i >= g.ide - 1) return;
+// calc_coef_w's adjoint in the same layout (32 columns x 8 level groups): a,
+// b, c of every level in parallel, the recurrence forwards (alpha, gamma) and
+// then its transpose (the cotangent of gamma flowing down the column) by one
+// warp from shared memory, the products of each level in parallel.  One
+// thread per column took 116 us at 240x240x41 (nine field passes): six
+// divisions by mut^2 per level in a serial chain, and local arrays.
+__global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
+    Grid g, const float* __restrict__ mut_, const float* __restrict__ cqw, const float* __restrict__ c2a,
+    const float* __restrict__ rdn, const float* __restrict__ rdnw, float dts, const float* __restrict__ abar,
+    const float* __restrict__ alphabar, const float* __restrict__ gammabar, float* __restrict__ mutbar,
+    float* __restrict__ cqwbar, float* __restrict__ c2abar, int i0) {
+  extern __shared__ float vs_smem[];
   const int nz = g.nz;
-  const int c = g.i2(j, i);
-  const size_t lev = (size_t)g.ny * g.nx;
+  const int tx = threadIdx.x % kVsTX, tk = threadIdx.x / kVsTX;
+  const int i = i0 + blockIdx.x * kVsTX + tx, j = g.jds + blockIdx.y;
+  const bool col = i >= g.ids && i < g.ide - 1;
+  const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
+  const int lev = g.ny * g.nx;
+  const int n = nz * kVsTX;
+  float* const sa = vs_smem + tx;                                // a
+  float *const sb = sa + n, *const sc = sa + 2 * n;              // b (then the level's own c2a term), c
+  float *const sl = sa + 3 * n, *const sm = sa + 4 * n;          // alpha, gamma
+  float *const sg = sa + 5 * n, *const st = sa + 6 * n;          // gammabar (then its total, then the mut^2 term),
+                                                                 // alphabar (then the level below's c2a term)
   const double cofd = (0.5 * (double)dts * G * (1.0 + (double)g.epssm)) * (0.5 * (double)dts * G * (1.0 + (double)g.epssm));
   const float cof = (float)cofd, cofm2 = (float)(-2.0 * cofd), cof2 = (float)(2.0 * cofd);
   const float mut = mut_[c];
-  const float mm = mut * mut;
+  const float mm = mut * mut, r_mm = __frcp_rn(mm);
   const float lid = g.top_lid ? 0.f : 1.f;
-  float ak[kMaxNz], bk[kMaxNz], ck[kMaxNz], al[kMaxNz], gm[kMaxNz];
-  // forward recomputation (k_coef_w's arithmetic)
-  const float c2t = c2a[(nz - 2) * lev + c], rwt = rdnw[nz - 2];
-  const float atop = cofm2 * (rwt * rwt) * c2t * lid / mm;
-  gm[0] = 0.f;
 #pragma unroll 4
-  for (int k = 1; k < nz - 1; ++k) {
-    const size_t p = k * lev + c;
-    const float cw = cqw[p];
-    ak[k] = k >= 2 ? -cw * cof * rdn[k] * rdnw[k - 1] * c2a[p - lev] / mm : 0.f;
-    bk[k] = 1.0f + cw * cof * rdn[k] * (rdnw[k] * c2a[p] / mm + rdnw[k - 1] * c2a[p - lev] / mm);
-    ck[k] = -cw * cof * rdn[k] * rdnw[k] * c2a[p] / mm;
-    al[k] = 1.0f / (bk[k] - ak[k] * gm[k - 1]);
-    gm[k] = ck[k] * al[k];
+  for (int k = 1 + tk; k < nz; k += kVsKT) {
+    const int p = k * lev + c;
+    st[k * kVsTX] = alphabar[p];
+    if (k == nz - 1) continue;
+    sg[k * kVsTX] = gammabar[p];
+    const float cw = cqw[p], c2k = c2a[p], c2m = c2a[p - lev];
+    const float rk = rdn[k], rwk = rdnw[k], rwm = rdnw[k - 1];
+    sa[k * kVsTX] = k >= 2 ? divc(-cw * cof * rk * rwm * c2m, mm, r_mm) : 0.f;
+    sb[k * kVsTX] = 1.0f + cw * cof * rk * (divc(rwk * c2k, mm, r_mm) + divc(rwm * c2m, mm, r_mm));
+    sc[k * kVsTX] = divc(-cw * cof * rk * rwk * c2k, mm, r_mm);
   }
-  const float btop = 1.0f + cof2 * (rwt * rwt) * c2t / mm;
-  const float altop = 1.0f / (btop - atop * gm[nz - 2]);
-  // reverse
+  float c2t = 0.f, atopb = 0.f;
+  if (tk == 0) {
+    c2t = c2a[(nz - 2) * lev + c];
+    atopb = abar[(nz - 1) * lev + c];
+  }
+  __syncthreads();
   float mmb = 0.f, c2tb = 0.f;
-  float gmb = 0.f;  // cotangent of gm[k] flowing down from level k+1
-  {
-    const float alb = alphabar[(nz - 1) * lev + c];
+  if (tk == 0) {
+    float gm = 0.f;
+    sm[0] = 0.f;
+#pragma unroll 8
+    for (int k = 1; k < nz - 1; ++k) {
+      const float al = __frcp_rn(sb[k * kVsTX] - sa[k * kVsTX] * gm);
+      gm = sc[k * kVsTX] * al;
+      sl[k * kVsTX] = al;
+      sm[k * kVsTX] = gm;
+    }
+    const float rwt = rdnw[nz - 2];
+    const float atop = divc(cofm2 * (rwt * rwt) * c2t * lid, mm, r_mm);
+    const float btop = 1.0f + divc(cof2 * (rwt * rwt) * c2t, mm, r_mm);
+    const float altop = __frcp_rn(btop - atop * gm);
+    const float alb = st[(nz - 1) * kVsTX];
     const float bb = -altop * altop * alb;
-    const float atb = abar[(nz - 1) * lev + c] + altop * altop * gm[nz - 2] * alb;
-    gmb = altop * altop * atop * alb;
+    const float atb = atopb + altop * altop * gm * alb;
     // btop = 1 + cof2 rwt^2 c2t / mm ; atop = cofm2 rwt^2 c2t lid / mm
-    c2tb += bb * cof2 * (rwt * rwt) / mm + atb * cofm2 * (rwt * rwt) * lid / mm;
-    mmb += -bb * (btop - 1.0f) / mm - atb * atop / mm;
+    c2tb = divc(bb * cof2 * (rwt * rwt), mm, r_mm) + divc(atb * cofm2 * (rwt * rwt) * lid, mm, r_mm);
+    mmb = divc(-bb * (btop - 1.0f), mm, r_mm) - divc(atb * atop, mm, r_mm);
+    float gmb = altop * altop * atop * alb;  // cotangent of gamma(k) flowing down from level k+1
+#pragma unroll 8
+    for (int k = nz - 2; k >= 1; --k) {
+      const float g_k = sg[k * kVsTX] + gmb;
+      sg[k * kVsTX] = g_k;
+      const float al = sl[k * kVsTX];
+      gmb = al * al * sa[k * kVsTX] * (st[k * kVsTX] + g_k * sc[k * kVsTX]);
+    }
+    sb[(nz - 1) * kVsTX] = c2tb;
   }
-  float c2b_next = 0.f;  // cotangent of c2a at level k (from the k+1 step's c2a(k) terms)
+  __syncthreads();
 #pragma unroll 4
-  for (int k = nz - 2; k >= 1; --k) {
-    const size_t p = k * lev + c;
-    const float cw = cqw[p];
-    const float g_k = gammabar[p] + gmb;               // total cotangent of gm[k]
-    const float ccb = g_k * al[k];
-    const float alb = alphabar[p] + g_k * ck[k];        // total cotangent of al[k]
-    const float a2 = al[k] * al[k];
+  for (int k = 1 + tk; k < nz - 1; k += kVsKT) {
+    const int p = k * lev + c;
+    const float cw = cqw[p], c2k = c2a[p], c2m = c2a[p - lev];
+    const float rk = rdn[k], rwk = rdnw[k], rwm = rdnw[k - 1];
+    const float ak = sa[k * kVsTX], bk = sb[k * kVsTX], ck = sc[k * kVsTX], al = sl[k * kVsTX];
+    const float g_k = sg[k * kVsTX];
+    const float ccb = g_k * al;
+    const float alb = st[k * kVsTX] + g_k * ck;
+    const float a2 = al * al;
     const float bb = -a2 * alb;
-    const float akb = (k >= 2 ? abar[p] : 0.f) + a2 * gm[k - 1] * alb;
-    gmb = a2 * ak[k] * alb;                             // to gm[k-1]
-    const float base = cof * rdn[k] / mm;
-    const float c2k = c2a[p], c2m = c2a[p - lev];
-    // cqw
-    float cwb = bb * base * (rdnw[k] * c2k + rdnw[k - 1] * c2m) - ccb * base * rdnw[k] * c2k;
-    if (k >= 2) cwb += -akb * base * rdnw[k - 1] * c2m;
-    cqwbar[p] += cwb;
-    // c2a(k) and c2a(k-1)
-    float c2kb = bb * cw * base * rdnw[k] - ccb * cw * base * rdnw[k] + c2b_next;
-    float c2mb = bb * cw * base * rdnw[k - 1];
-    if (k >= 2) c2mb += -akb * cw * base * rdnw[k - 1];
-    if (k == nz - 2) c2kb += c2tb;
-    c2abar[p] += c2kb;
-    c2b_next = c2mb;
-    // mm
-    mmb += -bb * (bk[k] - 1.0f) / mm - ccb * ck[k] / mm - (k >= 2 ? akb * ak[k] / mm : 0.f);
+    const float akb = (k >= 2 ? abar[p] : 0.f) + a2 * sm[(k - 1) * kVsTX] * alb;
+    const float base = divc(cof * rk, mm, r_mm);
+    float cwb = bb * base * (rwk * c2k + rwm * c2m) - ccb * base * rwk * c2k;
+    float c2mb = bb * cw * base * rwm;
+    if (k >= 2) {
+      cwb += -akb * base * rwm * c2m;
+      c2mb += -akb * cw * base * rwm;
+    }
+    if (col) cqwbar[p] += cwb;
+    st[k * kVsTX] = c2mb;
+    sb[k * kVsTX] = bb * cw * base * rwk - ccb * cw * base * rwk;
+    sg[k * kVsTX] = divc(-bb * (bk - 1.0f), mm, r_mm) - divc(ccb * ck, mm, r_mm) -
+                    (k >= 2 ? divc(akb * ak, mm, r_mm) : 0.f);
   }
-  c2abar[c] += c2b_next;  // c2a(0), from level 1
-  mutbar[c] += mmb * 2.0f * mut;
+  __syncthreads();
+  if (!col) return;
+#pragma unroll 4
+  for (int k = tk; k < nz - 1; k += kVsKT) {
+    float v = k == 0 ? 0.f : sb[k * kVsTX];
+    v += k == nz - 2 ? 0.f : st[(k + 1) * kVsTX];
+    if (k == nz - 2) v += sb[(nz - 1) * kVsTX];
+    c2abar[k * lev + c] += v;
+  }
+  if (tk == 0) {
+#pragma unroll 8
+    for (int k = nz - 2; k >= 1; --k) mmb += sg[k * kVsTX];
+    mutbar[c] += mmb * 2.0f * mut;
+  }
 }
 
 int launch_coef_w_adj(const Grid& g, const float* mut, const float* cqw, const float* c2a, const float* rdn,
                       const float* rdnw, float dts, const float* abar, const float* alphabar, const float* gammabar,
                       float* mutbar, float* cqwbar, float* c2abar, cudaStream_t st) {
-  const dim3 b2(32, 8);
-  k_coef_w_adj<<<col_grid(g, b2), b2, 0, st>>>(g, mut, cqw, c2a, rdn, rdnw, dts, abar, alphabar, gammabar, mutbar,
-                                               cqwbar, c2abar);
+  const int i0 = g.nx % 8 == 0 ? g.ids / 8 * 8 : g.ids;
+  const size_t smem = 7 * (size_t)g.nz * kVsTX * sizeof(float);
+  allow_smem(k_coef_w_adj, smem);
+  k_coef_w_adj<<<dim3((g.ide - 1 - i0 + kVsTX - 1) / kVsTX, g.jde - 1 - g.jds), kVsTX * kVsKT, smem, st>>>(
+      g, mut, cqw, c2a, rdn, rdnw, dts, abar, alphabar, gammabar, mutbar, cqwbar, c2abar, i0);
   return 1;
 }
 
