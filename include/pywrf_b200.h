@@ -494,6 +494,17 @@ int wrf_wsm6(const WrfGrid* g, float* th, float* qv, float* qc, float* qr, float
              float delt, float* rainnc, float* rainncv, float* snownc, float* snowncv,
              float* graupelnc, float* graupelncv, float* sr, void* stream);
 
+/* wrf_wsm6's computation with caller scratch: its column part and its point
+ * processes run as separate kernels (delt < 240 s; the fused kernel
+ * otherwise).  work holds wrf_wsm6_work_floats floats (may be null when that
+ * is 0) and must not overlap the other arrays. */
+int wrf_wsm6_work_floats(const WrfGrid* g, float delt, size_t* floats);
+int wrf_wsm6_work(const WrfGrid* g, float* th, float* qv, float* qc, float* qr, float* qi, float* qs,
+                  float* qg, const float* rho, const float* pii, const float* p, const float* dz8w,
+                  float delt, float* rainnc, float* rainncv, float* snownc, float* snowncv,
+                  float* graupelnc, float* graupelncv, float* sr, float* work, size_t work_floats,
+                  void* stream);
+
 /* wrf_wsm6's computation without caller scratch and without any device
  * allocation; no counterpart in the reference.  For callers that pass only
  * the scheme's own arrays and must not allocate device memory themselves:

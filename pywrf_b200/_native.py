@@ -212,6 +212,10 @@ def lib() -> ctypes.CDLL:
     L.wrf_coef_w_adj.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 5 + [ctypes.c_float] + [vp] * 6 + [vp]
     L.wrf_wsm6.restype = ip
     L.wrf_wsm6.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 11 + [ctypes.c_float] + [vp] * 7 + [vp]
+    L.wrf_wsm6_work_floats.restype = ip
+    L.wrf_wsm6_work_floats.argtypes = [ctypes.POINTER(WrfGridC), ctypes.c_float, ctypes.POINTER(ctypes.c_size_t)]
+    L.wrf_wsm6_work.restype = ip
+    L.wrf_wsm6_work.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 11 + [ctypes.c_float] + [vp] * 8 + [ctypes.c_size_t, vp]
     L.wrf_wsm6_noalloc.restype = ip
     L.wrf_wsm6_noalloc.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 11 + [ctypes.c_float] + [vp] * 7 + [vp]
     L.wrf_status_read.restype = ip

@@ -31,22 +31,31 @@ __device__ __forceinline__ float n0sfac_of(float t) {
   return fmaxf(fminf(wexp(F(mp::ALPHA) * (F(mp::T0C) - t)), F(mp::N0SMAX / mp::N0S)), 1.0f);
 }
 
+// Most points hold no rain, snow or graupel: the powers, exponentials and
+// divisions of a species (a few hundred instructions together) are formed
+// under the condition that lets the reference's `where` chain take them, so a
+// warp whose lanes all lie outside branches around them.  What is taken is
+// the same expression either way.
+
 // slope_wsm6 (wrf_physics.py:2048-2104); the rain caps serve all species
 __device__ __forceinline__ void slope_point(float q0, float q1, float q2, float den, float denfac, float t, Slope& o) {
-  const float n0 = n0sfac_of(t);
-  const float lam[3] = {wpow(F(mp::PIDN0R) / (q0 * den), 0.25f), wpow(F(mp::PIDN0S) * n0 / (q1 * den), 0.25f),
-                        wpow(F(mp::PIDN0G) / (q2 * den), 0.25f)};
   const float be[3] = {F(mp::BVTR), F(mp::BVTS), F(mp::BVTG)};
   const float pv[3] = {F(mp::PVTR), F(mp::PVTS), F(mp::PVTG)};
   const float qq[3] = {q0, q1, q2};
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
-    const bool small = qq[m] <= F(mp::QCRMIN);
-    const float a = small ? F(mp::RSLOPERMAX) : 1.0f / lam[m];
-    o.rs[m] = a;
-    o.rb[m] = small ? F(mp::RSLOPERBMAX) : wpow(a, be[m]);
-    o.r2[m] = small ? F(mp::RSLOPER2MAX) : a * a;
-    o.r3[m] = small ? F(mp::RSLOPER3MAX) : a * a * a;
+    o.rs[m] = F(mp::RSLOPERMAX);
+    o.rb[m] = F(mp::RSLOPERBMAX);
+    o.r2[m] = F(mp::RSLOPER2MAX);
+    o.r3[m] = F(mp::RSLOPER3MAX);
+    if (!(qq[m] <= F(mp::QCRMIN))) {
+      const float num = m == 0 ? F(mp::PIDN0R) : m == 1 ? F(mp::PIDN0S) * n0sfac_of(t) : F(mp::PIDN0G);
+      const float a = 1.0f / wpow(num / (qq[m] * den), 0.25f);
+      o.rs[m] = a;
+      o.rb[m] = wpow(a, be[m]);
+      o.r2[m] = a * a;
+      o.r3[m] = a * a * a;
+    }
     const float v = pv[m] * o.rb[m] * denfac;
     o.vt[m] = qq[m] <= 0.f ? 0.f : v;
   }
@@ -54,23 +63,20 @@ __device__ __forceinline__ void slope_point(float q0, float q1, float q2, float 
 
 // terminal velocities alone (wrf_physics.py:1988-2046)
 __device__ __forceinline__ float vt_rain(float qr, float den, float denfac) {
-  const float lam = wpow(F(mp::PIDN0R) / (qr * den), 0.25f);
-  const float rs = qr <= F(mp::QCRMIN) ? F(mp::RSLOPERMAX) : 1.0f / lam;
-  const float rb = qr <= F(mp::QCRMIN) ? F(mp::RSLOPERBMAX) : wpow(rs, F(mp::BVTR));
+  float rb = F(mp::RSLOPERBMAX);
+  if (!(qr <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0R) / (qr * den), 0.25f), F(mp::BVTR));
   const float v = F(mp::PVTR) * rb * denfac;
   return qr <= 0.f ? 0.f : v;
 }
 __device__ __forceinline__ float vt_snow(float qs, float den, float denfac, float t) {
-  const float lam = wpow(F(mp::PIDN0S) * n0sfac_of(t) / (qs * den), 0.25f);
-  const float rs = qs <= F(mp::QCRMIN) ? F(mp::RSLOPERMAX) : 1.0f / lam;
-  const float rb = qs <= F(mp::QCRMIN) ? F(mp::RSLOPERBMAX) : wpow(rs, F(mp::BVTS));
+  float rb = F(mp::RSLOPERBMAX);
+  if (!(qs <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0S) * n0sfac_of(t) / (qs * den), 0.25f), F(mp::BVTS));
   const float v = F(mp::PVTS) * rb * denfac;
   return qs <= 0.f ? 0.f : v;
 }
 __device__ __forceinline__ float vt_graup(float qg, float den, float denfac) {
-  const float lam = wpow(F(mp::PIDN0G) / (qg * den), 0.25f);
-  const float rs = qg <= F(mp::QCRMIN) ? F(mp::RSLOPERMAX) : 1.0f / lam;
-  const float rb = qg <= F(mp::QCRMIN) ? F(mp::RSLOPERBMAX) : wpow(rs, F(mp::BVTG));
+  float rb = F(mp::RSLOPERBMAX);
+  if (!(qg <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0G) / (qg * den), 0.25f), F(mp::BVTG));
   const float v = F(mp::PVTG) * rb * denfac;
   return qg <= 0.f ? 0.f : v;
 }
@@ -86,8 +92,8 @@ __device__ __forceinline__ void fpvs(float t, float p, float& qs0, float& qs1) {
   float a = fminf(w1, 0.99f * p);
   a = F(mp::EP2) * a / (p - a);
   qs0 = fmaxf(a, F(mp::QMIN));
-  const float w0 = F(mp::PSAT) * wexp(wlog(tr) * F(xai)) * wexp(F(xbi) * (1.0f - tr));
-  float b = t < F(ttp) ? w0 : w1;
+  float b = w1;
+  if (t < F(ttp)) b = F(mp::PSAT) * wexp(wlog(tr) * F(xai)) * wexp(F(xbi) * (1.0f - tr));
   b = fminf(b, 0.99f * p);
   b = F(mp::EP2) * b / (p - b);
   qs1 = fmaxf(b, F(mp::QMIN));
@@ -128,16 +134,17 @@ __device__ void wsm6_point(float& t, float& q, float& qc0, float& qc1, float& qr
       t = t + xlf3 / cpm * qc0;
       qc0 = 0.f;
     }
-    const float pfrzdtc = fminf(F(mp::PFRZ1) * (wexp(F(mp::PFRZ2) * fminf(supcol, 50.0f)) - 1.0f) * den / F(mp::DENR) /
-                                    F(mp::XNCR) * qc0 * qc0 * dtcld, qc0);
     if (supcol > 0.f && qc0 > F(mp::QMIN)) {
+      const float pfrzdtc = fminf(F(mp::PFRZ1) * (wexp(F(mp::PFRZ2) * fminf(supcol, 50.0f)) - 1.0f) * den /
+                                      F(mp::DENR) / F(mp::XNCR) * qc0 * qc0 * dtcld, qc0);
       qc1 = qc1 + pfrzdtc;
       t = t + xlf3 / cpm * pfrzdtc;
       qc0 = qc0 - pfrzdtc;
     }
-    const float pfrzdtr = fminf(F(20.0 * mp::PI * mp::PI * mp::PFRZ1 * mp::N0R * mp::DENR) / den *
-                                    (wexp(F(mp::PFRZ2) * fminf(supcol, 50.0f)) - 1.0f) * r30pre * r30pre * rs0pre * dtcld, qr0);
     if (supcol > 0.f && qr0 > 0.f) {
+      const float pfrzdtr = fminf(F(20.0 * mp::PI * mp::PI * mp::PFRZ1 * mp::N0R * mp::DENR) / den *
+                                      (wexp(F(mp::PFRZ2) * fminf(supcol, 50.0f)) - 1.0f) * r30pre * r30pre * rs0pre *
+                                      dtcld, qr0);
       qr2 = qr2 + pfrzdtr;
       t = t + xlf3 / cpm * pfrzdtr;
       qr0 = qr0 - pfrzdtr;
@@ -145,12 +152,17 @@ __device__ void wsm6_point(float& t, float& q, float& qc0, float& qc1, float& qr
   }
   Slope sl;
   slope_point(qr0, qr1, qr2, den, denfac, t, sl);
-  const float work1_0 = diffac(xl, p, t, den, qs0);
-  const float work1_1 = diffac(F(mp::XLS), p, t, den, qs1);
-  float work2 = venfac(p, t, den);
+  // diffac and venfac serve the processes of rain, snow, graupel and ice only
+  const bool precip = qr0 > 0.f || qr1 > 0.f || qr2 > 0.f;
+  float work1_0 = 1.f, work1_1 = 1.f, work2 = 0.f;
+  if (precip) {
+    work1_0 = diffac(xl, p, t, den, qs0);
+    work2 = venfac(p, t, den);
+  }
+  if (t0c - t > 0.f && (precip || qc1 > 0.f)) work1_1 = diffac(F(mp::XLS), p, t, den, qs1);
   float supsat = fmaxf(q, F(mp::QMIN)) - qs0;
-  float praut = F(mp::QCK1) * wpow(qc0, F(7.0 / 3.0));
-  praut = qc0 > F(mp::QC0) ? fminf(praut, qc0 / dtcld) : 0.f;
+  float praut = 0.f;
+  if (qc0 > F(mp::QC0)) praut = fminf(F(mp::QCK1) * wpow(qc0, F(7.0 / 3.0)), qc0 / dtcld);
   float pracw = (qr0 > F(mp::QCRMIN) && qc0 > F(mp::QMIN))
                     ? fminf(F(mp::PACRR) * sl.r3[0] * sl.rb[0] * qc0 * denfac, qc0 / dtcld) : 0.f;
   float prevp = 0.f;
@@ -166,21 +178,24 @@ __device__ void wsm6_point(float& t, float& q, float& qc0, float& qc1, float& qr
     if (c3) prevp = fminf(prevp, supsat / dtcld / 2.0f);
   }
   supcol = t0c - t;
-  const float n0sfac = fmaxf(fminf(wexp(F(mp::ALPHA) * supcol), F(mp::N0SMAX / mp::N0S)), 1.0f);
+  float n0sfac = 1.0f;
+  if (qr1 > 0.f) n0sfac = fmaxf(fminf(wexp(F(mp::ALPHA) * supcol), F(mp::N0SMAX / mp::N0S)), 1.0f);
   supsat = fmaxf(q, F(mp::QMIN)) - qs1;
   const float satdt = supsat / dtcld;
   bool ifsat = false;
-  const float xni = fminf(fmaxf(5.38e7f * wpow(den * fmaxf(qc1, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
-  const float eacrs = wexp(0.07f * (-supcol));
-  const float xmi = den * qc1 / xni;
-  const float diameter = fminf(F(mp::DICON) * sqrtf(xmi), F(mp::DIMAX));
-  const float vt2i = 1.49e4f * wpow(diameter, 1.31f);
+  float xni = 1.0e3f, diameter = 0.f, vt2i = 0.f;  // of the cloud ice: its processes need T < T0
+  if (supcol > 0.f && qc1 > 0.f) {
+    xni = fminf(fmaxf(5.38e7f * wpow(den * fmaxf(qc1, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+    const float xmi = den * qc1 / xni;
+    diameter = fminf(F(mp::DICON) * sqrtf(xmi), F(mp::DIMAX));
+    if (precip) vt2i = 1.49e4f * wpow(diameter, 1.31f);
+  }
   const float vt2r = F(mp::PVTR) * sl.rb[0] * denfac;
   const float vt2s = F(mp::PVTS) * sl.rb[1] * denfac;
   const float vt2g = F(mp::PVTG) * sl.rb[2] * denfac;
   const float qsum = fmaxf(qr1 + qr2, 1.0e-15f);
-  float vt2ave = (vt2s * qr1 + vt2g * qr2) / qsum;
-  if (!(qsum > 1.0e-15f)) vt2ave = 0.f;
+  float vt2ave = 0.f;
+  if (qsum > 1.0e-15f) vt2ave = (vt2s * qr1 + vt2g * qr2) / qsum;
   const bool cnd = supcol > 0.f && qc1 > F(mp::QMIN);
   const float pi_ = F(mp::PI);
   float praci = 0.f, piacr = 0.f, psaci = 0.f, pgaci = 0.f;
@@ -191,6 +206,7 @@ __device__ void wsm6_point(float& t, float& q, float& qc0, float& qc1, float& qr
                       (sl.r3[0] * sl.r3[0]) * sl.rb[0] / 24.0f / den, qr0 / dtcld);
   }
   if (qr1 > F(mp::QCRMIN) && cnd) {
+    const float eacrs = wexp(0.07f * (-supcol));
     const float acrfac = 2.0f * sl.r3[1] + 2.0f * diameter * sl.r2[1] + diameter * diameter * sl.rs[1];
     psaci = fminf(pi_ * qc1 * eacrs * F(mp::N0S) * n0sfac * fabsf(vt2ave - vt2i) * acrfac / 4.0f, qc1 / dtcld);
   }
@@ -701,19 +717,7 @@ __device__ void wsm6_column_w(const Seg<SEG, NS>& g, WCol<NS>& c, float delt, Pr
     cpm[s] = c.q[s] >= F(mp::QMIN) ? F(mp::CPV) * c.q[s] + (1.0f - c.q[s]) * F(mp::CPD)
                                    : F(mp::CPD * (1.0 - mp::QMIN) + mp::CPV * mp::QMIN);
     xl[s] = F(mp::XLV0) - F(mp::XLV1) * (c.t[s] - t0c);
-    const int k = g.k(s);
-    if (k < km) sc.dz[k] = c.delz[s];
   }
-  __syncwarp();
-  if (g.l == 0) {
-    float z = 0.f;
-    sc.zi[0] = z;
-    for (int k = 0; k < km; ++k) {
-      z = z + sc.dz[k];
-      sc.zi[k + 1] = z;
-    }
-  }
-  __syncwarp();
   const float dz0 = __shfl_sync(kFull, c.delz[0], 0, SEG);
   pr.rainncv = 0.f;
   pr.snowncv = 0.f;
@@ -723,88 +727,126 @@ __device__ void wsm6_column_w(const Seg<SEG, NS>& g, WCol<NS>& c, float delt, Pr
   const float dtcld = ((double)delt <= mp::DTCLDCR) ? delt : F(1.0 * (double)delt / loops);
   const int nloop = (int)loops;
   for (int loop = 0; loop < nloop; ++loop) {
+    bool mass = false;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      denfac[s] = sqrtf(1.0f / c.den[s] * F(mp::DEN0));
-      fpvs(c.t[s], c.p[s], qs0[s], qs1[s]);
-      Slope sl;
-      slope_point(c.qr0[s], c.qr1[s], c.qr2[s], c.den[s], denfac[s], c.t[s], sl);
-      const float qsum = fmaxf(c.qr1[s] + c.qr2[s], 1.0e-15f);
-      ww2[s] = qsum > 1.0e-15f ? (sl.vt[1] * c.qr1[s] + sl.vt[2] * c.qr2[s]) / qsum : 0.f;
-      ww[s] = c.qr0[s] <= 0.f ? 0.f : sl.vt[0];
-      rq[s] = c.den[s] * c.qr0[s];
-      rq2[s] = c.den[s] * c.qr1[s];
-      rq3[s] = c.den[s] * c.qr2[s];
-    }
-    // sedimentation of rain, then of snow + graupel
-    const float delq1 = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 1, sc);
-    float delq2, delq3;
-    nislfv6_w<SEG, NS>(g, c.den, denfac, c.t, c.delz, ww2, rq2, rq3, dtcld, 1, sc, &delq2, &delq3);
-    const float fall0 = delq1 / dz0 / dtcld, fall1 = delq2 / dz0 / dtcld, fall2 = delq3 / dz0 / dtcld;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const float den = c.den[s];
-      c.qr0[s] = fmaxf(rq[s] / den, 0.0f);
-      c.qr1[s] = fmaxf(rq2[s] / den, 0.0f);
-      c.qr2[s] = fmaxf(rq3[s] / den, 0.0f);
-      qr0s[s] = c.qr0[s];
-      Slope sl;
-      slope_point(c.qr0[s], c.qr1[s], c.qr2[s], den, denfac[s], c.t[s], sl);
-      rs0[s] = sl.rs[0];
-      r30[s] = sl.r3[0];
-      // melting of snow, then graupel
-      float t = c.t[s];
-      const float n0sfac = n0sfac_of(t);
-      const bool cond = t > t0c;
-      const float work2 = cond ? venfac(c.p[s], t, den) : 0.f;
-      const float xlf = F(mp::XLF0);
-      if (c.qr1[s] > 0.f && cond) {
-        const float coeres = sl.r2[1] * sqrtf(sl.rs[1] * sl.rb[1]);
-        float psmlt = xka(t, den) / xlf * (t0c - t) * F(mp::PI) / 2.0f * n0sfac *
-                      (F(mp::PRECS1) * sl.r2[1] + F(mp::PRECS2) * work2 * coeres) / den;
-        psmlt = fminf(fmaxf(psmlt * dtcld / 1.0f, -c.qr1[s] / 1.0f), 0.0f);
-        c.qr1[s] = c.qr1[s] + psmlt;
-        c.qr0[s] = c.qr0[s] - psmlt;
-        t = t + xlf / cpm[s] * psmlt;
+      mass |= g.k(s) < km && (c.qr0[s] > 0.f || c.qr1[s] > 0.f || c.qr2[s] > 0.f || c.qc1[s] > 0.f);
+      if constexpr (kPoint) {
+        denfac[s] = sqrtf(1.0f / c.den[s] * F(mp::DEN0));
+        fpvs(c.t[s], c.p[s], qs0[s], qs1[s]);
+        rs0[s] = F(mp::RSLOPERMAX);
+        r30[s] = F(mp::RSLOPER3MAX);
       }
-      if (c.qr2[s] > 0.f && cond) {
-        const float coeres = sl.r2[2] * sqrtf(sl.rs[2] * sl.rb[2]);
-        float pgmlt = xka(t, den) / xlf * (t0c - t) * (F(mp::PRECG1) * sl.r2[2] + F(mp::PRECG2) * work2 * coeres) / den;
-        pgmlt = fminf(fmaxf(pgmlt * dtcld / 1.0f, -c.qr2[s] / 1.0f), 0.0f);
-        c.qr2[s] = c.qr2[s] + pgmlt;
-        c.qr0[s] = c.qr0[s] - pgmlt;
-        t = t + xlf / cpm[s] * pgmlt;
-      }
-      c.t[s] = t;
-      // cloud-ice fall speed (ice number from the loop-start ice)
-      const float qi = c.qc1[s];
-      const float xni = fminf(fmaxf(5.387e7f * wpow(den * fmaxf(qi, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
-      float wt = fmaxf(fminf(F(mp::DICON) * sqrtf(den * qi / xni), F(mp::DIMAX)), 1.0e-25f);
-      wt = 1.49e4f * wexp(wlog(wt) * 1.31f);
-      ww[s] = qi <= 0.f ? 0.f : wt;
-      rq[s] = den * qi;
+      qr0s[s] = 0.f;
     }
-    const float delqi = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 0, sc);
+    // Nothing falls or melts in any column of the warp (the vote is over the
+    // whole warp, so every lane takes the same way): the sedimentation leaves
+    // zeros, the temperature and the precipitation as they are.
+    if (__ballot_sync(kFull, mass) != 0u) {
+      // depths and interface heights of the column
 #pragma unroll
-    for (int s = 0; s < NS; ++s) c.qc1[s] = fmaxf(rq[s] / c.den[s], 0.0f);
-    const float fallc = delqi / dz0 / dtcld;
-    const float fallsum = fall0 + fall1 + fall2 + fallc;
-    const float fallsum_qsi = fall1 + fallc;
-    const float fallsum_qg = fall2;
-    auto acc = [&](float fs) { return fs * dz0 / F(mp::DENR) * dtcld * 1000.0f; };
-    if (fallsum > 0.f) {
-      pr.rainncv = acc(fallsum) + pr.rainncv;
-      pr.rain = acc(fallsum) + pr.rain;
+      for (int s = 0; s < NS; ++s)
+        if (g.k(s) < km) sc.dz[g.k(s)] = c.delz[s];
+      __syncwarp();
+      if (g.l == 0) {
+        float z = 0.f;
+        sc.zi[0] = z;
+        for (int k = 0; k < km; ++k) {
+          z = z + sc.dz[k];
+          sc.zi[k + 1] = z;
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        if constexpr (!kPoint) denfac[s] = sqrtf(1.0f / c.den[s] * F(mp::DEN0));
+        Slope sl;
+        slope_point(c.qr0[s], c.qr1[s], c.qr2[s], c.den[s], denfac[s], c.t[s], sl);
+        const float qsum = fmaxf(c.qr1[s] + c.qr2[s], 1.0e-15f);
+        ww2[s] = qsum > 1.0e-15f ? (sl.vt[1] * c.qr1[s] + sl.vt[2] * c.qr2[s]) / qsum : 0.f;
+        ww[s] = c.qr0[s] <= 0.f ? 0.f : sl.vt[0];
+        rq[s] = c.den[s] * c.qr0[s];
+        rq2[s] = c.den[s] * c.qr1[s];
+        rq3[s] = c.den[s] * c.qr2[s];
+      }
+      // sedimentation of rain, then of snow + graupel
+      const float delq1 = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 1, sc);
+      float delq2, delq3;
+      nislfv6_w<SEG, NS>(g, c.den, denfac, c.t, c.delz, ww2, rq2, rq3, dtcld, 1, sc, &delq2, &delq3);
+      const float fall0 = delq1 / dz0 / dtcld, fall1 = delq2 / dz0 / dtcld, fall2 = delq3 / dz0 / dtcld;
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const float den = c.den[s];
+        c.qr0[s] = fmaxf(rq[s] / den, 0.0f);
+        c.qr1[s] = fmaxf(rq2[s] / den, 0.0f);
+        c.qr2[s] = fmaxf(rq3[s] / den, 0.0f);
+        qr0s[s] = c.qr0[s];
+        // melting of snow, then graupel
+        float t = c.t[s];
+        const bool cond = t > t0c;
+        const bool melt = cond && (c.qr1[s] > 0.f || c.qr2[s] > 0.f);
+        Slope sl;
+        if (kPoint || melt) slope_point(c.qr0[s], c.qr1[s], c.qr2[s], den, denfac[s], t, sl);
+        if constexpr (kPoint) {
+          rs0[s] = sl.rs[0];
+          r30[s] = sl.r3[0];
+        }
+        const float work2 = melt ? venfac(c.p[s], t, den) : 0.f;
+        const float xlf = F(mp::XLF0);
+        if (c.qr1[s] > 0.f && cond) {
+          const float n0sfac = n0sfac_of(t);
+          const float coeres = sl.r2[1] * sqrtf(sl.rs[1] * sl.rb[1]);
+          float psmlt = xka(t, den) / xlf * (t0c - t) * F(mp::PI) / 2.0f * n0sfac *
+                        (F(mp::PRECS1) * sl.r2[1] + F(mp::PRECS2) * work2 * coeres) / den;
+          psmlt = fminf(fmaxf(psmlt * dtcld / 1.0f, -c.qr1[s] / 1.0f), 0.0f);
+          c.qr1[s] = c.qr1[s] + psmlt;
+          c.qr0[s] = c.qr0[s] - psmlt;
+          t = t + xlf / cpm[s] * psmlt;
+        }
+        if (c.qr2[s] > 0.f && cond) {
+          const float coeres = sl.r2[2] * sqrtf(sl.rs[2] * sl.rb[2]);
+          float pgmlt = xka(t, den) / xlf * (t0c - t) * (F(mp::PRECG1) * sl.r2[2] + F(mp::PRECG2) * work2 * coeres) / den;
+          pgmlt = fminf(fmaxf(pgmlt * dtcld / 1.0f, -c.qr2[s] / 1.0f), 0.0f);
+          c.qr2[s] = c.qr2[s] + pgmlt;
+          c.qr0[s] = c.qr0[s] - pgmlt;
+          t = t + xlf / cpm[s] * pgmlt;
+        }
+        c.t[s] = t;
+        // cloud-ice fall speed (ice number from the loop-start ice)
+        const float qi = c.qc1[s];
+        ww[s] = 0.f;
+        if (!(qi <= 0.f)) {
+          const float xni = fminf(fmaxf(5.387e7f * wpow(den * fmaxf(qi, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+          const float wt = fmaxf(fminf(F(mp::DICON) * sqrtf(den * qi / xni), F(mp::DIMAX)), 1.0e-25f);
+          ww[s] = 1.49e4f * wexp(wlog(wt) * 1.31f);
+        }
+        rq[s] = den * qi;
+      }
+      const float delqi = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 0, sc);
+#pragma unroll
+      for (int s = 0; s < NS; ++s) c.qc1[s] = fmaxf(rq[s] / c.den[s], 0.0f);
+      const float fallc = delqi / dz0 / dtcld;
+      const float fallsum = fall0 + fall1 + fall2 + fallc;
+      const float fallsum_qsi = fall1 + fallc;
+      const float fallsum_qg = fall2;
+      auto acc = [&](float fs) { return fs * dz0 / F(mp::DENR) * dtcld * 1000.0f; };
+      if (fallsum > 0.f) {
+        pr.rainncv = acc(fallsum) + pr.rainncv;
+        pr.rain = acc(fallsum) + pr.rain;
+      }
+      if (fallsum_qsi > 0.f) {
+        pr.snowncv = acc(fallsum_qsi) + pr.snowncv;
+        pr.snow = acc(fallsum_qsi) + pr.snow;
+      }
+      if (fallsum_qg > 0.f) {
+        pr.graupelncv = acc(fallsum_qg) + pr.graupelncv;
+        pr.graupel = acc(fallsum_qg) + pr.graupel;
+      }
+      if (fallsum > 0.f) pr.sr = (pr.snowncv + pr.graupelncv) / (pr.rainncv + 1.0e-12f);
+    } else {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) c.qr0[s] = c.qr1[s] = c.qr2[s] = c.qc1[s] = 0.f;
     }
-    if (fallsum_qsi > 0.f) {
-      pr.snowncv = acc(fallsum_qsi) + pr.snowncv;
-      pr.snow = acc(fallsum_qsi) + pr.snow;
-    }
-    if (fallsum_qg > 0.f) {
-      pr.graupelncv = acc(fallsum_qg) + pr.graupelncv;
-      pr.graupel = acc(fallsum_qg) + pr.graupel;
-    }
-    if (fallsum > 0.f) pr.sr = (pr.snowncv + pr.graupelncv) / (pr.rainncv + 1.0e-12f);
     if constexpr (kPoint) {
 #pragma unroll
       for (int s = 0; s < NS; ++s)
@@ -1167,9 +1209,10 @@ __device__ __forceinline__ void wsm6_finish_point(const Grid& g, const S& s, int
     const float mpten = t / pii - th;
     T = T + mpten;
     s[WF_T][p] = T;
-    s[WF_H_DIABATIC][p] = mpten / dt;
-    s[WF_QV_DIABATIC][p] = (q - qvnew) / dt;
-    s[WF_QC_DIABATIC][p] = (qc0 - qcold) / dt;
+    const float r_dt = __frcp_rn(dt);
+    s[WF_H_DIABATIC][p] = divc(mpten, dt, r_dt);
+    s[WF_QV_DIABATIC][p] = divc(q - qvnew, dt, r_dt);
+    s[WF_QC_DIABATIC][p] = divc(qc0 - qcold, dt, r_dt);
     qvnew = q;
     M[n3 + p] = q;
     M[2 * n3 + p] = qc0;
@@ -1540,6 +1583,46 @@ int launch_wsm6(const Grid& g, float* const* f, float delt, cudaStream_t st) {
   return 1;
 }
 
+static double time_split(float delt) { return fmax((double)delt / mp::DTCLDCR, 1.0); }
+static int time_split_loops(float delt) { return (int)time_split(delt); }
+
+// the split form on caller arrays (one time-split loop): the column part, then
+// the point processes, with the two intermediates of the scheme's block in
+// scr_t and scr_qr0s
+static int launch_wsm6_split(const Grid& g, const Wsm6Args& a, float delt, float* scr_t, float* scr_qr0s,
+                             cudaStream_t st) {
+  const int ncol = g.ide - 2 - (g.ids + 1), nrow = g.jde - 2 - (g.jds + 1);
+  const dim3 b(32 * kWarpsPerBlock);
+  if (g.nz - 1 <= 47) {
+    constexpr int SPB = kWarpsPerBlock * 2;
+    k_wsm6_sed_args<16, 3><<<dim3((ncol + SPB - 1) / SPB, nrow), b, 0, st>>>(g, a, delt, scr_t, scr_qr0s);
+  } else {
+    constexpr int SPB = kWarpsPerBlock;
+    k_wsm6_sed_args<32, 2><<<dim3((ncol + SPB - 1) / SPB, nrow), b, 0, st>>>(g, a, delt, scr_t, scr_qr0s);
+  }
+  const float dtcld = ((double)delt <= mp::DTCLDCR) ? delt : (float)(1.0 * (double)delt / time_split(delt));
+  const dim3 b3(32, 4);
+  k_wsm6_finish_args<<<point_grid(g, b3), b3, 0, st>>>(g, a, dtcld, scr_t, scr_qr0s);
+  return 2;
+}
+
+// one intermediate field of the split form: the scheme's block
+static size_t wsm6_block_points(const Grid& g) {
+  return (size_t)(g.nz - 1) * (size_t)(g.jde - g.jds - 3) * (size_t)(g.ide - g.ids - 3);
+}
+
+size_t wsm6_work_floats(const Grid& g, float delt) { return time_split_loops(delt) == 1 ? 2 * wsm6_block_points(g) : 0; }
+
+// The split form with caller scratch where one time-split loop suffices: the
+// point processes on one thread per point branch on neighbouring points' states
+// instead of a column's levels, in a third of the fused kernel's registers.
+int launch_wsm6_work(const Grid& g, float* const* f, float delt, float* work, cudaStream_t st) {
+  if (time_split_loops(delt) != 1) return launch_wsm6(g, f, delt, st);
+  const Wsm6Args a{f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], f[9], f[10],
+                   f[11], f[12], f[13], f[14], f[15], f[16], f[17]};
+  return launch_wsm6_split(g, a, delt, work, work + wsm6_block_points(g), st);
+}
+
 // The scratch's device address is looked up by the first call in each CUDA
 // context (cudaGetSymbolAddress, with the context's device current) and kept
 // with that context's handle: after a device reset the new primary context
@@ -1561,15 +1644,11 @@ CtxGetCurrentFn ctx_get_current() {
 }  // namespace
 
 int launch_wsm6_noalloc(const Grid& g, float* const* f, float delt, cudaStream_t st, const char** err) {
-  const int km = g.nz - 1;
-  const int ncol = g.ide - 2 - (g.ids + 1), nrow = g.jde - 2 - (g.jds + 1);
-  const size_t npts = (size_t)km * (size_t)nrow * (size_t)ncol;
-  if (npts > kNoAllocMaxPoints) {
+  if (wsm6_block_points(g) > kNoAllocMaxPoints) {
     *err = "wrf_wsm6_noalloc: the scheme's block exceeds the fixed scratch (2097152 points per field)";
     return WRF_EINVAL;
   }
-  const double loops = fmax((double)delt / mp::DTCLDCR, 1.0);
-  if ((int)loops != 1) {
+  if (time_split_loops(delt) != 1) {
     *err = "wrf_wsm6_noalloc: delt >= 240 s needs two time-split loops; use wrf_wsm6";
     return WRF_EINVAL;
   }
@@ -1607,18 +1686,7 @@ int launch_wsm6_noalloc(const Grid& g, float* const* f, float delt, cudaStream_t
   }
   Wsm6Args a{f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8], f[9], f[10],
              f[11], f[12], f[13], f[14], f[15], f[16], f[17]};
-  const dim3 b(32 * kWarpsPerBlock);
-  if (km <= 47) {
-    constexpr int SPB = kWarpsPerBlock * 2;
-    k_wsm6_sed_args<16, 3><<<dim3((ncol + SPB - 1) / SPB, nrow), b, 0, st>>>(g, a, delt, base, base + kNoAllocMaxPoints);
-  } else {
-    constexpr int SPB = kWarpsPerBlock;
-    k_wsm6_sed_args<32, 2><<<dim3((ncol + SPB - 1) / SPB, nrow), b, 0, st>>>(g, a, delt, base, base + kNoAllocMaxPoints);
-  }
-  const float dtcld = ((double)delt <= mp::DTCLDCR) ? delt : (float)(1.0 * (double)delt / loops);
-  const dim3 b3(32, 4);
-  k_wsm6_finish_args<<<point_grid(g, b3), b3, 0, st>>>(g, a, dtcld, base, base + kNoAllocMaxPoints);
-  return 2;
+  return launch_wsm6_split(g, a, delt, base, base + kNoAllocMaxPoints, st);
 }
 
 

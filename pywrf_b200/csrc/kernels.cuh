@@ -180,6 +180,9 @@ int launch_bdy_final_op_adj(const Grid& g, const S& s, const S& b, cudaStream_t 
 // microphysics (k_wsm6.cu)
 int launch_physics(const Grid& g, const S& s, cudaStream_t st);
 int launch_wsm6(const Grid& g, float* const* f, float delt, cudaStream_t st);
+// the same with caller scratch of wsm6_work_floats(g, delt) floats
+size_t wsm6_work_floats(const Grid& g, float delt);
+int launch_wsm6_work(const Grid& g, float* const* f, float delt, float* work, cudaStream_t st);
 // WSM6 with a fixed file-scope device scratch (returns kernels or WRF_E*, *err set)
 int launch_wsm6_noalloc(const Grid& g, float* const* f, float delt, cudaStream_t st, const char** err);
 

@@ -1352,6 +1352,36 @@ int wrf_wsm6(const WrfGrid* gin, float* th, float* qv, float* qc, float* qr, flo
   return check_launch("wsm6");
 }
 
+int wrf_wsm6_work_floats(const WrfGrid* gin, float delt, size_t* floats) {
+  Grid g;
+  int rc = make_grid(gin, g);
+  if (rc) return rc;
+  if (!floats) return fail(WRF_EINVAL, "null argument");
+  if (!(delt > 0.f)) return fail(WRF_EINVAL, "delt must be > 0");
+  *floats = wsm6_work_floats(g, delt);
+  return WRF_OK;
+}
+
+int wrf_wsm6_work(const WrfGrid* gin, float* th, float* qv, float* qc, float* qr, float* qi, float* qs, float* qg,
+                  const float* rho, const float* pii, const float* p, const float* dz8w, float delt, float* rainnc,
+                  float* rainncv, float* snownc, float* snowncv, float* graupelnc, float* graupelncv, float* sr,
+                  float* work, size_t work_floats, void* stream) {
+  Grid g;
+  int rc = make_grid(gin, g);
+  if (rc) return rc;
+  float* f[18] = {th, qv, qc, qr, qi, qs, qg, const_cast<float*>(rho), const_cast<float*>(pii),
+                  const_cast<float*>(p), const_cast<float*>(dz8w), rainnc, rainncv, snownc, snowncv,
+                  graupelnc, graupelncv, sr};
+  for (float* x : f)
+    if (!x) return fail(WRF_EINVAL, "null argument");
+  if (!(delt > 0.f)) return fail(WRF_EINVAL, "delt must be > 0");
+  const size_t need = wsm6_work_floats(g, delt);
+  if (work_floats < need || (need && !work)) return fail(WRF_EINVAL, "wsm6_work: work too small");
+  cudaGetLastError();
+  launch_wsm6_work(g, f, delt, work, static_cast<cudaStream_t>(stream));
+  return check_launch("wsm6_work");
+}
+
 int wrf_wsm6_noalloc(const WrfGrid* gin, float* th, float* qv, float* qc, float* qr, float* qi, float* qs,
                      float* qg, const float* rho, const float* pii, const float* p, const float* dz8w, float delt,
                      float* rainnc, float* rainncv, float* snownc, float* snowncv, float* graupelnc,

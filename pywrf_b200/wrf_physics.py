@@ -65,13 +65,18 @@ def wsm6(th, q, qc, qr, qi, qs, qg, den, pii, p, delz, delt, g, cpd, cpv, rd, rv
     cg = _grid(nz, ny, nx, delt)
     ptr = lambda t: ctypes.c_void_p(t.data_ptr())
     with torch.cuda.device(th.device):
-        rc = N.lib().wrf_wsm6(ctypes.byref(cg), *[ptr(fields[k]) for k in ("th", "q", "qc", "qr", "qi", "qs", "qg", "den",
+        # the scheme's two intermediate fields, on the current stream
+        n = ctypes.c_size_t(0)
+        N.check(N.lib().wrf_wsm6_work_floats(ctypes.byref(cg), ctypes.c_float(float(delt)), ctypes.byref(n)),
+                "wrf_wsm6_work_floats")
+        work = torch.empty(n.value, dtype=torch.float32, device=th.device)
+        rc = N.lib().wrf_wsm6_work(ctypes.byref(cg), *[ptr(fields[k]) for k in ("th", "q", "qc", "qr", "qi", "qs", "qg", "den",
                                                                           "pii", "p", "delz")],
-                              ctypes.c_float(float(delt)),
-                              *[ptr(flat[k]) for k in ("rain", "rainncv", "snow", "snowncv", "graupel", "graupelncv",
-                                                       "sr")],
-                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
-    N.check(rc, "wrf_wsm6")
+                                   ctypes.c_float(float(delt)),
+                                   *[ptr(flat[k]) for k in ("rain", "rainncv", "snow", "snowncv", "graupel",
+                                                            "graupelncv", "sr")],
+                                   ptr(work), n.value, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    N.check(rc, "wrf_wsm6_work")
     return th, q, qc, qr, qi, qs, qg, rain, rainncv, snow, snowncv, graupel, graupelncv, sr, refl_10cm
 
 
