@@ -471,117 +471,115 @@ int launch_forces_terms(const Grid& g, const S& s, int terms, cudaStream_t st) {
 
 // -------------------------------------------- tendency accumulation + spec rows
 
-__global__ void k_addtend(Grid g, S s, int rk_step) {
-  WRF_POINT_INDEX(g, k, j, i);
+// A thread takes LZ levels of one column: its map factors' reciprocals (the
+// divisions by them in their correctly rounded form) and its place in the
+// specified rows are found once, and the rows' overrides sit behind one
+// branch.  The one-level form spent 700 instructions per warp on sixteen
+// field passes and was bound by their issue (86 % of the slots).
+template <bool R1, int LZ>
+__global__ void __launch_bounds__(128) k_addtend(Grid g, S s) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde, nz = g.nz, nx = g.nx, ny = g.ny;
+  if (i < ids || i >= ide || j < jds || j >= jde) return;
   const int c = g.i2(j, i);
-  const size_t p = (size_t)k * ny * nx + c;
-  const bool mass = j >= jds && j < jde - 1 && i >= ids && i < ide - 1;
-  auto ys0 = [&](int bid, int kk, int ii) { return s[bid][((size_t)kk * 5 + 0) * nx + ii]; };
-  auto xs0 = [&](int bid, int kk, int jj) { return s[bid][((size_t)kk * ny + jj) * 5]; };
-  // specified rows: field_tend = bdy_tend (y rows first, x columns overwrite)
-  auto spec = [&](float& t, int btxs, int ibe, int jbe) {
-    if (i >= ids && i < ibe && j == jds) t = ys0(btxs + 2, k, i);
-    if (i >= ids && i < ibe && j == jbe - 1) t = ys0(btxs + 3, k, i);
-    if (j >= jds && j < jbe && i == ids) t = xs0(btxs + 0, k, j);
-    if (j >= jds && j < jbe && i == ibe - 1) t = xs0(btxs + 1, k, j);
-  };
-  // operands first, then the specified-row overrides, then the stores (a
-  // store would hold back the later fields' loads)
-  const bool r1 = rk_step == 1;
-  const bool du = k < nz - 1 && j >= jds && j < jde - 1 && i >= ids && i < ide;
-  const bool dv = k < nz - 1 && j >= jds && j < jde && i >= ids && i < ide - 1;
-  const bool dt = mass && k < nz - 1;
-  const bool dmu = mass && k == 0;
-  float tfu = 0.f, usv = 0.f, mfuy = 1.f, rtu = 0.f;
-  if (du) {
-    tfu = s[WF_RU_TENDF][p];
-    mfuy = s[WF_MSFUY][c];
-    if (r1) usv = s[WF_U_SAVE][p];
-    rtu = s[WF_RU_TEND][p];
-  }
-  float tfv = 0.f, vsv = 0.f, mfvx = 0.f, mvxi = 0.f, rtv = 0.f;
-  if (dv) {
-    tfv = s[WF_RV_TENDF][p];
-    if (r1) {
-      vsv = s[WF_V_SAVE][p];
-      mfvx = s[WF_MSFVX][c];
+  const int lev = ny * nx;
+  const bool ur = j < jde - 1, vr = i < ide - 1, mass = ur && vr;
+  const bool edge = j == jds || j >= jde - 2 || i == ids || i >= ide - 2;
+  const float mfuy = ur ? __ldg(&s[WF_MSFUY][c]) : 1.f, mvxi = vr ? __ldg(&s[WF_MSFVX_INV][c]) : 0.f;
+  const float mfvx = R1 && vr ? __ldg(&s[WF_MSFVX][c]) : 0.f;
+  const float msfty = mass ? __ldg(&s[WF_MSFTY][c]) : 1.f, mut = mass ? __ldg(&s[WF_MUT][c]) : 0.f;
+  const float r_mfuy = __frcp_rn(mfuy), r_msfty = __frcp_rn(msfty);
+#pragma unroll 1
+  for (int q = 0; q < LZ; ++q) {
+    const int k = blockIdx.z * LZ + q;
+    if (k >= nz) break;
+    const int p = k * lev + c;
+    // specified rows: field_tend = bdy_tend (y rows first, x columns overwrite)
+    auto spec = [&](float& t, int btxs, int ibe, int jbe) {
+      if (i < ibe && j == jds) t = s[btxs + 2][(size_t)k * 5 * nx + i];
+      if (i < ibe && j == jbe - 1) t = s[btxs + 3][(size_t)k * 5 * nx + i];
+      if (j < jbe && i == ids) t = s[btxs + 0][((size_t)k * ny + j) * 5];
+      if (j < jbe && i == ibe - 1) t = s[btxs + 1][((size_t)k * ny + j) * 5];
+    };
+    // operands first, then the specified-row overrides, then the stores (a
+    // store would hold back the later fields' loads)
+    const bool half = k < nz - 1;
+    const bool du = half && ur, dv = half && vr, dt = half && mass, dmu = mass && k == 0;
+    float tfu = 0.f, usv = 0.f, rtu = 0.f, tfv = 0.f, vsv = 0.f, rtv = 0.f;
+    float tfw = 0.f, wsv = 0.f, rtw = 0.f, tfp = 0.f, phs = 0.f, rtp = 0.f;
+    float tft = 0.f, tsv = 0.f, rtt = 0.f, hd = 0.f, mut0 = 0.f, mutf0 = 0.f;
+    if (du) {
+      tfu = s[WF_RU_TENDF][p];
+      rtu = s[WF_RU_TEND][p];
+      if (R1) usv = s[WF_U_SAVE][p];
     }
-    mvxi = s[WF_MSFVX_INV][c];
-    rtv = s[WF_RV_TEND][p];
-  }
-  float msfty = 1.f, tfw = 0.f, wsv = 0.f, rtw = 0.f, tfp = 0.f, phs = 0.f, rtp = 0.f;
-  float tft = 0.f, tsv = 0.f, rtt = 0.f, mutc = 0.f, hd = 0.f, mut0 = 0.f, mutf0 = 0.f;
-  if (mass) {
-    msfty = s[WF_MSFTY][c];
-    tfw = s[WF_RW_TENDF][p];
-    rtw = s[WF_RW_TEND][p];
-    tfp = s[WF_PH_TENDF][p];
-    rtp = s[WF_PH_TEND][p];
-    if (r1) {
-      wsv = s[WF_W_SAVE][p];
-      phs = s[WF_PH_SAVE][p];
+    if (dv) {
+      tfv = s[WF_RV_TENDF][p];
+      rtv = s[WF_RV_TEND][p];
+      if (R1) vsv = s[WF_V_SAVE][p];
     }
-  }
-  if (dt) {
-    tft = s[WF_T_TENDF][p];
-    if (r1) tsv = s[WF_T_SAVE][p];
-    rtt = s[WF_T_TEND][p];
-    mutc = s[WF_MUT][c];
-    hd = s[WF_H_DIABATIC][p];
-  }
-  if (dmu) {
-    mut0 = s[WF_MU_TEND][c];
-    mutf0 = s[WF_MU_TENDF][c];
-  }
-  float ou = 0.f, ov = 0.f, ow = 0.f, oph = 0.f, ot = 0.f, omu = 0.f;
-  if (du) {  // u
-    if (r1) tfu = tfu + usv * mfuy;
-    ou = rtu + tfu / mfuy;
-    spec(ou, WF_U_BTXS, ide, jde - 1);
-  }
-  if (dv) {  // v
-    if (r1) tfv = tfv + vsv * mfvx;
-    ov = rtv + tfv * mvxi;
-    spec(ov, WF_V_BTXS, ide - 1, jde);
-  }
-  if (mass) {
-    if (r1) tfw = tfw + wsv * msfty;
-    ow = rtw + tfw / msfty;
-    if (r1) tfp = tfp + phs;
-    oph = rtp + tfp / msfty;
-    spec(oph, WF_PH_BTXS, ide - 1, jde - 1);
-  }
-  if (dt) {
-    if (r1) tft = tft + tsv;
-    ot = rtt + tft / msfty + mutc * hd / msfty;
-    spec(ot, WF_T_BTXS, ide - 1, jde - 1);
-  }
-  if (dmu) {
-    omu = mut0 + mutf0;
-    spec(omu, WF_MU_BTXS, ide - 1, jde - 1);
-  }
-  if (du) {
-    if (r1) s[WF_RU_TENDF][p] = tfu;
-    s[WF_RU_TEND][p] = ou;
-  }
-  if (dv) {
-    if (r1) s[WF_RV_TENDF][p] = tfv;
-    s[WF_RV_TEND][p] = ov;
-  }
-  if (mass) {
-    if (r1) {
-      s[WF_RW_TENDF][p] = tfw;
-      s[WF_PH_TENDF][p] = tfp;
+    if (mass) {
+      tfw = s[WF_RW_TENDF][p];
+      rtw = s[WF_RW_TEND][p];
+      tfp = s[WF_PH_TENDF][p];
+      rtp = s[WF_PH_TEND][p];
+      if (R1) {
+        wsv = s[WF_W_SAVE][p];
+        phs = s[WF_PH_SAVE][p];
+      }
     }
-    s[WF_RW_TEND][p] = ow;
-    s[WF_PH_TEND][p] = oph;
+    if (dt) {
+      tft = s[WF_T_TENDF][p];
+      rtt = s[WF_T_TEND][p];
+      hd = s[WF_H_DIABATIC][p];
+      if (R1) tsv = s[WF_T_SAVE][p];
+    }
+    if (dmu) {
+      mut0 = s[WF_MU_TEND][c];
+      mutf0 = s[WF_MU_TENDF][c];
+    }
+    if (R1) {
+      tfu = tfu + usv * mfuy;
+      tfv = tfv + vsv * mfvx;
+      tfw = tfw + wsv * msfty;
+      tfp = tfp + phs;
+      tft = tft + tsv;
+    }
+    float ou = rtu + divc(tfu, mfuy, r_mfuy);
+    float ov = rtv + tfv * mvxi;
+    const float ow = rtw + divc(tfw, msfty, r_msfty);
+    float oph = rtp + divc(tfp, msfty, r_msfty);
+    float ot = rtt + divc(tft, msfty, r_msfty) + divc(mut * hd, msfty, r_msfty);
+    float omu = mut0 + mutf0;
+    if (edge) {
+      if (du) spec(ou, WF_U_BTXS, ide, jde - 1);
+      if (dv) spec(ov, WF_V_BTXS, ide - 1, jde);
+      if (mass) spec(oph, WF_PH_BTXS, ide - 1, jde - 1);
+      if (dt) spec(ot, WF_T_BTXS, ide - 1, jde - 1);
+      if (dmu) spec(omu, WF_MU_BTXS, ide - 1, jde - 1);
+    }
+    if (du) {
+      if (R1) s[WF_RU_TENDF][p] = tfu;
+      s[WF_RU_TEND][p] = ou;
+    }
+    if (dv) {
+      if (R1) s[WF_RV_TENDF][p] = tfv;
+      s[WF_RV_TEND][p] = ov;
+    }
+    if (mass) {
+      if (R1) {
+        s[WF_RW_TENDF][p] = tfw;
+        s[WF_PH_TENDF][p] = tfp;
+      }
+      s[WF_RW_TEND][p] = ow;
+      s[WF_PH_TEND][p] = oph;
+    }
+    if (dt) {
+      if (R1) s[WF_T_TENDF][p] = tft;
+      s[WF_T_TEND][p] = ot;
+    }
+    if (dmu) s[WF_MU_TEND][c] = omu;
   }
-  if (dt) {
-    if (r1) s[WF_T_TENDF][p] = tft;
-    s[WF_T_TEND][p] = ot;
-  }
-  if (dmu) s[WF_MU_TEND][c] = omu;
 }
 
 // stand-alone advect_scalar on caller arrays (s carries msftx, fnm, fnp, rdnw)
@@ -607,8 +605,19 @@ int launch_advect_forces(const Grid& g, const S& s, cudaStream_t st) {
 }
 
 int launch_addtend(const Grid& g, const S& s, int rk_step, cudaStream_t st) {
+  // four levels per thread once a quarter of the points still fills the GPU
+  // (eight blocks of 128 threads on each of 148 SMs)
   const dim3 b3(32, 4);
-  k_addtend<<<point_grid(g, b3), b3, 0, st>>>(g, s, rk_step);
+  dim3 gr = point_grid(g, b3);
+  const bool deep = g.n3() >= 4 * (size_t)148 * 8 * 128;
+  if (deep) gr.z = (g.nz + 3) / 4;
+  if (rk_step == 1) {
+    if (deep) k_addtend<true, 4><<<gr, b3, 0, st>>>(g, s);
+    else k_addtend<true, 1><<<gr, b3, 0, st>>>(g, s);
+  } else {
+    if (deep) k_addtend<false, 4><<<gr, b3, 0, st>>>(g, s);
+    else k_addtend<false, 1><<<gr, b3, 0, st>>>(g, s);
+  }
   return 1;
 }
 
