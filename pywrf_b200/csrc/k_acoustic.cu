@@ -1125,8 +1125,9 @@ int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st) {
     for (int e = 0; e < kUvNO && ok; ++e)
       ok = tma::encode_f32_4d(&a.own[e], s[fo[e]], g.nx, g.ny, g.nz, 1, kUvOW, kUvOH, &err);
     if (ok) {
-      a.nchunk = min((g.nz - 1 + kUvKCH - 1) / kUvKCH, g.nz - 1);
-      const dim3 gr((g.ide + 1 - g.ids + kUvTX - 1) / kUvTX, (g.jde - g.jds + kUvTY - 1) / kUvTY, a.nchunk);
+      const int bx = (g.ide + 1 - g.ids + kUvTX - 1) / kUvTX, by = (g.jde - g.jds + kUvTY - 1) / kUvTY;
+      a.nchunk = level_chunks(g.nz - 1, bx * by, kUvKCH, 4);
+      const dim3 gr(bx, by, a.nchunk);
       k_advance_uv_tma<<<gr, dim3(kUvTX, kUvTY), 0, st>>>(g, s, dts, a);
       return 1;
     }

@@ -4,7 +4,7 @@
 // stage's coupled velocities.
 //
 // A block of TX x TY threads owns (TX-1) x (TY-1) columns and marches up
-// through KCH levels.  For each level the species' values of the tile and its
+// through its chunk of levels.  For each level the species' values of the tile and its
 // halo are staged in shared memory together with everything else the level
 // reads (the thread's face velocities, the rom of its top face, the column
 // value three levels up and, when accumulating, its tendency): cp.async,
@@ -29,7 +29,7 @@ struct AdvArgs {
   const float* q[6];
   float* tend[6];
   const float *ru, *rv, *rom;
-  int ngroup;
+  int ngroup, nchunk;
 };
 
 // y face jf (between rows jf-1 and jf) from the tile column, rows STRIDE
@@ -127,7 +127,8 @@ __global__ void __launch_bounds__(kAdvTX * kAdvTY) k_advect_tiled(Grid g, S s, A
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde;
   const size_t lev = (size_t)ny * nx;
   const int grp = blockIdx.z % a.ngroup;
-  const int k0 = (blockIdx.z / a.ngroup) * kAdvKCH, k1 = min(k0 + kAdvKCH, g.nz);
+  const int chunk = blockIdx.z / a.ngroup;
+  const int k0 = chunk * g.nz / a.nchunk, k1 = (chunk + 1) * g.nz / a.nchunk;
   const float* qs[NSP];
   float* ts[NSP];
 #pragma unroll
@@ -348,8 +349,8 @@ __global__ void __launch_bounds__(kTTX * kTTY, WRF_ADV_MINB) k_advect_tma(Grid g
     q_hi = min(k0 + kTRing - 1, k1) - 1;
     a_hi = min(k0 + kARing - 1, k1) - 1;
   }
-  // column windows q(k-3 .. k+3), the values q(k1 .. k1+2) above the chunk
-  // (read directly; the rings hold the chunk's own levels) and the flux
+  // column windows q(k-3 .. k+3), the next values above the window that the
+  // chunk's own levels do not hold (read directly) and the flux
   // through the bottom face
   float win[NSP][7], wtop[NSP][3], fbot[NSP];
   const float rbot = cell && k0 < nz ? __ldg(&a.romg[k0 * lev + c]) : 0.f;
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(kTTX * kTTY, WRF_ADV_MINB) k_advect_tma(Grid g
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const int kk = k1 + d;
+      const int kk = max(k1, k0 + 3) + d;
       wtop[m][d] = (cell && kk < nz) ? __ldg(&q[kk * lev + c]) : 0.f;
     }
     fbot[m] = zface(ktf, fnm, fnp, win[m], k0, k0, rbot);
@@ -687,7 +688,7 @@ __device__ __forceinline__ void advect_mom_block(const Grid& g, const S& s, cons
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const int kk = k1 + d;
+    const int kk = max(k1, k0 + 3) + d;
     wtop[d] = (cell && kk < nz) ? __ldg(&qg[kk * lev + c]) : 0.f;
   }
   float fbot, rprev = 0.f;
@@ -866,10 +867,11 @@ namespace {
 // arrays are 16-byte aligned (the encoder checks the bases)
 bool tma_form(const Grid& g) { return kernel_form() == WRF_FORM_FAST && g.nx % 4 == 0 && g.ids >= 0 && g.jds >= 0; }
 
-int nchunks(const Grid& g) { return (g.nz + kTKCH - 1) / kTKCH; }
-
-dim3 tma_grid(const Grid& g, int ngroup) {
-  return dim3((g.ide - g.ids + kTTX - 1) / kTTX, (g.jde - g.jds + kTTY - 1) / kTTY, ngroup * nchunks(g));
+// ngroup blocks per tile and chunk; sets *nchunk
+dim3 tma_grid(const Grid& g, int ngroup, int* nchunk) {
+  const int bx = (g.ide - g.ids + kTTX - 1) / kTTX, by = (g.jde - g.jds + kTTY - 1) / kTTY;
+  *nchunk = level_chunks(g.nz, bx * by * ngroup, kTKCH, 4);
+  return dim3(bx, by, ngroup * *nchunk);
 }
 
 bool aux_maps(AdvTmaArgs& a, const Grid& g, const float* ru, const float* rv, const float* rom) {
@@ -900,9 +902,10 @@ int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaS
       !tma::encode_f32_4d(&a.rom, s[WF_WW], g.nx, g.ny, g.nz, 1, kMW, kMH, &err))
     return 0;
   a.romg = s[WF_WW];
-  a.nchunk = min((g.nz - 1 + kMomKCH - 1) / kMomKCH, g.nz - 1);
   a.comp0 = comp0;
-  const dim3 gr((g.ide - g.ids + kTTX - 1) / kTTX, (g.jde - g.jds + kTTY - 1) / kTTY, ncomp * a.nchunk);
+  const int bx = (g.ide - g.ids + kTTX - 1) / kTTX, by = (g.jde - g.jds + kTTY - 1) / kTTY;
+  a.nchunk = level_chunks(g.nz - 1, bx * by * ncomp, kMomKCH, 4);
+  const dim3 gr(bx, by, ncomp * a.nchunk);
   k_advect_mom_tma<<<gr, dim3(kTTX, kTTY), 0, st>>>(g, s, a);
   return 1;
 }
@@ -923,8 +926,8 @@ int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st) {
       a.qw0 = 1;
       a.tw0 = 1;
       a.ngroup = 3;
-      a.nchunk = nchunks(g);
-      k_advect_tma<2, false><<<tma_grid(g, 3), dim3(kTTX, kTTY), 0, st>>>(g, s, a);
+      const dim3 gr = tma_grid(g, 3, &a.nchunk);
+      k_advect_tma<2, false><<<gr, dim3(kTTX, kTTY), 0, st>>>(g, s, a);
       return 1;
     }
   }
@@ -938,8 +941,9 @@ int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st) {
   a.rom = s[WF_WW_M];
   a.ngroup = 3;
   const dim3 b(kAdvTX, kAdvTY);
-  const dim3 gr((g.ide - g.ids + kAdvCX - 1) / kAdvCX, (g.jde - g.jds + kAdvCY - 1) / kAdvCY,
-                3 * ((g.nz + kAdvKCH - 1) / kAdvKCH));
+  const int bx = (g.ide - g.ids + kAdvCX - 1) / kAdvCX, by = (g.jde - g.jds + kAdvCY - 1) / kAdvCY;
+  a.nchunk = level_chunks(g.nz, 3 * bx * by, kAdvKCH, 4);
+  const dim3 gr(bx, by, 3 * a.nchunk);
   k_advect_tiled<2, false><<<gr, b, 0, st>>>(g, s, a);
   return 1;
 }
@@ -957,8 +961,8 @@ int launch_advect_theta_tiled(const Grid& g, const S& s, cudaStream_t st) {
       a.qw0 = 0;
       a.tw0 = 0;
       a.ngroup = 1;
-      a.nchunk = nchunks(g);
-      k_advect_tma<1, true><<<tma_grid(g, 1), dim3(kTTX, kTTY), 0, st>>>(g, s, a);
+      const dim3 gr = tma_grid(g, 1, &a.nchunk);
+      k_advect_tma<1, true><<<gr, dim3(kTTX, kTTY), 0, st>>>(g, s, a);
       return 1;
     }
   }
@@ -970,8 +974,9 @@ int launch_advect_theta_tiled(const Grid& g, const S& s, cudaStream_t st) {
   a.rom = s[WF_WW];
   a.ngroup = 1;
   const dim3 b(kAdvTX, kAdvTY);
-  const dim3 gr((g.ide - g.ids + kAdvCX - 1) / kAdvCX, (g.jde - g.jds + kAdvCY - 1) / kAdvCY,
-                (g.nz + kAdvKCH - 1) / kAdvKCH);
+  const int bx = (g.ide - g.ids + kAdvCX - 1) / kAdvCX, by = (g.jde - g.jds + kAdvCY - 1) / kAdvCY;
+  a.nchunk = level_chunks(g.nz, bx * by, kAdvKCH, 4);
+  const dim3 gr(bx, by, a.nchunk);
   k_advect_tiled<1, true><<<gr, b, 0, st>>>(g, s, a);
   return 1;
 }

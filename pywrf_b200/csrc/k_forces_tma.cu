@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
       } else {
         t = 0.f;
       }
-      t = t + mut * gf * cur.w / msfty;
+      t = t + divc(mut * gf * cur.w, msfty, rm);
       const bool top = (k == nz - 1);
       float fly_c, fly_n, flx_c, flx_e;
       if (!top) {
@@ -274,30 +274,30 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
         flx_c = muu_c * (cfn * u_c + cfn1 * __ldg(&s[WF_U][q3])) * mux_c;
         flx_e = muu_e * (cfn * u_e + cfn1 * __ldg(&s[WF_U][q3 + 1])) * mux_e;
       }
-      const float ky = top ? (float)(0.5 * g.rdyd) : (float)(0.25 * g.rdyd);
+      const float kym = divc(top ? (float)(0.5 * g.rdyd) : (float)(0.25 * g.rdyd), msfty, rm);
       const float* ph = PH0 + oQ;
       const float* phb = PHB0 + oQ;
       if (j >= jds + 3 && j < jde - 4) {
         const float dd = d6s(ph, kFQW) + 45.0f * (phb[kFQW] - phb[-kFQW]) - 9.0f * (phb[2 * kFQW] - phb[-2 * kFQW]) +
                          (phb[3 * kFQW] - phb[-3 * kFQW]);
-        t = t - (ky / msfty) * ((fly_n + fly_c) * (float)(1.0 / 60.0) * dd);
+        t = t - kym * ((fly_n + fly_c) * (float)(1.0 / 60.0) * dd);
       } else if (j == jds + 2 || j == jde - 4) {
         const float dd = 8.0f * (ph[kFQW] - ph[-kFQW]) - (ph[2 * kFQW] - ph[-2 * kFQW]) +
                          8.0f * (phb[kFQW] - phb[-kFQW]) - (phb[2 * kFQW] - phb[-2 * kFQW]);
-        t = t - (ky / msfty) * ((fly_n + fly_c) * (float)(1.0 / 12.0) * dd);
+        t = t - kym * ((fly_n + fly_c) * (float)(1.0 / 12.0) * dd);
       } else if (j == jds + 1 || j == jde - 3) {
         const float dp1 = phb[kFQW] - phb[0] + ph[kFQW] - ph[0];
         const float dp0 = phb[0] - phb[-kFQW] + ph[0] - ph[-kFQW];
-        t = t - (ky / msfty) * (fly_n * dp1 + fly_c * dp0);
+        t = t - kym * (fly_n * dp1 + fly_c * dp0);
       }
-      const float kx = top ? (float)(0.5 * g.rdxd) : (float)(0.25 * g.rdxd);
+      const float kxm = divc(top ? (float)(0.5 * g.rdxd) : (float)(0.25 * g.rdxd), msfty, rm);
       if (i >= ids + 3 && i < ide - 4) {
         const float dd = d6s(ph, 1) + 45.0f * (phb[1] - phb[-1]) - 9.0f * (phb[2] - phb[-2]) + (phb[3] - phb[-3]);
-        t = t - (kx / msfty) * ((flx_e + flx_c) * (float)(1.0 / 60.0) * dd);
+        t = t - kxm * ((flx_e + flx_c) * (float)(1.0 / 60.0) * dd);
       } else if (i == ids + 1 || i == ide - 3) {
         const float dp1 = phb[1] - phb[0] + ph[1] - ph[0];
         const float dp0 = phb[0] - phb[-1] + ph[0] - ph[-1];
-        t = t - (kx / msfty) * (flx_e * dp1 + flx_c * dp0);
+        t = t - kxm * (flx_e * dp1 + flx_c * dp0);
       }
       o_ph = t;
     }
@@ -333,14 +333,12 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
     }
     // ---------------- pg_buoy_w (wrf_dynamics.py:2424-2460); cqw becomes 1/(1+cqw)
     if (mass && k >= 1 && k < nz - 1) {
+      const float cq1 = __frcp_rn(1.0f + cur.cqw);
+      const float cq2 = cur.cqw * cq1;
       if (k == nz - 2) {  // the top level, from the unmodified cqw of level nz-2
-        const float cq1 = 1.0f / (1.0f + cur.cqw);
-        const float cq2 = cur.cqw * cq1;
         const float rwt_top = (k + 1 < k1) ? nxt.rwt : s[WF_RW_TEND][(size_t)(k + 1) * lev + c];
         o_rwt = rwt_top + rm * gf * (cq1 * 2.0f * __ldg(&rdnw[nz - 2]) * (-pk_c) - mu_c - cq2 * mub);
       }
-      const float cq1 = 1.0f / (1.0f + cur.cqw);
-      const float cq2 = cur.cqw * cq1;
       o_cqw = cq1;
       o_rw = cur.rwt + rm * gf * (cq1 * __ldg(&rdn[k]) * (pk_c - p_c) - mu_c - cq2 * mub);
     }
@@ -441,10 +439,11 @@ int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st) {
   const int f[kFNM] = {WF_U, WF_V, WF_RU, WF_RV, WF_RW, WF_ALT, WF_AL, WF_PB, WF_PHP, WF_P};
   for (int e = 0; e < kFNM; ++e)
     if (!tma::encode_f32_4d(&a.m[e], s[f[e]], g.nx, g.ny, g.nz, 1, kFMW, kFMH, &err)) return 0;
-  a.nchunk = min((g.nz + kFKCH - 1) / kFKCH, g.nz);
+  const int bx = (g.ide - g.ids + kFTX - 1) / kFTX, by = (g.jde - g.jds + kFTY - 1) / kFTY;
+  a.nchunk = level_chunks(g.nz, bx * by, kFKCH, 2);
   const size_t dyn = (size_t)kFRing * kFSlot * sizeof(float) + 128;
   if (cudaFuncSetAttribute(k_forces_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess) return 0;
-  const dim3 gr((g.ide - g.ids + kFTX - 1) / kFTX, (g.jde - g.jds + kFTY - 1) / kFTY, a.nchunk);
+  const dim3 gr(bx, by, a.nchunk);
   k_forces_tma<<<gr, dim3(kFTX, kFTY), dyn, st>>>(g, s, a);
   return 1;
 }

@@ -135,6 +135,20 @@ __device__ __forceinline__ bool ring_point(const Grid& g, int r, int& j, int& i)
 inline bool ring_fits(const Grid& g) { return g.jde - g.jds >= 10 && g.ide - g.ids >= 11; }
 inline int ring_size(const Grid& g) { return 10 * (g.ide + 1 - g.ids) + (g.jde - g.jds - 10) * 11; }
 
+// Level chunks of a launch whose blocks march up through their levels: at
+// most `most` levels per chunk, and fewer (down to one) while the launch's
+// blocks would leave part of the 148 SMs without the `resident` blocks that
+// fit there.  A level costs a
+// block a few microseconds of latency whatever the grid, so on small domains
+// the chunk's length is the kernel's time; each chunk re-reads the values
+// below and above it, which only shows once the chip is full.
+inline int level_chunks(int nlev, int blocks_per_chunk, int most, int resident) {
+  const int few = (nlev + most - 1) / most;
+  const int fill = (148 * resident + blocks_per_chunk - 1) / blocks_per_chunk;
+  const int n = few > fill ? few : fill;
+  return n < nlev ? n : nlev;
+}
+
 inline dim3 point_grid(const Grid& g, dim3 b) { return dim3((g.nx + b.x - 1) / b.x, (g.ny + b.y - 1) / b.y, g.nz); }
 inline dim3 col_grid(const Grid& g, dim3 b) { return dim3((g.nx + b.x - 1) / b.x, (g.ny + b.y - 1) / b.y, 1); }
 
