@@ -140,6 +140,13 @@
 #include "relax.cuh"
 
 namespace wrf {
+
+// dynamic shared memory above 48 KB has to be allowed kernel by kernel
+template <typename K>
+static void allow_smem(K kernel, size_t bytes) {
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 namespace {
 
 // dPhi/dq at stencil offset o = m - f of a 5th-order face (o in [-3, 2]),
@@ -670,59 +677,84 @@ __device__ __forceinline__ bool mut_in(const Grid& g, int j, int i) {
   return j >= g.jds + 1 && j < g.jde - 2 && i >= g.ids + 1 && i < g.ide - 2;
 }
 
-__device__ __forceinline__ float mut_dvdxi(const Grid& g, const S& s, int k, int j, int i) {
-  const int nx = g.nx;
-  const size_t c = (size_t)j * nx + i, p = (size_t)k * g.ny * nx + c;
-  const float vn = s[WF_V][p + nx] + s[WF_MUV][c + nx] * s[WF_V_SAVE][p + nx] * s[WF_MSFVX_INV][c + nx];
-  const float vs = s[WF_V][p] + s[WF_MUV][c] * s[WF_V_SAVE][p] * s[WF_MSFVX_INV][c];
-  const float ue = s[WF_U][p + 1] + s[WF_MUU][c + 1] * s[WF_U_SAVE][p + 1] / s[WF_MSFUY][c + 1];
-  const float uw = s[WF_U][p] + s[WF_MUU][c] * s[WF_U_SAVE][p] / s[WF_MSFUY][c];
-  return s[WF_MSFTX][c] * s[WF_MSFTY][c] * (g.rdy * (vn - vs) + g.rdx * (ue - uw));
-}
+// The column kernels of this operator: a block owns 32 adjacent columns of one
+// row (a warp's lanes) and 8 level groups (its warps).  What a level needs from
+// memory is loaded over levels in parallel; the vertical sums and scans run
+// from shared memory ([nz][32] arrays), one warp each, in the reference's
+// order.  One thread per column took 97 (forward), 116 and 132 us (the two
+// column passes of the reverse) at 240x240x41 and hardly less at 101x101x35,
+// a memory round trip every few levels.
+constexpr int kMutTX = 32, kMutKT = 8;
 
-// a column's forward values: dvdxi, dmdt and the new ww (ww' = W - ww_1)
-struct MutCol {
-  float dv[kMaxNz], wwp[kMaxNz];
-  float dmdt;
+// dvdxi of a column's levels, its two-dimensional factors loaded once
+struct MutDiv {
+  float muvn, mvin, muv0, mvi0, muup, mfup, r_mfup, muu0, mfu0, r_mfu0, msf;
+  __device__ __forceinline__ MutDiv(const Grid& g, const S& s, int c) {
+    const int nx = g.nx;
+    muvn = s[WF_MUV][c + nx];
+    mvin = s[WF_MSFVX_INV][c + nx];
+    muv0 = s[WF_MUV][c];
+    mvi0 = s[WF_MSFVX_INV][c];
+    muup = s[WF_MUU][c + 1];
+    mfup = s[WF_MSFUY][c + 1];
+    muu0 = s[WF_MUU][c];
+    mfu0 = s[WF_MSFUY][c];
+    msf = s[WF_MSFTX][c] * s[WF_MSFTY][c];
+    r_mfup = __frcp_rn(mfup);
+    r_mfu0 = __frcp_rn(mfu0);
+  }
+  __device__ __forceinline__ float at(const Grid& g, const S& s, int p) const {
+    const int nx = g.nx;
+    const float* u = s[WF_U];
+    const float* v = s[WF_V];
+    const float* u1 = s[WF_U_SAVE];
+    const float* v1 = s[WF_V_SAVE];
+    const float vn = __ldg(v + p + nx) + muvn * __ldg(v1 + p + nx) * mvin;
+    const float vs = __ldg(v + p) + muv0 * __ldg(v1 + p) * mvi0;
+    const float ue = __ldg(u + p + 1) + divc(muup * __ldg(u1 + p + 1), mfup, r_mfup);
+    const float uw = __ldg(u + p) + divc(muu0 * __ldg(u1 + p), mfu0, r_mfu0);
+    return msf * (g.rdy * (vn - vs) + g.rdx * (ue - uw));
+  }
 };
 
-constexpr int kMutChunk = 8;  // levels whose loads a column kernel issues together
-
-__device__ void mut_column(const Grid& g, const S& s, int j, int i, MutCol& m) {
-  const int ktf = g.nz - 1;
-  const size_t lev = (size_t)g.ny * g.nx, c = (size_t)j * g.nx + i;
+// the scan of ww over the column's levels: sw[k] becomes W(k) (ww'(k) = W(k)
+// - ww_1(k)) from the divergences sdv; every thread of the block takes part
+__device__ __forceinline__ void mut_scan(const Grid& g, const S& s, bool in, int c, float dmdt, const float* sdv,
+                                         float* sw) {
+  const int ktf = g.nz - 1, tk = threadIdx.y;
   const float* dnw = s[WF_DNW];
-  m.dmdt = 0.f;
-#pragma unroll 8
-  for (int k = 0; k < ktf; ++k) {
-    m.dv[k] = mut_dvdxi(g, s, k, j, i);
-    m.dmdt = m.dmdt + dnw[k] * m.dv[k];
+  if (in) {
+    const float mt = s[WF_MU_TEND][c], msfty = s[WF_MSFTY][c], r_msfty = __frcp_rn(msfty);
+    for (int k = 1 + tk; k < ktf; k += kMutKT)
+      sw[k * kMutTX] = divc(__ldg(dnw + k - 1) * (dmdt + sdv[(k - 1) * kMutTX] + mt), msfty, r_msfty);
   }
-  const float mt = s[WF_MU_TEND][c], msfty = s[WF_MSFTY][c];
-  float W = s[WF_WW][c];
-  m.wwp[0] = W - s[WF_WW1][c];
+  __syncthreads();
+  if (in && tk == 0) {
+    float W = s[WF_WW][c];
+    sw[0] = W;
 #pragma unroll 8
-  for (int k = 1; k < ktf; ++k) {
-    W = W - dnw[k - 1] * (m.dmdt + m.dv[k - 1] + mt) / msfty;
-    m.wwp[k] = W - s[WF_WW1][k * lev + c];
+    for (int k = 1; k < ktf; ++k) {
+      W = W - sw[k * kMutTX];
+      sw[k * kMutTX] = W;
+    }
   }
+  __syncthreads();
 }
 
-// the cotangents of wdtn(kk), kk in [1, ktf), and of ww'(k), k in [0, ktf)
-__device__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dts, int j, int i, const MutCol& m,
-                           float* wdb, float* wwb) {
-  const int ktf = g.nz - 1;
-  const size_t lev = (size_t)g.ny * g.nx, c = (size_t)j * g.nx + i;
-  const float dm = dts * s[WF_MSFTY][c];
-  const float* rdnw = s[WF_RDNW];
+// the cotangents of wdtn(k), k in [1, ktf), and of ww'(k), k in [0, ktf), of
+// one level (p: the point, dm = dts msfty)
+__device__ __forceinline__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dm, int k, int p, float& wdb,
+                                           float& wwb) {
+  const int lev = g.ny * g.nx;
   const float* t1 = s[WF_T_SAVE];
-#pragma unroll 8
-  for (int k = 0; k < ktf; ++k) {
-    wdb[k] = 0.f;
-    if (k >= 1) wdb[k] = -dm * rdnw[k - 1] * b[WF_T][(k - 1) * lev + c] + dm * rdnw[k] * b[WF_T][k * lev + c];
-    const float tavg = k >= 1 ? s[WF_FNM][k] * t1[k * lev + c] + s[WF_FNP][k] * t1[(k - 1) * lev + c] : 0.f;
-    wwb[k] = b[WF_WW][k * lev + c] + (k >= 1 ? wdb[k] * tavg : 0.f);
+  const float* rdnw = s[WF_RDNW];
+  wdb = 0.f;
+  float tavg = 0.f;
+  if (k >= 1) {
+    wdb = -dm * __ldg(rdnw + k - 1) * b[WF_T][p - lev] + dm * __ldg(rdnw + k) * b[WF_T][p];
+    tavg = __ldg(s[WF_FNM] + k) * __ldg(t1 + p) + __ldg(s[WF_FNP] + k) * __ldg(t1 + p - lev);
   }
+  wwb = b[WF_WW][p] + (k >= 1 ? wdb * tavg : 0.f);
 }
 
 // mu' is the new mu; the cotangent reaching it from mu', muts', muave'
@@ -733,85 +765,115 @@ __device__ __forceinline__ float mut_mu_bar(const Grid& g, const S& b, size_t c)
 
 }  // namespace
 
-__global__ void k_advance_mu_t(Grid g, S s, float dts) {
-  WRF_COLUMN_INDEX(g, j, i);
-  if (!mut_in(g, j, i)) return;
-  const int ktf = g.nz - 1, nx = g.nx;
-  const size_t lev = (size_t)g.ny * nx, c = (size_t)j * nx + i;
-  MutCol m;
-  mut_column(g, s, j, i, m);
-  const float ep1 = (float)(1.0 + (double)g.epssm), em1 = (float)(1.0 - (double)g.epssm);
-  const float mu0 = s[WF_MU][c], mt = s[WF_MU_TEND][c];
-  const float mu1 = mu0 + dts * (m.dmdt + mt);
-  s[WF_MU][c] = mu1;
-  s[WF_MUDF][c] = m.dmdt + mt;
-  s[WF_MUTS][c] = s[WF_MUT][c] + mu1;
-  s[WF_MUAVE][c] = 0.5f * (ep1 * mu1 + em1 * mu0);
-  for (int k = 0; k < ktf; ++k) s[WF_WW][k * lev + c] = m.wwp[k];
+__global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, float dts) {
+  extern __shared__ float mut_smem[];
+  const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx;
+  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const bool in = mut_in(g, j, i);
+  const int c = in ? j * nx + i : 0;
+  float* const sdv = mut_smem + threadIdx.x;
+  float* const sw = sdv + nz * kMutTX;
+  __shared__ float sdm[kMutTX];
+  if (in) {
+    const MutDiv d(g, s, c);
+#pragma unroll 4
+    for (int k = tk; k < ktf; k += kMutKT) sdv[k * kMutTX] = d.at(g, s, k * lev + c);
+  }
+  __syncthreads();
+  if (in && tk == 0) {
+    float dmdt = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < ktf; ++k) dmdt = dmdt + __ldg(s[WF_DNW] + k) * sdv[k * kMutTX];
+    sdm[threadIdx.x] = dmdt;
+    const float ep1 = (float)(1.0 + (double)g.epssm), em1 = (float)(1.0 - (double)g.epssm);
+    const float mu0 = s[WF_MU][c], mt = s[WF_MU_TEND][c], mut = s[WF_MUT][c];
+    const float mu1 = mu0 + dts * (dmdt + mt);
+    s[WF_MU][c] = mu1;
+    s[WF_MUDF][c] = dmdt + mt;
+    s[WF_MUTS][c] = mut + mu1;
+    s[WF_MUAVE][c] = 0.5f * (ep1 * mu1 + em1 * mu0);
+  }
+  __syncthreads();
+  mut_scan(g, s, in, c, sdm[threadIdx.x], sdv, sw);
+  if (in) {
+#pragma unroll 4
+    for (int k = tk; k < ktf; k += kMutKT) sw[k * kMutTX] = sw[k * kMutTX] - __ldg(s[WF_WW1] + k * lev + c);
+  }
+  __syncthreads();
+  if (!in) return;
   const float msfty = s[WF_MSFTY][c], msftx = s[WF_MSFTX][c], rdx = g.rdx, rdy = g.rdy;
   const float* t1 = s[WF_T_SAVE];
   const float* u = s[WF_U];
   const float* v = s[WF_V];
-  auto wdtn = [&](int k) {
-    if (k < 1 || k >= ktf) return 0.f;
-    return m.wwp[k] * (s[WF_FNM][k] * t1[k * lev + c] + s[WF_FNP][k] * t1[(k - 1) * lev + c]);
-  };
-  // kMutChunk levels at a time, every load of the block before its stores
-  for (int k0 = 0; k0 < ktf; k0 += kMutChunk) {
-    float tk[kMutChunk], tt[kMutChunk], h[kMutChunk], rd[kMutChunk], wd[kMutChunk + 1];
+  const float* fnm = s[WF_FNM];
+  const float* fnp = s[WF_FNP];
+  // every load of a thread's levels before its stores, four levels at a time
+  for (int kb = tk; kb < ktf; kb += 4 * kMutKT) {
+    float tk_[4], tt[4], h[4], wd[4];
 #pragma unroll
-    for (int q = 0; q <= kMutChunk; ++q) wd[q] = wdtn(k0 + q);
-#pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      const size_t p = (size_t)(k < ktf ? k : 0) * lev + c;
-      tk[q] = s[WF_T][p];
+    for (int q = 0; q < 4; ++q) {
+      const int k = kb + q * kMutKT;
+      if (k >= ktf) continue;
+      const int p = k * lev + c;
+      tk_[q] = s[WF_T][p];
       tt[q] = s[WF_T_TEND][p];
-      h[q] = 0.5f * rdy * (v[p + nx] * (t1[p + nx] + t1[p]) - v[p] * (t1[p] + t1[p - nx])) +
-             0.5f * rdx * (u[p + 1] * (t1[p + 1] + t1[p]) - u[p] * (t1[p] + t1[p - 1]));
-      rd[q] = s[WF_RDNW][k < ktf ? k : 0];
+      const float tc = __ldg(t1 + p);
+      h[q] = 0.5f * rdy * (__ldg(v + p + nx) * (__ldg(t1 + p + nx) + tc) - __ldg(v + p) * (tc + __ldg(t1 + p - nx))) +
+             0.5f * rdx * (__ldg(u + p + 1) * (__ldg(t1 + p + 1) + tc) - __ldg(u + p) * (tc + __ldg(t1 + p - 1)));
+      const float up = k + 1 < ktf ? sw[(k + 1) * kMutTX] * (__ldg(fnm + k + 1) * __ldg(t1 + p + lev) + __ldg(fnp + k + 1) * tc) : 0.f;
+      const float dn = k >= 1 ? sw[k * kMutTX] * (__ldg(fnm + k) * tc + __ldg(fnp + k) * __ldg(t1 + p - lev)) : 0.f;
+      wd[q] = up - dn;
     }
 #pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      if (k >= ktf) break;
-      const size_t p = k * lev + c;
-      s[WF_T_2SAVE][p] = tk[q];
-      const float t1v = tk[q] + msfty * dts * tt[q];
-      s[WF_T][p] = t1v - dts * msfty * (msftx * h[q] + rd[q] * (wd[q + 1] - wd[q]));
+    for (int q = 0; q < 4; ++q) {
+      const int k = kb + q * kMutKT;
+      if (k >= ktf) continue;
+      const int p = k * lev + c;
+      s[WF_WW][p] = sw[k * kMutTX];
+      s[WF_T_2SAVE][p] = tk_[q];
+      const float t1v = tk_[q] + msfty * dts * tt[q];
+      s[WF_T][p] = t1v - dts * msfty * (msftx * h[q] + __ldg(s[WF_RDNW] + k) * wd[q]);
     }
   }
 }
 
-__global__ void k_advance_mu_t_adj_dv(Grid g, S s, S b, float dts, int ref_no_grad, float* work) {
-  WRF_COLUMN_INDEX(g, j, i);
-  if (!mut_in(g, j, i)) return;
-  const int ktf = g.nz - 1;
-  const size_t lev = (size_t)g.ny * g.nx, c = (size_t)j * g.nx + i;
-  MutCol m;
-  mut_column(g, s, j, i, m);
-  float wdb[kMaxNz], wwb[kMaxNz], qb[kMaxNz];
-  mut_ww_bar(g, s, b, dts, j, i, m, wdb, wwb);
-  const float msfty = s[WF_MSFTY][c];
-  float S_ = 0.f, qsum = 0.f;
-#pragma unroll 8
-  for (int k = ktf - 1; k >= 1; --k) {
-    S_ += wwb[k];
-    qb[k - 1] = -s[WF_DNW][k - 1] / msfty * S_;
-    qsum += qb[k - 1];
-  }
-  const float dmdtb = qsum + (ref_no_grad ? 0.f : dts * mut_mu_bar(g, b, c) + b[WF_MUDF][c]);
-  for (int k0 = 0; k0 < ktf; k0 += kMutChunk) {  // dnw loaded before the block's stores
-    float dn[kMutChunk];
-#pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) dn[q] = s[WF_DNW][k0 + q < ktf ? k0 + q : 0];
-#pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      if (k >= ktf) break;
-      work[k * lev + c] = (k <= ktf - 2 ? qb[k] : 0.f) + dn[q] * dmdtb;
+__global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, S s, S b, float dts, int ref_no_grad,
+                                                                        float* work) {
+  extern __shared__ float mut_smem[];
+  const int ktf = g.nz - 1, nx = g.nx, lev = g.ny * nx;
+  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const bool in = mut_in(g, j, i);
+  const int c = in ? j * nx + i : 0;
+  float* const swb = mut_smem + threadIdx.x;  // wwb, then qb one level down
+  __shared__ float sdm[kMutTX];
+  if (in) {
+    const float dm = dts * s[WF_MSFTY][c];
+#pragma unroll 4
+    for (int k = 1 + tk; k < ktf; k += kMutKT) {
+      float wdb, wwb;
+      mut_ww_bar(g, s, b, dm, k, k * lev + c, wdb, wwb);
+      swb[k * kMutTX] = wwb;
     }
   }
+  __syncthreads();
+  if (in && tk == 0) {
+    const float msfty = s[WF_MSFTY][c], r_msfty = __frcp_rn(msfty);
+    float S_ = 0.f, qsum = 0.f;
+#pragma unroll 8
+    for (int k = ktf - 1; k >= 1; --k) {
+      S_ += swb[k * kMutTX];
+      const float qb = divc(-__ldg(s[WF_DNW] + k - 1), msfty, r_msfty) * S_;
+      swb[k * kMutTX] = qb;  // of level k - 1
+      qsum += qb;
+    }
+    sdm[threadIdx.x] = qsum + (ref_no_grad ? 0.f : dts * mut_mu_bar(g, b, c) + b[WF_MUDF][c]);
+  }
+  __syncthreads();
+  if (!in) return;
+  const float dmdtb = sdm[threadIdx.x];
+#pragma unroll 4
+  for (int k = tk; k < ktf; k += kMutKT)
+    work[k * lev + c] = (k <= ktf - 2 ? swb[(k + 1) * kMutTX] : 0.f) + __ldg(s[WF_DNW] + k) * dmdtb;
 }
 
 __global__ void k_advance_mu_t_adj_pt(Grid g, S s, S b, float dts, const float* work) {
@@ -855,96 +917,126 @@ __global__ void k_advance_mu_t_adj_pt(Grid g, S s, S b, float dts, const float* 
   if (t1b != 0.f) b[WF_T_SAVE][p] += t1b;
 }
 
-__global__ void k_advance_mu_t_adj_col(Grid g, S s, S b, float dts, int ref_no_grad, const float* work) {
-  WRF_COLUMN_INDEX(g, j, i);
-  const int ktf = g.nz - 1, nx = g.nx;
-  const size_t lev = (size_t)g.ny * nx, c = (size_t)j * nx + i;
-  const float rdx = g.rdx, rdy = g.rdy;
+// (b[WF_T] is rewritten here, so this runs after the two passes above)
+__global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g, S s, S b, float dts, int ref_no_grad,
+                                                                         const float* work) {
+  extern __shared__ float mut_smem[];
+  const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx, n = nz * kMutTX;
+  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const bool in = mut_in(g, j, i);
   // muu, muv: the u / v terms of the divergence at this column
-  {
+  const bool w = i >= 1 && mut_in(g, j, i - 1), sth = mut_in(g, j - 1, i), any = w || in || sth;
+  const int c = any ? j * nx + i : 0;
+  float *const sdv = mut_smem + threadIdx.x, *const sw = sdv + n;            // dvdxi, W
+  float *const sq = sdv + 2 * n, *const sr = sdv + 3 * n;                    // muu, muv terms
+  float *const swb = sdv + 4 * n, *const swd = sdv + 5 * n;                  // wwb, wdb
+  __shared__ float sdm[kMutTX], sqs[kMutTX], sws[kMutTX];
+  if (any) {
+    const float rdx = g.rdx, rdy = g.rdy;
+    const float mw = w ? s[WF_MSFTX][c - 1] * s[WF_MSFTY][c - 1] : 0.f;
+    const float mo = in ? s[WF_MSFTX][c] * s[WF_MSFTY][c] : 0.f;
+    const float ms = sth ? s[WF_MSFTX][c - nx] * s[WF_MSFTY][c - nx] : 0.f;
+    const float mfu = s[WF_MSFUY][c], r_mfu = __frcp_rn(mfu), mvi = s[WF_MSFVX_INV][c];
+#pragma unroll 4
+    for (int k = tk; k < ktf; k += kMutKT) {
+      const int p = k * lev + c;
+      const float wo = in ? __ldg(work + p) : 0.f;
+      float ub = 0.f, vb = 0.f;
+      if (w) ub += mw * rdx * __ldg(work + p - 1);
+      if (in) ub -= mo * rdx * wo;
+      if (sth) vb += ms * rdy * __ldg(work + p - nx);
+      if (in) vb -= mo * rdy * wo;
+      sq[k * kMutTX] = divc(ub * __ldg(s[WF_U_SAVE] + p), mfu, r_mfu);
+      sr[k * kMutTX] = vb * __ldg(s[WF_V_SAVE] + p) * mvi;
+    }
+  }
+  if (in) {
+    const MutDiv d(g, s, c);
+    const float dm = dts * s[WF_MSFTY][c];
+#pragma unroll 2
+    for (int k = tk; k < ktf; k += kMutKT) {
+      const int p = k * lev + c;
+      sdv[k * kMutTX] = d.at(g, s, p);
+      float wdb, wwb;
+      mut_ww_bar(g, s, b, dm, k, p, wdb, wwb);
+      swb[k * kMutTX] = wwb;
+      swd[k * kMutTX] = wdb;
+    }
+  }
+  __syncthreads();
+  // one warp per sum: dmdt; muu and muv; the sums over ww's cotangent (the
+  // scan passes every ww' cotangent down to ww(0))
+  if (in && tk == 0) {
+    float dmdt = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < ktf; ++k) dmdt = dmdt + __ldg(s[WF_DNW] + k) * sdv[k * kMutTX];
+    sdm[threadIdx.x] = dmdt;
+  } else if (any && tk == 1) {
     float amuu = 0.f, amuv = 0.f;
-    const bool w = i >= 1 && mut_in(g, j, i - 1), o = mut_in(g, j, i), sth = j >= 1 && mut_in(g, j - 1, i);
-    if (w || o || sth) {
-      const float mw = w ? s[WF_MSFTX][c - 1] * s[WF_MSFTY][c - 1] : 0.f;
-      const float mo = o ? s[WF_MSFTX][c] * s[WF_MSFTY][c] : 0.f;
-      const float ms = sth ? s[WF_MSFTX][c - nx] * s[WF_MSFTY][c - nx] : 0.f;
 #pragma unroll 8
-      for (int k = 0; k < ktf; ++k) {
-        const size_t p = k * lev + c;
-        float ub = 0.f, vb = 0.f;
-        if (w) ub += mw * rdx * work[p - 1];
-        if (o) ub -= mo * rdx * work[p];
-        if (sth) vb += ms * rdy * work[p - nx];
-        if (o) vb -= mo * rdy * work[p];
-        amuu += ub * s[WF_U_SAVE][p] / s[WF_MSFUY][c];
-        amuv += vb * s[WF_V_SAVE][p] * s[WF_MSFVX_INV][c];
-      }
-      if (amuu != 0.f) b[WF_MUU][c] += amuu;
-      if (amuv != 0.f) b[WF_MUV][c] += amuv;
+    for (int k = 0; k < ktf; ++k) {
+      amuu += sq[k * kMutTX];
+      amuv += sr[k * kMutTX];
     }
+    if (amuu != 0.f) b[WF_MUU][c] += amuu;
+    if (amuv != 0.f) b[WF_MUV][c] += amuv;
+  } else if (in && tk == 2) {
+    const float msfty = s[WF_MSFTY][c], r_msfty = __frcp_rn(msfty);
+    float wsum = 0.f, qsum = 0.f, S_ = 0.f;
+#pragma unroll 8
+    for (int k = ktf - 1; k >= 1; --k) {
+      S_ += swb[k * kMutTX];
+      qsum += divc(-__ldg(s[WF_DNW] + k - 1), msfty, r_msfty) * S_;
+    }
+#pragma unroll 8
+    for (int k = 0; k < ktf; ++k) wsum += swb[k * kMutTX];
+    sqs[threadIdx.x] = qsum;
+    sws[threadIdx.x] = wsum;
   }
-  if (!mut_in(g, j, i)) return;
-  MutCol m;
-  mut_column(g, s, j, i, m);
-  float wdb[kMaxNz], wwb[kMaxNz];
-  mut_ww_bar(g, s, b, dts, j, i, m, wdb, wwb);
+  __syncthreads();
+  mut_scan(g, s, in, c, in ? sdm[threadIdx.x] : 0.f, sdv, sw);
+  if (!in) return;
   const float msfty = s[WF_MSFTY][c];
-  // ww, ww_1 (the scan passes every ww' cotangent down to ww(0))
-  float wsum = 0.f, qsum = 0.f, S_ = 0.f;
-#pragma unroll 8
-  for (int k = ktf - 1; k >= 1; --k) {
-    S_ += wwb[k];
-    qsum += -s[WF_DNW][k - 1] / msfty * S_;
-  }
-  // (the arrays may alias as far as the compiler knows: each block of
-  // kMutChunk levels loads everything it reads before its first store, so
-  // the loads issue together)
-  for (int k0 = 0; k0 < ktf; k0 += kMutChunk) {
-    float w1[kMutChunk];
-#pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) w1[q] = k0 + q < ktf ? b[WF_WW1][(k0 + q) * lev + c] : 0.f;
-#pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      if (k >= ktf) break;
-      wsum += wwb[k];
-      b[WF_WW1][k * lev + c] = w1[q] - wwb[k];
-      if (k >= 1) b[WF_WW][k * lev + c] = 0.f;
-    }
-  }
-  b[WF_WW][c] = wsum;
-  // theta: t_ave = t, ft, the vertical fluxes' t_1 (t_1(k) takes level k's
-  // fnm term, then level k + 1's fnp term)
   const float* fnm = s[WF_FNM];
   const float* fnp = s[WF_FNP];
-  for (int k0 = 0; k0 < ktf; k0 += kMutChunk) {
-    float tb[kMutChunk], tt[kMutChunk], t2s[kMutChunk], tsv[kMutChunk], fm[kMutChunk], fp[kMutChunk];
+  const float* ww1 = s[WF_WW1];
+  // theta: t_ave = t, ft, the vertical fluxes' t_1 (t_1(k) takes level k's
+  // fnm term, then level k + 1's fnp term); ww, ww_1.  Two levels' loads
+  // before their stores.
+  for (int kb = tk; kb < ktf; kb += 2 * kMutKT) {
+    float w1b[2], tb[2], tt[2], t2s[2], tsv[2], wk[2], wu[2];
 #pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      const size_t p = (size_t)(k < ktf ? k : 0) * lev + c;
-      tb[q] = k < ktf ? b[WF_T][p] : 0.f;
-      tt[q] = k < ktf ? b[WF_T_TEND][p] : 0.f;
-      t2s[q] = k < ktf ? b[WF_T_2SAVE][p] : 0.f;
-      tsv[q] = k < ktf ? b[WF_T_SAVE][p] : 0.f;
-      fm[q] = k >= 1 && k < ktf ? fnm[k] : 0.f;
-      fp[q] = k + 1 < ktf ? fnp[k + 1] : 0.f;
+    for (int q = 0; q < 2; ++q) {
+      const int k = kb + q * kMutKT;
+      if (k >= ktf) continue;
+      const int p = k * lev + c;
+      w1b[q] = b[WF_WW1][p];
+      tb[q] = b[WF_T][p];
+      tt[q] = b[WF_T_TEND][p];
+      t2s[q] = b[WF_T_2SAVE][p];
+      tsv[q] = b[WF_T_SAVE][p];
+      wk[q] = sw[k * kMutTX] - __ldg(ww1 + p);
+      wu[q] = k + 1 < ktf ? sw[(k + 1) * kMutTX] - __ldg(ww1 + p + lev) : 0.f;
     }
 #pragma unroll
-    for (int q = 0; q < kMutChunk; ++q) {
-      const int k = k0 + q;
-      if (k >= ktf) break;
-      const size_t p = k * lev + c;
+    for (int q = 0; q < 2; ++q) {
+      const int k = kb + q * kMutKT;
+      if (k >= ktf) continue;
+      const int p = k * lev + c;
+      b[WF_WW1][p] = w1b[q] - swb[k * kMutTX];
+      b[WF_WW][p] = k >= 1 ? 0.f : sws[threadIdx.x];
       b[WF_T_TEND][p] = tt[q] + msfty * dts * tb[q];
       b[WF_T][p] = tb[q] + t2s[q];
       b[WF_T_2SAVE][p] = 0.f;
       float x = tsv[q];
-      if (k >= 1) x += wdb[k] * m.wwp[k] * fm[q];
-      if (k + 1 < ktf) x += wdb[k + 1] * m.wwp[k + 1] * fp[q];
+      if (k >= 1) x += swd[k * kMutTX] * wk[q] * __ldg(fnm + k);
+      if (k + 1 < ktf) x += swd[(k + 1) * kMutTX] * wu[q] * __ldg(fnp + k + 1);
       b[WF_T_SAVE][p] = x;
     }
   }
   // the mu update
+  if (tk != 0) return;
+  const float qsum = sqs[threadIdx.x];
   if (ref_no_grad) {
     b[WF_MU_TEND][c] += qsum;
   } else {
@@ -959,18 +1051,24 @@ __global__ void k_advance_mu_t_adj_col(Grid g, S s, S b, float dts, int ref_no_g
   }
 }
 
+// the rows of the updated columns (more: those above them, which muv's cotangent reaches)
+static dim3 mut_grid(const Grid& g, int more) {
+  return dim3((g.ide - 1 + kMutTX - 1) / kMutTX, g.jde - 3 - g.jds + more);
+}
+
 int launch_advance_mu_t(const Grid& g, const S& s, float dts, cudaStream_t st) {
-  const dim3 b2(32, 4);
-  k_advance_mu_t<<<col_grid(g, b2), b2, 0, st>>>(g, s, dts);
+  k_advance_mu_t<<<mut_grid(g, 0), dim3(kMutTX, kMutKT), 2 * (size_t)g.nz * kMutTX * sizeof(float), st>>>(g, s, dts);
   return 1;
 }
 
 int launch_advance_mu_t_adj(const Grid& g, const S& s, const S& b, float dts, int ref_no_grad, float* work,
                             cudaStream_t st) {
   const dim3 b2(32, 4), b3(32, 4);
-  k_advance_mu_t_adj_dv<<<col_grid(g, b2), b2, 0, st>>>(g, s, b, dts, ref_no_grad, work);
+  const size_t col = (size_t)g.nz * kMutTX * sizeof(float);
+  k_advance_mu_t_adj_dv<<<mut_grid(g, 0), dim3(kMutTX, kMutKT), col, st>>>(g, s, b, dts, ref_no_grad, work);
   k_advance_mu_t_adj_pt<<<point_grid(g, b3), b3, 0, st>>>(g, s, b, dts, work);
-  k_advance_mu_t_adj_col<<<col_grid(g, b2), b2, 0, st>>>(g, s, b, dts, ref_no_grad, work);
+  allow_smem(k_advance_mu_t_adj_col, 6 * col);
+  k_advance_mu_t_adj_col<<<mut_grid(g, 1), dim3(kMutTX, kMutKT), 6 * col, st>>>(g, s, b, dts, ref_no_grad, work);
   return 3;
 }
 
@@ -1697,13 +1795,6 @@ int launch_vsolve_w(int ncol, int nz, const float* x, const float* a, const floa
   k_vsolve_w<<<(ncol + kVsTX - 1) / kVsTX, kVsTX * kVsKT, 4 * nz * kVsTX * sizeof(float), st>>>(ncol, nz, x, a, alpha,
                                                                                                 gamma, w);
   return 1;
-}
-
-// a kernel whose dynamic shared memory can pass 48 KB has its limit raised
-// once per device
-template <typename K>
-static void allow_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 int launch_vsolve_w_adj(int ncol, int nz, const float* x, const float* a, const float* alpha, const float* gamma,
