@@ -255,6 +255,20 @@ int wrf_halo(const WrfGrid* g, float* field, char var, int two_d, void* stream);
  * the cotangent of the field before the copies (a separate array). */
 int wrf_halo_adj(const WrfGrid* g, const float* field_bar, float* in_bar, char var, int two_d, void* stream);
 /* wrf_boundary.py:358-400 zero_grad_bdy of w (all levels), in place. */
+/* out[f] = the halo copies of in[f] (stagger letter vars[f], two_d[f] as for
+ * wrf_halo; 'Z': zero_grad_bdy of w) for a batch of n fields, out of place,
+ * and the adjoint (in_bar[f] written, not accumulated); every out array is
+ * distinct from all the in arrays */
+int wrf_halo_copy(const WrfGrid* g, int n, const float* const* in, float* const* out, const char* vars,
+                  const int* two_d, void* stream);
+int wrf_halo_copy_adj(const WrfGrid* g, int n, const float* const* out_bar, float* const* in_bar, const char* vars,
+                      const int* two_d, void* stream);
+/* rk_scalar_tend's advection of the moisture species (slots 1..6 of moist and
+ * advect_tend, [7][nz][ny][nx]) by the mass fluxes: the points of [0, nz) x
+ * [jds, jde) x [ids, ide) of those slots are written */
+int wrf_advect_moist(const WrfGrid* g, const float* moist, float* advect_tend, const float* ru, const float* rv,
+                     const float* rom, const float* msftx, const float* fzm, const float* fzp, const float* rdzw,
+                     void* stream);
 int wrf_zero_grad_w(const WrfGrid* g, float* w, void* stream);
 /* Its adjoint: w_bar is added (+=) into in_bar (a separate array). */
 int wrf_zero_grad_w_adj(const WrfGrid* g, const float* w_bar, float* in_bar, void* stream);

@@ -136,6 +136,12 @@ def lib() -> ctypes.CDLL:
     L.wrf_halo.argtypes = [ctypes.POINTER(WrfGridC), vp, ctypes.c_char, ip, vp]
     L.wrf_halo_adj.restype = ip
     L.wrf_halo_adj.argtypes = [ctypes.POINTER(WrfGridC), vp, vp, ctypes.c_char, ip, vp]
+    pp = ctypes.POINTER(vp)
+    for nm in ("wrf_halo_copy", "wrf_halo_copy_adj"):
+        getattr(L, nm).restype = ip
+        getattr(L, nm).argtypes = [ctypes.POINTER(WrfGridC), ip, pp, pp, ctypes.c_char_p, ctypes.POINTER(ip), vp]
+    L.wrf_advect_moist.restype = ip
+    L.wrf_advect_moist.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 10
     L.wrf_zero_grad_w.restype = ip
     L.wrf_zero_grad_w.argtypes = [ctypes.POINTER(WrfGridC), vp, vp]
     L.wrf_zero_grad_w_adj.restype = ip

@@ -576,6 +576,116 @@ def zero_grad_w(w, rdx=1.0 / 9000.0, rdy=1.0 / 9000.0):
     return ZeroGradW.apply((rdx, rdy), w)
 
 
+class Halos(torch.autograd.Function):
+    """The halo copies of several fields in one launch each way: ``scal`` =
+    (vars, rdx, rdy), one letter of ``vars`` per tensor: a stagger letter of
+    :func:`halo`, 'Z' for zero_grad_bdy of w, or for a [7, nz, ny, nx]
+    moisture array 'M' (slots 1..6 as 'p', slot 0 copied)."""
+
+    @staticmethod
+    def _call(name, cg, letters, ins, outs):
+        pi, po, vs, td = [], [], [], []
+        for var, a, b in zip(letters, ins, outs):
+            if var == "M":
+                step = a.numel() // 7 * 4
+                for m in range(1, 7):
+                    pi.append(a.data_ptr() + m * step)
+                    po.append(b.data_ptr() + m * step)
+                    vs.append("p")
+                    td.append(0)
+                b[0].copy_(a[0])
+            else:
+                pi.append(a.data_ptr())
+                po.append(b.data_ptr())
+                vs.append(var)
+                td.append(int(a.dim() == 2))
+        n = len(pi)
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with torch.cuda.device(ins[0].device):
+            rc = getattr(N.lib(), name)(ctypes.byref(cg), n, (ctypes.c_void_p * n)(*pi), (ctypes.c_void_p * n)(*po),
+                                        "".join(vs).encode(), (ctypes.c_int * n)(*td), stream)
+        N.check(rc, name)
+
+    @staticmethod
+    def forward(ctx, scal, *fields):
+        ctx.set_materialize_grads(False)
+        _cuda_only(*fields)
+        letters = str(scal[0])
+        if len(letters) != len(fields):
+            raise ValueError("one letter per field")
+        shape = next((f.shape[-3:] for f in fields if f.dim() > 2), (12,) + tuple(fields[0].shape[-2:]))
+        for var, f in zip(letters, fields):
+            want = shape[1:] if f.dim() == 2 else ((7,) + tuple(shape) if var == "M" else shape)
+            if tuple(f.shape) != tuple(want):
+                raise ValueError(f"halos: a field of shape {tuple(f.shape)} where {tuple(want)} is expected")
+        cg = scalar_grid(shape, float(scal[1]), float(scal[2]))
+        outs = tuple(torch.empty_like(f) for f in fields)
+        Halos._call("wrf_halo_copy", cg, letters, [f.detach() for f in fields], outs)
+        ctx.cg, ctx.letters = cg, letters
+        return outs
+
+    @staticmethod
+    def backward(ctx, *gouts):
+        some = [q for q, gq in enumerate(gouts) if gq is not None]
+        gins = [None] * len(gouts)
+        if some:
+            gs = [gouts[q].contiguous() for q in some]
+            bs = [torch.empty_like(gq) for gq in gs]
+            Halos._call("wrf_halo_copy_adj", ctx.cg, "".join(ctx.letters[q] for q in some), gs, bs)
+            for q, b in zip(some, bs):
+                gins[q] = b
+        return (None,) + tuple(gins)
+
+
+def halos(fields: Sequence[torch.Tensor], letters: str, rdx=1.0 / 9000.0, rdy=1.0 / 9000.0):
+    """Differentiable halo copies of ``fields`` by ``letters`` (:class:`Halos`);
+    returns the new fields."""
+    return Halos.apply((letters, rdx, rdy), *fields)
+
+
+class AdvectMoist(torch.autograd.Function):
+    """The advection of qv .. qg (slots 1..6 of a [7, nz, ny, nx] array) by
+    (ru, rv, rom), as the step's advect_tend: zero outside the advected
+    points (pywrf/wrf_dynamics.py:3982-4051)."""
+
+    @staticmethod
+    def forward(ctx, moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx: float, rdy: float):
+        _cuda_only(moist, ru, rv, rom, msftx, fnm, fnp, rdnw)
+        cg = scalar_grid(ru.shape, rdx, rdy)
+        out = torch.zeros_like(moist)
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with torch.cuda.device(moist.device):
+            rc = N.lib().wrf_advect_moist(ctypes.byref(cg), _ptr(moist), _ptr(out), _ptr(ru), _ptr(rv), _ptr(rom),
+                                          _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw), stream)
+        N.check(rc, "wrf_advect_moist")
+        ctx.save_for_backward(moist, ru, rv, rom, msftx, fnm, fnp, rdnw)
+        ctx.cg = cg
+        return out
+
+    @staticmethod
+    def backward(ctx, gout):
+        moist, ru, rv, rom, msftx, fnm, fnp, rdnw = ctx.saved_tensors
+        gout = gout.contiguous()
+        qb, rub, rvb, romb = _zeros(moist, ru, ru, ru)
+        n = ctypes.c_size_t(0)
+        N.check(N.lib().wrf_advect_scalar_adj_work(ctypes.byref(ctx.cg), ctypes.byref(n)), "work")
+        work = torch.empty(int(n.value), dtype=torch.float32, device=moist.device)
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with torch.cuda.device(moist.device):
+            for m in range(1, 7):  # the species share the fluxes' cotangents
+                rc = N.lib().wrf_advect_scalar_adj(ctypes.byref(ctx.cg), _ptr(moist[m]), _ptr(ru), _ptr(rv),
+                                                   _ptr(rom), _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw),
+                                                   _ptr(gout[m]), _ptr(qb[m]), _ptr(rub), _ptr(rvb), _ptr(romb),
+                                                   _ptr(work), n, stream)
+                N.check(rc, "wrf_advect_scalar_adj")
+        return qb, rub, rvb, romb, None, None, None, None, None, None
+
+
+def advect_moist(moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx, rdy):
+    """Differentiable moisture advection on the GPU (:class:`AdvectMoist`)."""
+    return AdvectMoist.apply(moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx, rdy)
+
+
 AW_INPUTS = ("w", "rw_tend", "ww", "w_save", "u", "v", "muave", "muts", "mut", "t_2ave", "t_2", "t_1", "ph", "ph_1",
              "phb", "ph_tend", "ht", "c2a", "cqw", "alt", "a", "alpha", "gamma")
 AW_DATA = ("msftx", "msfty", "fnm", "fnp", "rdnw", "rdn")
@@ -959,15 +1069,11 @@ def acoustic_substep(st: dict, data: dict, iteration: int, nsub: int, dts: float
     s["ru_m"], s["rv_m"], s["ww_m"] = sumflux({k: s[k] for k in SF_INPUTS}, {k: data[k] for k in SF_DATA},
                                               iteration, nsub, rdx, rdy)
     s["ph"] = spec_bdyupdate_ph({k: s[k] for k in SPH_INPUTS}, dts, rdx, rdy)
-    s["w"] = zero_grad_w(s["w"], rdx, rdy)
     pr_in = {"al": s["al"], "p": s["p"], "ph": s["ph"], "alt": s["alt"], "t_2": s["t"], "t_1": s["t_save"],
              "c2a": s["c2a"], "pm1": s["pm1"], "mu": s["mu"], "mut": s["muts"]}
     s["al"], s["p"], s["pm1"] = calc_p_rho(pr_in, data["rdnw"], smdiv, iteration, rdx, rdy)
-    s["ph"] = halo(s["ph"], "w", rdx, rdy)
-    s["al"] = halo(s["al"], "p", rdx, rdy)
-    s["p"] = halo(s["p"], "p", rdx, rdy)
-    for k in ("muts", "mu", "mudf"):
-        s[k] = halo(s[k], "t", rdx, rdy)
+    names = ("w", "ph", "al", "p", "muts", "mu", "mudf")
+    s.update(zip(names, halos([s[k] for k in names], "Zwppttt", rdx, rdy)))
     return s
 
 
@@ -1091,16 +1197,15 @@ def acoustic_stage(st: dict, data: dict, rk_step: int, nsub: int, dts: float, *,
     s["al"], s["p"], s["pm1"] = calc_p_rho(pr, data["rdnw"], smdiv, 0, rdx, rdy)
     s["a"], s["alpha"], s["gamma"] = coef_w(s["mut"], s["cqw"], s["c2a"], data["rdn"], data["rdnw"], dts, epssm,
                                             top_lid, rdx, rdy)
-    for k, var in (("ru_tend", "u"), ("rv_tend", "v"), ("ph", "w"), ("al", "p"), ("p", "p"), ("t_1", "t"),
-                   ("t_save", "t"), ("mu_1", "t"), ("mu", "t"), ("mudf", "t")):
-        s[k] = halo(s[k], var, rdx, rdy)
+    names = ("ru_tend", "rv_tend", "ph", "al", "p", "t_1", "t_save", "mu_1", "mu", "mudf")
+    s.update(zip(names, halos([s[k] for k in names], "uvwppttttt", rdx, rdy)))
     sc = dict(epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3, rdx=rdx, rdy=rdy)
     for it in range(1, nsub + 1):
         s = acoustic_substep(s, data, it, nsub, dts, **sc)
     s = small_step_finish(s, data, dts, nsub, rk_step, rdx, rdy)
     if rk_step == 3:
-        for k, var in (("ru_m", "u"), ("rv_m", "v"), ("ww_m", "w"), ("mut", "t"), ("muts", "t")):
-            s[k] = halo(s[k], var, rdx, rdy)
+        names = ("ru_m", "rv_m", "ww_m", "mut", "muts")
+        s.update(zip(names, halos([s[k] for k in names], "uvwtt", rdx, rdy)))
     return s
 
 
@@ -1220,6 +1325,60 @@ def horizontal_diffusion(var: str, field, tend, mut, xk, data: dict, rdx, rdy, b
     """Differentiable ``tend + horizontal_diffusion(field)``; ``data`` maps
     the map factors of HDIFF_DATA."""
     return HorizontalDiffusion.apply((var, rdx, rdy), field, tend, mut, xk, base, *[data[k] for k in HDIFF_DATA])
+
+
+class MoistDiffusion(torch.autograd.Function):
+    """tend' = tend + horizontal_diffusion of qv .. qg (slots 1..6 of [7, nz,
+    ny, nx] arrays) with the column mass and eddy viscosity they share;
+    ``scal`` = (rdx, rdy), then the seven map factors of HDIFF_DATA."""
+
+    @staticmethod
+    def forward(ctx, scal, moist, tend, mut, xk, *maps):
+        _cuda_only(moist, tend, mut, xk, *maps)
+        cg = scalar_grid(xk.shape, float(scal[0]), float(scal[1]))
+        out = tend.detach().clone()
+        tab = _table(dict(zip(HDIFF_DATA, maps)))
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with torch.cuda.device(moist.device):
+            for m in range(1, 7):
+                rc = N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, b"m", _ptr(moist[m]), None, _ptr(mut),
+                                                      _ptr(xk), _ptr(out[m]), stream)
+                N.check(rc, "wrf_horizontal_diffusion")
+        ctx.cg = cg
+        ctx.save_for_backward(moist, mut, xk, *maps)
+        return out
+
+    @staticmethod
+    def backward(ctx, gout):
+        moist, mut, xk, *maps = ctx.saved_tensors
+        gout = gout.contiguous()
+        fb, mb, kb = _zeros(moist, mut, xk)
+        tab = _table(dict(zip(HDIFF_DATA, maps)))
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with torch.cuda.device(moist.device):
+            for m in range(1, 7):  # the species share the mass's and the viscosity's cotangents
+                rc = N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(ctx.cg), tab, b"m", _ptr(moist[m]), None,
+                                                          _ptr(mut), _ptr(xk), _ptr(gout[m]), _ptr(fb[m]), _ptr(mb),
+                                                          _ptr(kb), stream)
+                N.check(rc, "wrf_horizontal_diffusion_adj")
+        return (None, fb, gout, mb, kb) + (None,) * len(HDIFF_DATA)
+
+
+class PutSlot(torch.autograd.Function):
+    """A [7, nz, ny, nx] array with one slot replaced by a field."""
+
+    @staticmethod
+    def forward(ctx, slot: int, moist, field):
+        out = moist.detach().clone()
+        out[slot].copy_(field)
+        ctx.slot = slot
+        return out
+
+    @staticmethod
+    def backward(ctx, gout):
+        gm = gout.clone()
+        gm[ctx.slot].zero_()
+        return None, gm, gout[ctx.slot].contiguous()
 
 
 class MassWeight(torch.autograd.Function):
@@ -1344,15 +1503,13 @@ def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts:
         raise ValueError("the first stage's relaxation needs dtbc")
     s = dict(st)
     s.update(prep({k: s[k] for k in PREP_FIELDS}, {k: data[k] for k in PREP_DATA}, 127, rdx, rdy))
-    for k, var in (("ru", "u"), ("rv", "v"), ("rw", "w"), ("ww", "w"), ("php", "w"), ("alt", "t"), ("p", "p"),
-                   ("muu", "u"), ("muv", "v"), ("mut", "t"), ("al", "p"), ("ph", "w")):
-        s[k] = halo(s[k], var, rdx, rdy)
+    names = ("ru", "rv", "rw", "ww", "php", "alt", "p", "muu", "muv", "mut", "al", "ph")
+    s.update(zip(names, halos([s[k] for k in names], "uvwwwtpuvtpw", rdx, rdy)))
     if rk_step == 1:
         for k in ("ru_tendf", "rv_tendf", "rw_tendf", "ph_tendf", "t_tendf", "mu_tendf", "moist_tend"):
             s[k] = torch.zeros_like(st[k])
         s["xkmh"], s["xkhh"] = eddy_viscosity(s, data, rdx, rdy, cf1, cf2, cf3)
-        s["xkmh"] = halo(s["xkmh"], "t", rdx, rdy)
-        s["xkhh"] = halo(s["xkhh"], "t", rdx, rdy)
+        s["xkmh"], s["xkhh"] = halos([s["xkmh"], s["xkhh"]], "tt", rdx, rdy)
     for k in ("ru_tend", "rv_tend", "rw_tend", "t_tend", "ph_tend", "u_save", "v_save", "w_save", "ph_save",
               "t_save", "mu_tend", "mu_save"):
         s[k] = torch.zeros_like(st[k])
@@ -1412,32 +1569,25 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
     calc_p_rho_phi and, before the last stage, the halo copies."""
     s = dict(st)
     moist = s["moist"]
-    adv = [torch.zeros_like(moist[0])]
-    for im in range(1, 7):
-        adv.append(advect_scalar(moist[im], torch.zeros_like(moist[im]), s["ru_m"], s["rv_m"], s["ww_m"],
-                                 data["msftx"], data["fnm"], data["fnp"], data["rdnw"], rdx, rdy))
-    s["advect_tend"] = torch.stack(adv)
+    s["advect_tend"] = advect_moist(moist, s["ru_m"], s["rv_m"], s["ww_m"], data["msftx"], data["fnm"], data["fnp"],
+                                    data["rdnw"], rdx, rdy)
     if rk_step == 1:
         if bt is None or dtbc is None:
             raise ValueError("the first stage's qv relaxation needs its boundary arrays and dtbc")
-        hd = {k: data[k] for k in HDIFF_DATA}
-        mt = s["moist_tend"]
-        tends = [mt[0]] + [horizontal_diffusion("m", moist[im], mt[im], s["muts"], s["xkhh"], hd, rdx, rdy)
-                           for im in range(1, 7)]
+        mt = MoistDiffusion.apply((rdx, rdy), moist, s["moist_tend"], s["muts"], s["xkhh"],
+                                  *[data[k] for k in HDIFF_DATA])
         nz = moist.shape[1]
         rq = mass_weight(moist[1], s["mut"], nz - 1, rdx, rdy)
-        tends[1] = spec_bdytend(relax_bdytend(rq, tends[1], "t", dtbc, bt["q"]), bt["q"], "t", rdx, rdy)
-        s["moist_tend"] = torch.stack(tends)
-    op = _MoistUpdate(rk_step, dt_rk, moist[0])
+        qv = spec_bdytend(relax_bdytend(rq, mt[1], "t", dtbc, bt["q"]), bt["q"], "t", rdx, rdy)
+        s["moist_tend"] = PutSlot.apply(1, mt, qv)
+    op = _MoistUpdate(rk_step, dt_rk, s["u"])
     cg = scalar_grid(s["u"].shape, rdx, rdy)
     dd = {"msfty": data["msfty"], "ru_m": s["ru_m"].detach(), "rv_m": s["rv_m"].detach(), "rdnw": data["rdnw"]}
     outs = _TableOp.apply(op, cg, *[s[k] for k in op.fields], *[dd[k] for k in op.data])
     s.update(dict(zip(op.outputs, outs)))
     if rk_step < 3:
-        for k, var in (("u", "U"), ("v", "V"), ("w", "w"), ("t", "p"), ("ph", "w"), ("mu", "t")):
-            s[k] = halo(s[k], var, rdx, rdy)
-        m = s["moist"]
-        s["moist"] = torch.stack([m[0]] + [halo(m[im], "p", rdx, rdy) for im in range(1, 7)])
+        names = ("u", "v", "w", "t", "ph", "mu", "moist")
+        s.update(zip(names, halos([s[k] for k in names], "UVwpwtM", rdx, rdy)))
     return s
 
 
@@ -1490,11 +1640,8 @@ def step_end(st: dict, data: dict, bdy: dict, dtbc: float, *, cf1: float, cf2: f
     qv and set_w_surface.  ``bdy`` maps 'u', 'v', 't', 'ph', 'qv' to their
     boundary arrays (xs .. tye)."""
     s = dict(st)
-    for k, var in (("u_1", "U"), ("u", "U"), ("v_1", "V"), ("v", "V"), ("w_1", "w"), ("w", "w"), ("t_1", "p"),
-                   ("t", "p"), ("ph_1", "w"), ("ph", "w"), ("mu_1", "t"), ("mu", "t")):
-        s[k] = halo(s[k], var, rdx, rdy)
-    m = s["moist"]
-    s["moist"] = torch.stack([m[0]] + [halo(m[im], "p", rdx, rdy) for im in range(1, 7)])
+    names = ("u_1", "u", "v_1", "v", "w_1", "w", "t_1", "t", "ph_1", "ph", "mu_1", "mu", "moist")
+    s.update(zip(names, halos([s[k] for k in names], "UUVVwwppwwttM", rdx, rdy)))
     op = _BdyFinal()
     cg = scalar_grid(s["u"].shape, rdx, rdy)
     cg.cf1, cg.cf2, cg.cf3 = float(cf1), float(cf2), float(cf3)

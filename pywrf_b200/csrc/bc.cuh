@@ -26,6 +26,19 @@ int launch_bc(const Grid& g, const BcBatch& b, cudaStream_t st);
 // (k_adjoint_bc.cu: the incoming cotangent ibar is accumulated)
 int launch_halo(const Grid& g, float* field, char var, bool two_d, cudaStream_t st);
 int launch_halo_adj(const Grid& g, const float* fbar, float* ibar, char var, bool two_d, cudaStream_t st);
+// out = halo copies of in (or zero_grad_bdy(w) of it: zg), and its adjoint, for
+// a batch of fields in one launch each (k_adjoint_bc.cu)
+struct HaloItem {
+  const float* in;
+  float* out;
+  BcItem bc;
+  int zg;
+};
+struct HaloBatch {
+  int n = 0;
+  HaloItem item[kBcMax];
+};
+int launch_halo_copy(const Grid& g, const HaloBatch& b, bool adj, cudaStream_t st);
 int launch_zero_grad_w(const Grid& g, float* w, cudaStream_t st);
 int launch_zero_grad_w_adj(const Grid& g, const float* fbar, float* ibar, cudaStream_t st);
 

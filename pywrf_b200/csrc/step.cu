@@ -884,6 +884,28 @@ bool halo_var(char v) {
 }
 }  // namespace
 
+int wrf_advect_moist(const WrfGrid* gin, const float* moist, float* advect_tend, const float* ru, const float* rv,
+                     const float* rom, const float* msftx, const float* fzm, const float* fzp, const float* rdzw,
+                     void* stream) {
+  Grid g;
+  int rc = make_grid(gin, g);
+  if (rc) return rc;
+  if (!moist || !advect_tend || !ru || !rv || !rom || !msftx || !fzm || !fzp || !rdzw)
+    return fail(WRF_EINVAL, "null argument");
+  S s{};
+  s.f[WF_MOIST] = const_cast<float*>(moist);
+  s.f[WF_ADVECT_TEND] = advect_tend;
+  s.f[WF_RU_M] = const_cast<float*>(ru);
+  s.f[WF_RV_M] = const_cast<float*>(rv);
+  s.f[WF_WW_M] = const_cast<float*>(rom);
+  s.f[WF_MSFTX] = const_cast<float*>(msftx);
+  s.f[WF_FNM] = const_cast<float*>(fzm);
+  s.f[WF_FNP] = const_cast<float*>(fzp);
+  s.f[WF_RDNW] = const_cast<float*>(rdzw);
+  cudaGetLastError();
+  launch_advect_moist(g, s, static_cast<cudaStream_t>(stream));
+  return check_launch("advect_moist");
+}
 int wrf_halo(const WrfGrid* gin, float* field, char var, int two_d, void* stream) {
   Grid g;
   int rc = make_grid(gin, g);
@@ -906,6 +928,41 @@ int wrf_halo_adj(const WrfGrid* gin, const float* field_bar, float* in_bar, char
   return check_launch("halo_adj");
 }
 
+// the batch of wrf_halo_copy / wrf_halo_copy_adj, in chunks the kernel's
+// parameters hold and of at most 65535 (field, level) pairs
+static int halo_copy(const WrfGrid* gin, int n, const float* const* in, float* const* out, const char* vars,
+                     const int* two_d, bool adj, void* stream) {
+  Grid g;
+  int rc = make_grid(gin, g);
+  if (rc) return rc;
+  if (n < 1 || !in || !out || !vars || !two_d) return fail(WRF_EINVAL, "halo_copy: null argument or empty batch");
+  for (int f = 0; f < n; ++f) {
+    if (!in[f] || !out[f] || in[f] == out[f]) return fail(WRF_EINVAL, "halo_copy: two distinct arrays needed");
+    if (vars[f] != 'Z' && !halo_var(vars[f])) return fail(WRF_EINVAL, "halo_copy: unknown stagger letter");
+    if (vars[f] == 'Z' && two_d[f]) return fail(WRF_EINVAL, "halo_copy: zero_grad_bdy is for w");
+  }
+  cudaGetLastError();
+  for (int f0 = 0; f0 < n; f0 += kBcMax) {
+    HaloBatch b;
+    for (int f = f0; f < n && f < f0 + kBcMax; ++f) {
+      HaloItem& h = b.item[b.n++];
+      h.in = in[f];
+      h.out = out[f];
+      h.zg = vars[f] == 'Z' ? 1 : 0;
+      h.bc = bc_item(g, nullptr, h.zg ? 'w' : vars[f], two_d[f] != 0);
+    }
+    launch_halo_copy(g, b, adj, static_cast<cudaStream_t>(stream));
+  }
+  return check_launch("halo_copy");
+}
+int wrf_halo_copy(const WrfGrid* gin, int n, const float* const* in, float* const* out, const char* vars,
+                  const int* two_d, void* stream) {
+  return halo_copy(gin, n, in, out, vars, two_d, false, stream);
+}
+int wrf_halo_copy_adj(const WrfGrid* gin, int n, const float* const* out_bar, float* const* in_bar, const char* vars,
+                      const int* two_d, void* stream) {
+  return halo_copy(gin, n, out_bar, in_bar, vars, two_d, true, stream);
+}
 int wrf_zero_grad_w(const WrfGrid* gin, float* w, void* stream) {
   Grid g;
   int rc = make_grid(gin, g);
