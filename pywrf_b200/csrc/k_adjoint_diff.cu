@@ -27,21 +27,32 @@ __device__ __forceinline__ void acc(float* a, size_t q, float v) {
   if (v != 0.f) atomicAdd(a + q, v);
 }
 
+enum { DV_U = 0, DV_V = 1, DV_W = 2, DV_M = 3 };
+
+// the points of coefficient e's (x minus, x plus, y minus, y plus) averages
+__host__ __device__ constexpr int mass_points(int var, int e) {
+  return var == DV_U ? (e < 2 ? 1 : 4) : var == DV_V ? (e < 2 ? 4 : 0) : var == DV_W ? 4 : 2;
+}
+__host__ __device__ constexpr int visc_points(int var, int e) {
+  return var == DV_U ? (e < 2 ? 1 : 4) : var == DV_V ? (e < 2 ? 4 : 1) : var == DV_W ? 4 : 2;
+}
+
 // one of the four coefficients: value = ratio * mavg * kavg * rd with the
-// averages over nm mut points (dj, di) and nk viscosity points (dk, dj, di),
-// each weighted by wm / wk
+// averages over mass_points mut points (dj, di) and visc_points viscosity
+// points (dk, dj, di), each weighted by wm / wk.  The variable is a template
+// parameter of everything below, so that the points are constants of the
+// unrolled code: as run-time lists they lived in local memory, and the
+// kernels (174 us forward, 207 us reverse per field at 240x240x41) waited on
+// them.
 struct Coef {
-  float ratio, rd, wm, wk;
-  int nm, nk;
-  bool kfirst;  // the viscosity average multiplies before the mass average
+  float ratio, rd, wm, wk, mavg;
   int mj[4], mi[4], kk[4], kj[4], ki[4];
 };
 
-enum { DV_U = 0, DV_V = 1, DV_W = 2, DV_M = 3 };
-
-// the four coefficients (x minus, x plus, y minus, y plus) of variable var at
-// column c, in the reference's formulas
-__device__ void diff_coefs(const Grid& g, const S& s, int var, int c, Coef (&cf)[4]) {
+// the four coefficients of variable VAR at column c, in the reference's
+// formulas
+template <int VAR>
+__device__ __forceinline__ void diff_coefs(const Grid& g, const S& s, const float* mut, int c, Coef (&cf)[4]) {
   const int nx = g.nx;
   const float* msftx = s[WF_MSFTX];
   const float* msfty = s[WF_MSFTY];
@@ -50,55 +61,63 @@ __device__ void diff_coefs(const Grid& g, const S& s, int var, int c, Coef (&cf)
   const float* msfvx = s[WF_MSFVX];
   const float* msfvy = s[WF_MSFVY];
   const float* msfvi = s[WF_MSFVX_INV];
-  auto set = [](Coef& a, float ratio, float rd, float wm, float wk, int nm, int nk) {
-    a.ratio = ratio; a.rd = rd; a.wm = wm; a.wk = wk; a.nm = nm; a.nk = nk; a.kfirst = false;
+  auto set = [](Coef& a, float ratio, float rd, float wm, float wk) {
+    a.ratio = ratio; a.rd = rd; a.wm = wm; a.wk = wk;
   };
   auto mp = [](Coef& a, int e, int dj, int di) { a.mj[e] = dj; a.mi[e] = di; };
   auto kp = [](Coef& a, int e, int dk, int dj, int di) { a.kk[e] = dk; a.kj[e] = dj; a.ki[e] = di; };
   const float rdx = g.rdx, rdy = g.rdy;
-  if (var == DV_U) {
-    set(cf[0], msftx[c - 1] / msfty[c - 1], rdx, 1.f, 1.f, 1, 1); mp(cf[0], 0, 0, -1); kp(cf[0], 0, 0, 0, -1);
-    set(cf[1], msftx[c] / msfty[c], rdx, 1.f, 1.f, 1, 1); mp(cf[1], 0, 0, 0); kp(cf[1], 0, 0, 0, 0);
+  if constexpr (VAR == DV_U) {
+    set(cf[0], msftx[c - 1] / msfty[c - 1], rdx, 1.f, 1.f); mp(cf[0], 0, 0, -1); kp(cf[0], 0, 0, 0, -1);
+    set(cf[1], msftx[c] / msfty[c], rdx, 1.f, 1.f); mp(cf[1], 0, 0, 0); kp(cf[1], 0, 0, 0, 0);
+#pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int d = e == 0 ? -1 : 1;
-      set(cf[2 + e], (msfuy[c] + msfuy[c + d * nx]) / (msfux[c] + msfux[c + d * nx]), rdy, 0.25f, 0.25f, 4, 4);
+      set(cf[2 + e], (msfuy[c] + msfuy[c + d * nx]) / (msfux[c] + msfux[c + d * nx]), rdy, 0.25f, 0.25f);
       mp(cf[2 + e], 0, 0, 0); mp(cf[2 + e], 1, d, 0); mp(cf[2 + e], 2, d, -1); mp(cf[2 + e], 3, 0, -1);
       kp(cf[2 + e], 0, 0, 0, 0); kp(cf[2 + e], 1, 0, d, 0); kp(cf[2 + e], 2, 0, d, -1); kp(cf[2 + e], 3, 0, 0, -1);
     }
-  } else if (var == DV_V) {
+  } else if constexpr (VAR == DV_V) {
+#pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int d = e == 0 ? -1 : 1;
-      set(cf[e], (msfvx[c] + msfvx[c + d]) / (msfvy[c] + msfvy[c + d]), rdx, 0.25f, 0.25f, 4, 4);
+      set(cf[e], (msfvx[c] + msfvx[c + d]) / (msfvy[c] + msfvy[c + d]), rdx, 0.25f, 0.25f);
       mp(cf[e], 0, 0, 0); mp(cf[e], 1, -1, 0); mp(cf[e], 2, -1, d); mp(cf[e], 3, 0, d);
       kp(cf[e], 0, 0, 0, 0); kp(cf[e], 1, 0, -1, 0); kp(cf[e], 2, 0, -1, d); kp(cf[e], 3, 0, 0, d);
     }
-    set(cf[2], msfty[c - nx] / msftx[c - nx], rdy, 0.f, 1.f, 0, 1); kp(cf[2], 0, 0, -1, 0);
-    set(cf[3], msfty[c] / msftx[c], rdy, 0.f, 1.f, 0, 1); kp(cf[3], 0, 0, 0, 0);
-  } else if (var == DV_W) {
+    set(cf[2], msfty[c - nx] / msftx[c - nx], rdy, 0.f, 1.f); kp(cf[2], 0, 0, -1, 0);
+    set(cf[3], msfty[c] / msftx[c], rdy, 0.f, 1.f); kp(cf[3], 0, 0, 0, 0);
+  } else if constexpr (VAR == DV_W) {
     // 0.25 (m(a) + m(b) + m(a) + m(b)): the pair is listed twice, as the
     // reference sums it
-    set(cf[0], msfux[c] / msfuy[c], rdx, 0.25f, 0.25f, 4, 4);
+    set(cf[0], msfux[c] / msfuy[c], rdx, 0.25f, 0.25f);
     mp(cf[0], 0, 0, 0); mp(cf[0], 1, 0, -1); mp(cf[0], 2, 0, 0); mp(cf[0], 3, 0, -1);
     kp(cf[0], 0, 0, 0, 0); kp(cf[0], 1, 0, 0, -1); kp(cf[0], 2, -1, 0, 0); kp(cf[0], 3, -1, 0, -1);
-    set(cf[1], msfux[c + 1] / msfuy[c + 1], rdx, 0.25f, 0.25f, 4, 4);
+    set(cf[1], msfux[c + 1] / msfuy[c + 1], rdx, 0.25f, 0.25f);
     mp(cf[1], 0, 0, 1); mp(cf[1], 1, 0, 0); mp(cf[1], 2, 0, 1); mp(cf[1], 3, 0, 0);
     kp(cf[1], 0, 0, 0, 1); kp(cf[1], 1, 0, 0, 0); kp(cf[1], 2, -1, 0, 1); kp(cf[1], 3, -1, 0, 0);
-    set(cf[2], msfvy[c] / msfvx[c], rdy, 0.25f, 0.25f, 4, 4);
+    set(cf[2], msfvy[c] / msfvx[c], rdy, 0.25f, 0.25f);
     mp(cf[2], 0, 0, 0); mp(cf[2], 1, -1, 0); mp(cf[2], 2, 0, 0); mp(cf[2], 3, -1, 0);
     kp(cf[2], 0, 0, 0, 0); kp(cf[2], 1, 0, -1, 0); kp(cf[2], 2, -1, 0, 0); kp(cf[2], 3, -1, -1, 0);
-    set(cf[3], msfvy[c + nx] / msfvx[c + nx], rdy, 0.25f, 0.25f, 4, 4);
+    set(cf[3], msfvy[c + nx] / msfvx[c + nx], rdy, 0.25f, 0.25f);
     mp(cf[3], 0, 1, 0); mp(cf[3], 1, 0, 0); mp(cf[3], 2, 1, 0); mp(cf[3], 3, 0, 0);
     kp(cf[3], 0, 0, 1, 0); kp(cf[3], 1, 0, 0, 0); kp(cf[3], 2, -1, 1, 0); kp(cf[3], 3, -1, 0, 0);
   } else {
-    set(cf[0], msfux[c] / msfuy[c], rdx, 0.5f, 0.5f, 2, 2);
+    set(cf[0], msfux[c] / msfuy[c], rdx, 0.5f, 0.5f);
     mp(cf[0], 0, 0, 0); mp(cf[0], 1, 0, -1); kp(cf[0], 0, 0, 0, 0); kp(cf[0], 1, 0, 0, -1);
-    set(cf[1], msfux[c + 1] / msfuy[c + 1], rdx, 0.5f, 0.5f, 2, 2);
+    set(cf[1], msfux[c + 1] / msfuy[c + 1], rdx, 0.5f, 0.5f);
     mp(cf[1], 0, 0, 1); mp(cf[1], 1, 0, 0); kp(cf[1], 0, 0, 0, 1); kp(cf[1], 1, 0, 0, 0);
-    set(cf[2], msfvy[c] * msfvi[c], rdy, 0.5f, 0.5f, 2, 2);
+    set(cf[2], msfvy[c] * msfvi[c], rdy, 0.5f, 0.5f);
     mp(cf[2], 0, 0, 0); mp(cf[2], 1, -1, 0); kp(cf[2], 0, 0, 0, 0); kp(cf[2], 1, 0, -1, 0);
-    set(cf[3], msfvy[c + nx] * msfvi[c + nx], rdy, 0.5f, 0.5f, 2, 2);
+    set(cf[3], msfvy[c + nx] * msfvi[c + nx], rdy, 0.5f, 0.5f);
     mp(cf[3], 0, 1, 0); mp(cf[3], 1, 0, 0); kp(cf[3], 0, 0, 1, 0); kp(cf[3], 1, 0, 0, 0);
-    for (int e = 0; e < 4; ++e) cf[e].kfirst = true;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float ms = 0.f;
+#pragma unroll
+    for (int q = 0; q < mass_points(VAR, e); ++q) ms = ms + __ldg(mut + c + cf[e].mj[q] * nx + cf[e].mi[q]);
+    cf[e].mavg = mass_points(VAR, e) ? cf[e].wm * ms : 1.f;
   }
 }
 
@@ -114,23 +133,26 @@ __device__ __forceinline__ bool diff_region(const Grid& g, int var, int k, int j
 
 struct DiffPoint {
   float kx[4];   // the coefficients
-  float mavg[4], kavg[4];
+  float kavg[4];
   float d[4];    // dxm, dxp, dym, dyp
   float mr[2];   // mrdx, mrdy
 };
 
-__device__ void diff_point(const Grid& g, const S& s, int var, const float* f, const float* base, const float* mut,
-                           const float* K, int k, int c, size_t p, const Coef (&cf)[4], DiffPoint& o) {
-  const int nx = g.nx;
-  const size_t lev = (size_t)g.ny * nx;
+template <int VAR>
+__device__ __forceinline__ void diff_point(const Grid& g, const S& s, const float* __restrict__ f,
+                                           const float* __restrict__ base, const float* __restrict__ K, int c, int p,
+                                           const Coef (&cf)[4], DiffPoint& o) {
+  const int nx = g.nx, lev = g.ny * nx;
+#pragma unroll
   for (int e = 0; e < 4; ++e) {
-    float ms = 0.f, ks = 0.f;
-    for (int q = 0; q < cf[e].nm; ++q) ms = ms + mut[c + cf[e].mj[q] * nx + cf[e].mi[q]];
-    for (int q = 0; q < cf[e].nk; ++q) ks = ks + K[p + (long)cf[e].kk[q] * (long)lev + cf[e].kj[q] * nx + cf[e].ki[q]];
-    o.mavg[e] = cf[e].nm ? cf[e].wm * ms : 1.f;
+    float ks = 0.f;
+#pragma unroll
+    for (int q = 0; q < visc_points(VAR, e); ++q)
+      ks = ks + __ldg(K + p + cf[e].kk[q] * lev + cf[e].kj[q] * nx + cf[e].ki[q]);
     o.kavg[e] = cf[e].wk * ks;
-    o.kx[e] = cf[e].kfirst ? cf[e].ratio * o.kavg[e] * o.mavg[e] * cf[e].rd
-                           : cf[e].ratio * o.mavg[e] * o.kavg[e] * cf[e].rd;
+    // a mass-point scalar's viscosity average multiplies before the mass average
+    o.kx[e] = VAR == DV_M ? cf[e].ratio * o.kavg[e] * cf[e].mavg * cf[e].rd
+                          : cf[e].ratio * cf[e].mavg * o.kavg[e] * cf[e].rd;
   }
   const float cc = f[p];
   const float xm = f[p - 1], xp = f[p + 1], ym = f[p - nx], yp = f[p + nx];
@@ -146,8 +168,8 @@ __device__ void diff_point(const Grid& g, const S& s, int var, const float* f, c
     o.d[2] = cc - ym;
     o.d[3] = yp - cc;
   }
-  const float* m1 = var == DV_U ? s[WF_MSFUX] : (var == DV_V ? s[WF_MSFVX] : s[WF_MSFTX]);
-  const float* m2 = var == DV_U ? s[WF_MSFUY] : (var == DV_V ? s[WF_MSFVY] : s[WF_MSFTY]);
+  const float* m1 = VAR == DV_U ? s[WF_MSFUX] : (VAR == DV_V ? s[WF_MSFVX] : s[WF_MSFTX]);
+  const float* m2 = VAR == DV_U ? s[WF_MSFUY] : (VAR == DV_V ? s[WF_MSFVY] : s[WF_MSFTY]);
   o.mr[0] = m1[c] * m2[c] * g.rdx;
   o.mr[1] = m1[c] * m2[c] * g.rdy;
 }
@@ -155,19 +177,23 @@ __device__ void diff_point(const Grid& g, const S& s, int var, const float* f, c
 // a thread takes one column's levels [z0, z0 + kHdiffLevels) of the
 // diffusion region: the column's coefficients once, then its levels
 constexpr int kHdiffLevels = 8;
-__global__ void k_hdiff_op(Grid g, S s, int var, const float* f, const float* base, const float* mut, const float* K,
-                           float* tend) {
+template <int VAR>
+__global__ void __launch_bounds__(128) k_hdiff_op(Grid g, S s, const float* __restrict__ f,
+                                                  const float* __restrict__ base, const float* __restrict__ mut,
+                                                  const float* __restrict__ K, float* __restrict__ tend) {
+  constexpr int var = VAR;
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int z0 = blockIdx.z * kHdiffLevels;
   if (i >= g.nx || j >= g.ny || !diff_region(g, var, g.nz - 2, j, i)) return;
   const int c = g.i2(j, i);
   Coef cf[4];
-  diff_coefs(g, s, var, c, cf);
+  diff_coefs<VAR>(g, s, mut, c, cf);
+#pragma unroll 2
   for (int k = z0; k < z0 + kHdiffLevels && k < g.nz; ++k) {
     if (!diff_region(g, var, k, j, i)) continue;
-    const size_t p = (size_t)k * g.ny * g.nx + c;
+    const int p = k * g.ny * g.nx + c;
     DiffPoint o;
-    diff_point(g, s, var, f, base, mut, K, k, c, p, cf, o);
+    diff_point<VAR>(g, s, f, base, K, c, p, cf, o);
     tend[p] = tend[p] + (o.mr[0] * (o.kx[1] * o.d[1] - o.kx[0] * o.d[0]) + o.mr[1] * (o.kx[3] * o.d[3] - o.kx[2] * o.d[2]));
   }
 }
@@ -178,10 +204,12 @@ __global__ void k_hdiff_op(Grid g, S s, int var, const float* f, const float* ba
 // (the cotangent outputs are distinct from every operand and from each
 // other: __restrict__ lets a level's loads run ahead of the previous
 // level's atomic adds)
-__global__ void k_hdiff_op_adj(Grid g, S s, int var, const float* __restrict__ f, const float* __restrict__ base,
+template <int VAR>
+__global__ void __launch_bounds__(128) k_hdiff_op_adj(Grid g, S s, const float* __restrict__ f, const float* __restrict__ base,
                                const float* __restrict__ mut, const float* __restrict__ K,
                                const float* __restrict__ tbar, float* __restrict__ fbar, float* __restrict__ mutbar,
                                float* __restrict__ Kbar) {
+  constexpr int var = VAR;
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int z0 = blockIdx.z * kHdiffLevels;
   if (i >= g.nx || j >= g.ny || !diff_region(g, var, g.nz - 2, j, i)) return;
@@ -189,7 +217,7 @@ __global__ void k_hdiff_op_adj(Grid g, S s, int var, const float* __restrict__ f
   const size_t lev = (size_t)g.ny * nx;
   const int c = g.i2(j, i);
   Coef cf[4];
-  diff_coefs(g, s, var, c, cf);
+  diff_coefs<VAR>(g, s, mut, c, cf);
   float wm[4] = {0.f, 0.f, 0.f, 0.f};  // the mass averages' cotangents, per edge
   const float sgn[4] = {-1.f, 1.f, -1.f, 1.f};
 #pragma unroll 2
@@ -199,7 +227,7 @@ __global__ void k_hdiff_op_adj(Grid g, S s, int var, const float* __restrict__ f
     const float T = tbar[p];
     if (T == 0.f) continue;
     DiffPoint o;
-    diff_point(g, s, var, f, base, mut, K, k, c, p, cf, o);
+    diff_point<VAR>(g, s, f, base, K, c, (int)p, cf, o);
     // d/d(differences): +-mr * k..
     const float gx0 = -o.mr[0] * o.kx[0] * T, gx1 = o.mr[0] * o.kx[1] * T;
     const float gy0 = -o.mr[1] * o.kx[2] * T, gy1 = o.mr[1] * o.kx[3] * T;
@@ -217,10 +245,11 @@ __global__ void k_hdiff_op_adj(Grid g, S s, int var, const float* __restrict__ f
       const float mr = e < 2 ? o.mr[0] : o.mr[1];
       const float kb = sgn[e] * mr * o.d[e] * T;  // cotangent of k..
       const float base_c = cf[e].ratio * cf[e].rd * kb;
-      if (cf[e].nm) wm[e] += base_c * o.kavg[e] * cf[e].wm;
+      if (mass_points(VAR, e)) wm[e] += base_c * o.kavg[e] * cf[e].wm;
       if (Kbar) {
-        const float wkb = base_c * o.mavg[e] * cf[e].wk;
-        for (int q = 0; q < cf[e].nk; ++q)
+        const float wkb = base_c * cf[e].mavg * cf[e].wk;
+#pragma unroll
+        for (int q = 0; q < visc_points(VAR, e); ++q)
           acc(Kbar, p + (long)cf[e].kk[q] * (long)lev + cf[e].kj[q] * nx + cf[e].ki[q], wkb);
       }
     }
@@ -228,7 +257,8 @@ __global__ void k_hdiff_op_adj(Grid g, S s, int var, const float* __restrict__ f
   if (mutbar)
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      for (int q = 0; q < cf[e].nm; ++q) acc(mutbar, c + cf[e].mj[q] * nx + cf[e].mi[q], wm[e]);
+#pragma unroll
+      for (int q = 0; q < mass_points(VAR, e); ++q) acc(mutbar, c + cf[e].mj[q] * nx + cf[e].mi[q], wm[e]);
 }
 
 // ---- the eddy viscosities ----
@@ -480,17 +510,21 @@ __global__ void k_mass_weight_adj(Grid g, const float* f, const float* mut, cons
 // var: 'u', 'v', 'w' or 'm' (a scalar; with base, theta's diffusion about it)
 int launch_hdiff_op(const Grid& g, const S& s, char var, const float* f, const float* base, const float* mut,
                     const float* K, float* tend, cudaStream_t st) {
-  const int v = var == 'u' ? DV_U : (var == 'v' ? DV_V : (var == 'w' ? DV_W : DV_M));
   const dim3 b3(32, 4), grid((g.nx + 31) / 32, (g.ny + 3) / 4, (g.nz + kHdiffLevels - 1) / kHdiffLevels);
-  k_hdiff_op<<<grid, b3, 0, st>>>(g, s, v, f, base, mut, K, tend);
+  if (var == 'u') k_hdiff_op<DV_U><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tend);
+  else if (var == 'v') k_hdiff_op<DV_V><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tend);
+  else if (var == 'w') k_hdiff_op<DV_W><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tend);
+  else k_hdiff_op<DV_M><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tend);
   return 1;
 }
 
 int launch_hdiff_op_adj(const Grid& g, const S& s, char var, const float* f, const float* base, const float* mut,
                         const float* K, const float* tbar, float* fbar, float* mutbar, float* Kbar, cudaStream_t st) {
-  const int v = var == 'u' ? DV_U : (var == 'v' ? DV_V : (var == 'w' ? DV_W : DV_M));
   const dim3 b3(32, 4), grid((g.nx + 31) / 32, (g.ny + 3) / 4, (g.nz + kHdiffLevels - 1) / kHdiffLevels);
-  k_hdiff_op_adj<<<grid, b3, 0, st>>>(g, s, v, f, base, mut, K, tbar, fbar, mutbar, Kbar);
+  if (var == 'u') k_hdiff_op_adj<DV_U><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tbar, fbar, mutbar, Kbar);
+  else if (var == 'v') k_hdiff_op_adj<DV_V><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tbar, fbar, mutbar, Kbar);
+  else if (var == 'w') k_hdiff_op_adj<DV_W><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tbar, fbar, mutbar, Kbar);
+  else k_hdiff_op_adj<DV_M><<<grid, b3, 0, st>>>(g, s, f, base, mut, K, tbar, fbar, mutbar, Kbar);
   return 1;
 }
 
