@@ -131,8 +131,8 @@ __device__ void fpvs(const T& t, const T& p, T& qs0, T& qs1) {
   T a = vmin(w1, 0.99f * p);
   a = F(EP2) * a / (p - a);
   qs0 = vmax(a, F(QMIN));
-  const T w0 = F(PSAT) * vexp(vlog(tr) * F(xai)) * vexp(F(xbi) * (1.0f - tr));
-  T b = val(t) < F(ttp) ? w0 : w1;
+  T b = w1;
+  if (val(t) < F(ttp)) b = F(PSAT) * vexp(vlog(tr) * F(xai)) * vexp(F(xbi) * (1.0f - tr));
   b = vmin(b, 0.99f * p);
   b = F(EP2) * b / (p - b);
   qs1 = vmax(b, F(QMIN));
@@ -206,36 +206,24 @@ __device__ void remap(const Col<T>& C, int km, int qa, int out) {
   }
 }
 
-// the mass that left through the ground (wrf_physics.py:1361-1374)
-template <class T>
-__device__ T surface_flux(const Col<T>& C, int km, int qa) {
-  T precip = cst<T>(0.f);
-  for (int k = 0; k < km; ++k) {
-    const float z0 = val(C(A_ZA, k)), z1 = val(C(A_ZA, k + 1));
-    if (z0 < 0.f && z1 < 0.f) precip = precip + C(qa, k) * C(A_DZA, k);
-    if (z0 < 0.f && z1 > 0.f) precip = precip + C(qa, k) * (0.0f - C(A_ZA, k));
-  }
-  return precip;
-}
-
 // nislfv_rain_plm (kind 0, rain; kind 2, cloud ice with iter 0) and
 // nislfv_rain_plm6 (kind 1: snow in r1 and graupel in r2 with the shared
 // mass-weighted speed): the cell speeds are in A_W1, the masses (den q) in
-// r1 (and r2), replaced by the sedimented masses; returns the first
-// species' surface flux
+// r1 (and r2), replaced by the sedimented masses.  (The surface flux feeds
+// the precipitation accumulators only, which are not differentiated.)
 template <class T>
-__device__ T nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float dt, int iter) {
-  T allold = cst<T>(0.f);
-  for (int k = 0; k < km; ++k) allold = allold + C(r1, k);
+__device__ void nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float dt, int iter) {
+  float allold = 0.f;
+  for (int k = 0; k < km; ++k) allold = allold + val(C(r1, k));
   if (kind == 1)
-    for (int k = 0; k < km; ++k) allold = allold + C(r2, k);
-  if (!(val(allold) > 0.f)) {
+    for (int k = 0; k < km; ++k) allold = allold + val(C(r2, k));
+  if (!(allold > 0.f)) {
     // nothing to fall: the scheme's result is zero (value and derivatives)
     for (int k = 0; k < km; ++k) {
       C(r1, k) = cst<T>(0.f);
       if (kind == 1) C(r2, k) = cst<T>(0.f);
     }
-    return cst<T>(0.f);
+    return;
   }
   C(A_ZI, 0) = cst<T>(0.f);
   for (int k = 0; k < km; ++k) C(A_ZI, k + 1) = C(A_ZI, k) + C(A_DELZ, k);
@@ -273,18 +261,11 @@ __device__ T nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float dt,
       }
     }
   }
-  const bool ok = val(allold) > 0.f;
-  T precip = cst<T>(0.f);
   for (int sp = 0; sp < (kind == 1 ? 2 : 1); ++sp) {
     const int qa = sp == 0 ? A_QA : A_QA2, r = sp == 0 ? r1 : r2;
     C(qa, km - 1) = cst<T>(0.f);
     remap(C, km, qa, r);
-    const T pr = surface_flux(C, km, qa);
-    if (sp == 0) precip = pr;
-    if (!ok)
-      for (int k = 0; k < km; ++k) C(r, k) = cst<T>(0.f);
   }
-  return ok ? precip : cst<T>(0.f);
 }
 
 // the rates' limiter: where source > value (and cnd), every listed rate is
@@ -337,9 +318,15 @@ __device__ void point_processes(T& t, T& q, T& qc, T& qi, T& qr, T& qs, T& qg, c
   // rates
   Slope3<T> sl;
   slope3(qr, qs, qg, den, t, sl);
-  const T work1_0 = diffac(xl, p, t, den, qs0);
-  const T work1_1 = diffac(F(XLS), p, t, den, qs1);
-  T work2 = venfac(p, t, den);
+  // (terms of processes that cannot act at this point are not formed: most
+  // points hold no precipitation, and these are most of the work)
+  const bool precip = val(qr) > 0.f || val(qs) > 0.f || val(qg) > 0.f;
+  T work1_0 = cst<T>(1.f), work1_1 = cst<T>(1.f), work2 = zero;
+  if (precip) {
+    work1_0 = diffac(xl, p, t, den, qs0);
+    work2 = venfac(p, t, den);
+  }
+  if (val(t) < F(T0C) && (precip || val(qi) > 0.f)) work1_1 = diffac(F(XLS), p, t, den, qs1);
   T supsat = vmax(q, F(QMIN)) - qs0;
   T praut = zero, pracw = zero, prevp = zero;
   if (val(qc) > F(QC0)) praut = vmin(F(QCK1) * vpow(qc, 7.0f / 3.0f), qc / dtcld);
@@ -356,15 +343,18 @@ __device__ void point_processes(T& t, T& q, T& qc, T& qi, T& qr, T& qs, T& qg, c
     }
   }
   supcol = F(T0C) - t;
-  const T n0s = vmax(vmin(vexp(F(ALPHA) * supcol), F(N0SMAX / N0S)), 1.0f);
+  T n0s = cst<T>(1.f);
+  if (val(qs) > 0.f) n0s = vmax(vmin(vexp(F(ALPHA) * supcol), F(N0SMAX / N0S)), 1.0f);
   supsat = vmax(q, F(QMIN)) - qs1;
   const T satdt = supsat / dtcld;
   bool ifsat = false;
-  const T xni = vmin(vmax(5.38e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
-  const T eacrs = vexp(0.07f * (-supcol));
-  const T xmi = den * qi / xni;
-  const T diameter = vmin(F(DICON) * vsqrt(xmi), F(DIMAX));
-  const T vt2i = 1.49e4f * vpow(diameter, 1.31f);
+  T xni = cst<T>(1.0e3f), diameter = zero, vt2i = zero;
+  if (val(supcol) > 0.f && val(qi) > 0.f) {
+    xni = vmin(vmax(5.38e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+    const T xmi = den * qi / xni;
+    diameter = vmin(F(DICON) * vsqrt(xmi), F(DIMAX));
+    if (precip) vt2i = 1.49e4f * vpow(diameter, 1.31f);
+  }
   const T vt2r = F(PVTR) * sl.rb[0] * denfac;
   const T vt2s = F(PVTS) * sl.rb[1] * denfac;
   const T vt2g = F(PVTG) * sl.rb[2] * denfac;
@@ -383,6 +373,7 @@ __device__ void point_processes(T& t, T& q, T& qc, T& qi, T& qr, T& qs, T& qg, c
                    qr / dtcld);
     }
     if (val(qs) > F(QCRMIN)) {
+      const T eacrs = vexp(0.07f * (-supcol));
       const T acrfac = 2.0f * sl.r3[1] + 2.0f * diameter * sl.r2[1] + diameter * diameter * sl.rs[1];
       psaci = vmin(F(PI) * qi * eacrs * F(N0S) * n0s * vabs(vt2ave - vt2i) * acrfac / 4.0f, qi / dtcld);
     }
@@ -560,6 +551,12 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
   const float dtcld = delt <= F(DTCLDCR) ? delt : delt / loops;
   const int nloop = (int)loops;
   for (int it = 0; it < nloop; ++it) {
+    bool rain = false, snow = false, ice = false;
+    for (int k = 0; k < km; ++k) {
+      rain |= val(C(A_QR, k)) > 0.f;
+      snow |= val(C(A_QS, k)) > 0.f || val(C(A_QG, k)) > 0.f;
+      ice |= val(C(A_QI, k)) > 0.f;
+    }
     for (int k = 0; k < km; ++k) {
       const T den = C(A_DEN, k), t = C(A_T, k), q = C(A_Q, k);
       const T denfac = vsqrt(1.0f / den * F(DEN0));
@@ -570,16 +567,19 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
       C(A_QS1, k) = qs1;
       C(A_RH0, k) = vmax(q / qs0, F(QMIN));
       C(A_RH1, k) = vmax(q / qs1, F(QMIN));
-      C(A_XNI, k) = vmin(vmax(5.387e7f * vpow(den * vmax(C(A_QI, k), F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+      const T qi = C(A_QI, k);
+      if (val(qi) > 0.f)
+        C(A_XNI, k) = vmin(vmax(5.387e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
       const T qr = C(A_QR, k), qs = C(A_QS, k), qg = C(A_QG, k);
       C(A_W1, k) = vt_of(0, qr, den, denfac, t);
       const T qsum = vmax(qs + qg, 1.0e-15f);
       C(A_W2, k) = val(qsum) > 1.0e-15f
                        ? (vt_of(1, qs, den, denfac, t) * qs + vt_of(2, qg, den, denfac, t) * qg) / qsum
                        : cst<T>(0.f);
-      C(A_R1, k) = den * qr;
-      C(A_R2, k) = den * qs;
-      C(A_R3, k) = den * qg;
+      // (the masses of a species that the column does not hold fall nowhere)
+      C(A_R1, k) = rain ? den * qr : cst<T>(0.f);
+      C(A_R2, k) = snow ? den * qs : cst<T>(0.f);
+      C(A_R3, k) = snow ? den * qg : cst<T>(0.f);
     }
     nislfv(C, km, 0, A_R1, -1, dtcld, 1);
     for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_W2, k);
@@ -589,14 +589,15 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
       const T den = C(A_DEN, k), p = C(A_P, k), cpm = C(A_CPM, k);
       T qr = vmax(C(A_R1, k) / den, 0.0f), qs = vmax(C(A_R2, k) / den, 0.0f), qg = vmax(C(A_R3, k) / den, 0.0f);
       T t = C(A_T, k);
+      // melting of snow, then graupel (elsewhere only rain's slope is read)
+      const bool warm = val(t) > F(T0C) && (val(qs) > 0.f || val(qg) > 0.f);
+      const T none = cst<T>(0.f);
       Slope3<T> sl;
-      slope3(qr, qs, qg, den, t, sl);
+      slope3(qr, warm ? qs : none, warm ? qg : none, den, t, sl);
       C(A_SR3, k) = sl.r3[0];
       C(A_SRS, k) = sl.rs[0];
-      const T n0s = n0sfac(t);
-      // melting of snow, then graupel
-      const bool warm = val(t) > F(T0C);
       if (warm) {
+        const T n0s = val(qs) > 0.f ? n0sfac(t) : none;
         const T work2 = venfac(p, t, den);
         if (val(qs) > 0.f) {
           const T coeres = sl.r2[1] * vsqrt(sl.rs[1] * sl.rb[1]);
@@ -628,7 +629,7 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
         T wt = vmax(vmin(F(DICON) * vsqrt(den * qi / C(A_XNI, k)), F(DIMAX)), 1.0e-25f);
         C(A_W1, k) = 1.49e4f * vexp(vlog(wt) * 1.31f);
       }
-      C(A_R1, k) = den * qi;
+      C(A_R1, k) = ice ? den * qi : cst<T>(0.f);
     }
     nislfv(C, km, 2, A_R1, -1, dtcld, 0);
     if (stop_at_points) {
@@ -865,9 +866,12 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, 
 // cotangents from the outputs' (yb: theta, qv .. qg, h_diabatic) and adds
 // them into the adjoints of those entries of the column's tape, which
 // k_mp_tape_rev then sweeps.  The level's processes read no other level, so
-// the chain a thread runs is one level's, not the column's.  vo (when its T
-// is not null) receives the level's output values.
-constexpr int kPointInputs = 21;
+// the chain a thread runs is one level's, not the column's.  Only the inputs
+// of the processes that are taped are seeded (packed over the passes: a
+// species that is absent is a constant); theta, its initial value and the
+// Exner function enter the finish alone, whose derivatives are written out.
+// vo (when its T is not null) receives the level's output values.
+constexpr int kPointInputs = 21, kPointSeeds = 18;
 template <int N>
 __global__ void __launch_bounds__(128) k_mp_points_adj(Grid g, S yb, Tv* ws, TapeCtx tc, int c0, int nc, S vo,
                                                        const int* done, const int* used, float dt) {
@@ -900,37 +904,51 @@ __global__ void __launch_bounds__(128) k_mp_points_adj(Grid g, S yb, Tv* ws, Tap
   const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
   const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
   using D = Dual<N>;
-  for (int j0 = 0; j0 < kPointInputs; j0 += N) {
-    D x[kPointInputs];
+  int seeds = 0;  // the taped inputs, as a bit mask
 #pragma unroll
-    for (int q = 0; q < kPointInputs; ++q) {
+  for (int q = 0; q < kPointSeeds; ++q) seeds |= in[q].id >= 0 && in[q].s != 0.f ? 1 << q : 0;
+  const bool values = vo[WF_T] != nullptr;
+  for (int pass = 0; pass == 0 || seeds; ++pass) {
+    int at[N];  // the inputs seeded in this pass
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+      at[d] = seeds ? __ffs(seeds) - 1 : -1;
+      seeds &= seeds - 1;
+    }
+    D x[kPointSeeds];
+#pragma unroll
+    for (int q = 0; q < kPointSeeds; ++q) {
       x[q] = dconst<N>(in[q].v);
 #pragma unroll
-      for (int d = 0; d < N; ++d)
-        if (q == j0 + d) x[q].d[d] = 1.f;
+      for (int d = 0; d < N; ++d) x[q].d[d] = q == at[d] ? 1.f : 0.f;
     }
     D tt = x[0], qv = x[1], qc = x[2], qi = x[3], qr = x[4], qs = x[5], qg = x[6];
     Slope3<D> sl0;
     sl0.r3[0] = x[16];
     sl0.rs[0] = x[17];
     point_processes(tt, qv, qc, qi, qr, qs, qg, x[7], x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15], sl0, dtcld);
-    // moist_physics_finish_em at the level
-    const D mpten = tt / x[20] - x[19];
-    const D tnew = x[18] + mpten;
-    const D h = mpten / dt;
+    // moist_physics_finish_em at the level: mpten = t / pii - th is added to
+    // theta and gives h_diabatic = mpten / dt
+    const float rp = 1.0f / in[20].v, ympten = yt + yh / dt;
 #pragma unroll
     for (int d = 0; d < N; ++d) {
-      const float v = yt * tnew.d[d] + yh * h.d[d] + ym[1] * qv.d[d] + ym[2] * qc.d[d] + ym[3] * qr.d[d] +
+      const float v = ympten * (tt.d[d] * rp) + ym[1] * qv.d[d] + ym[2] * qc.d[d] + ym[3] * qr.d[d] +
                       ym[4] * qi.d[d] + ym[5] * qs.d[d] + ym[6] * qg.d[d];
 #pragma unroll
-      for (int q = 0; q < kPointInputs; ++q)
-        if (q == j0 + d) cot[q] += v;
+      for (int q = 0; q < kPointSeeds; ++q)
+        if (q == at[d]) cot[q] = v;
     }
-    if (j0 == 0 && vo[WF_T]) {
-      vo[WF_T][p] = tnew.v;
-      vo[WF_H_DIABATIC][p] = h.v;
-      const float mv[7] = {0.f, qv.v, qc.v, qr.v, qi.v, qs.v, qg.v};
-      for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = mv[m];
+    if (pass == 0) {
+      const float mpten = tt.v / in[20].v - in[19].v;
+      cot[18] = yt;
+      cot[19] = -ympten;
+      cot[20] = -ympten * (tt.v * rp) * rp;
+      if (values) {
+        vo[WF_T][p] = in[18].v + mpten;
+        vo[WF_H_DIABATIC][p] = mpten / dt;
+        const float mv[7] = {0.f, qv.v, qc.v, qr.v, qi.v, qs.v, qg.v};
+        for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = mv[m];
+      }
     }
   }
 #pragma unroll
@@ -954,48 +972,50 @@ __global__ void __launch_bounds__(kSweepBlock) k_mp_tape_rev(Grid g, S b, TapeCt
   for (int idx = 0; idx < nin; ++idx) put_input_cot(g, b, cp.c2, idx, __ldcg(tc.adj(idx, lane)));
 }
 
-// one pass of forward-mode tangents over the columns that the tape left
-// undone: the inputs with indices [pass N, pass N + N) of each column are
-// seeded and their cotangents formed from the outputs' cotangents yb
+// the passes of forward-mode tangents over the columns that the tape left
+// undone (usually none: one launch finds that out): each pass seeds the inputs
+// with indices [pass N, pass N + N) and forms their cotangents from the
+// outputs' cotangents yb
 template <int N>
-__global__ void __launch_bounds__(64) k_mp_tangent(Grid g, S s, S yb, S b, int pass, float dt, Dual<N>* ws,
-                                                   int ncol, const int* done) {
+__global__ void __launch_bounds__(64) k_mp_tangent(Grid g, S s, S yb, S b, float dt, Dual<N>* ws, int ncol,
+                                                   const int* done) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   ColPos cp;
   if (col >= ncol || !col_pos(g, col, cp) || done[col] || !cp.run) return;
-  const int nin = mp_inputs(g), j0 = pass * N;
-  if (j0 >= nin) return;
+  const int nin = mp_inputs(g);
   const int km = g.nz - 1, c2 = cp.c2;
   const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3();
   using T = Dual<N>;
   const Col<T> C{ws + col, ncol, km + 1};
-  prep_column(g, s, C, c2, [&](int idx, float v) {
-    T x = dconst<N>(v);
-    const int d = idx - j0;
-    if (d >= 0 && d < N) x.d[d] = 1.f;
-    return x;
-  });
-  wsm6_column(C, km, dt, true);
-  float acc[N];
+  for (int j0 = 0; j0 < nin; j0 += N) {
+    prep_column(g, s, C, c2, [&](int idx, float v) {
+      T x = dconst<N>(v);
+      const int d = idx - j0;
+      if (d >= 0 && d < N) x.d[d] = 1.f;
+      return x;
+    });
+    wsm6_column(C, km, dt, true);
+    float acc[N];
 #pragma unroll
-  for (int n = 0; n < N; ++n) acc[n] = 0.f;
-  for (int k = 0; k < km; ++k) {
-    finish_level(C, k, dt);
-    const size_t p = k * lev + c2;
-    const T tnew = C(A_TIN, k), h = C(A_TH, k);
-    const float yt = yb[WF_T][p], yh = yb[WF_H_DIABATIC][p];
+    for (int n = 0; n < N; ++n) acc[n] = 0.f;
+    for (int k = 0; k < km; ++k) {
+      finish_level(C, k, dt);
+      const size_t p = k * lev + c2;
+      const T tnew = C(A_TIN, k), h = C(A_TH, k);
+      const float yt = yb[WF_T][p], yh = yb[WF_H_DIABATIC][p];
 #pragma unroll
-    for (int n = 0; n < N; ++n) acc[n] += yt * tnew.d[n] + yh * h.d[n];
-    for (int m = 1; m < 7; ++m) {
-      const T qo = C(moist_slot(m), k);
-      const float y = yb[WF_MOIST][m * n3 + p];
+      for (int n = 0; n < N; ++n) acc[n] += yt * tnew.d[n] + yh * h.d[n];
+      for (int m = 1; m < 7; ++m) {
+        const T qo = C(moist_slot(m), k);
+        const float y = yb[WF_MOIST][m * n3 + p];
 #pragma unroll
-      for (int n = 0; n < N; ++n) acc[n] += y * qo.d[n];
+        for (int n = 0; n < N; ++n) acc[n] += y * qo.d[n];
+      }
     }
-  }
 #pragma unroll
-  for (int n = 0; n < N; ++n)
-    if (j0 + n < nin) put_input_cot(g, b, c2, j0 + n, acc[n]);
+    for (int n = 0; n < N; ++n)
+      if (j0 + n < nin) put_input_cot(g, b, c2, j0 + n, acc[n]);
+  }
 }
 
 }  // namespace mpt
@@ -1095,12 +1115,8 @@ int launch_physics_adj(const Grid& g, const S& s, const S& post, const S& b, flo
   }
   // the columns whose tape outgrew the capacity, by tangent passes
   auto* ws = reinterpret_cast<Dual<kMpDirections>*>(work + w.region);
-  const int passes = (mpt::mp_inputs(g) + kMpDirections - 1) / kMpDirections;
-  for (int pass = 0; pass < passes; ++pass) {
-    mpt::k_mp_tangent<kMpDirections><<<(w.ncol + 63) / 64, 64, 0, st>>>(g, s, yb, b, pass, dt, ws, w.ncol, done);
-    ++n;
-  }
-  return n;
+  mpt::k_mp_tangent<kMpDirections><<<(w.ncol + 63) / 64, 64, 0, st>>>(g, s, yb, b, dt, ws, w.ncol, done);
+  return n + 1;
 }
 
 }  // namespace wrf

@@ -30,7 +30,7 @@
 
 namespace wrf {
 
-constexpr int kTapeBlock = 64;
+constexpr int kTapeBlock = 32;
 constexpr int kTapeMaxEntries = 0xffff;  // operand indices fit in 16 bits
 
 // an entry: x the packed operand indices, y and z the partials (float
