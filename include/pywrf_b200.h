@@ -632,6 +632,18 @@ int wrf_rowsum_bf16(const void* a, int rows, int cols, float* out, void* stream)
  * refreshes the bf16 copy wb [r][c] and the transposed copy wtb [c][r] (either may be NULL) */
 int wrf_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int r, int c,
              void* wb, void* wtb, float lr, float beta1, float beta2, float eps, float wd, int step, void* stream);
+/* the same for a batch of matrices, in one launch */
+typedef struct WrfAdamItem {
+  float* w;
+  const float* gpart;
+  float *m, *v;
+  void *wb, *wtb;
+  long long split_stride;
+  int nsplit, r, c;
+  float wd;
+} WrfAdamItem;
+int wrf_adam_batch(int n, const WrfAdamItem* items, float lr, float beta1, float beta2, float eps, int step,
+                   void* stream);
 /* out [c][r] = a [r][c]^T (bf16) */
 int wrf_transpose_bf16(const void* a, int r, int c, void* out, void* stream);
 

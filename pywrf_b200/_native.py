@@ -40,6 +40,12 @@ WRF_MLP_LAYERS = 4
 EPI_F32, EPI_BIAS_GELU, EPI_GELU_BWD, EPI_BF16 = 0, 1, 2, 3
 
 
+class WrfAdamItemC(ctypes.Structure):
+    _fields_ = [("w", ctypes.c_void_p), ("gpart", ctypes.c_void_p), ("m", ctypes.c_void_p), ("v", ctypes.c_void_p),
+                ("wb", ctypes.c_void_p), ("wtb", ctypes.c_void_p), ("split_stride", ctypes.c_longlong),
+                ("nsplit", ctypes.c_int), ("r", ctypes.c_int), ("c", ctypes.c_int), ("wd", ctypes.c_float)]
+
+
 class WrfMlpNetC(ctypes.Structure):
     """``WrfMlpNet`` of include/pywrf_b200.h"""
     _fields_ = [("dims", ctypes.c_int * (WRF_MLP_LAYERS + 1)), ("w", ctypes.c_void_p * WRF_MLP_LAYERS),
@@ -252,6 +258,8 @@ def lib() -> ctypes.CDLL:
     L.wrf_rowsum_bf16.argtypes = [vp, ip, ip, vp, vp]
     L.wrf_adam.restype = ip
     L.wrf_adam.argtypes = [vp, vp, ip, ll, vp, vp, ip, ip, vp, vp, f32, f32, f32, f32, f32, ip, vp]
+    L.wrf_adam_batch.restype = ip
+    L.wrf_adam_batch.argtypes = [ip, ctypes.POINTER(WrfAdamItemC), f32, f32, f32, f32, ip, vp]
     L.wrf_transpose_bf16.restype = ip
     L.wrf_transpose_bf16.argtypes = [vp, ip, ip, vp, vp]
     _lib = L

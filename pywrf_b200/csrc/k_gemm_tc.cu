@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 //                      accumulator empty
 // Every wait is bounded and also gives up once another role has aborted.
 #ifndef WRF_GEMM_PEPI
-#define WRF_GEMM_PEPI 8
+#define WRF_GEMM_PEPI 16
 #endif
 // kPEpi epilogue warps (a multiple of 4): warp 2 + e drains lane group
 // (2 + e) % 4, columns chunks e / 4, e / 4 + kPEpi / 4, ...

@@ -142,22 +142,35 @@ __global__ void __launch_bounds__(256) k_mse_grad(const float* y, const float* t
   __shared__ float tile[32][33];
   __shared__ float red[8];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
+  const int n0 = blockIdx.x * 32;
   float acc = 0.f;
-  for (int r = ty; r < 32; r += 8) {
-    const int m = m0 + r, n = n0 + tx;
-    float d = 0.f;
-    if (m < M && n < N) {
-      if (n < nvalid) d = y[(size_t)m * N + n] - t[(size_t)m * N + n];
-      dy[(size_t)m * N + n] = __float2bfloat16_rn(scale * d);
+  // four tiles down the rows per block: the blocks' sums meet in one word
+  for (int q = 0; q < 4; ++q) {
+    const int m0 = (blockIdx.y * 4 + q) * 32;
+    if (m0 >= M) break;
+    float yv[4], tv[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = m0 + ty + 8 * r, n = n0 + tx;
+      const bool in = m < M && n < nvalid;
+      yv[r] = in ? y[(size_t)m * N + n] : 0.f;
+      tv[r] = in ? t[(size_t)m * N + n] : 0.f;
     }
-    acc += d * d;
-    tile[r][tx] = scale * d;
-  }
-  __syncthreads();
-  for (int r = ty; r < 32; r += 8) {
-    const int n = n0 + r, m = m0 + tx;
-    if (n < N && m < M) dyt[(size_t)n * M + m] = __float2bfloat16_rn(tile[tx][r]);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = m0 + ty + 8 * r, n = n0 + tx;
+      const float d = yv[r] - tv[r];
+      if (m < M && n < N) dy[(size_t)m * N + n] = __float2bfloat16_rn(scale * d);
+      acc += d * d;
+      tile[ty + 8 * r][tx] = scale * d;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int n = n0 + ty + 8 * r, m = m0 + tx;
+      if (n < N && m < M) dyt[(size_t)n * M + m] = __float2bfloat16_rn(tile[tx][ty + 8 * r]);
+    }
+    __syncthreads();
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (tx == 0) red[ty] = acc;
@@ -184,28 +197,106 @@ __global__ void __launch_bounds__(256) k_rowsum_bf16(const __nv_bfloat16* a, int
   }
 }
 
+// The same sums in the same order, for rows of whole 16-byte words: a warp
+// takes a row, a lane the partial sums of eight of the threads above (every
+// 256th column each), so that a row arrives in 16-byte loads.  The form above
+// has one 2-byte load per thread and trip in a chain of 32: 17.7 us for 512
+// rows of 8192, the time of eight of the network's products.
+__global__ void __launch_bounds__(128) k_rowsum_bf16_v8(const __nv_bfloat16* a, int rows, int cols, float* out) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const uint4* row = reinterpret_cast<const uint4*>(a + (size_t)r * cols);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+  for (int c = lane; c < cols / 8; c += 32) {
+    const uint4 w = __ldg(row + c);
+    const unsigned u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      acc[2 * q] += __uint_as_float(u[q] << 16);
+      acc[2 * q + 1] += __uint_as_float(u[q] & 0xffff0000u);
+    }
+  }
+  // the threads' butterfly: offsets 16 and 8 are lanes 2 and 1 apart here
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 2);
+    acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 1);
+  }
+  const float s4 = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+  float sum = 0.f;
+  for (int q = 0; q < 8; ++q) sum += __shfl_sync(0xffffffffu, s4, 4 * q);
+  if (lane == 0) out[r] = sum;
+}
+
 // Adam (with decoupled weight decay) on fp32 master parameters; the gradient
 // is the sum of nsplit partial sums split_stride apart
-__global__ void k_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int R, int C,
-                       __nv_bfloat16* wb, __nv_bfloat16* wtb, float lr, float b1, float b2, float eps, float wd,
-                       float bc1, float bc2) {
-  const long long n = (long long)R * C;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    float gsum = 0.f;
-    for (int s = 0; s < nsplit; ++s) gsum += gpart[s * split_stride + e];
-    const float mm = b1 * m[e] + (1.0f - b1) * gsum;
-    const float vv = b2 * v[e] + (1.0f - b2) * gsum * gsum;
-    m[e] = mm;
-    v[e] = vv;
-    float ww = w[e];
-    ww = ww - lr * ((mm / bc1) / (sqrtf(vv / bc2) + eps) + wd * ww);
-    w[e] = ww;
+// A launch takes a batch of matrices; a block one 32 x 32 tile of one of them,
+// so that the transposed copy is written along its rows too.
+__global__ void __launch_bounds__(256) k_adam(AdamBatch b, float lr, float b1, float b2, float eps, float bc1, float bc2) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  int f = 0;
+  while (f + 1 < b.n && (int)blockIdx.x >= b.first[f + 1]) ++f;
+  const AdamItem it = b.item[f];
+  const int tiles_c = (it.c + 31) / 32, t = blockIdx.x - b.first[f];
+  const int r0 = t / tiles_c * 32, c0 = t % tiles_c * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const bool col = c0 + tx < it.c;
+  float gs[4], mv[4], vv[4], wv[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = r0 + ty + 8 * q;
+    gs[q] = 0.f;
+    if (r >= it.r || !col) continue;
+    const long long e = (long long)r * it.c + c0 + tx;
+    mv[q] = it.m[e];
+    vv[q] = it.v[e];
+    wv[q] = it.w[e];
+    const float* gp = it.g + e;
+#pragma unroll 8
+    for (int s = 0; s < it.nsplit; ++s) gs[q] += __ldg(gp + s * it.split_stride);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = r0 + ty + 8 * q;
+    if (r >= it.r || !col) continue;
+    const long long e = (long long)r * it.c + c0 + tx;
+    const float mm = b1 * mv[q] + (1.0f - b1) * gs[q];
+    const float nv = b2 * vv[q] + (1.0f - b2) * gs[q] * gs[q];
+    it.m[e] = mm;
+    it.v[e] = nv;
+    const float ww = wv[q] - lr * ((mm / bc1) / (sqrtf(nv / bc2) + eps) + it.wd * wv[q]);
+    it.w[e] = ww;
     const __nv_bfloat16 hb = __float2bfloat16_rn(ww);
-    if (wb) wb[e] = hb;
-    if (wtb) {
-      const long long r = e / C, c = e - r * C;
-      wtb[c * R + r] = hb;
-    }
+    if (it.wb) static_cast<__nv_bfloat16*>(it.wb)[e] = hb;
+    tile[ty + 8 * q][tx] = hb;
+  }
+  if (!it.wtb) return;
+  __syncthreads();
+  __nv_bfloat16* wt = static_cast<__nv_bfloat16*>(it.wtb);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int c = c0 + ty + 8 * q, r = r0 + tx;
+    if (c < it.c && r < it.r) wt[(long long)c * it.r + r] = tile[tx][ty + 8 * q];
+  }
+}
+
+// the same with two columns (4 bytes) per thread, 64 x 64 tiles; R and C even
+__global__ void __launch_bounds__(256) k_transpose_bf16x2(const __nv_bfloat162* a, int R, int C, __nv_bfloat162* out) {
+  __shared__ __nv_bfloat16 tile[64][66];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int r = r0 + ty + 8 * q, c = c0 + 2 * tx;
+    if (r < R && c < C) *reinterpret_cast<__nv_bfloat162*>(&tile[ty + 8 * q][2 * tx]) = a[((size_t)r * C + c) / 2];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = c0 + ty + 8 * q, r = r0 + 2 * tx;
+    if (c < C && r < R)
+      out[((size_t)c * R + r) / 2] = __halves2bfloat162(tile[2 * tx][ty + 8 * q], tile[2 * tx + 1][ty + 8 * q]);
   }
 }
 
@@ -275,28 +366,37 @@ int launch_mlp_normalize(const MlpLayout& L, const float* norm, const float* raw
 
 int launch_mse_grad(const float* y, const float* t, int M, int N, int nvalid, float scale, void* dy, void* dyt,
                     float* loss, cudaStream_t st) {
-  const dim3 grid((N + 31) / 32, (M + 31) / 32);
+  const dim3 grid((N + 31) / 32, (M + 127) / 128);
   k_mse_grad<<<grid, 256, 0, st>>>(y, t, M, N, nvalid, scale, static_cast<__nv_bfloat16*>(dy),
                                    static_cast<__nv_bfloat16*>(dyt), loss);
   return 1;
 }
 
 int launch_rowsum_bf16(const void* a, int rows, int cols, float* out, cudaStream_t st) {
-  k_rowsum_bf16<<<rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(a), cols, out);
+  const auto* p = static_cast<const __nv_bfloat16*>(a);
+  if (cols % 8 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0)
+    k_rowsum_bf16_v8<<<(rows + 3) / 4, 128, 0, st>>>(p, rows, cols, out);
+  else
+    k_rowsum_bf16<<<rows, 256, 0, st>>>(p, cols, out);
   return 1;
 }
 
-int launch_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int R, int C,
-                void* wb, void* wtb, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2,
-                cudaStream_t st) {
-  const long long n = (long long)R * C;
-  const int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-  k_adam<<<blocks, 256, 0, st>>>(w, gpart, nsplit, split_stride, m, v, R, C, static_cast<__nv_bfloat16*>(wb),
-                                 static_cast<__nv_bfloat16*>(wtb), lr, b1, b2, eps, wd, bc1, bc2);
+int launch_adam(AdamBatch& b, float lr, float b1, float b2, float eps, float bc1, float bc2, cudaStream_t st) {
+  int blocks = 0;
+  for (int f = 0; f < b.n; ++f) {
+    b.first[f] = blocks;
+    blocks += (b.item[f].r + 31) / 32 * ((b.item[f].c + 31) / 32);
+  }
+  k_adam<<<blocks, 256, 0, st>>>(b, lr, b1, b2, eps, bc1, bc2);
   return 1;
 }
 
 int launch_transpose_bf16(const void* a, int R, int C, void* out, cudaStream_t st) {
+  if (R % 2 == 0 && C % 2 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(out)) % 4 == 0) {
+    k_transpose_bf16x2<<<dim3((C + 63) / 64, (R + 63) / 64), 256, 0, st>>>(
+        static_cast<const __nv_bfloat162*>(a), R, C, static_cast<__nv_bfloat162*>(out));
+    return 1;
+  }
   const dim3 grid((C + 31) / 32, (R + 31) / 32);
   k_transpose_bf16<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(a), R, C, static_cast<__nv_bfloat16*>(out));
   return 1;

@@ -85,9 +85,26 @@ int launch_mlp_normalize(const MlpLayout& L, const float* norm, const float* raw
 int launch_mse_grad(const float* y, const float* t, int M, int N, int nvalid, float scale, void* dy, void* dyt,
                     float* loss, cudaStream_t st);
 int launch_rowsum_bf16(const void* a, int rows, int cols, float* out, cudaStream_t st);
-int launch_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int R, int C,
-                void* wb, void* wtb, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2,
-                cudaStream_t st);
+// one matrix of an Adam step: fp32 master w [r][c] with its moments m, v, the
+// gradient as nsplit partial sums split_stride apart, the bf16 copies wb, wtb
+// (or null), the weight decay wd; and a batch of them (first: each one's
+// first block, set by the launch)
+struct AdamItem {
+  float* w;
+  const float* g;
+  float *m, *v;
+  void *wb, *wtb;
+  long long split_stride;
+  int nsplit, r, c;
+  float wd;
+};
+constexpr int kAdamMax = 16;
+struct AdamBatch {
+  int n = 0;
+  int first[kAdamMax];
+  AdamItem item[kAdamMax];
+};
+int launch_adam(AdamBatch& b, float lr, float b1, float b2, float eps, float bc1, float bc2, cudaStream_t st);
 int launch_transpose_bf16(const void* a, int R, int C, void* out, cudaStream_t st);
 // the network's four products on m rows: x -> h0 -> h1 -> h0 -> y (bias + GELU fused)
 int launch_mlp_forward(const MlpNetDev& net, const void* x, int m, void* h0, void* h1, float* y, int* errflag,

@@ -1636,15 +1636,31 @@ int wrf_rowsum_bf16(const void* a, int rows, int cols, float* out, void* stream)
                     "rowsum_bf16");
 }
 
-int wrf_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int r, int c,
-             void* wb, void* wtb, float lr, float beta1, float beta2, float eps, float wd, int step, void* stream) {
-  if (!w || !gpart || !m || !v || r < 1 || c < 1 || nsplit < 1 || step < 1)
-    return fail(WRF_EINVAL, "null argument, empty matrix, or step < 1");
+int wrf_adam_batch(int n, const WrfAdamItem* items, float lr, float beta1, float beta2, float eps, int step,
+                   void* stream) {
+  if (n < 1 || !items || step < 1) return fail(WRF_EINVAL, "null argument, empty batch, or step < 1");
+  for (int f = 0; f < n; ++f) {
+    const WrfAdamItem& i = items[f];
+    if (!i.w || !i.gpart || !i.m || !i.v || i.r < 1 || i.c < 1 || i.nsplit < 1)
+      return fail(WRF_EINVAL, "null argument or empty matrix");
+  }
   const float bc1 = (float)(1.0 - pow((double)beta1, step)), bc2 = (float)(1.0 - pow((double)beta2, step));
   cudaGetLastError();
-  return ret_launch(launch_adam(w, gpart, nsplit, split_stride, m, v, r, c, wb, wtb, lr, beta1, beta2, eps, wd, bc1,
-                                bc2, static_cast<cudaStream_t>(stream)),
-                    nullptr, "adam");
+  for (int f0 = 0; f0 < n; f0 += kAdamMax) {
+    AdamBatch b;
+    for (int f = f0; f < n && f < f0 + kAdamMax; ++f) {
+      const WrfAdamItem& i = items[f];
+      b.item[b.n++] = AdamItem{i.w, i.gpart, i.m, i.v, i.wb, i.wtb, i.split_stride, i.nsplit, i.r, i.c, i.wd};
+    }
+    launch_adam(b, lr, beta1, beta2, eps, bc1, bc2, static_cast<cudaStream_t>(stream));
+  }
+  return check_launch("adam");
+}
+
+int wrf_adam(float* w, const float* gpart, int nsplit, long long split_stride, float* m, float* v, int r, int c,
+             void* wb, void* wtb, float lr, float beta1, float beta2, float eps, float wd, int step, void* stream) {
+  const WrfAdamItem one{w, gpart, m, v, wb, wtb, split_stride, nsplit, r, c, wd};
+  return wrf_adam_batch(1, &one, lr, beta1, beta2, eps, step, stream);
 }
 
 int wrf_transpose_bf16(const void* a, int r, int c, void* out, void* stream) {

@@ -242,13 +242,15 @@ class Trainer:
         net = self.net
         net.adam_step += 1
         s = _stream_handle(None)
+        items = (N.WrfAdamItemC * (2 * LAYERS))()  # every layer's weights and bias in one launch
         for i in range(LAYERS):
             r, c = net.dims[i + 1], net.dims[i]
-            N.check(self.lib.wrf_adam(_p(net.w32[i]), _p(self.gw[i]), self.splits[i], r * c, _p(net.mw[i]),
-                                      _p(net.vw[i]), r, c, _p(net.wb[i]), _p(net.wtb[i]), self.lr, b1, b2, eps,
-                                      self.wd, net.adam_step, s), "adam")
-            N.check(self.lib.wrf_adam(_p(net.b32[i]), _p(self.gb[i]), 1, r, _p(net.mb[i]), _p(net.vb[i]), 1, r,
-                                      None, None, self.lr, b1, b2, eps, 0.0, net.adam_step, s), "adam")
+            items[2 * i] = N.WrfAdamItemC(net.w32[i].data_ptr(), self.gw[i].data_ptr(), net.mw[i].data_ptr(),
+                                          net.vw[i].data_ptr(), net.wb[i].data_ptr(), net.wtb[i].data_ptr(), r * c,
+                                          self.splits[i], r, c, self.wd)
+            items[2 * i + 1] = N.WrfAdamItemC(net.b32[i].data_ptr(), self.gb[i].data_ptr(), net.mb[i].data_ptr(),
+                                              net.vb[i].data_ptr(), None, None, r, 1, 1, r, 0.0)
+        N.check(self.lib.wrf_adam_batch(2 * LAYERS, items, self.lr, b1, b2, eps, net.adam_step, s), "adam")
 
     def step(self, x: torch.Tensor, t: torch.Tensor) -> None:
         self.forward(x)
