@@ -8,6 +8,7 @@
 //   k_mu_uv_1 / k_ssfinish  calc_mu_uv_1, small_step_finish
 // The vertical recurrences (mass divergence sum, ww scan, Thomas sweeps) run
 // sequentially per column in the reference's order.
+#include <type_traits>
 #include "kernels.cuh"
 #include "tma.cuh"
 
@@ -508,18 +509,20 @@ constexpr int kColTX = 16, kColKT = 16;
 #define WRF_COL_MINB 4
 #endif
 template <int NQ>
-__global__ void __launch_bounds__(kColTX * kColKT, WRF_COL_MINB) k_acoustic_col(Grid g, S s, float dts, int iteration, int nsub) {
-  __shared__ float sdw[kMaxNz][kColTX], sww[kMaxNz][kColTX], st2av[kMaxNz][kColTX], srhs[kMaxNz][kColTX];
-  __shared__ float sa[kMaxNz][kColTX], salpha[kMaxNz][kColTX], sgamma[kMaxNz][kColTX], sph[kMaxNz][kColTX];
-  __shared__ float swd[kMaxNz][kColTX];
+__global__ void __launch_bounds__(kColTX * kColKT, WRF_COL_MINB) k_acoustic_col(Grid g, S s, float dts, int iteration, int nsub,
+                                                                             int i0) {
+  constexpr int NZ = NQ * kColKT;  // nz <= NZ
+  __shared__ float sdw[NZ][kColTX], sww[NZ][kColTX], st2av[NZ][kColTX], srhs[NZ][kColTX];
+  __shared__ float sa[NZ][kColTX], salpha[NZ][kColTX], sgamma[NZ][kColTX], sph[NZ][kColTX];
+  __shared__ float swd[NZ][kColTX];
   __shared__ float pdnw[kMaxNz], prdnw[kMaxNz], prdn[kMaxNz], pfnm[kMaxNz], pfnp[kMaxNz];
   __shared__ float smuave[kColTX], smuts[kColTX], smu[kColTX];
   const int nz = g.nz, kend = nz - 1, nx = g.nx;
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde;
   const int tx = threadIdx.x % kColTX, tk = threadIdx.x / kColTX;
-  const int i = ids + blockIdx.x * kColTX + tx;
+  const int i = i0 + blockIdx.x * kColTX + tx;      // i0 <= ids: whole sectors where the rows allow it
   const int j = jds + blockIdx.y;
-  const bool col = i < ide;                         // j < jde by the grid
+  const bool col = i >= ids && i < ide;             // j < jde by the grid
   const bool inner = col && j >= jds + 1 && j < jde - 2 && i >= ids + 1 && i < ide - 2;
   const bool spec = col && (((j == jds || j == jde - 2) && i < ide - 1) || (j >= jds + 1 && j < jde - 2 && (i == ids || i == ide - 2)));
   const bool mass = inner || spec;
@@ -999,6 +1002,451 @@ __global__ void __launch_bounds__(kColTX * kColKT, WRF_COL_MINB) k_acoustic_col(
 }
 
 
+// The same update with one thread per column, for domains whose columns fill
+// the GPU by themselves (acoustic_col_marches below).  Three sweeps per
+// column, no block barriers: up (the divergence of every level and its sum,
+// and the flux averages of u and v), up again (ww, theta, the right-hand
+// sides and the Thomas forward sweep, each level as soon as its neighbours
+// are known, the values of the levels around it carried in registers), down
+// (the back substitution, phi, and calc_p_rho of each level).  Only two
+// column arrays are kept, in shared memory ([nz][32] each): the divergence,
+// overwritten by the eliminated right-hand side of w, and the right-hand side
+// of phi.  The operands of a few levels are loaded together, so each resident
+// warp keeps about twenty 128-byte lines in flight.  The tiled form above
+// issues a third more instructions (predicates, addresses and reciprocals per
+// level group, the sweeps by one warp of eight; 75 million warp instructions
+// against 57 at 240x240x41) behind ten block barriers, but starts more loads
+// at once where the columns are few.  Per launch, tiled and marching: 140 and
+// 165 us at 240x240x41, 251 and 253 at 320x320x41, 411 and 374 at 320x320x61,
+// 1091 and 828 at 512x512x61.
+// The arithmetic is that of the tiled form, operation for operation.
+constexpr int kMarchTX = 32;
+
+__global__ void __launch_bounds__(kMarchTX, 13) k_acoustic_march(Grid g, S s, float dts, int iteration, int nsub,
+                                                                 int i0) {
+  extern __shared__ float march_smem[];
+  const int nz = g.nz, kend = nz - 1, nx = g.nx;
+  const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde;
+  const int i = i0 + blockIdx.x * kMarchTX + threadIdx.x, j = jds + blockIdx.y;
+  // the profiles: dnw, rdnw, rdn, fnm, fnp
+  __shared__ float pd[5][kMaxNz];
+  for (int e = threadIdx.x; e < nz; e += kMarchTX) {
+    pd[0][e] = __ldg(&s[WF_DNW][e]);
+    pd[1][e] = __ldg(&s[WF_RDNW][e]);
+    pd[2][e] = __ldg(&s[WF_RDN][e]);
+    pd[3][e] = __ldg(&s[WF_FNM][e]);
+    pd[4][e] = __ldg(&s[WF_FNP][e]);
+  }
+  __syncwarp();
+  if (i < ids || i >= ide) return;
+  float* const sy = march_smem + threadIdx.x;           // divergence, then y of the Thomas sweep
+  float* const sr = sy + nz * kMarchTX;                 // right-hand side of phi
+  const bool inner = j >= jds + 1 && j < jde - 2 && i >= ids + 1 && i < ide - 2;
+  const bool spec = ((j == jds || j == jde - 2) && i < ide - 1) || (j >= jds + 1 && j < jde - 2 && (i == ids || i == ide - 2));
+  const int c = g.i2(j, i);
+  const int lev = g.ny * nx;
+  const float* __restrict__ u = s[WF_U];
+  const float* __restrict__ v = s[WF_V];
+  const float* __restrict__ t1 = s[WF_T_SAVE];
+  const float* __restrict__ ft = s[WF_T_TEND];
+  const float* __restrict__ ww1 = s[WF_WW1];
+  const float* __restrict__ ph1 = s[WF_PH_SAVE];
+  const float* __restrict__ phb = s[WF_PHB];
+  const float* __restrict__ pht = s[WF_PH_TEND];
+  const float* __restrict__ c2a = s[WF_C2A];
+  const float* __restrict__ alt = s[WF_ALT];
+  float* t = s[WF_T];
+  float* ww = s[WF_WW];
+  float* ph = s[WF_PH];
+  const bool last = iteration == nsub;
+  const float fsub = (float)nsub, r_nsub = __frcp_rn(fsub);
+  const float msftx = __ldg(&s[WF_MSFTX][c]), msfty = __ldg(&s[WF_MSFTY][c]);
+  const float mut = __ldg(&s[WF_MUT][c]);
+  const float mu_tend = __ldg(&s[WF_MU_TEND][c]);
+  const float ep = g.epssm;
+  const float ep1 = (float)(1.0 + (double)ep), em1 = (float)(1.0 - (double)ep);
+
+  // --- sweep 1: flux averages of u and v (all columns), divergence (inner)
+  float dmdt = 0.f;
+  {
+    float* ru_m = s[WF_RU_M];
+    float* rv_m = s[WF_RV_M];
+    const float* __restrict__ u1 = s[WF_U_SAVE];
+    const float* __restrict__ v1 = s[WF_V_SAVE];
+    const bool ur = j < jde - 1, vr = i < ide - 1;
+    const float muu0 = __ldg(&s[WF_MUU][c]), mfu0 = __ldg(&s[WF_MSFUY][c]);
+    const float muv0 = __ldg(&s[WF_MUV][c]), mvi0 = __ldg(&s[WF_MSFVX_INV][c]);
+    const float muup = inner ? __ldg(&s[WF_MUU][c + 1]) : 0.f, mfup = inner ? __ldg(&s[WF_MSFUY][c + 1]) : 1.f;
+    const float muvn = inner ? __ldg(&s[WF_MUV][c + nx]) : 0.f, mvin = inner ? __ldg(&s[WF_MSFVX_INV][c + nx]) : 0.f;
+    const float r_mfup = __frcp_rn(mfup), r_mfu0 = __frcp_rn(mfu0);
+    const float msf = msftx * msfty, rdx = g.rdx, rdy = g.rdy;
+    constexpr int B = 4;
+    struct Ops { float u0, v0, u10, v10, ue, u1e, vn, v1n, a, b; };
+    auto load = [&](int k, Ops& o) {
+      const int p = k * lev + c;
+      const bool lv = k < kend;
+      o.u0 = lv ? __ldg(u + p) : 0.f;
+      o.v0 = lv ? __ldg(v + p) : 0.f;
+      const bool sv = lv && (inner || last);
+      o.u10 = sv ? __ldg(u1 + p) : 0.f;
+      o.v10 = sv ? __ldg(v1 + p) : 0.f;
+      const bool in = lv && inner;
+      o.ue = in ? __ldg(u + p + 1) : 0.f;
+      o.u1e = in ? __ldg(u1 + p + 1) : 0.f;
+      o.vn = in ? __ldg(v + p + nx) : 0.f;
+      o.v1n = in ? __ldg(v1 + p + nx) : 0.f;
+      o.a = iteration == 1 ? 0.f : ru_m[p];
+      o.b = iteration == 1 ? 0.f : rv_m[p];
+    };
+    for (int kb = 0; kb < nz; kb += B) {
+      Ops o[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (kb + q < nz) load(kb + q, o[q]);
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int k = kb + q;
+        if (k >= nz) continue;
+        const int p = k * lev + c;
+        float a = o[q].a, b = o[q].b;
+        if (k < kend) {
+          if (ur) a = a + o[q].u0;
+          if (vr) b = b + o[q].v0;
+          if (last) {
+            if (ur) a = divc(a, fsub, r_nsub) + divc(muu0 * o[q].u10, mfu0, r_mfu0);
+            if (vr) b = divc(b, fsub, r_nsub) + muv0 * o[q].v10 * mvi0;
+          }
+        }
+        ru_m[p] = a;
+        rv_m[p] = b;
+        if (inner && k < kend) {
+          const float dw = msf * (rdy * ((o[q].vn + muvn * o[q].v1n * mvin) - (o[q].v0 + muv0 * o[q].v10 * mvi0)) +
+                                  rdx * ((o[q].ue + divc(muup * o[q].u1e, mfup, r_mfup)) -
+                                         (o[q].u0 + divc(muu0 * o[q].u10, mfu0, r_mfu0))));
+          sy[k * kMarchTX] = dw;
+          dmdt = dmdt + pd[0][k] * dw;
+        }
+      }
+    }
+  }
+  float* ww_m = s[WF_WW_M];
+  float* al = s[WF_AL];
+  float* pp = s[WF_P];
+  float* pm1 = s[WF_PM1];
+  if (inner) {
+    const float* __restrict__ ca = s[WF_A];
+    const float* __restrict__ calpha = s[WF_ALPHA];
+    const float* __restrict__ cgamma = s[WF_GAMMA];
+    const float* __restrict__ rw = s[WF_RW_TEND];
+    const float* __restrict__ cqw = s[WF_CQW];
+    float* w = s[WF_W];
+    float* t2a = s[WF_T_2SAVE];
+    const float r_msfty = __frcp_rn(msfty), r_mut = __frcp_rn(mut);
+    float mu = s[WF_MU][c];
+    const float muave_old = mu;
+    mu = mu + dts * (dmdt + mu_tend);
+    const float muts = mut + mu;
+    const float muave = 0.5f * (ep1 * mu + em1 * muave_old);
+    s[WF_MU][c] = mu;
+    s[WF_MUDF][c] = dmdt + mu_tend;
+    s[WF_MUTS][c] = muts;
+    s[WF_MUAVE][c] = muave;
+    const float r_muts = __frcp_rn(muts);
+    const float cy = (float)(0.5 * g.rdyd), cx = (float)(0.5 * g.rdxd);
+    const float cw = (float)(0.5 * G * (1.0 - (double)ep));
+    const float msft_inv = 1.0f / msfty;
+    const float cp = (float)(0.5 * (double)dts * G);
+    const float cq = (float)((double)dts * G);
+    // lower boundary of w: the terrain slope and near-surface winds
+    float w0;
+    {
+      const float* __restrict__ ht = s[WF_HT];
+      auto cv = [&](int cc) { return g.cf1 * __ldg(&v[cc]) + g.cf2 * __ldg(&v[lev + cc]) + g.cf3 * __ldg(&v[2 * lev + cc]); };
+      auto cu = [&](int cc) { return g.cf1 * __ldg(&u[cc]) + g.cf2 * __ldg(&u[lev + cc]) + g.cf3 * __ldg(&u[2 * lev + cc]); };
+      const float h0 = __ldg(&ht[c]);
+      w0 = msfty * 0.5f * g.rdy * ((__ldg(&ht[c + nx]) - h0) * cv(c + nx) + (h0 - __ldg(&ht[c - nx])) * cv(c)) +
+           msftx * 0.5f * g.rdx * ((__ldg(&ht[c + 1]) - h0) * cu(c + 1) + (h0 - __ldg(&ht[c - 1])) * cu(c));
+    }
+    // --- sweep 2.  Step k: ww(k+1), theta(k), the phi right-hand side r(k),
+    // and with it w's right-hand side at m = k - 1 and its elimination.
+    struct Ops {
+      float ww1n, t1n, p1n, pbn;                              // level k + 1
+      float told, ft, vn, tn, v0, ts, ue, te, u0, tw;         // level k
+      float ph, pt, w, wm, ww1;
+      float c2, alt, rw, cq, a, al;                           // level m = k - 1
+    };
+    // E: a step near the column's ends; between them every condition on the
+    // level holds
+    auto load = [&](auto edge, int k, Ops& o) {
+      constexpr bool E = decltype(edge)::value;
+      const int p = k * lev + c, m = p - lev;
+      o.wm = iteration == 1 ? 0.f : ww_m[p];
+      o.ww1 = last ? __ldg(ww1 + p) : 0.f;
+      o.ph = ph[p];
+      if (!E || k < kend) {
+        o.ww1n = !E || k + 1 < kend ? __ldg(ww1 + p + lev) : ww[p + lev];
+        o.t1n = !E || k + 1 < kend ? __ldg(t1 + p + lev) : 0.f;
+        o.told = t[p];
+        o.ft = __ldg(ft + p);
+        o.vn = __ldg(v + p + nx);
+        o.tn = __ldg(t1 + p + nx);
+        o.v0 = __ldg(v + p);
+        o.ts = __ldg(t1 + p - nx);
+        o.ue = __ldg(u + p + 1);
+        o.te = __ldg(t1 + p + 1);
+        o.u0 = __ldg(u + p);
+        o.tw = __ldg(t1 + p - 1);
+        o.p1n = __ldg(ph1 + p + lev);
+        o.pbn = __ldg(phb + p + lev);
+      }
+      if (!E || k >= 1) {
+        o.pt = __ldg(pht + p);
+        o.w = w[p];
+        o.c2 = __ldg(c2a + m);
+        o.alt = __ldg(alt + m);
+      }
+      if (!E || k >= 2) {
+        o.rw = __ldg(rw + m);
+        o.cq = __ldg(cqw + m);
+        o.a = __ldg(ca + m);
+        o.al = __ldg(calpha + m);
+      }
+    };
+    const float rw_top = __ldg(rw + kend * lev + c), a_top = __ldg(ca + kend * lev + c),
+                al_top = __ldg(calpha + kend * lev + c);
+    float scan = ww[c];              // the ww scan, ww1 not yet taken off
+    float wwk = scan - __ldg(ww1 + c);
+    ww[c] = wwk;
+    float t1k = __ldg(t1 + c), p1k = __ldg(ph1 + c), pbk = __ldg(phb + c);
+    float wdn = 0.f, swk = 0.f;      // wdtn(k), wdwn(k)
+    float rm = 0.f, phm = 0.f, avm = 0.f, wm1 = 0.f;   // r, phi, t_2ave, w at k - 1
+    float X = 0.f, Tq = 0.f;         // the pressure and buoyancy terms at m - 1
+    float y = w0;
+    auto step = [&](auto edge, int k, const Ops& o, Ops& n) {
+      constexpr bool E = decltype(edge)::value;
+      if (!E || k < kend) load(edge, k + 1, n);
+      const int p = k * lev + c;
+      const float rdk = pd[1][k], fk = pd[3][k], fpk = pd[4][k];
+      float cc = o.wm + wwk;
+      if (last) cc = divc(cc, fsub, r_nsub) + o.ww1;
+      float wwn = 0.f, swn = 0.f, avk = 0.f;
+      if (!E || k < kend) {
+        float wup = 0.f;
+        if (!E || k + 1 < kend) {
+          scan = scan - divc(pd[0][k] * (dmdt + sy[k * kMarchTX] + mu_tend), msfty, r_msfty);
+          wwn = scan - o.ww1n;
+          ww[p + lev] = wwn;
+          wup = wwn * (pd[3][k + 1] * o.t1n + pd[4][k + 1] * t1k);
+        } else {
+          wwn = o.ww1n;  // ww at the top level stays
+        }
+        float tt = o.told + msfty * dts * o.ft;
+        const float hy = cy * (o.vn * (o.tn + t1k) - o.v0 * (t1k + o.ts));
+        const float hx = cx * (o.ue * (o.te + t1k) - o.u0 * (t1k + o.tw));
+        tt = tt - dts * msfty * (msftx * (hy + hx) + rdk * (wup - wdn));
+        t[p] = tt;
+        avk = 0.5f * (ep1 * tt + em1 * o.told);
+        avk = (avk + muave * (float)T0) / (muts * ((float)T0 + t1k));
+        t2a[p] = avk;
+        swn = 0.5f * (wwn + wwk) * rdk * (o.p1n - p1k + o.pbn - pbk);
+        wdn = wup;
+        t1k = o.t1n;
+        p1k = o.p1n;
+        pbk = o.pbn;
+      }
+      ww_m[p] = cc;
+      float r = 0.f;
+      if (!E || k >= 1) {
+        r = dts * (o.pt + cw * o.w);
+        if (!E || k < kend) r = r - dts * (fk * swn + fpk * swk);
+        r = o.ph + divc(msfty * r, mut, r_mut);
+        const float rdm = pd[1][k - 1];
+        const float X1 = divc(o.c2 * rdm, mut, r_mut) * (ep1 * (r - rm) + em1 * (o.ph - phm));
+        const float T1 = o.c2 * o.alt * avm;
+        if (!E || k >= 2) {
+          const float rdn_m = pd[2][k - 1];
+          const float wl = wm1 + dts * o.rw + msft_inv * o.cq * (cp * rdn_m * (X1 - X)) +
+                           cq * msft_inv * (rdn_m * (T1 - Tq) - muave);
+          y = (wl - o.a * y) * o.al;
+          sy[(k - 1) * kMarchTX] = y;
+        }
+        if (E && k == kend) {
+          const float cm = (float)(-0.5 * (double)dts * G);
+          const float wl = o.w + dts * rw_top +
+                           msft_inv * (divc(cm, mut, r_mut) * (rdm * rdm) * 2.0f * o.c2 *
+                                           (ep1 * (r - rm) + em1 * (o.ph - phm)) -
+                                       cq * (2.0f * rdm * o.c2 * o.alt * avm + muave));
+          y = (wl - a_top * y) * al_top;
+        }
+        X = X1;
+        Tq = T1;
+        wm1 = o.w;
+      }
+      sr[k * kMarchTX] = r;
+      rm = r;
+      phm = o.ph;
+      avm = avk;
+      wwk = wwn;
+      swk = swn;
+    };
+    {
+      const std::true_type ends{};
+      const std::false_type between{};
+      Ops A, B;
+      load(ends, 0, A);
+      step(ends, 0, A, B);
+      step(ends, 1, B, A);
+      int k = 2;
+      for (; k + 1 <= kend - 3; k += 2) {
+        step(between, k, A, B);
+        step(between, k + 1, B, A);
+      }
+      for (; k <= kend; k += 2) {
+        step(ends, k, A, B);
+        if (k < kend) step(ends, k + 1, B, A);
+      }
+    }
+    // --- sweep 3: back substitution, damping, phi; calc_p_rho of each level
+    struct Down { float gm, p1, pb, ws, alt, t1, c2, t, pm; };
+    const float* __restrict__ wsave = s[WF_W_SAVE];
+    auto load3 = [&](int k, Down& o) {
+      const int p = k * lev + c;
+      if (k >= 1) {
+        o.p1 = __ldg(ph1 + p);
+        o.pb = __ldg(phb + p);
+        o.ws = __ldg(wsave + p);
+      } else {
+        o.ws = ph[p];  // phi(0) stays
+      }
+      if (k < kend) {
+        o.gm = __ldg(cgamma + p);
+        o.alt = __ldg(alt + p);
+        o.t1 = __ldg(t1 + p);
+        o.c2 = __ldg(c2a + p);
+        o.t = t[p];
+        o.pm = pm1[p];
+      }
+    };
+    const float gf = (float)G;
+    constexpr float r_g = 1.0f / (float)G, r_hd = 1.0f / 5000.0f;
+    const float hdepth = 5000.0f;
+    const float dampmag = (float)((double)dts * 0.2);
+    const float hpi = (float)(0.5 * 3.14159265359);
+    float hbot = 0.f, wn = 0.f, phn = 0.f;
+    auto down = [&](int k, const Down& o, Down& n) {
+      if (k >= 1) load3(k - 1, n);
+      const int p = k * lev + c;
+      float phk;
+      if (k == 0) {
+        w[c] = w0;
+        phk = o.ws;
+      } else {
+        const float hk = divc(o.p1 + o.pb, gf, r_g);
+        if (k == kend) {
+          hbot = hk - hdepth;
+          wn = y;
+        } else {
+          wn = sy[k * kMarchTX] - o.gm * wn;
+        }
+        float dwd = 0.f;
+        if (hk >= hbot) {
+          const float sn = sinf(divc(hpi * (hk - hbot), hdepth, r_hd));
+          dwd = dampmag * (sn * sn);
+        }
+        const float num = wn - dwd * mut * o.ws;
+        const float wk = dwd == 0.f ? num : num / (1.0f + dwd);  // x / 1 == x
+        w[p] = wk;
+        phk = sr[k * kMarchTX] + divc(msfty * 0.5f * dts * gf * ep1 * wk, muts, r_muts);
+        ph[p] = phk;
+      }
+      if (k < kend) {
+        const float alk = -r_muts * (o.alt * mu + pd[1][k] * (phn - phk));
+        al[p] = alk;
+        const float pnew = o.c2 * (o.alt * (o.t - mu * o.t1) / (muts * ((float)T0 + o.t1)) - alk);
+        pp[p] = pnew + g.smdiv * (pnew - o.pm);
+        pm1[p] = pnew;
+      }
+      phn = phk;
+    };
+    {
+      Down A, B;
+      load3(kend, A);
+      for (int k = kend; k >= 0; k -= 2) {
+        down(k, A, B);
+        if (k >= 1) down(k - 1, B, A);
+      }
+    }
+  } else if (spec) {
+    const float mu = s[WF_MU][c] + dts * mu_tend;
+    const float muts = s[WF_MUTS][c] + dts * mu_tend;
+    s[WF_MU][c] = mu;
+    s[WF_MUTS][c] = muts;
+    const float r_muts = __frcp_rn(muts);
+    const float mu_old = muts - dts * mu_tend;
+    float phm = 0.f, altm = 0.f, t1m = 0.f, c2m = 0.f, tm = 0.f, pmm = 0.f;
+    constexpr int B = 4;
+    for (int kb = 0; kb < nz; kb += B) {
+      float ov[B][11];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int k = kb + q, p = k * lev + c;
+        if (k >= nz) continue;
+        ov[q][0] = ph[p];
+        ov[q][1] = __ldg(pht + p);
+        ov[q][2] = __ldg(ph1 + p);
+        ov[q][3] = iteration == 1 ? 0.f : ww_m[p];
+        ov[q][4] = ww[p];
+        ov[q][5] = last ? __ldg(ww1 + p) : 0.f;
+        if (k >= kend) continue;
+        ov[q][6] = t[p] + dts * __ldg(ft + p);
+        ov[q][7] = __ldg(alt + p);
+        ov[q][8] = __ldg(t1 + p);
+        ov[q][9] = __ldg(c2a + p);
+        ov[q][10] = pm1[p];
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int k = kb + q, p = k * lev + c;
+        if (k >= nz) continue;
+        float cc = ov[q][3] + ov[q][4];
+        if (last) cc = divc(cc, fsub, r_nsub) + ov[q][5];
+        ww_m[p] = cc;
+        const float phk = divc(ov[q][0] * mu_old, muts, r_muts) + divc(dts * ov[q][1], muts, r_muts) +
+                          ov[q][2] * (divc(mu_old, muts, r_muts) - 1.0f);
+        ph[p] = phk;
+        if (k < kend) t[p] = ov[q][6];
+        if (k >= 1) {  // calc_p_rho of the level below
+          const int pm = p - lev;
+          const float alk = -r_muts * (altm * mu + pd[1][k - 1] * (phk - phm));
+          al[pm] = alk;
+          const float pnew = c2m * (altm * (tm - mu * t1m) / (muts * ((float)T0 + t1m)) - alk);
+          pp[pm] = pnew + g.smdiv * (pnew - pmm);
+          pm1[pm] = pnew;
+        }
+        phm = phk;
+        tm = ov[q][6];
+        altm = ov[q][7];
+        t1m = ov[q][8];
+        c2m = ov[q][9];
+        pmm = ov[q][10];
+      }
+    }
+  } else if (iteration == 1) {  // outside the mass columns the flux average only starts at zero
+    for (int k = 0; k < nz; ++k) ww_m[k * lev + c] = 0.f;
+  }
+}
+
+// The marching form takes one wave of at most 13 warps per SM whose length is
+// the column's chain of levels (110 us per launch at 41 levels however few the
+// columns), so it pays from about one and a half such waves on: at 400x400x41
+// 397 us against 405 for the tiled form, at 320x320x61 374 against 411, at
+// 512x512x61 828 against 1091; at 240x240x41 165 against 140.
+static bool acoustic_col_marches(const Grid& g) {
+  return kernel_form() == WRF_FORM_FAST &&
+         2LL * (g.ide - g.ids) * (g.jde - g.jds) >= 3LL * 148 * 13 * kMarchTX;
+}
+
+
 __global__ void k_mu_uv_1(Grid g, S s) {
   WRF_COLUMN_INDEX(g, j, i);
   const int c = g.i2(j, i);
@@ -1138,11 +1586,19 @@ int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st) {
 }
 
 int launch_acoustic_col(const Grid& g, const S& s, float dts, int iteration, int nsub, cudaStream_t st) {
-  const dim3 gc((g.ide - g.ids + kColTX - 1) / kColTX, g.jde - g.jds);
-  if (g.nz <= 3 * kColKT)
-    k_acoustic_col<3><<<gc, kColTX * kColKT, 0, st>>>(g, s, dts, iteration, nsub);
+  const int i0 = g.nx % 8 == 0 ? g.ids / 8 * 8 : g.ids;
+  if (acoustic_col_marches(g)) {
+    k_acoustic_march<<<dim3((g.ide - i0 + kMarchTX - 1) / kMarchTX, g.jde - g.jds), kMarchTX,
+                       2 * (size_t)g.nz * kMarchTX * sizeof(float), st>>>(g, s, dts, iteration, nsub, i0);
+    return 1;
+  }
+  const dim3 gc((g.ide - i0 + kColTX - 1) / kColTX, g.jde - g.jds);
+  if (g.nz <= 2 * kColKT)
+    k_acoustic_col<2><<<gc, kColTX * kColKT, 0, st>>>(g, s, dts, iteration, nsub, i0);
+  else if (g.nz <= 3 * kColKT)
+    k_acoustic_col<3><<<gc, kColTX * kColKT, 0, st>>>(g, s, dts, iteration, nsub, i0);
   else
-    k_acoustic_col<4><<<gc, kColTX * kColKT, 0, st>>>(g, s, dts, iteration, nsub);
+    k_acoustic_col<4><<<gc, kColTX * kColKT, 0, st>>>(g, s, dts, iteration, nsub, i0);
   return 1;
 }
 
