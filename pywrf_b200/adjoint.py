@@ -68,6 +68,7 @@ operators keeps no tape of the forward's intermediates.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Callable, Sequence
 
 import torch
@@ -197,11 +198,18 @@ UV_DATA = ("msfux", "msfuy", "msfvx", "msfvx_inv", "msfvy", "fnm", "fnp", "rdnw"
 
 def _table(named: dict):
     """A state table (WrfState) holding the given fields by name."""
-    names = N.field_names()
-    arr = (ctypes.c_void_p * len(names))()
+    index = _field_index()
+    arr = (ctypes.c_void_p * len(index))()
     for k, t in named.items():
-        arr[names.index(k)] = _ptr(t).value
+        if not (t.is_cuda and t.dtype is torch.float32 and t.is_contiguous()):
+            raise TypeError("a contiguous float32 CUDA tensor is required (no CPU path)")
+        arr[index[k]] = t.data_ptr()
     return arr
+
+
+@functools.lru_cache(maxsize=1)
+def _field_index() -> dict:
+    return {k: q for q, k in enumerate(N.field_names())}
 
 
 def _zeros(*likes):
@@ -1048,33 +1056,8 @@ def acoustic_substep(st: dict, data: dict, iteration: int, nsub: int, dts: float
     after the substep (a new dict).  Differentiable end to end: every piece
     is a hand-written reverse kernel, and the chain keeps only the operators'
     inputs."""
-    s = dict(st)
-    u, v = advance_uv({k: s[k] for k in UV_INPUTS}, {k: data[k] for k in UV_DATA}, dts, emdiv, cf1, cf2, cf3, rdx,
-                      rdy)
-    s["u"], s["v"] = u, v
-    mt_in = {"ww": s["ww"], "ww_1": s["ww1"], "u": u, "u_1": s["u_save"], "v": v, "v_1": s["v_save"], "t": s["t"],
-             "t_1": s["t_save"], "t_ave": s["t_2save"], "ft": s["t_tend"], "mu": s["mu"], "mut": s["mut"],
-             "muave": s["muave"], "muts": s["muts"], "muu": s["muu"], "muv": s["muv"], "mudf": s["mudf"],
-             "mu_tend": s["mu_tend"]}
-    mt = advance_mu_t(mt_in, {k: data[k] for k in MUT_DATA}, dts, epssm, rdx, rdy)
-    s.update(ww=mt["ww"], t=mt["t"], t_2save=mt["t_ave"], muave=mt["muave"], muts=mt["muts"], mudf=mt["mudf"],
-             mu=mt["mu"])
-    s["t"] = spec_bdyupdate(s["t"], s["t_tend"], dts, "t", rdx, rdy)
-    s["mu"] = spec_bdyupdate(s["mu"], s["mu_tend"], dts, "m", rdx, rdy)
-    s["muts"] = spec_bdyupdate(s["muts"], s["mu_tend"], dts, "m", rdx, rdy)
-    aw_in = {k: s[k] for k in AW_INPUTS if k not in ("t_2ave", "t_2", "t_1", "ph_1")}
-    aw_in.update(t_2ave=s["t_2save"], t_2=s["t"], t_1=s["t_save"], ph_1=s["ph_save"])
-    aw = advance_w(aw_in, {k: data[k] for k in AW_DATA}, dts, epssm, cf1, cf2, cf3, rdx, rdy)
-    s.update(t_2save=aw["t_2ave"], w=aw["w"], ph=aw["ph"])
-    s["ru_m"], s["rv_m"], s["ww_m"] = sumflux({k: s[k] for k in SF_INPUTS}, {k: data[k] for k in SF_DATA},
-                                              iteration, nsub, rdx, rdy)
-    s["ph"] = spec_bdyupdate_ph({k: s[k] for k in SPH_INPUTS}, dts, rdx, rdy)
-    pr_in = {"al": s["al"], "p": s["p"], "ph": s["ph"], "alt": s["alt"], "t_2": s["t"], "t_1": s["t_save"],
-             "c2a": s["c2a"], "pm1": s["pm1"], "mu": s["mu"], "mut": s["muts"]}
-    s["al"], s["p"], s["pm1"] = calc_p_rho(pr_in, data["rdnw"], smdiv, iteration, rdx, rdy)
-    names = ("w", "ph", "al", "p", "muts", "mu", "mudf")
-    s.update(zip(names, halos([s[k] for k in names], "Zwppttt", rdx, rdy)))
-    return s
+    cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3)
+    return _run_chain(_substep_ops({**data, "_like3": st["ww"]}, iteration, nsub, dts), cg, st)
 
 
 class _TableOp(torch.autograd.Function):
@@ -1111,6 +1094,406 @@ class _TableOp(torch.autograd.Function):
         with torch.cuda.device(saved[0].device):
             N.check(op.adj(ctx.cg, _table(named), _table(bars), stream), op.name + "_adj")
         return (None, None) + tuple(bars[k] for k in op.fields) + (None,) * len(op.data)
+
+
+# ---- chains: a sequence of operators on one state, reversed on one table of
+# cotangents ----
+#
+# Composed from one autograd Function per operator, a step hands every field
+# that several operators read to the autograd engine, which adds their
+# cotangents up field by field, and every Function clears buffers for the
+# cotangents it adds into and copies those it rewrites: at 240x240x41 about a
+# third of the launches of a step's reverse, and most of its time on the host.
+# The reverse kernels accumulate into their operands' cotangents and rewrite
+# their results' cotangents to those of the values they replaced, so a whole
+# sequence of them runs on one table; the engine sees the sequence's ends only.
+
+class _Bars(dict):
+    """The cotangents of a chain's state by name; those not yet reached are
+    zero and are allocated when an operator asks for them."""
+
+    def need(self, likes: dict) -> dict:
+        missing = [k for k in likes if self.get(k) is None]
+        self.update(zip(missing, _zeros(*[likes[k] for k in missing])))
+        return {k: self[k] for k in likes}
+
+
+class _ChainOp:
+    """One operator of a chain: ``reads`` are the state names its reverse
+    needs (their values on entry are kept), ``writes`` those it replaces.
+    ``forward(cg, st, out, stream)`` fills ``out`` (copies of the written
+    fields, updated in place; with ``fresh``, uninitialised) and
+    ``backward(cg, saved, bars, stream)`` turns the written names' cotangents
+    into those of the values on entry and adds the rest."""
+    fresh = False
+
+    def __init__(self, reads, writes, forward, backward, fresh=False, fill=None):
+        self.reads, self.writes, self.forward, self.backward = tuple(reads), tuple(writes), forward, backward
+        self.fresh, self.fill = fresh, fill
+
+
+def _rc(rc, name):
+    N.check(rc, name)
+
+
+def _table_chain_op(op, data: dict):
+    """A chain operator from a state-table operator (see :class:`_TableOp`)."""
+    const = {k: data[k] for k in op.data}
+
+    def fwd(cg, st, out, stream):
+        _rc(op.fwd(cg, _table({**const, **{k: st[k] for k in op.fields}, **out}), stream), op.name)
+
+    def bwd(cg, saved, bars, stream):
+        likes = {k: saved[k] for k in op.fields}
+        _rc(op.adj(cg, _table({**const, **likes}), _table(bars.need(likes)), stream), op.name + "_adj")
+
+    return _ChainOp(op.fields, op.outputs, fwd, bwd)
+
+
+class _CallOp:
+    """A state-table operator from two library calls (for the operators
+    whose stand-alone Functions call the library directly)."""
+
+    def __init__(self, name, fields, outputs, data, fwd, adj):
+        self.name, self.fields, self.outputs, self.data, self.fwd, self.adj = name, fields, outputs, data, fwd, adj
+
+
+class _Chain(torch.autograd.Function):
+    """The operators ``ops`` in order on the state fields ``names``; returns
+    the final values of ``outs``."""
+
+    @staticmethod
+    def forward(ctx, ops, cg, names, outs, *tensors):
+        ctx.set_materialize_grads(False)
+        _cuda_only(*tensors)
+        st = {k: v.detach() for k, v in zip(names, tensors)}
+        kept = {}     # id of a kept tensor -> its place among the saved ones
+        saved, places = [], []
+        own = set()   # ids of this chain's tensors that nothing has kept
+        with torch.cuda.device(tensors[0].device):
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            for op in ops:
+                at = []
+                for k in op.reads:
+                    v = st[k]
+                    if id(v) not in kept:
+                        kept[id(v)] = len(saved)
+                        saved.append(v)
+                        own.discard(id(v))
+                    at.append(kept[id(v)])
+                places.append(at)
+                out = {}
+                for k in op.writes:
+                    if op.fresh:
+                        like = st[op.fill or k]
+                        out[k] = torch.empty_like(like)
+                    elif id(st[k]) in own:
+                        out[k] = st[k]
+                    else:
+                        out[k] = st[k].clone()
+                op.forward(cg, st, out, stream)
+                for k, v in out.items():
+                    st[k] = v
+                    own.add(id(v))
+        ctx.save_for_backward(*saved)
+        ctx.ops, ctx.cg, ctx.names, ctx.outs, ctx.places = ops, cg, names, outs, places
+        ctx.device = tensors[0].device
+        return tuple(st[k] for k in outs)
+
+    @staticmethod
+    def backward(ctx, *gouts):
+        saved = ctx.saved_tensors  # read once (checkpoint unpacks each saved tensor once)
+        bars = _Bars()
+        for k, gk in zip(ctx.outs, gouts):
+            if gk is not None:
+                bars[k] = gk.contiguous().clone()
+        with torch.cuda.device(ctx.device):
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            for op, at in zip(reversed(ctx.ops), reversed(ctx.places)):
+                op.backward(ctx.cg, {k: saved[q] for k, q in zip(op.reads, at)}, bars, stream)
+        need = ctx.needs_input_grad[4:]
+        return (None, None, None, None) + tuple(bars.get(k) if w else None for k, w in zip(ctx.names, need))
+
+
+def _run_chain(ops, cg, st: dict) -> dict:
+    """``st`` after the chain: the fields the operators write replaced."""
+    names, made = {}, set()
+    for op in ops:
+        for k in op.reads + ((op.fill,) if op.fill else op.writes):
+            if k not in made:
+                names[k] = None
+        made.update(op.writes)
+    outs = tuple(k for k in dict.fromkeys(k for op in ops for k in op.writes) if not k.startswith("_"))
+    new = _Chain.apply(tuple(ops), cg, tuple(names), outs, *[st[k] for k in names])
+    return {**st, **dict(zip(outs, new))}
+
+
+def _zero_op(name, like):
+    """``name`` starts from zero (shaped like the state field ``like``)."""
+    def fwd(cg, st, out, stream):
+        out[name].zero_()
+
+    def bwd(cg, saved, bars, stream):
+        bars.pop(name, None)
+
+    return _ChainOp((), (name,), fwd, bwd, fresh=True, fill=like)
+
+
+def _halo_op(names, letters):
+    """The halo copies of ``names`` (:class:`Halos`), out of place."""
+    def fwd(cg, st, out, stream):
+        Halos._call("wrf_halo_copy", cg, letters, [st[k] for k in names], [out[k] for k in names])
+
+    def bwd(cg, saved, bars, stream):
+        some = [q for q, k in enumerate(names) if bars.get(k) is not None]
+        if some:
+            gs = [bars[names[q]] for q in some]
+            new = [torch.empty_like(v) for v in gs]
+            Halos._call("wrf_halo_copy_adj", cg, "".join(letters[q] for q in some), gs, new)
+            bars.update((names[q], v) for q, v in zip(some, new))
+
+    return _ChainOp((), names, fwd, bwd, fresh=True)
+
+
+def _spec_update_op(field, tend, dt, var):
+    def fwd(cg, st, out, stream):
+        _rc(N.lib().wrf_spec_bdyupdate(ctypes.byref(cg), _ptr(out[field]), _ptr(st[tend]), dt, var.encode(), stream),
+            "wrf_spec_bdyupdate")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(field) is not None:
+            b = bars.need({tend: saved[tend]})
+            _rc(N.lib().wrf_spec_bdyupdate_adj(ctypes.byref(cg), _ptr(bars[field]), _ptr(b[tend]), dt, var.encode(),
+                                               stream), "wrf_spec_bdyupdate_adj")
+
+    return _ChainOp((tend,), (field,), fwd, bwd)
+
+
+def _spec_tend_op(tend, bt: dict, var):
+    def fwd(cg, st, out, stream):
+        _rc(N.lib().wrf_spec_bdytend(ctypes.byref(cg), _ptr(out[tend]), _ptr(bt["txs"]), _ptr(bt["txe"]),
+                                     _ptr(bt["tys"]), _ptr(bt["tye"]), var.encode(), stream), "wrf_spec_bdytend")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(tend) is not None:
+            _rc(N.lib().wrf_spec_bdytend_adj(ctypes.byref(cg), _ptr(bars[tend]), var.encode(), stream),
+                "wrf_spec_bdytend_adj")
+
+    return _ChainOp((), (tend,), fwd, bwd)
+
+
+def _relax_op(field, tend, bdy: dict, var, dtbc):
+    """tend += relax_bdytend(field); 'm' (mu) is 2-D: the library relaxes one
+    level of it."""
+    arr = (ctypes.c_void_p * 8)(*[_ptr(bdy[k]).value for k in BDY_NAMES])
+    keep = [bdy[k] for k in BDY_NAMES]
+
+    def fwd(cg, st, out, stream):
+        assert keep
+        _rc(N.lib().wrf_relax_bdytend(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), arr, var.encode(),
+                                      float(dtbc), stream), "wrf_relax_bdytend")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(tend) is not None:
+            b = bars.need({field: saved[field]})
+            _rc(N.lib().wrf_relax_bdytend_adj(ctypes.byref(cg), _ptr(bars[tend]), _ptr(b[field]), var.encode(),
+                                              stream), "wrf_relax_bdytend_adj")
+
+    return _ChainOp((field,), (tend,), fwd, bwd)
+
+
+def _mass_weight_op(field, mass, out_name, nk):
+    def fwd(cg, st, out, stream):
+        out[out_name].zero_()
+        _rc(N.lib().wrf_mass_weight(ctypes.byref(cg), _ptr(st[field]), _ptr(st[mass]), _ptr(out[out_name]), nk,
+                                    stream), "wrf_mass_weight")
+
+    def bwd(cg, saved, bars, stream):
+        gk = bars.pop(out_name, None)
+        if gk is not None:
+            b = bars.need(saved)
+            _rc(N.lib().wrf_mass_weight_adj(ctypes.byref(cg), _ptr(saved[field]), _ptr(saved[mass]), _ptr(gk),
+                                            _ptr(b[field]), _ptr(b[mass]), nk, stream), "wrf_mass_weight_adj")
+
+    return _ChainOp((field, mass), (out_name,), fwd, bwd, fresh=True, fill=field)
+
+
+def _advect_work(cg, name, like):
+    n = ctypes.c_size_t(0)
+    _rc(getattr(N.lib(), name)(ctypes.byref(cg), ctypes.byref(n)), "work")
+    return torch.empty(int(n.value), dtype=torch.float32, device=like.device), n
+
+
+def _advect_momentum_op(component, field, tend, data: dict):
+    msf = data[("msfux", "msfvy", "msftx")[component]]
+    m2 = _ptr(data["msfvx"]) if component == 1 else None
+    rdz = data["rdn" if component == 2 else "rdnw"]
+    fnm, fnp = data["fnm"], data["fnp"]
+
+    def fwd(cg, st, out, stream):
+        _rc(N.lib().wrf_advect_momentum(ctypes.byref(cg), component, _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
+                                        _ptr(st["rv"]), _ptr(st["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
+                                        _ptr(rdz), 0, stream), "wrf_advect_momentum")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(tend) is None:
+            return
+        b = bars.need(saved)
+        work, n = _advect_work(cg, "wrf_advect_momentum_adj_work", saved[field])
+        _rc(N.lib().wrf_advect_momentum_adj(ctypes.byref(cg), component, _ptr(saved[field]), _ptr(saved["ru"]),
+                                            _ptr(saved["rv"]), _ptr(saved["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
+                                            _ptr(rdz), _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
+                                            _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n, stream),
+            "wrf_advect_momentum_adj")
+
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd)
+
+
+def _advect_scalar_op(field, tend, data: dict):
+    const = [_ptr(data[k]) for k in ("msftx", "fnm", "fnp", "rdnw")]
+
+    def fwd(cg, st, out, stream):
+        _rc(N.lib().wrf_advect_scalar(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
+                                      _ptr(st["rv"]), _ptr(st["ww"]), *const, stream), "wrf_advect_scalar")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(tend) is None:
+            return
+        b = bars.need(saved)
+        work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved[field])
+        _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved[field]), _ptr(saved["ru"]), _ptr(saved["rv"]),
+                                          _ptr(saved["ww"]), *const, _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
+                                          _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n, stream),
+            "wrf_advect_scalar_adj")
+
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd)
+
+
+def _advect_moist_op(data: dict):
+    """advect_tend = the moisture's advection by the averaged fluxes, which
+    carry no cotangent past the update they feed (:class:`AdvectMoist`)."""
+    const = [_ptr(data[k]) for k in ("msftx", "fnm", "fnp", "rdnw")]
+    fluxes = ("ru_m", "rv_m", "ww_m")
+
+    def fwd(cg, st, out, stream):
+        out["advect_tend"].zero_()
+        _rc(N.lib().wrf_advect_moist(ctypes.byref(cg), _ptr(st["moist"]), _ptr(out["advect_tend"]),
+                                     *[_ptr(st[k]) for k in fluxes], *const, stream), "wrf_advect_moist")
+
+    def bwd(cg, saved, bars, stream):
+        gk = bars.pop("advect_tend", None)
+        if gk is None:
+            return
+        b = bars.need(saved)
+        work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved["ru_m"])
+        for m in range(1, 7):
+            _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved["moist"][m]),
+                                              *[_ptr(saved[k]) for k in fluxes], *const, _ptr(gk[m]),
+                                              _ptr(b["moist"][m]), *[_ptr(b[k]) for k in fluxes], _ptr(work), n,
+                                              stream), "wrf_advect_scalar_adj")
+
+    return _ChainOp(("moist",) + fluxes, ("advect_tend",), fwd, bwd, fresh=True, fill="moist")
+
+
+def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
+    """tend += horizontal_diffusion(field); ``field`` "moist": its six
+    species into the slots of ``tend``."""
+    const = {k: data[k] for k in HDIFF_DATA}
+    bp = None if base is None else _ptr(base)
+
+    def each(v):
+        return [v[m] for m in range(1, 7)] if v.dim() == 4 else [v]
+
+    def fwd(cg, st, out, stream):
+        tab = _table(const)
+        for f, o in zip(each(st[field]), each(out[tend])):
+            _rc(N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp, _ptr(st[mass]),
+                                                 _ptr(st[visc]), _ptr(o), stream), "wrf_horizontal_diffusion")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get(tend) is None:
+            return
+        b = bars.need(saved)
+        tab = _table(const)
+        for f, gk, fb in zip(each(saved[field]), each(bars[tend]), each(b[field])):
+            _rc(N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp,
+                                                     _ptr(saved[mass]), _ptr(saved[visc]), _ptr(gk), _ptr(fb),
+                                                     _ptr(b[mass]), _ptr(b[visc]), stream),
+                "wrf_horizontal_diffusion_adj")
+
+    return _ChainOp((field, mass, visc), (tend,), fwd, bwd)
+
+
+def _coef_w_op(dts, data: dict):
+    names = ("a", "alpha", "gamma")
+
+    def fwd(cg, st, out, stream):
+        for k in names:
+            out[k].zero_()
+        _rc(N.lib().wrf_coef_w(ctypes.byref(cg), _ptr(st["mut"]), _ptr(st["cqw"]), _ptr(st["c2a"]),
+                               _ptr(data["rdn"]), _ptr(data["rdnw"]), float(dts), *[_ptr(out[k]) for k in names],
+                               stream), "wrf_coef_w")
+
+    def bwd(cg, saved, bars, stream):
+        gs = bars.need({k: saved["cqw"] for k in names})
+        b = bars.need(saved)
+        _rc(N.lib().wrf_coef_w_adj(ctypes.byref(cg), _ptr(saved["mut"]), _ptr(saved["cqw"]), _ptr(saved["c2a"]),
+                                   _ptr(data["rdn"]), _ptr(data["rdnw"]), float(dts), *[_ptr(gs[k]) for k in names],
+                                   _ptr(b["mut"]), _ptr(b["cqw"]), _ptr(b["c2a"]), stream), "wrf_coef_w_adj")
+        for k in names:
+            del bars[k]
+
+    return _ChainOp(("mut", "cqw", "c2a"), names, fwd, bwd, fresh=True, fill="cqw")
+
+
+def _substep_ops(data: dict, iteration: int, nsub: int, dts: float) -> list:
+    """The operators of one acoustic substep, in the reference's order."""
+    L = N.lib()
+    by = ctypes.byref
+    field = lambda names, ren: tuple(ren.get(k, k) for k in names)  # noqa: E731
+
+    def work_like(tab_adj, like):
+        return lambda cg, tab, btab, stream: tab_adj(cg, tab, btab, torch.empty_like(like), stream)
+
+    ws3 = data["_like3"]
+    uv = _CallOp("wrf_advance_uv", UV_INPUTS, ("u", "v"), UV_DATA,
+                 lambda cg, tab, s: L.wrf_advance_uv(by(cg), tab, dts, s),
+                 lambda cg, tab, b, s: L.wrf_advance_uv_adj(by(cg), tab, b, dts, s))
+    mt = _CallOp("wrf_advance_mu_t", field(MUT_INPUTS, _MUT_FIELD), field(MUT_OUTPUTS, _MUT_FIELD), MUT_DATA,
+                 lambda cg, tab, s: L.wrf_advance_mu_t(by(cg), tab, dts, s),
+                 work_like(lambda cg, tab, b, w, s: L.wrf_advance_mu_t_adj(by(cg), tab, b, dts, 0, _ptr(w), s),
+                           ws3))
+    aw = _CallOp("wrf_advance_w", field(AW_INPUTS, _AW_FIELD), field(AW_OUTPUTS, _AW_FIELD), AW_DATA,
+                 lambda cg, tab, s: L.wrf_advance_w(by(cg), tab, dts, s),
+                 work_like(lambda cg, tab, b, w, s: L.wrf_advance_w_adj(by(cg), tab, b, dts, _ptr(w), s),
+                           data["msftx"]))
+    sf = _CallOp("wrf_sumflux", SF_INPUTS, SF_INPUTS[:3], SF_DATA,
+                 lambda cg, tab, s: L.wrf_sumflux(by(cg), tab, iteration, nsub, s),
+                 lambda cg, tab, b, s: L.wrf_sumflux_adj(by(cg), tab, b, iteration, nsub, s))
+    sp = _CallOp("wrf_spec_bdyupdate_ph", SPH_INPUTS, ("ph",), (),
+                 lambda cg, tab, s: L.wrf_spec_bdyupdate_ph(by(cg), tab, dts, s),
+                 lambda cg, tab, b, s: L.wrf_spec_bdyupdate_ph_adj(by(cg), tab, b, dts, s))
+    ops = [_table_chain_op(uv, data), _table_chain_op(mt, data)]
+    ops += [_spec_update_op("t", "t_tend", dts, "t"), _spec_update_op("mu", "mu_tend", dts, "m"),
+            _spec_update_op("muts", "mu_tend", dts, "m")]
+    ops += [_table_chain_op(aw, data), _table_chain_op(sf, data), _table_chain_op(sp, data), _p_rho_op(data, iteration)]
+    ops.append(_halo_op(("w", "ph", "al", "p", "muts", "mu", "mudf"), "Zwppttt"))
+    return ops
+
+
+def _p_rho_op(data: dict, step: int):
+    ren = tuple(_PRHO_FIELD.get(k, k) for k in PRHO_INPUTS)
+    return _table_chain_op(_CallOp("wrf_calc_p_rho", ren, ("al", "p", "pm1"), ("rdnw",),
+                                   lambda cg, tab, s: N.lib().wrf_calc_p_rho(ctypes.byref(cg), tab, step, s),
+                                   lambda cg, tab, b, s: N.lib().wrf_calc_p_rho_adj(ctypes.byref(cg), tab, b, step,
+                                                                                    s)), data)
+
+
+def _chain_grid(shape, rdx, rdy, **scal):
+    cg = scalar_grid(shape, rdx, rdy)
+    for k, v in scal.items():
+        setattr(cg, k, v if k == "top_lid" else float(v))
+    return cg
 
 
 class _SmallStepPrep:
@@ -1191,22 +1574,23 @@ def acoustic_stage(st: dict, data: dict, rk_step: int, nsub: int, dts: float, *,
     with small_step_finish, and at the last stage the halo copies of the
     averaged fluxes and column masses.  ``st`` maps every field these read;
     returns the state after the stage."""
-    s = small_step_prep(st, data, rk_step, rdx, rdy)
-    pr = {"al": s["al"], "p": s["p"], "ph": s["ph"], "alt": s["alt"], "t_2": s["t"], "t_1": s["t_save"],
-          "c2a": s["c2a"], "pm1": s["pm1"], "mu": s["mu"], "mut": s["muts"]}
-    s["al"], s["p"], s["pm1"] = calc_p_rho(pr, data["rdnw"], smdiv, 0, rdx, rdy)
-    s["a"], s["alpha"], s["gamma"] = coef_w(s["mut"], s["cqw"], s["c2a"], data["rdn"], data["rdnw"], dts, epssm,
-                                            top_lid, rdx, rdy)
-    names = ("ru_tend", "rv_tend", "ph", "al", "p", "t_1", "t_save", "mu_1", "mu", "mudf")
-    s.update(zip(names, halos([s[k] for k in names], "uvwppttttt", rdx, rdy)))
-    sc = dict(epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3, rdx=rdx, rdy=rdy)
+    cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3,
+                     top_lid=int(bool(top_lid)))
+    return _run_chain(_acoustic_ops(st, data, rk_step, nsub, dts), cg, st)
+
+
+def _acoustic_ops(st: dict, data: dict, rk_step: int, nsub: int, dts: float) -> list:
+    """The operators of :func:`acoustic_stage`."""
+    nz, ny, nx = st["u"].shape
+    dev = st["u"].device
+    ops = [_table_chain_op(_SmallStepPrep(rk_step, ny, nx, dev), data), _p_rho_op(data, 0), _coef_w_op(dts, data),
+           _halo_op(("ru_tend", "rv_tend", "ph", "al", "p", "t_1", "t_save", "mu_1", "mu", "mudf"), "uvwppttttt")]
     for it in range(1, nsub + 1):
-        s = acoustic_substep(s, data, it, nsub, dts, **sc)
-    s = small_step_finish(s, data, dts, nsub, rk_step, rdx, rdy)
+        ops += _substep_ops({**data, "_like3": st["ww"]}, it, nsub, dts)
+    ops.append(_table_chain_op(_SmallStepFinish(dts, nsub, rk_step, ny, nx, dev), data))
     if rk_step == 3:
-        names = ("ru_m", "rv_m", "ww_m", "mut", "muts")
-        s.update(zip(names, halos([s[k] for k in names], "uvwtt", rdx, rdy)))
-    return s
+        ops.append(_halo_op(("ru_m", "rv_m", "ww_m", "mut", "muts"), "uvwtt"))
+    return ops
 
 
 class _Addtend:
@@ -1464,23 +1848,17 @@ DYN_DATA = tuple(dict.fromkeys(STAGE_DATA + PREP_DATA + FORCES_DATA + _Addtend.d
                                HDIFF_DATA + ("t_init",)))
 
 
-def _first_stage_diffusion(s: dict, data: dict, bdy: dict, dtbc: float, rdx, rdy) -> dict:
+def _first_stage_ops(data: dict, bdy: dict, dtbc: float, nz: int) -> list:
     """The first stage's horizontal diffusion of u, v, w and theta into the
     physics tendencies and the lateral relaxation into the saved fields
     (pywrf/solver.py:1112-1203)."""
-    hd = {k: data[k] for k in HDIFF_DATA}
-    for name in ("u", "v", "w"):
-        s[f"r{name}_tendf"] = horizontal_diffusion(name, s[name], s[f"r{name}_tendf"], s["mut"], s["xkmh"], hd,
-                                                   rdx, rdy)
-    s["t_tendf"] = horizontal_diffusion("m", s["t"], s["t_tendf"], s["mut"], s["xkhh"], hd, rdx, rdy,
-                                        base=data["t_init"])
-    nz = s["u"].shape[0]
-    s["u_save"] = relax_bdytend(s["ru"], s["u_save"], "u", dtbc, bdy["u"])
-    s["v_save"] = relax_bdytend(s["rv"], s["v_save"], "v", dtbc, bdy["v"])
-    s["ph_save"] = relax_bdytend(mass_weight(s["ph"], s["mut"], nz, rdx, rdy), s["ph_save"], "h", dtbc, bdy["h"])
-    s["t_save"] = relax_bdytend(mass_weight(s["t"], s["mut"], nz, rdx, rdy), s["t_save"], "t", dtbc, bdy["t"])
-    s["mu_tend"] = relax_bdytend(s["mu"][None], s["mu_tend"][None], "m", dtbc, bdy["m"])[0]
-    return s
+    ops = [_diffusion_op(k, k, f"r{k}_tendf", "mut", "xkmh", data) for k in ("u", "v", "w")]
+    ops.append(_diffusion_op("m", "t", "t_tendf", "mut", "xkhh", data, base=data["t_init"]))
+    ops += [_relax_op("ru", "u_save", bdy["u"], "u", dtbc), _relax_op("rv", "v_save", bdy["v"], "v", dtbc)]
+    for k, var in (("ph", "h"), ("t", "t")):
+        ops += [_mass_weight_op(k, "mut", "_mass", nz), _relax_op("_mass", f"{k}_save", bdy[var], var, dtbc)]
+    ops.append(_relax_op("mu", "mu_tend", bdy["m"], "m", dtbc))
+    return ops
 
 
 def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts: float, *, epssm: float,
@@ -1501,39 +1879,34 @@ def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts:
         raise ValueError("rk_step is 1, 2 or 3")
     if rk_step == 1 and dtbc is None:
         raise ValueError("the first stage's relaxation needs dtbc")
-    s = dict(st)
-    s.update(prep({k: s[k] for k in PREP_FIELDS}, {k: data[k] for k in PREP_DATA}, 127, rdx, rdy))
-    names = ("ru", "rv", "rw", "ww", "php", "alt", "p", "muu", "muv", "mut", "al", "ph")
-    s.update(zip(names, halos([s[k] for k in names], "uvwwwtpuvtpw", rdx, rdy)))
+    L, by = N.lib(), ctypes.byref
+    cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3,
+                     cfn=cfn, cfn1=cfn1)
+    ops = [_table_chain_op(_CallOp("wrf_prep", PREP_FIELDS, PREP_OUTPUTS, PREP_DATA,
+                                   lambda c, tab, s: L.wrf_prep(by(c), tab, 127, s),
+                                   lambda c, tab, b, s: L.wrf_prep_adj(by(c), tab, b, 127, s)), data),
+           _halo_op(("ru", "rv", "rw", "ww", "php", "alt", "p", "muu", "muv", "mut", "al", "ph"), "uvwwwtpuvtpw")]
+    zeros = ("ru_tend", "rv_tend", "rw_tend", "t_tend", "ph_tend", "u_save", "v_save", "w_save", "ph_save", "t_save",
+             "mu_tend", "mu_save")
     if rk_step == 1:
-        for k in ("ru_tendf", "rv_tendf", "rw_tendf", "ph_tendf", "t_tendf", "mu_tendf", "moist_tend"):
-            s[k] = torch.zeros_like(st[k])
-        s["xkmh"], s["xkhh"] = eddy_viscosity(s, data, rdx, rdy, cf1, cf2, cf3)
-        s["xkmh"], s["xkhh"] = halos([s["xkmh"], s["xkhh"]], "tt", rdx, rdy)
-    for k in ("ru_tend", "rv_tend", "rw_tend", "t_tend", "ph_tend", "u_save", "v_save", "w_save", "ph_save",
-              "t_save", "mu_tend", "mu_save"):
-        s[k] = torch.zeros_like(st[k])
-    z = lambda k: s[k]  # noqa: E731
-    s["ru_tend"] = advect_momentum(0, s["u"], z("ru_tend"), s["ru"], s["rv"], s["ww"], data["msfux"], None,
-                                   data["fnm"], data["fnp"], data["rdnw"], rdx, rdy)
-    s["rv_tend"] = advect_momentum(1, s["v"], z("rv_tend"), s["ru"], s["rv"], s["ww"], data["msfvy"], data["msfvx"],
-                                   data["fnm"], data["fnp"], data["rdnw"], rdx, rdy)
-    s["rw_tend"] = advect_momentum(2, s["w"], z("rw_tend"), s["ru"], s["rv"], s["ww"], data["msftx"], None,
-                                   data["fnm"], data["fnp"], data["rdn"], rdx, rdy)
-    s["t_tend"] = advect_scalar(s["t"], z("t_tend"), s["ru"], s["rv"], s["ww"], data["msftx"], data["fnm"],
-                                data["fnp"], data["rdnw"], rdx, rdy)
-    outs = forces({k: s[k] for k in FORCES_INPUTS}, {k: data[k] for k in FORCES_DATA}, 31, rdx, rdy, cf1, cf2, cf3,
-                  cfn, cfn1)
-    s.update(dict(zip(FORCES_OUTPUTS, outs)))
+        tendf = ("ru_tendf", "rv_tendf", "rw_tendf", "ph_tendf", "t_tendf", "mu_tendf", "moist_tend")
+        ops += [_zero_op(k, k) for k in tendf]
+        ops += [_table_chain_op(_EddyViscosity(st["u"]), data), _halo_op(("xkmh", "xkhh"), "tt")]
+    ops += [_zero_op(k, k) for k in zeros]
+    ops += [_advect_momentum_op(0, "u", "ru_tend", data), _advect_momentum_op(1, "v", "rv_tend", data),
+            _advect_momentum_op(2, "w", "rw_tend", data), _advect_scalar_op("t", "t_tend", data)]
+    ops.append(_table_chain_op(_CallOp("wrf_forces", FORCES_INPUTS, FORCES_OUTPUTS, FORCES_DATA,
+                                       lambda c, tab, s: L.wrf_forces(by(c), tab, 31, s),
+                                       lambda c, tab, b, s: L.wrf_forces_adj(by(c), tab, b, 31, s)), data))
     if rk_step == 1:
-        s = _first_stage_diffusion(s, data, bt, dtbc, rdx, rdy)
-    s = addtend(s, data, rk_step, rdx, rdy)
+        ops += _first_stage_ops(data, bt, dtbc, st["u"].shape[0])
+    ops.append(_table_chain_op(_Addtend(rk_step), data))
+    s = _run_chain(ops, cg, st)
     if theta_bias is not None:
         s["t_tend"] = s["t_tend"] + theta_bias
-    for k, var in (("ru_tend", "u"), ("rv_tend", "v"), ("ph_tend", "h"), ("t_tend", "t"), ("mu_tend", "m")):
-        s[k] = spec_bdytend(s[k], bt[var], var, rdx, rdy)
-    return acoustic_stage(s, data, rk_step, nsub, dts, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2,
-                          cf3=cf3, rdx=rdx, rdy=rdy)
+    ops = [_spec_tend_op(k, bt[var], var) for k, var in (("ru_tend", "u"), ("rv_tend", "v"), ("ph_tend", "h"),
+                                                         ("t_tend", "t"), ("mu_tend", "m"))]
+    return _run_chain(ops + _acoustic_ops(s, data, rk_step, nsub, dts), cg, s)
 
 
 class _MoistUpdate:
@@ -1567,28 +1940,47 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
     and specified tendency of qv (``bt['q']``: its eight boundary arrays,
     ``dtbc`` the boundary time); rk_update_scalar, flow_dep_bdy of qc .. qg,
     calc_p_rho_phi and, before the last stage, the halo copies."""
-    s = dict(st)
-    moist = s["moist"]
-    s["advect_tend"] = advect_moist(moist, s["ru_m"], s["rv_m"], s["ww_m"], data["msftx"], data["fnm"], data["fnp"],
-                                    data["rdnw"], rdx, rdy)
+    if rk_step == 1 and (bt is None or dtbc is None):
+        raise ValueError("the first stage's qv relaxation needs its boundary arrays and dtbc")
+    cg = scalar_grid(st["u"].shape, rdx, rdy)
+    ops = [_advect_moist_op(data)]
     if rk_step == 1:
-        if bt is None or dtbc is None:
-            raise ValueError("the first stage's qv relaxation needs its boundary arrays and dtbc")
-        mt = MoistDiffusion.apply((rdx, rdy), moist, s["moist_tend"], s["muts"], s["xkhh"],
-                                  *[data[k] for k in HDIFF_DATA])
-        nz = moist.shape[1]
-        rq = mass_weight(moist[1], s["mut"], nz - 1, rdx, rdy)
-        qv = spec_bdytend(relax_bdytend(rq, mt[1], "t", dtbc, bt["q"]), bt["q"], "t", rdx, rdy)
-        s["moist_tend"] = PutSlot.apply(1, mt, qv)
-    op = _MoistUpdate(rk_step, dt_rk, s["u"])
-    cg = scalar_grid(s["u"].shape, rdx, rdy)
-    dd = {"msfty": data["msfty"], "ru_m": s["ru_m"].detach(), "rv_m": s["rv_m"].detach(), "rdnw": data["rdnw"]}
-    outs = _TableOp.apply(op, cg, *[s[k] for k in op.fields], *[dd[k] for k in op.data])
-    s.update(dict(zip(op.outputs, outs)))
+        ops.append(_diffusion_op("m", "moist", "moist_tend", "muts", "xkhh", data))
+        ops += _relax_qv_ops(st["u"].shape[0], bt["q"], dtbc)
+    # the averaged fluxes enter flow_dep_bdy by their sign alone: data
+    dd = {"msfty": data["msfty"], "ru_m": st["ru_m"].detach(), "rv_m": st["rv_m"].detach(), "rdnw": data["rdnw"]}
+    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk, st["u"]), dd))
     if rk_step < 3:
-        names = ("u", "v", "w", "t", "ph", "mu", "moist")
-        s.update(zip(names, halos([s[k] for k in names], "UVwpwtM", rdx, rdy)))
-    return s
+        ops.append(_halo_op(("u", "v", "w", "t", "ph", "mu", "moist"), "UVwpwtM"))
+    return _run_chain(ops, cg, st)
+
+
+def _relax_qv_ops(nz: int, bdy: dict, dtbc: float) -> list:
+    """qv's lateral relaxation and specified tendency into its slot of
+    moist_tend (pywrf/solver.py:1600-1640)."""
+    arr = (ctypes.c_void_p * 8)(*[_ptr(bdy[k]).value for k in BDY_NAMES])
+    L, by = N.lib(), ctypes.byref
+
+    def fwd(cg, st, out, stream):
+        tend = out["moist_tend"][1]
+        mass = torch.zeros_like(tend)
+        _rc(L.wrf_mass_weight(by(cg), _ptr(st["moist"][1]), _ptr(st["mut"]), _ptr(mass), nz - 1, stream),
+            "wrf_mass_weight")
+        _rc(L.wrf_relax_bdytend(by(cg), _ptr(mass), _ptr(tend), arr, b"t", float(dtbc), stream), "wrf_relax_bdytend")
+        _rc(L.wrf_spec_bdytend(by(cg), _ptr(tend), *[_ptr(bdy[k]) for k in ("txs", "txe", "tys", "tye")], b"t",
+                               stream), "wrf_spec_bdytend")
+
+    def bwd(cg, saved, bars, stream):
+        if bars.get("moist_tend") is None:
+            return
+        b, gk = bars.need(saved), bars["moist_tend"][1]
+        _rc(L.wrf_spec_bdytend_adj(by(cg), _ptr(gk), b"t", stream), "wrf_spec_bdytend_adj")
+        mass = torch.zeros_like(gk)
+        _rc(L.wrf_relax_bdytend_adj(by(cg), _ptr(gk), _ptr(mass), b"t", stream), "wrf_relax_bdytend_adj")
+        _rc(L.wrf_mass_weight_adj(by(cg), _ptr(saved["moist"][1]), _ptr(saved["mut"]), _ptr(mass),
+                                  _ptr(b["moist"][1]), _ptr(b["mut"]), nz - 1, stream), "wrf_mass_weight_adj")
+
+    return [_ChainOp(("moist", "mut"), ("moist_tend",), fwd, bwd)]
 
 
 RK_STATE = tuple(dict.fromkeys(DYN_STATE + _MoistUpdate.fields + ("ru_m", "rv_m", "ww_m")))
