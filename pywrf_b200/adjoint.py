@@ -79,10 +79,24 @@ from .config import Grid
 from .state import make_cgrid
 
 
-def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
-    if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+def _ptr(t: torch.Tensor) -> int:
+    """The address of a contiguous float32 CUDA tensor."""
+    if not (t.is_cuda and t.dtype is torch.float32 and t.is_contiguous()):
         raise TypeError("a contiguous float32 CUDA tensor is required (no CPU path)")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+# The device is named by its index: from a torch.device (or none at all)
+# current_stream and device each take several microseconds to find it, which
+# is most of what a small operator's call spends outside its kernels.
+def _stream(t: torch.Tensor) -> int:
+    """The handle of the stream that is current on the tensor's device."""
+    return torch.cuda.current_stream(t.get_device()).cuda_stream
+
+
+def _on(t: torch.Tensor):
+    """The tensor's device as the current one."""
+    return torch.cuda.device(t.get_device())
 
 
 def _cuda_only(*ts) -> None:
@@ -94,7 +108,13 @@ def _cuda_only(*ts) -> None:
 
 
 def scalar_grid(shape, rdx: float, rdy: float):
-    """The C grid record of the solver's 5-cell frame for a field of ``shape``."""
+    """The C grid record of the solver's 5-cell frame for a field of ``shape``
+    (the caller's own copy)."""
+    return N.WrfGridC.from_buffer_copy(_frame(tuple(shape), float(rdx), float(rdy)))
+
+
+@functools.lru_cache(maxsize=64)
+def _frame(shape, rdx: float, rdy: float):
     nz, ny, nx = shape
     g = Grid.make(nx, ny, nz, 1.0 / float(rdx), 1.0 / float(rdy), 1.0)
     cg = make_cgrid(g, {"cf1": 0.0, "cf2": 0.0, "cf3": 0.0, "cfn": 0.0, "cfn1": 0.0})
@@ -103,18 +123,24 @@ def scalar_grid(shape, rdx: float, rdy: float):
     return cg
 
 
+@functools.lru_cache(maxsize=64)
+def _advect_work_floats(shape) -> int:
+    n = ctypes.c_size_t(0)
+    N.check(N.lib().wrf_advect_scalar_adj_work(ctypes.byref(_frame(shape, 1.0, 1.0)), ctypes.byref(n)), "work")
+    return n.value
+
+
 class AdvectScalar(torch.autograd.Function):
     """out = tendency + flux-form advection of ``field`` by (ru, rv, rom)."""
 
     @staticmethod
     def forward(ctx, field, tendency, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx: float, rdy: float):
-        _cuda_only(field, tendency, ru, rv, rom, msftx, fnm, fnp, rdnw)
+        q, _, *rest = [_ptr(t) for t in (field, tendency, ru, rv, rom, msftx, fnm, fnp, rdnw)]
         cg = scalar_grid(field.shape, rdx, rdy)
         out = tendency.detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
-            rc = N.lib().wrf_advect_scalar(ctypes.byref(cg), _ptr(field), _ptr(out), _ptr(ru), _ptr(rv), _ptr(rom),
-                                           _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw), stream)
+        stream = _stream(field)
+        with _on(field):
+            rc = N.lib().wrf_advect_scalar(ctypes.byref(cg), q, out.data_ptr(), *rest, stream)
         N.check(rc, "wrf_advect_scalar")
         ctx.save_for_backward(field, ru, rv, rom, msftx, fnm, fnp, rdnw)
         ctx.cg = cg
@@ -125,11 +151,10 @@ class AdvectScalar(torch.autograd.Function):
         field, ru, rv, rom, msftx, fnm, fnp, rdnw = ctx.saved_tensors
         gout = gout.contiguous()
         qb, rub, rvb, romb = _zeros(field, field, field, field)
-        n = ctypes.c_size_t(0)
-        N.check(N.lib().wrf_advect_scalar_adj_work(ctypes.byref(ctx.cg), ctypes.byref(n)), "work")
-        work = torch.empty(int(n.value), dtype=torch.float32, device=field.device)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        n = _advect_work_floats(tuple(field.shape))
+        work = torch.empty(n, dtype=torch.float32, device=field.device)
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_advect_scalar_adj(ctypes.byref(ctx.cg), _ptr(field), _ptr(ru), _ptr(rv), _ptr(rom),
                                                _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw), _ptr(gout), _ptr(qb),
                                                _ptr(rub), _ptr(rvb), _ptr(romb), _ptr(work), n, stream)
@@ -157,8 +182,8 @@ class AdvectMomentum(torch.autograd.Function):
         cg = scalar_grid(field.shape, rdx, rdy)
         out = tendency.detach().clone()
         m2 = _ptr(msf2) if msf2 is not None else None
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_advect_momentum(ctypes.byref(cg), int(component), _ptr(field), _ptr(out), _ptr(ru),
                                              _ptr(rv), _ptr(rom), _ptr(msf), m2, _ptr(fzm), _ptr(fzp), _ptr(rdz),
                                              0, stream)
@@ -176,8 +201,8 @@ class AdvectMomentum(torch.autograd.Function):
         n = ctypes.c_size_t(0)
         N.check(N.lib().wrf_advect_momentum_adj_work(ctypes.byref(ctx.cg), ctypes.byref(n)), "work")
         work = torch.empty(int(n.value), dtype=torch.float32, device=field.device)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_advect_momentum_adj(ctypes.byref(ctx.cg), ctx.component, _ptr(field), _ptr(ru), _ptr(rv),
                                                  _ptr(rom), _ptr(msf), m2, _ptr(fzm), _ptr(fzp), _ptr(rdz), _ptr(gout),
                                                  _ptr(qb), _ptr(rub), _ptr(rvb), _ptr(romb), _ptr(work), n, stream)
@@ -222,9 +247,19 @@ def _zeros(*likes):
     buf = torch.zeros(sum(sizes), dtype=torch.float32, device=likes[0].device)
     out, o = [], 0
     for t, n in zip(likes, sizes):
-        out.append(buf[o:o + t.numel()].view(t.shape))
+        out.append(torch.as_strided(buf, t.shape, _packed(t), o))
         o += n
     return out
+
+
+def _packed(t: torch.Tensor) -> tuple:
+    """The strides of ``t``'s shape without gaps."""
+    if t.is_contiguous():
+        return t.stride()
+    s = [1]
+    for n in reversed(t.shape[1:]):
+        s.append(s[-1] * n)
+    return tuple(reversed(s))
 
 
 def _bars(named: dict, fields, grads: dict) -> dict:
@@ -256,8 +291,8 @@ class AdvanceUV(torch.autograd.Function):
         cg.emdiv, cg.cf1, cg.cf2, cg.cf3 = emdiv, cf1, cf2, cf3
         u_new, v_new = named["u"].detach().clone(), named["v"].detach().clone()
         tab = _table({**named, "u": u_new, "v": v_new})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(u_new.device):
+        stream = _stream(u_new)
+        with _on(u_new):
             rc = N.lib().wrf_advance_uv(ctypes.byref(cg), tab, dts, stream)
         N.check(rc, "wrf_advance_uv")
         ctx.save_for_backward(*tensors)
@@ -273,8 +308,8 @@ class AdvanceUV(torch.autograd.Function):
         gv = bars["v"] if gv is None else gv.contiguous()
         tab = _table(named)
         btab = _table({"u": gu, "v": gv, **bars})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gu.device):
+        stream = _stream(gu)
+        with _on(gu):
             rc = N.lib().wrf_advance_uv_adj(ctypes.byref(ctx.cg), tab, btab, ctx.dts, stream)
         N.check(rc, "wrf_advance_uv_adj")
         return (None, gu, gv) + tuple(bars[k] for k in UV_INPUTS[2:]) + (None,) * len(UV_DATA)
@@ -316,8 +351,8 @@ class Forces(torch.autograd.Function):
         cg.cf1, cg.cf2, cg.cf3, cg.cfn, cg.cfn1 = cf1, cf2, cf3, cfn, cfn1
         outs = {k: named[k].detach().clone() for k in FORCES_OUTPUTS}
         tab = _table({**named, **outs})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(outs["ph_tend"].device):
+        stream = _stream(outs["ph_tend"])
+        with _on(outs["ph_tend"]):
             rc = N.lib().wrf_forces(ctypes.byref(cg), tab, terms, stream)
         N.check(rc, "wrf_forces")
         ctx.save_for_backward(*tensors)
@@ -329,8 +364,8 @@ class Forces(torch.autograd.Function):
         tensors = ctx.saved_tensors
         named = dict(zip(FORCES_INPUTS + FORCES_DATA, tensors))
         bars = _bars(named, FORCES_INPUTS, dict(zip(FORCES_OUTPUTS, gouts)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(bars["u"].device):
+        stream = _stream(bars["u"])
+        with _on(bars["u"]):
             rc = N.lib().wrf_forces_adj(ctypes.byref(ctx.cg), _table(named), _table(bars), ctx.terms, stream)
         N.check(rc, "wrf_forces_adj")
         return (None,) + tuple(bars[k] for k in FORCES_INPUTS) + (None,) * len(FORCES_DATA)
@@ -367,8 +402,8 @@ class Sumflux(torch.autograd.Function):
         named = dict(zip(SF_INPUTS + SF_DATA, tensors))
         cg = scalar_grid(named["u"].shape, float(scal[2]), float(scal[3]))
         outs = {k: named[k].detach().clone() for k in SF_INPUTS[:3]}
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(named["u"].device):
+        stream = _stream(named["u"])
+        with _on(named["u"]):
             rc = N.lib().wrf_sumflux(ctypes.byref(cg), _table({**named, **outs}), iteration, nsub, stream)
         N.check(rc, "wrf_sumflux")
         ctx.save_for_backward(*tensors)
@@ -379,8 +414,8 @@ class Sumflux(torch.autograd.Function):
     def backward(ctx, *gouts):
         named = dict(zip(SF_INPUTS + SF_DATA, ctx.saved_tensors))
         bars = _bars(named, SF_INPUTS, dict(zip(SF_INPUTS[:3], gouts)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(bars["u"].device):
+        stream = _stream(bars["u"])
+        with _on(bars["u"]):
             rc = N.lib().wrf_sumflux_adj(ctypes.byref(ctx.cg), _table(named), _table(bars), ctx.it[0], ctx.it[1],
                                          stream)
         N.check(rc, "wrf_sumflux_adj")
@@ -403,8 +438,8 @@ class SpecUpdate(torch.autograd.Function):
         shape = field.shape if field.dim() == 3 else (12,) + tuple(field.shape)
         cg = scalar_grid(shape, float(scal[2]), float(scal[3]))
         out = field.detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_spec_bdyupdate(ctypes.byref(cg), _ptr(out), _ptr(tend), dt, var.encode(), stream)
         N.check(rc, "wrf_spec_bdyupdate")
         ctx.cg, ctx.dt, ctx.var = cg, dt, var
@@ -414,8 +449,8 @@ class SpecUpdate(torch.autograd.Function):
     def backward(ctx, gout):
         gout = gout.contiguous()
         tb = torch.zeros_like(gout)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gout.device):
+        stream = _stream(gout)
+        with _on(gout):
             rc = N.lib().wrf_spec_bdyupdate_adj(ctypes.byref(ctx.cg), _ptr(gout), _ptr(tb), ctx.dt, ctx.var.encode(),
                                                 stream)
         N.check(rc, "wrf_spec_bdyupdate_adj")
@@ -440,8 +475,8 @@ class SpecUpdatePh(torch.autograd.Function):
         named = dict(zip(SPH_INPUTS, tensors))
         cg = scalar_grid(named["ph"].shape, float(scal[1]), float(scal[2]))
         out = named["ph"].detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(out.device):
+        stream = _stream(out)
+        with _on(out):
             rc = N.lib().wrf_spec_bdyupdate_ph(ctypes.byref(cg), _table({**named, "ph": out}), float(scal[0]), stream)
         N.check(rc, "wrf_spec_bdyupdate_ph")
         ctx.save_for_backward(*tensors)
@@ -452,8 +487,8 @@ class SpecUpdatePh(torch.autograd.Function):
     def backward(ctx, gout):
         named = dict(zip(SPH_INPUTS, ctx.saved_tensors))
         bars = _bars(named, SPH_INPUTS, {"ph": gout})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gout.device):
+        stream = _stream(gout)
+        with _on(gout):
             rc = N.lib().wrf_spec_bdyupdate_ph_adj(ctypes.byref(ctx.cg), _table(named), _table(bars), ctx.dt, stream)
         N.check(rc, "wrf_spec_bdyupdate_ph_adj")
         return (None,) + tuple(bars[k] for k in SPH_INPUTS)
@@ -488,8 +523,8 @@ class Prep(torch.autograd.Function):
         named = dict(zip(PREP_FIELDS + PREP_DATA, tensors))
         cg = scalar_grid(named["u"].shape, float(scal[1]), float(scal[2]))
         outs = {k: named[k].detach().clone() for k in PREP_OUTPUTS}
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(named["u"].device):
+        stream = _stream(named["u"])
+        with _on(named["u"]):
             rc = N.lib().wrf_prep(ctypes.byref(cg), _table({**named, **outs}), ops, stream)
         N.check(rc, "wrf_prep")
         ctx.save_for_backward(*tensors)
@@ -500,8 +535,8 @@ class Prep(torch.autograd.Function):
     def backward(ctx, *gouts):
         named = dict(zip(PREP_FIELDS + PREP_DATA, ctx.saved_tensors))
         bars = _bars(named, PREP_FIELDS, dict(zip(PREP_OUTPUTS, gouts)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(bars["u"].device):
+        stream = _stream(bars["u"])
+        with _on(bars["u"]):
             rc = N.lib().wrf_prep_adj(ctypes.byref(ctx.cg), _table(named), _table(bars), ctx.ops, stream)
         N.check(rc, "wrf_prep_adj")
         return (None,) + tuple(bars[k] for k in PREP_FIELDS) + (None,) * len(PREP_DATA)
@@ -529,8 +564,8 @@ class Halo(torch.autograd.Function):
         shape = (12,) + tuple(field.shape) if two_d else field.shape
         cg = scalar_grid(shape, float(scal[1]), float(scal[2]))
         out = field.detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_halo(ctypes.byref(cg), _ptr(out), var.encode(), int(two_d), stream)
         N.check(rc, "wrf_halo")
         ctx.cg, ctx.var, ctx.two_d = cg, var, two_d
@@ -540,8 +575,8 @@ class Halo(torch.autograd.Function):
     def backward(ctx, gout):
         gout = gout.contiguous()
         gin = torch.zeros_like(gout)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gout.device):
+        stream = _stream(gout)
+        with _on(gout):
             rc = N.lib().wrf_halo_adj(ctypes.byref(ctx.cg), _ptr(gout), _ptr(gin), ctx.var.encode(), int(ctx.two_d),
                                       stream)
         N.check(rc, "wrf_halo_adj")
@@ -561,8 +596,8 @@ class ZeroGradW(torch.autograd.Function):
         _cuda_only(w)
         cg = scalar_grid(w.shape, float(scal[0]), float(scal[1]))
         out = w.detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(w.device):
+        stream = _stream(w)
+        with _on(w):
             rc = N.lib().wrf_zero_grad_w(ctypes.byref(cg), _ptr(out), stream)
         N.check(rc, "wrf_zero_grad_w")
         ctx.cg = cg
@@ -572,8 +607,8 @@ class ZeroGradW(torch.autograd.Function):
     def backward(ctx, gout):
         gout = gout.contiguous()
         gin = torch.zeros_like(gout)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gout.device):
+        stream = _stream(gout)
+        with _on(gout):
             rc = N.lib().wrf_zero_grad_w_adj(ctypes.byref(ctx.cg), _ptr(gout), _ptr(gin), stream)
         N.check(rc, "wrf_zero_grad_w_adj")
         return None, gin
@@ -608,8 +643,8 @@ class Halos(torch.autograd.Function):
                 vs.append(var)
                 td.append(int(a.dim() == 2))
         n = len(pi)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(ins[0].device):
+        stream = _stream(ins[0])
+        with _on(ins[0]):
             rc = getattr(N.lib(), name)(ctypes.byref(cg), n, (ctypes.c_void_p * n)(*pi), (ctypes.c_void_p * n)(*po),
                                         "".join(vs).encode(), (ctypes.c_int * n)(*td), stream)
         N.check(rc, name)
@@ -651,49 +686,6 @@ def halos(fields: Sequence[torch.Tensor], letters: str, rdx=1.0 / 9000.0, rdy=1.
     return Halos.apply((letters, rdx, rdy), *fields)
 
 
-class AdvectMoist(torch.autograd.Function):
-    """The advection of qv .. qg (slots 1..6 of a [7, nz, ny, nx] array) by
-    (ru, rv, rom), as the step's advect_tend: zero outside the advected
-    points (pywrf/wrf_dynamics.py:3982-4051)."""
-
-    @staticmethod
-    def forward(ctx, moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx: float, rdy: float):
-        _cuda_only(moist, ru, rv, rom, msftx, fnm, fnp, rdnw)
-        cg = scalar_grid(ru.shape, rdx, rdy)
-        out = torch.zeros_like(moist)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(moist.device):
-            rc = N.lib().wrf_advect_moist(ctypes.byref(cg), _ptr(moist), _ptr(out), _ptr(ru), _ptr(rv), _ptr(rom),
-                                          _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw), stream)
-        N.check(rc, "wrf_advect_moist")
-        ctx.save_for_backward(moist, ru, rv, rom, msftx, fnm, fnp, rdnw)
-        ctx.cg = cg
-        return out
-
-    @staticmethod
-    def backward(ctx, gout):
-        moist, ru, rv, rom, msftx, fnm, fnp, rdnw = ctx.saved_tensors
-        gout = gout.contiguous()
-        qb, rub, rvb, romb = _zeros(moist, ru, ru, ru)
-        n = ctypes.c_size_t(0)
-        N.check(N.lib().wrf_advect_scalar_adj_work(ctypes.byref(ctx.cg), ctypes.byref(n)), "work")
-        work = torch.empty(int(n.value), dtype=torch.float32, device=moist.device)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(moist.device):
-            for m in range(1, 7):  # the species share the fluxes' cotangents
-                rc = N.lib().wrf_advect_scalar_adj(ctypes.byref(ctx.cg), _ptr(moist[m]), _ptr(ru), _ptr(rv),
-                                                   _ptr(rom), _ptr(msftx), _ptr(fnm), _ptr(fnp), _ptr(rdnw),
-                                                   _ptr(gout[m]), _ptr(qb[m]), _ptr(rub), _ptr(rvb), _ptr(romb),
-                                                   _ptr(work), n, stream)
-                N.check(rc, "wrf_advect_scalar_adj")
-        return qb, rub, rvb, romb, None, None, None, None, None, None
-
-
-def advect_moist(moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx, rdy):
-    """Differentiable moisture advection on the GPU (:class:`AdvectMoist`)."""
-    return AdvectMoist.apply(moist, ru, rv, rom, msftx, fnm, fnp, rdnw, rdx, rdy)
-
-
 AW_INPUTS = ("w", "rw_tend", "ww", "w_save", "u", "v", "muave", "muts", "mut", "t_2ave", "t_2", "t_1", "ph", "ph_1",
              "phb", "ph_tend", "ht", "c2a", "cqw", "alt", "a", "alpha", "gamma")
 AW_DATA = ("msftx", "msfty", "fnm", "fnp", "rdnw", "rdn")
@@ -718,8 +710,8 @@ class AdvanceW(torch.autograd.Function):
         cg.epssm, cg.cf1, cg.cf2, cg.cf3 = epssm, cf1, cf2, cf3
         outs = {k: named[k].detach().clone() for k in AW_OUTPUTS}
         tab = _table({_AW_FIELD.get(k, k): v for k, v in {**named, **outs}.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(outs["w"].device):
+        stream = _stream(outs["w"])
+        with _on(outs["w"]):
             rc = N.lib().wrf_advance_w(ctypes.byref(cg), tab, dts, stream)
         N.check(rc, "wrf_advance_w")
         ctx.save_for_backward(*tensors)
@@ -734,8 +726,8 @@ class AdvanceW(torch.autograd.Function):
         work = torch.empty_like(named["ht"])
         tab = _table({_AW_FIELD.get(k, k): v for k, v in named.items()})
         btab = _table({_AW_FIELD.get(k, k): v for k, v in bars.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(work.device):
+        stream = _stream(work)
+        with _on(work):
             rc = N.lib().wrf_advance_w_adj(ctypes.byref(ctx.cg), tab, btab, ctx.dts, _ptr(work), stream)
         N.check(rc, "wrf_advance_w_adj")
         return (None,) + tuple(bars[k] for k in AW_INPUTS) + (None,) * len(AW_DATA)
@@ -774,8 +766,8 @@ class AdvanceMuT(torch.autograd.Function):
         cg.epssm = epssm
         outs = {k: named[k].detach().clone() for k in MUT_OUTPUTS}
         tab = _table({_MUT_FIELD.get(k, k): v for k, v in {**named, **outs}.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(outs["ww"].device):
+        stream = _stream(outs["ww"])
+        with _on(outs["ww"]):
             rc = N.lib().wrf_advance_mu_t(ctypes.byref(cg), tab, dts, stream)
         N.check(rc, "wrf_advance_mu_t")
         ctx.save_for_backward(*tensors)
@@ -790,8 +782,8 @@ class AdvanceMuT(torch.autograd.Function):
         work = torch.empty_like(named["ww"])
         tab = _table({_MUT_FIELD.get(k, k): v for k, v in named.items()})
         btab = _table({_MUT_FIELD.get(k, k): v for k, v in bars.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(work.device):
+        stream = _stream(work)
+        with _on(work):
             rc = N.lib().wrf_advance_mu_t_adj(ctypes.byref(ctx.cg), tab, btab, ctx.dts, ctx.ref_no_grad, _ptr(work),
                                               stream)
         N.check(rc, "wrf_advance_mu_t_adj")
@@ -828,8 +820,8 @@ class CalcPRho(torch.autograd.Function):
         cg.smdiv = smdiv
         outs = {k: named[k].detach().clone() for k in ("al", "p", "pm1")}
         tab = _table({_PRHO_FIELD.get(k, k): v for k, v in {**named, **outs}.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(outs["p"].device):
+        stream = _stream(outs["p"])
+        with _on(outs["p"]):
             rc = N.lib().wrf_calc_p_rho(ctypes.byref(cg), tab, step, stream)
         N.check(rc, "wrf_calc_p_rho")
         ctx.save_for_backward(*tensors)
@@ -845,8 +837,8 @@ class CalcPRho(torch.autograd.Function):
         bars = {k: v for k, v in allb.items() if k not in out_b}
         tab = _table({_PRHO_FIELD.get(k, k): v for k, v in named.items()})
         btab = _table({_PRHO_FIELD.get(k, k): v for k, v in {**out_b, **bars}.items()})
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(named["p"].device):
+        stream = _stream(named["p"])
+        with _on(named["p"]):
             rc = N.lib().wrf_calc_p_rho_adj(ctypes.byref(ctx.cg), tab, btab, ctx.step, stream)
         N.check(rc, "wrf_calc_p_rho_adj")
         allb = {**out_b, **bars}
@@ -873,9 +865,9 @@ class RelaxBdytend(torch.autograd.Function):
         # the frame's minimum depth, and the library relaxes one level
         cg = scalar_grid((12, ny, nx) if variable == "m" else field.shape, 1.0 / 9000.0, 1.0 / 9000.0)
         out = tendency.detach().clone()
-        arr = (ctypes.c_void_p * 8)(*[_ptr(b).value for b in bdy8])
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        arr = (ctypes.c_void_p * 8)(*[_ptr(b) for b in bdy8])
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_relax_bdytend(ctypes.byref(cg), _ptr(field), _ptr(out), arr, variable.encode(),
                                            float(dtbc), stream)
         N.check(rc, "wrf_relax_bdytend")
@@ -888,8 +880,8 @@ class RelaxBdytend(torch.autograd.Function):
     def backward(ctx, gout):
         gout = gout.contiguous()
         fb = torch.zeros(ctx.shape, dtype=torch.float32, device=ctx.device)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(ctx.device):
+        stream = _stream(fb)
+        with _on(fb):
             rc = N.lib().wrf_relax_bdytend_adj(ctypes.byref(ctx.cg), _ptr(gout), _ptr(fb), ctx.variable.encode(),
                                                stream)
         N.check(rc, "wrf_relax_bdytend_adj")
@@ -907,13 +899,13 @@ class VSolveW(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, a, alpha, gamma):
-        _cuda_only(x, a, alpha, gamma)
+        ptrs = [_ptr(t) for t in (x, a, alpha, gamma)]
         nz = x.shape[0]
         ncol = x.numel() // nz
         w = torch.empty_like(x)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(x.device):
-            rc = N.lib().wrf_vsolve_w(ncol, nz, _ptr(x), _ptr(a), _ptr(alpha), _ptr(gamma), _ptr(w), stream)
+        stream = _stream(x)
+        with _on(x):
+            rc = N.lib().wrf_vsolve_w(ncol, nz, *ptrs, w.data_ptr(), stream)
         N.check(rc, "wrf_vsolve_w")
         ctx.save_for_backward(x, a, alpha, gamma)
         return w
@@ -925,8 +917,8 @@ class VSolveW(torch.autograd.Function):
         ncol = x.numel() // nz
         gw = gw.contiguous()
         gx, ga, gal, gg = _zeros(x, x, x, x)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(x.device):
+        stream = _stream(x)
+        with _on(x):
             rc = N.lib().wrf_vsolve_w_adj(ncol, nz, _ptr(x), _ptr(a), _ptr(alpha), _ptr(gamma), _ptr(gw), _ptr(gx),
                                           _ptr(ga), _ptr(gal), _ptr(gg), stream)
         N.check(rc, "wrf_vsolve_w_adj")
@@ -947,15 +939,16 @@ class CoefW(torch.autograd.Function):
         # checks hand out zeros from one shared buffer) instead of one
         # zero-filled tensor each, which backward would then clone
         ctx.set_materialize_grads(False)
-        _cuda_only(mut, cqw, c2a, rdn, rdnw)
+        ptrs = [_ptr(t) for t in (mut, cqw, c2a, rdn, rdnw)]
         cg = scalar_grid(cqw.shape, rdx, rdy)
         cg.epssm = float(epssm)
         cg.top_lid = int(bool(top_lid))
-        a, alpha, gamma = (torch.zeros_like(cqw) for _ in range(3))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(cqw.device):
-            rc = N.lib().wrf_coef_w(ctypes.byref(cg), _ptr(mut), _ptr(cqw), _ptr(c2a), _ptr(rdn), _ptr(rdnw),
-                                    float(dts), _ptr(a), _ptr(alpha), _ptr(gamma), stream)
+        a, alpha, gamma = (torch.empty_like(cqw) for _ in range(3))
+        torch._foreach_zero_([a, alpha, gamma])  # one launch
+        stream = _stream(cqw)
+        with _on(cqw):
+            rc = N.lib().wrf_coef_w(ctypes.byref(cg), *ptrs, float(dts), a.data_ptr(), alpha.data_ptr(),
+                                    gamma.data_ptr(), stream)
         N.check(rc, "wrf_coef_w")
         ctx.save_for_backward(mut, cqw, c2a, rdn, rdnw)
         ctx.cg, ctx.dts = cg, float(dts)
@@ -968,8 +961,8 @@ class CoefW(torch.autograd.Function):
         ga = z if ga is None else ga.contiguous()
         galpha = z if galpha is None else galpha.contiguous()
         ggamma = z if ggamma is None else ggamma.contiguous()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(cqw.device):
+        stream = _stream(cqw)
+        with _on(cqw):
             rc = N.lib().wrf_coef_w_adj(ctypes.byref(ctx.cg), _ptr(mut), _ptr(cqw), _ptr(c2a), _ptr(rdn), _ptr(rdnw),
                                         ctx.dts, _ptr(ga), _ptr(galpha), _ptr(ggamma), _ptr(mb), _ptr(cb), _ptr(c2b),
                                         stream)
@@ -1077,8 +1070,8 @@ class _TableOp(torch.autograd.Function):
         _cuda_only(*tensors)
         named = dict(zip(op.fields + op.data, tensors))
         outs = {k: named[k].detach().clone() for k in op.outputs}
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(tensors[0].device):
+        stream = _stream(tensors[0])
+        with _on(tensors[0]):
             N.check(op.fwd(cg, _table({**named, **outs}), stream), op.name)
         ctx.save_for_backward(*tensors)
         ctx.op, ctx.cg = op, cg
@@ -1090,8 +1083,8 @@ class _TableOp(torch.autograd.Function):
         saved = ctx.saved_tensors  # read once (checkpoint unpacks each saved tensor once)
         named = dict(zip(op.fields + op.data, saved))
         bars = _bars(named, op.fields, dict(zip(op.outputs, gouts)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(saved[0].device):
+        stream = _stream(saved[0])
+        with _on(saved[0]):
             N.check(op.adj(ctx.cg, _table(named), _table(bars), stream), op.name + "_adj")
         return (None, None) + tuple(bars[k] for k in op.fields) + (None,) * len(op.data)
 
@@ -1170,8 +1163,8 @@ class _Chain(torch.autograd.Function):
         kept = {}     # id of a kept tensor -> its place among the saved ones
         saved, places = [], []
         own = set()   # ids of this chain's tensors that nothing has kept
-        with torch.cuda.device(tensors[0].device):
-            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with _on(tensors[0]):
+            stream = _stream(tensors[0])
             for op in ops:
                 at = []
                 for k in op.reads:
@@ -1197,7 +1190,7 @@ class _Chain(torch.autograd.Function):
                     own.add(id(v))
         ctx.save_for_backward(*saved)
         ctx.ops, ctx.cg, ctx.names, ctx.outs, ctx.places = ops, cg, names, outs, places
-        ctx.device = tensors[0].device
+        ctx.device = tensors[0].get_device()
         return tuple(st[k] for k in outs)
 
     @staticmethod
@@ -1208,7 +1201,7 @@ class _Chain(torch.autograd.Function):
             if gk is not None:
                 bars[k] = gk.contiguous().clone()
         with torch.cuda.device(ctx.device):
-            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            stream = torch.cuda.current_stream(ctx.device).cuda_stream
             for op, at in zip(reversed(ctx.ops), reversed(ctx.places)):
                 op.backward(ctx.cg, {k: saved[q] for k, q in zip(op.reads, at)}, bars, stream)
         need = ctx.needs_input_grad[4:]
@@ -1285,11 +1278,10 @@ def _spec_tend_op(tend, bt: dict, var):
 def _relax_op(field, tend, bdy: dict, var, dtbc):
     """tend += relax_bdytend(field); 'm' (mu) is 2-D: the library relaxes one
     level of it."""
-    arr = (ctypes.c_void_p * 8)(*[_ptr(bdy[k]).value for k in BDY_NAMES])
-    keep = [bdy[k] for k in BDY_NAMES]
+    arrays = [bdy[k] for k in BDY_NAMES]
 
     def fwd(cg, st, out, stream):
-        assert keep
+        arr = (ctypes.c_void_p * 8)(*[_ptr(v) for v in arrays])
         _rc(N.lib().wrf_relax_bdytend(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), arr, var.encode(),
                                       float(dtbc), stream), "wrf_relax_bdytend")
 
@@ -1326,11 +1318,12 @@ def _advect_work(cg, name, like):
 
 def _advect_momentum_op(component, field, tend, data: dict):
     msf = data[("msfux", "msfvy", "msftx")[component]]
-    m2 = _ptr(data["msfvx"]) if component == 1 else None
+    msf2 = data["msfvx"] if component == 1 else None
     rdz = data["rdn" if component == 2 else "rdnw"]
     fnm, fnp = data["fnm"], data["fnp"]
 
     def fwd(cg, st, out, stream):
+        m2 = None if msf2 is None else _ptr(msf2)
         _rc(N.lib().wrf_advect_momentum(ctypes.byref(cg), component, _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
                                         _ptr(st["rv"]), _ptr(st["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
                                         _ptr(rdz), 0, stream), "wrf_advect_momentum")
@@ -1339,6 +1332,7 @@ def _advect_momentum_op(component, field, tend, data: dict):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
+        m2 = None if msf2 is None else _ptr(msf2)
         work, n = _advect_work(cg, "wrf_advect_momentum_adj_work", saved[field])
         _rc(N.lib().wrf_advect_momentum_adj(ctypes.byref(cg), component, _ptr(saved[field]), _ptr(saved["ru"]),
                                             _ptr(saved["rv"]), _ptr(saved["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
@@ -1350,11 +1344,11 @@ def _advect_momentum_op(component, field, tend, data: dict):
 
 
 def _advect_scalar_op(field, tend, data: dict):
-    const = [_ptr(data[k]) for k in ("msftx", "fnm", "fnp", "rdnw")]
+    const = [data[k] for k in ("msftx", "fnm", "fnp", "rdnw")]
 
     def fwd(cg, st, out, stream):
         _rc(N.lib().wrf_advect_scalar(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
-                                      _ptr(st["rv"]), _ptr(st["ww"]), *const, stream), "wrf_advect_scalar")
+                                      _ptr(st["rv"]), _ptr(st["ww"]), *map(_ptr, const), stream), "wrf_advect_scalar")
 
     def bwd(cg, saved, bars, stream):
         if bars.get(tend) is None:
@@ -1362,7 +1356,7 @@ def _advect_scalar_op(field, tend, data: dict):
         b = bars.need(saved)
         work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved[field])
         _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved[field]), _ptr(saved["ru"]), _ptr(saved["rv"]),
-                                          _ptr(saved["ww"]), *const, _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
+                                          _ptr(saved["ww"]), *map(_ptr, const), _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
                                           _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n, stream),
             "wrf_advect_scalar_adj")
 
@@ -1370,15 +1364,16 @@ def _advect_scalar_op(field, tend, data: dict):
 
 
 def _advect_moist_op(data: dict):
-    """advect_tend = the moisture's advection by the averaged fluxes, which
-    carry no cotangent past the update they feed (:class:`AdvectMoist`)."""
-    const = [_ptr(data[k]) for k in ("msftx", "fnm", "fnp", "rdnw")]
+    """advect_tend = the advection of qv .. qg (slots 1..6) by the averaged
+    fluxes, zero outside the advected points (pywrf/wrf_dynamics.py:
+    3982-4051)."""
+    const = [data[k] for k in ("msftx", "fnm", "fnp", "rdnw")]
     fluxes = ("ru_m", "rv_m", "ww_m")
 
     def fwd(cg, st, out, stream):
         out["advect_tend"].zero_()
         _rc(N.lib().wrf_advect_moist(ctypes.byref(cg), _ptr(st["moist"]), _ptr(out["advect_tend"]),
-                                     *[_ptr(st[k]) for k in fluxes], *const, stream), "wrf_advect_moist")
+                                     *[_ptr(st[k]) for k in fluxes], *map(_ptr, const), stream), "wrf_advect_moist")
 
     def bwd(cg, saved, bars, stream):
         gk = bars.pop("advect_tend", None)
@@ -1388,7 +1383,7 @@ def _advect_moist_op(data: dict):
         work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved["ru_m"])
         for m in range(1, 7):
             _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved["moist"][m]),
-                                              *[_ptr(saved[k]) for k in fluxes], *const, _ptr(gk[m]),
+                                              *[_ptr(saved[k]) for k in fluxes], *map(_ptr, const), _ptr(gk[m]),
                                               _ptr(b["moist"][m]), *[_ptr(b[k]) for k in fluxes], _ptr(work), n,
                                               stream), "wrf_advect_scalar_adj")
 
@@ -1399,13 +1394,12 @@ def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
     """tend += horizontal_diffusion(field); ``field`` "moist": its six
     species into the slots of ``tend``."""
     const = {k: data[k] for k in HDIFF_DATA}
-    bp = None if base is None else _ptr(base)
 
     def each(v):
         return [v[m] for m in range(1, 7)] if v.dim() == 4 else [v]
 
     def fwd(cg, st, out, stream):
-        tab = _table(const)
+        tab, bp = _table(const), None if base is None else _ptr(base)
         for f, o in zip(each(st[field]), each(out[tend])):
             _rc(N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp, _ptr(st[mass]),
                                                  _ptr(st[visc]), _ptr(o), stream), "wrf_horizontal_diffusion")
@@ -1414,7 +1408,7 @@ def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
-        tab = _table(const)
+        tab, bp = _table(const), None if base is None else _ptr(base)
         for f, gk, fb in zip(each(saved[field]), each(bars[tend]), each(b[field])):
             _rc(N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp,
                                                      _ptr(saved[mass]), _ptr(saved[visc]), _ptr(gk), _ptr(fb),
@@ -1633,8 +1627,8 @@ class SpecBdytend(torch.autograd.Function):
         shape = (12,) + tuple(tend.shape) if tend.dim() == 2 else tend.shape
         cg = scalar_grid(shape, float(scal[1]), float(scal[2]))
         out = tend.detach().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(tend.device):
+        stream = _stream(tend)
+        with _on(tend):
             rc = N.lib().wrf_spec_bdytend(ctypes.byref(cg), _ptr(out), _ptr(txs), _ptr(txe), _ptr(tys), _ptr(tye),
                                           var.encode(), stream)
         N.check(rc, "wrf_spec_bdytend")
@@ -1644,8 +1638,8 @@ class SpecBdytend(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         gin = gout.contiguous().clone()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(gin.device):
+        stream = _stream(gin)
+        with _on(gin):
             rc = N.lib().wrf_spec_bdytend_adj(ctypes.byref(ctx.cg), _ptr(gin), ctx.var.encode(), stream)
         N.check(rc, "wrf_spec_bdytend_adj")
         return None, gin, None, None, None, None
@@ -1676,9 +1670,9 @@ class HorizontalDiffusion(torch.autograd.Function):
         cg = scalar_grid(field.shape, float(scal[1]), float(scal[2]))
         out = tend.detach().clone()
         tab = _table(dict(zip(HDIFF_DATA, maps)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        stream = _stream(field)
         bp = None if base is None else _ptr(base)
-        with torch.cuda.device(field.device):
+        with _on(field):
             rc = N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, var.encode(), _ptr(field), bp, _ptr(mut),
                                                   _ptr(xk), _ptr(out), stream)
         N.check(rc, "wrf_horizontal_diffusion")
@@ -1695,9 +1689,9 @@ class HorizontalDiffusion(torch.autograd.Function):
         gout = gout.contiguous()
         fb, mb, kb = _zeros(field, mut, xk)
         tab = _table(dict(zip(HDIFF_DATA, maps)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        stream = _stream(field)
         bp = None if base is None else _ptr(base)
-        with torch.cuda.device(field.device):
+        with _on(field):
             rc = N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(ctx.cg), tab, ctx.var.encode(), _ptr(field), bp,
                                                       _ptr(mut), _ptr(xk), _ptr(gout), _ptr(fb), _ptr(mb), _ptr(kb),
                                                       stream)
@@ -1711,60 +1705,6 @@ def horizontal_diffusion(var: str, field, tend, mut, xk, data: dict, rdx, rdy, b
     return HorizontalDiffusion.apply((var, rdx, rdy), field, tend, mut, xk, base, *[data[k] for k in HDIFF_DATA])
 
 
-class MoistDiffusion(torch.autograd.Function):
-    """tend' = tend + horizontal_diffusion of qv .. qg (slots 1..6 of [7, nz,
-    ny, nx] arrays) with the column mass and eddy viscosity they share;
-    ``scal`` = (rdx, rdy), then the seven map factors of HDIFF_DATA."""
-
-    @staticmethod
-    def forward(ctx, scal, moist, tend, mut, xk, *maps):
-        _cuda_only(moist, tend, mut, xk, *maps)
-        cg = scalar_grid(xk.shape, float(scal[0]), float(scal[1]))
-        out = tend.detach().clone()
-        tab = _table(dict(zip(HDIFF_DATA, maps)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(moist.device):
-            for m in range(1, 7):
-                rc = N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, b"m", _ptr(moist[m]), None, _ptr(mut),
-                                                      _ptr(xk), _ptr(out[m]), stream)
-                N.check(rc, "wrf_horizontal_diffusion")
-        ctx.cg = cg
-        ctx.save_for_backward(moist, mut, xk, *maps)
-        return out
-
-    @staticmethod
-    def backward(ctx, gout):
-        moist, mut, xk, *maps = ctx.saved_tensors
-        gout = gout.contiguous()
-        fb, mb, kb = _zeros(moist, mut, xk)
-        tab = _table(dict(zip(HDIFF_DATA, maps)))
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(moist.device):
-            for m in range(1, 7):  # the species share the mass's and the viscosity's cotangents
-                rc = N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(ctx.cg), tab, b"m", _ptr(moist[m]), None,
-                                                          _ptr(mut), _ptr(xk), _ptr(gout[m]), _ptr(fb[m]), _ptr(mb),
-                                                          _ptr(kb), stream)
-                N.check(rc, "wrf_horizontal_diffusion_adj")
-        return (None, fb, gout, mb, kb) + (None,) * len(HDIFF_DATA)
-
-
-class PutSlot(torch.autograd.Function):
-    """A [7, nz, ny, nx] array with one slot replaced by a field."""
-
-    @staticmethod
-    def forward(ctx, slot: int, moist, field):
-        out = moist.detach().clone()
-        out[slot].copy_(field)
-        ctx.slot = slot
-        return out
-
-    @staticmethod
-    def backward(ctx, gout):
-        gm = gout.clone()
-        gm[ctx.slot].zero_()
-        return None, gm, gout[ctx.slot].contiguous()
-
-
 class MassWeight(torch.autograd.Function):
     """out = field * mut on levels below nk of the mass points, zero elsewhere
     (mass_weight, pywrf/wrf_boundary.py:408-414); ``scal`` = (nk, rdx, rdy)."""
@@ -1775,8 +1715,8 @@ class MassWeight(torch.autograd.Function):
         nk = int(scal[0])
         cg = scalar_grid(field.shape, float(scal[1]), float(scal[2]))
         out = torch.zeros_like(field)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             N.check(N.lib().wrf_mass_weight(ctypes.byref(cg), _ptr(field), _ptr(mut), _ptr(out), nk, stream),
                     "wrf_mass_weight")
         ctx.cg, ctx.nk = cg, nk
@@ -1788,8 +1728,8 @@ class MassWeight(torch.autograd.Function):
         field, mut = ctx.saved_tensors
         gout = gout.contiguous()
         fb, mb = _zeros(field, mut)
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        with torch.cuda.device(field.device):
+        stream = _stream(field)
+        with _on(field):
             rc = N.lib().wrf_mass_weight_adj(ctypes.byref(ctx.cg), _ptr(field), _ptr(mut), _ptr(gout), _ptr(fb),
                                              _ptr(mb), ctx.nk, stream)
         N.check(rc, "wrf_mass_weight_adj")
@@ -1958,10 +1898,11 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
 def _relax_qv_ops(nz: int, bdy: dict, dtbc: float) -> list:
     """qv's lateral relaxation and specified tendency into its slot of
     moist_tend (pywrf/solver.py:1600-1640)."""
-    arr = (ctypes.c_void_p * 8)(*[_ptr(bdy[k]).value for k in BDY_NAMES])
     L, by = N.lib(), ctypes.byref
+    arrays = [bdy[k] for k in BDY_NAMES]
 
     def fwd(cg, st, out, stream):
+        arr = (ctypes.c_void_p * 8)(*[_ptr(v) for v in arrays])
         tend = out["moist_tend"][1]
         mass = torch.zeros_like(tend)
         _rc(L.wrf_mass_weight(by(cg), _ptr(st["moist"][1]), _ptr(st["mut"]), _ptr(mass), nz - 1, stream),
