@@ -5,7 +5,8 @@
 // vabs, sel, val) runs both on float (the plain value) and on Dual<N> (the
 // value and N tangents at once).  Comparisons take the value, so branches and
 // selections follow the value path exactly: the derivative is that of the
-// branch taken.
+// branch taken.  Values round as the float code's; the tangents' products
+// and sums are fused, and a division by a constant is divc's.
 #pragma once
 #include "wrf_common.cuh"
 
@@ -60,7 +61,7 @@ __device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, const Dual<N>& b)
   Dual<N> r;
   r.v = a.v * b.v;
 #pragma unroll
-  for (int n = 0; n < N; ++n) r.d[n] = a.d[n] * b.v + a.v * b.d[n];
+  for (int n = 0; n < N; ++n) r.d[n] = fmaf(a.v, b.d[n], a.d[n] * b.v);
   return r;
 }
 template <int N>
@@ -69,7 +70,7 @@ __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, const Dual<N>& b)
   r.v = a.v / b.v;
   const float ib = 1.0f / b.v;
 #pragma unroll
-  for (int n = 0; n < N; ++n) r.d[n] = (a.d[n] - r.v * b.d[n]) * ib;
+  for (int n = 0; n < N; ++n) r.d[n] = fmaf(-r.v, b.d[n], a.d[n]) * ib;
   return r;
 }
 // mixed with a constant
@@ -117,8 +118,9 @@ template <int N>
 __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, float b) {
   Dual<N> r;
   r.v = a.v / b;
+  const float rb = __frcp_rn(b);
 #pragma unroll
-  for (int n = 0; n < N; ++n) r.d[n] = a.d[n] / b;
+  for (int n = 0; n < N; ++n) r.d[n] = divc(a.d[n], b, rb);
   return r;
 }
 template <int N>

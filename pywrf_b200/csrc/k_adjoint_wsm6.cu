@@ -13,13 +13,17 @@
 // interface fall speeds, departure cells and overlap remap.  The derivative
 // is that of the branch taken.
 //
-// The reverse product is taken in reverse mode: the column runs once on
-// taped scalars (tape.cuh), the outputs' cotangents seed the adjoints of
-// their entries, and one reverse sweep yields every input's cotangent.
-// With one time-split loop (split mode) the tape stops before the point
-// processes: those read only their own level, so each level's are reversed
-// on a thread of its own by forward-mode tangents and added into the
-// adjoints of the tape entries its inputs come from, before the sweep.
+// With one time-split loop (the ordinary case) only the sedimentation couples
+// the levels, so the block is reversed in two parts.  The masses that fall
+// are taped column by column (tape.cuh) in the columns that hold some.  All
+// else -- prep, the saturation ratios, melting, the point processes, finish --
+// is reversed per level on a thread of its own by forward-mode tangents with
+// respect to the level's nine inputs (temperature, vapour, cloud water,
+// pressure, density and the four fallen masses): the cotangents of the fallen
+// masses seed the tape, whose one reverse sweep gives the falling species'.
+// With several loops the whole column runs on taped scalars, the outputs'
+// cotangents seed the adjoints of their entries, and one reverse sweep yields
+// every input's cotangent.
 // Columns are taped in chunks that bound the tape's memory.  A column whose
 // tape outgrows the capacity is finished by forward-mode tangents instead:
 // the same code on Dual<N> numbers with N inputs seeded per pass, the
@@ -48,7 +52,10 @@ struct Col {
 enum {
   A_TIN, A_TH, A_PII, A_T, A_Q, A_QC, A_QI, A_QR, A_QS, A_QG, A_DEN, A_P, A_DELZ, A_CPM, A_XL, A_DENFAC, A_QS0,
   A_QS1, A_RH0, A_RH1, A_XNI, A_R1, A_R2, A_R3, A_W1, A_W2, A_ZI, A_WI, A_ZA, A_DZA, A_QA, A_QA2, A_WD, A_WWW,
-  A_SR3, A_SRS, A_COUNT
+  A_SR3, A_SRS, A_COUNT,
+  // with one time-split loop: the fallen cloud ice, and (float arrays in
+  // their slots) the level's temperature, Exner function, density and depth
+  A_RI = A_SR3, B_T = A_TIN, B_PII = A_TH, B_DEN = A_PII, B_DELZ = A_CPM
 };
 
 template <class T>
@@ -532,11 +539,42 @@ __device__ void point_processes(T& t, T& q, T& qc, T& qi, T& qr, T& qs, T& qg, c
   if (val(qi) <= F(QMIN)) qi = zero;
 }
 
+// melting of snow, then graupel (wrf_physics.py:415-470) at one level, and
+// rain's slope before it (the others' are read where they melt only)
+template <class T>
+__device__ void melt_level(T& t, T& qr, T& qs, T& qg, const T& den, const T& p, const T& cpm, Slope3<T>& sl,
+                           float dtcld) {
+  const float xlf = F(XLF0);
+  const bool warm = val(t) > F(T0C) && (val(qs) > 0.f || val(qg) > 0.f);
+  const T none = cst<T>(0.f);
+  slope3(qr, warm ? qs : none, warm ? qg : none, den, t, sl);
+  if (!warm) return;
+  const T n0s = val(qs) > 0.f ? n0sfac(t) : none;
+  const T work2 = venfac(p, t, den);
+  if (val(qs) > 0.f) {
+    const T coeres = sl.r2[1] * vsqrt(sl.rs[1] * sl.rb[1]);
+    T ps = xka(t, den) / xlf * (F(T0C) - t) * F(PI) / 2.0f * n0s *
+           (F(PRECS1) * sl.r2[1] + F(PRECS2) * work2 * coeres) / den;
+    ps = vmin(vmax(ps * dtcld / 1.0f, -qs / 1.0f), 0.0f);
+    qs = qs + ps;
+    qr = qr - ps;
+    t = t + xlf / cpm * ps;
+  }
+  if (val(qg) > 0.f) {
+    const T coeres = sl.r2[2] * vsqrt(sl.rs[2] * sl.rb[2]);
+    T pg = xka(t, den) / xlf * (F(T0C) - t) * (F(PRECG1) * sl.r2[2] + F(PRECG2) * work2 * coeres) / den;
+    pg = vmin(vmax(pg * dtcld / 1.0f, -qg / 1.0f), 0.0f);
+    qg = qg + pg;
+    qr = qr - pg;
+    t = t + xlf / cpm * pg;
+  }
+}
+
 // wsm6 (wrf_physics.py:137-1214) on one column of km levels: the arrays
 // A_T (temperature), A_Q, A_QC, A_QI, A_QR, A_QS, A_QG, A_DEN, A_P and
 // A_DELZ hold the inputs and receive the results
 template <class T>
-__device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead = false, bool stop_at_points = false) {
+__device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead = false) {
   for (int k = 0; k < km; ++k) {
     const T q = C(A_Q, k), t = C(A_T, k);
     C(A_CPM, k) = val(q) >= F(QMIN) ? F(CPV) * q + (1.0f - q) * F(CPD) : cst<T>(F(CPD * (1.0 - QMIN) + CPV * QMIN));
@@ -584,39 +622,14 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
     nislfv(C, km, 0, A_R1, -1, dtcld, 1);
     for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_W2, k);
     nislfv(C, km, 1, A_R2, A_R3, dtcld, 1);
-    const float xlf = F(XLF0);
     for (int k = 0; k < km; ++k) {
       const T den = C(A_DEN, k), p = C(A_P, k), cpm = C(A_CPM, k);
       T qr = vmax(C(A_R1, k) / den, 0.0f), qs = vmax(C(A_R2, k) / den, 0.0f), qg = vmax(C(A_R3, k) / den, 0.0f);
       T t = C(A_T, k);
-      // melting of snow, then graupel (elsewhere only rain's slope is read)
-      const bool warm = val(t) > F(T0C) && (val(qs) > 0.f || val(qg) > 0.f);
-      const T none = cst<T>(0.f);
       Slope3<T> sl;
-      slope3(qr, warm ? qs : none, warm ? qg : none, den, t, sl);
+      melt_level(t, qr, qs, qg, den, p, cpm, sl, dtcld);
       C(A_SR3, k) = sl.r3[0];
       C(A_SRS, k) = sl.rs[0];
-      if (warm) {
-        const T n0s = val(qs) > 0.f ? n0sfac(t) : none;
-        const T work2 = venfac(p, t, den);
-        if (val(qs) > 0.f) {
-          const T coeres = sl.r2[1] * vsqrt(sl.rs[1] * sl.rb[1]);
-          T ps = xka(t, den) / xlf * (F(T0C) - t) * F(PI) / 2.0f * n0s *
-                 (F(PRECS1) * sl.r2[1] + F(PRECS2) * work2 * coeres) / den;
-          ps = vmin(vmax(ps * dtcld / 1.0f, -qs / 1.0f), 0.0f);
-          qs = qs + ps;
-          qr = qr - ps;
-          t = t + xlf / cpm * ps;
-        }
-        if (val(qg) > 0.f) {
-          const T coeres = sl.r2[2] * vsqrt(sl.rs[2] * sl.rb[2]);
-          T pg = xka(t, den) / xlf * (F(T0C) - t) * (F(PRECG1) * sl.r2[2] + F(PRECG2) * work2 * coeres) / den;
-          pg = vmin(vmax(pg * dtcld / 1.0f, -qg / 1.0f), 0.0f);
-          qg = qg + pg;
-          qr = qr - pg;
-          t = t + xlf / cpm * pg;
-        }
-      }
       C(A_QR, k) = qr;
       C(A_QS, k) = qs;
       C(A_QG, k) = qg;
@@ -632,12 +645,6 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
       C(A_R1, k) = ice ? den * qi : cst<T>(0.f);
     }
     nislfv(C, km, 2, A_R1, -1, dtcld, 0);
-    if (stop_at_points) {
-      // (one time-split loop only) the point processes' inputs stay in the
-      // column arrays, cloud ice from its sedimented mass in A_QI
-      for (int k = 0; k < km; ++k) C(A_QI, k) = vmax(C(A_R1, k) / C(A_DEN, k), 0.0f);
-      return;
-    }
     for (int k = 0; k < km; ++k) {
       T t = C(A_T, k), q = C(A_Q, k), qc = C(A_QC, k), qr = C(A_QR, k), qs = C(A_QS, k), qg = C(A_QG, k);
       const T den = C(A_DEN, k);
@@ -783,7 +790,7 @@ __device__ __forceinline__ void put_input_cot(const Grid& g, const S& b, int c2,
 // cotangents are (or, after k_mp_tape_rev, will be) written: not when the
 // tape outgrew the capacity.
 __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, float dt, Tv* ws, TapeCtx tc,
-                                                        int c0, int nc, S vo, int* done, int* used, bool split) {
+                                                        int c0, int nc, S vo, int* done, int* used) {
   if (threadIdx.x == 0) g_tape = tc;
   __syncthreads();
   const int lane = tape_lane(), col = c0 + lane;
@@ -821,16 +828,6 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, 
   const Col<Tv> C{ws + lane, tc.stride, km + 1};
   tape_reserve(mp_inputs(g));
   prep_column(g, s, C, c2, [](int idx, float v) { return Tv{v, idx, 1.f}; });
-  if (split) {
-    // the point processes and finish are reversed per level by
-    // k_mp_points_adj, which seeds this tape's entries
-    wsm6_column(C, km, dt, false, true);
-    const int n = g_tape_n[threadIdx.x];
-    used[col] = n;
-    for (int k = 0; k < km; ++k) b[WF_H_DIABATIC][k * lev + c2] = 0.f;
-    if (n > tc.cap) done[col] = 0;
-    return;
-  }
   wsm6_column(C, km, dt);
   for (int k = 0; k < km; ++k) finish_level(C, k, dt);
   const int n = g_tape_n[threadIdx.x];
@@ -858,107 +855,334 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, 
   }
 }
 
-// The point processes and finish of one level of a column taped in split
-// mode, reversed by forward-mode tangents: one thread per (column, level)
-// reads the level's inputs from the column arrays k_mp_tape left (their
-// values, and the tape entries they are multiples of), evaluates the level
-// in Dual<N> arithmetic with N inputs seeded per pass, forms the inputs'
-// cotangents from the outputs' (yb: theta, qv .. qg, h_diabatic) and adds
-// them into the adjoints of those entries of the column's tape, which
-// k_mp_tape_rev then sweeps.  The level's processes read no other level, so
-// the chain a thread runs is one level's, not the column's.  Only the inputs
-// of the processes that are taped are seeded (packed over the passes: a
-// species that is absent is a constant); theta, its initial value and the
-// Exner function enter the finish alone, whose derivatives are written out.
-// vo (when its T is not null) receives the level's output values.
-constexpr int kPointInputs = 21, kPointSeeds = 18;
-template <int N>
-__global__ void __launch_bounds__(128) k_mp_points_adj(Grid g, S yb, Tv* ws, TapeCtx tc, int c0, int nc, S vo,
-                                                       const int* done, const int* used, float dt) {
+// ---- one time-split loop: the sedimentation on a tape, the rest per level
+
+// the level's values that the kernels below share (float arrays in the slots
+// of the column arrays)
+struct Base {
+  float* base;
+  int ncol, kst;
+  __device__ __forceinline__ float& operator()(int a, int k) const {
+    return base[(size_t)a * kst * ncol * (sizeof(Tv) / sizeof(float)) + (size_t)k * ncol];
+  }
+};
+__device__ __forceinline__ Base base_of(Tv* ws, int lane, int stride, int kst) {
+  return Base{reinterpret_cast<float*>(ws) + lane, stride, kst};
+}
+
+// the falling species that a column holds at some level
+enum { FALL_RAIN = 1, FALL_SNOW = 2, FALL_ICE = 4 };
+
+// moist_physics_prep_em of one level per thread (neighbouring threads take
+// neighbouring columns); flags[col] (zero on entry) collects the species that
+// fall.  Columns outside WSM6's block pass t and q through and set
+// h_diabatic to zero.
+__global__ void __launch_bounds__(128) k_mp_levels(Grid g, S s, S yb, S b, Tv* ws, int stride, int c0, int nc, S vo,
+                                                   int* flags) {
   const int km = g.nz - 1;
-  // neighbouring threads take neighbouring columns at one level: their
-  // column-array reads coalesce, and their branches mostly agree
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = (int)(t / nc), lane = (int)(t - (long long)k * nc);
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = (int)(x / nc), lane = (int)(x - (long long)k * nc);
   if (k >= km) return;
   const int col = c0 + lane;
-  const int n = used[col];
-  if (!done[col] || n == 0 || n > tc.cap) return;
   ColPos cp;
   col_pos(g, col, cp);
-  const Col<Tv> C{ws + lane, tc.stride, km + 1};
-  const int arr[kPointInputs] = {A_T,  A_Q,   A_QC,  A_QI,  A_QR,  A_QS,  A_QG,  A_DEN, A_P,  A_DENFAC, A_CPM,
-                                 A_XL, A_QS0, A_QS1, A_RH0, A_RH1, A_SR3, A_SRS, A_TIN, A_TH, A_PII};
-  Tv in[kPointInputs];
-#pragma unroll
-  for (int q = 0; q < kPointInputs; ++q) in[q] = C(arr[q], k);
   const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
-  const float yt = yb[WF_T][p], yh = yb[WF_H_DIABATIC][p];
+  if (!cp.run) {
+    b[WF_T][p] = yb[WF_T][p];
+    for (int m = 1; m < 7; ++m) b[WF_MOIST][m * n3 + p] = yb[WF_MOIST][m * n3 + p];
+    b[WF_H_DIABATIC][p] = 0.f;
+    if (vo[WF_T]) {
+      vo[WF_T][p] = s[WF_T][p];
+      for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = s[WF_MOIST][m * n3 + p];
+      vo[WF_H_DIABATIC][p] = 0.f;
+    }
+    return;
+  }
+  const Base B = base_of(ws, lane, stride, km + 1);
+  const float pii = wpow((s[WF_P][p] + s[WF_PB][p]) / (float)P0, F(RCP));
+  B(B_PII, k) = pii;
+  B(B_T, k) = (s[WF_T][p] + (float)T0) * pii;
+  B(B_DEN, k) = 1.0f / (s[WF_AL][p] + s[WF_ALB][p]);
+  B(B_DELZ, k) = (s[WF_PH][p + lev] + s[WF_PHB][p + lev]) / (float)G - (s[WF_PH][p] + s[WF_PHB][p]) / (float)G;
+  const float* q = s[WF_MOIST];
+  const int f = (q[3 * n3 + p] > 0.f ? FALL_RAIN : 0) | (q[5 * n3 + p] > 0.f || q[6 * n3 + p] > 0.f ? FALL_SNOW : 0) |
+                (q[4 * n3 + p] > 0.f ? FALL_ICE : 0);
+  if (f) atomicOr(&flags[col], f);
+}
+
+// the inputs of a column's sedimentation tape, km levels each
+enum { I_T, I_DEN, I_DELZ, I_QR, I_QI, I_QS, I_QG, I_COUNT };
+
+// The sedimentation of the columns that hold falling species, taped: one
+// thread per column, the species' fallen masses (den q; zero for a species
+// that the column does not hold) left in A_R1 (rain), A_R2 (snow), A_R3
+// (graupel) and A_RI.  used[col] holds the column's flags on entry and
+// receives the entries its tape took, 0 without a tape; done[col] whether
+// the column's cotangents will be written by the kernels that follow: not
+// when the tape outgrew the capacity.  The rest of the column's taped code
+// (saturation ratios, melting) went to the per-level tangents: a third of
+// the entries, and none at all in columns where nothing falls.
+__global__ void __launch_bounds__(kTapeBlock) k_mp_fall(Grid g, S s, float dt, Tv* ws, TapeCtx tc, int c0, int nc,
+                                                        int* done, int* used) {
+  if (threadIdx.x == 0) g_tape = tc;
+  __syncthreads();
+  const int lane = tape_lane(), col = c0 + lane;
+  ColPos cp;
+  if (lane >= nc || !col_pos(g, col, cp)) return;
+  const int flags = used[col], km = g.nz - 1;
+  used[col] = 0;
+  const bool room = tc.cap >= mp_inputs(g);
+  done[col] = room || !cp.run;
+  if (!cp.run || !flags || !room) return;
+  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3();
+  const bool rain = flags & FALL_RAIN, snow = flags & FALL_SNOW, ice = flags & FALL_ICE;
+  const Col<Tv> C{ws + lane, tc.stride, km + 1};
+  const Base B = base_of(ws, lane, tc.stride, km + 1);
+  const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
+  const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
+  tape_reserve(I_COUNT * km);
+  auto in = [&](int f, int k, float v) { return Tv{v, f * km + k, 1.f}; };
+  const Tv none = cst<Tv>(0.f);
+  for (int k = 0; k < km; ++k) {
+    const size_t p = k * lev + cp.c2;
+    const float* q = s[WF_MOIST] + p;
+    const Tv t = in(I_T, k, B(B_T, k)), den = in(I_DEN, k, B(B_DEN, k));
+    const Tv qr = vmax(in(I_QR, k, q[3 * n3]), 0.0f), qi = vmax(in(I_QI, k, q[4 * n3]), 0.0f);
+    const Tv qs = vmax(in(I_QS, k, q[5 * n3]), 0.0f), qg = vmax(in(I_QG, k, q[6 * n3]), 0.0f);
+    C(A_T, k) = t;
+    C(A_DEN, k) = den;
+    C(A_DELZ, k) = in(I_DELZ, k, B(B_DELZ, k));
+    const Tv denfac = rain || snow ? vsqrt(1.0f / den * F(DEN0)) : none;
+    C(A_DENFAC, k) = denfac;
+    C(A_W1, k) = rain ? vt_of(0, qr, den, denfac, t) : none;
+    const Tv qsum = vmax(qs + qg, 1.0e-15f);
+    C(A_W2, k) = snow && val(qsum) > 1.0e-15f
+                     ? (vt_of(1, qs, den, denfac, t) * qs + vt_of(2, qg, den, denfac, t) * qg) / qsum
+                     : none;
+    C(A_R1, k) = rain ? den * qr : none;
+    C(A_R2, k) = snow ? den * qs : none;
+    C(A_R3, k) = snow ? den * qg : none;
+    C(A_RI, k) = ice ? den * qi : none;
+    // cloud ice's speed (of this level alone) waits in A_XNI
+    Tv wi = none;
+    if (val(qi) > 0.f) {
+      const Tv xni = vmin(vmax(5.387e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+      const Tv wt = vmax(vmin(F(DICON) * vsqrt(den * qi / xni), F(DIMAX)), 1.0e-25f);
+      wi = 1.49e4f * vexp(vlog(wt) * 1.31f);
+    }
+    C(A_XNI, k) = wi;
+  }
+  if (rain) nislfv(C, km, 0, A_R1, -1, dtcld, 1);
+  if (snow) {
+    for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_W2, k);
+    nislfv(C, km, 1, A_R2, A_R3, dtcld, 1);
+  }
+  if (ice) {
+    for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_XNI, k);
+    nislfv(C, km, 2, A_RI, -1, dtcld, 0);
+  }
+  const int n = g_tape_n[threadIdx.x];
+  used[col] = n;
+  if (n > tc.cap) done[col] = 0;
+}
+
+// All but the sedimentation of one level, reversed by forward-mode tangents:
+// one thread per (column, level) evaluates the level in Dual<N> arithmetic
+// with N of its nine inputs seeded per pass -- temperature, vapour, cloud
+// water, pressure, density and the fallen masses -- forms their cotangents
+// from the outputs' (yb: theta, qv .. qg, h_diabatic), adds those of the
+// fallen masses into the adjoints of the tape entries they come from, and
+// writes prep's inputs' cotangents (the falling species' own are the tape's).
+// vo (when its T is not null) receives the level's output values.
+//
+// The evaluation is a chain of powers, divisions and selections: what counts
+// is how often it runs.  Only inputs that can act are seeded, packed over the
+// passes (nine at most, where the saturation ratios, slopes and heat
+// capacities as inputs of their own made eighteen), and a level with nothing
+// to condense, freeze or fall runs it not at all: its derivatives are the
+// identity.
+enum { X_T, X_Q, X_QC, X_P, X_DEN, X_RR, X_RS, X_RG, X_RI, X_COUNT };
+template <int N>
+__global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, Tv* ws, TapeCtx tc, int c0, int nc,
+                                                       S vo, const int* done, const int* used, float dt) {
+  const int km = g.nz - 1;
+  const long long xt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = (int)(xt / nc), lane = (int)(xt - (long long)k * nc);
+  if (k >= km) return;
+  const int col = c0 + lane;
+  ColPos cp;
+  col_pos(g, col, cp);
+  if (!cp.run || !done[col]) return;
+  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
+  const Base B = base_of(ws, lane, tc.stride, km + 1);
+  const float pfull = s[WF_P][p] + s[WF_PB][p], tin = s[WF_T][p], pii = B(B_PII, k);
+  float v[X_COUNT];
+  v[X_T] = B(B_T, k);
+  v[X_Q] = s[WF_MOIST][n3 + p];
+  v[X_QC] = s[WF_MOIST][2 * n3 + p];
+  v[X_P] = pfull;
+  v[X_DEN] = B(B_DEN, k);
+  Tv fall[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) fall[q] = cst<Tv>(0.f);
+  if (used[col] > 0) {
+    const Col<Tv> C{ws + lane, tc.stride, km + 1};
+    fall[0] = C(A_R1, k);
+    fall[1] = C(A_R2, k);
+    fall[2] = C(A_R3, k);
+    fall[3] = C(A_RI, k);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[X_RR + q] = fall[q].v;
+  const float yt = yb[WF_T][p];
   float ym[7];
 #pragma unroll
   for (int m = 1; m < 7; ++m) ym[m] = yb[WF_MOIST][m * n3 + p];
-  float cot[kPointInputs];
+  const float th = tin + (float)T0, rp = 1.0f / pii;
+  // moist_physics_finish_em: mpten = t / pii - th is added to theta and
+  // gives h_diabatic = mpten / dt
+  const float ympten = yt + yb[WF_H_DIABATIC][p] / dt;
+  float qs0, qs1;
+  fpvs(v[X_T], pfull, qs0, qs1);
+  const float qm = vmax(v[X_Q], F(QMIN));
+  // no hydrometeors, no condensation; no nucleation of ice
+  const bool dry = v[X_QC] <= 0.f && v[X_RR] == 0.f && v[X_RS] == 0.f && v[X_RG] == 0.f && v[X_RI] == 0.f;
+  const bool no_ice = qm <= qs1 || v[X_T] >= F(T0C);
+  const bool quiet = dry && no_ice && qm < qs0;
+  float cot[X_COUNT];
 #pragma unroll
-  for (int q = 0; q < kPointInputs; ++q) cot[q] = 0.f;
-  // the time-split loop's step (one loop: dt itself up to the split step)
-  const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
-  const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
-  using D = Dual<N>;
-  int seeds = 0;  // the taped inputs, as a bit mask
-#pragma unroll
-  for (int q = 0; q < kPointSeeds; ++q) seeds |= in[q].id >= 0 && in[q].s != 0.f ? 1 << q : 0;
-  const bool values = vo[WF_T] != nullptr;
-  for (int pass = 0; pass == 0 || seeds; ++pass) {
-    int at[N];  // the inputs seeded in this pass
-#pragma unroll
-    for (int d = 0; d < N; ++d) {
-      at[d] = seeds ? __ffs(seeds) - 1 : -1;
-      seeds &= seeds - 1;
+  for (int q = 0; q < X_COUNT; ++q) cot[q] = 0.f;
+  float tout = v[X_T];
+  if (quiet) {
+    cot[X_Q] = ym[1];
+    const float rden = 1.0f / v[X_DEN];
+    cot[X_RR] = ym[3] * rden;
+    cot[X_RS] = ym[5] * rden;
+    cot[X_RG] = ym[6] * rden;
+    if (vo[WF_T]) {
+      vo[WF_MOIST][n3 + p] = v[X_Q];
+      for (int m = 2; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = 0.f;
     }
-    D x[kPointSeeds];
+  } else {
+    // the time-split loop's step (one loop: dt itself up to the split step)
+    const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
+    const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
+    using D = Dual<N>;
+    int seeds = 1 << X_T | 1 << X_Q | 1 << X_P;
+    if (!(v[X_QC] < 0.f)) seeds |= 1 << X_QC;
+    if (!(dry && no_ice)) seeds |= 1 << X_DEN;
 #pragma unroll
-    for (int q = 0; q < kPointSeeds; ++q) {
-      x[q] = dconst<N>(in[q].v);
+    for (int q = 0; q < 4; ++q)
+      if (fall[q].id >= 0) seeds |= 1 << (X_RR + q);
+#pragma unroll 1
+    for (int pass = 0; seeds; ++pass) {
+      int at[N];  // the inputs seeded in this pass
 #pragma unroll
-      for (int d = 0; d < N; ++d) x[q].d[d] = q == at[d] ? 1.f : 0.f;
-    }
-    D tt = x[0], qv = x[1], qc = x[2], qi = x[3], qr = x[4], qs = x[5], qg = x[6];
-    Slope3<D> sl0;
-    sl0.r3[0] = x[16];
-    sl0.rs[0] = x[17];
-    point_processes(tt, qv, qc, qi, qr, qs, qg, x[7], x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15], sl0, dtcld);
-    // moist_physics_finish_em at the level: mpten = t / pii - th is added to
-    // theta and gives h_diabatic = mpten / dt
-    const float rp = 1.0f / in[20].v, ympten = yt + yh / dt;
+      for (int d = 0; d < N; ++d) {
+        at[d] = seeds ? __ffs(seeds) - 1 : -1;
+        seeds &= seeds - 1;
+      }
+      auto seed = [&](int q) {
+        D x = dconst<N>(v[q]);
 #pragma unroll
-    for (int d = 0; d < N; ++d) {
-      const float v = ympten * (tt.d[d] * rp) + ym[1] * qv.d[d] + ym[2] * qc.d[d] + ym[3] * qr.d[d] +
-                      ym[4] * qi.d[d] + ym[5] * qs.d[d] + ym[6] * qg.d[d];
+        for (int d = 0; d < N; ++d) x.d[d] = q == at[d] ? 1.f : 0.f;
+        return x;
+      };
+      D t = seed(X_T), q = seed(X_Q), qc = vmax(seed(X_QC), 0.0f);
+      const D pp = seed(X_P), den = seed(X_DEN);
+      const D cpm = val(q) >= F(QMIN) ? F(CPV) * q + (1.0f - q) * F(CPD) : cst<D>(F(CPD * (1.0 - QMIN) + CPV * QMIN));
+      const D xl = F(XLV0) - F(XLV1) * (t - F(T0C));
+      const D denfac = vsqrt(1.0f / den * F(DEN0));
+      D s0, s1;
+      fpvs(t, pp, s0, s1);
+      const D rh0 = vmax(q / s0, F(QMIN)), rh1 = vmax(q / s1, F(QMIN));
+      D qr = vmax(seed(X_RR) / den, 0.0f), qs = vmax(seed(X_RS) / den, 0.0f), qg = vmax(seed(X_RG) / den, 0.0f);
+      Slope3<D> sl0;
+      melt_level(t, qr, qs, qg, den, pp, cpm, sl0, dtcld);
+      D qi = vmax(seed(X_RI) / den, 0.0f);
+      point_processes(t, q, qc, qi, qr, qs, qg, den, pp, denfac, cpm, xl, s0, s1, rh0, rh1, sl0, dtcld);
 #pragma unroll
-      for (int q = 0; q < kPointSeeds; ++q)
-        if (q == at[d]) cot[q] = v;
-    }
-    if (pass == 0) {
-      const float mpten = tt.v / in[20].v - in[19].v;
-      cot[18] = yt;
-      cot[19] = -ympten;
-      cot[20] = -ympten * (tt.v * rp) * rp;
-      if (values) {
-        vo[WF_T][p] = in[18].v + mpten;
-        vo[WF_H_DIABATIC][p] = mpten / dt;
-        const float mv[7] = {0.f, qv.v, qc.v, qr.v, qi.v, qs.v, qg.v};
-        for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = mv[m];
+      for (int d = 0; d < N; ++d) {
+        const float c = ympten * (t.d[d] * rp) + ym[1] * q.d[d] + ym[2] * qc.d[d] + ym[3] * qr.d[d] +
+                        ym[4] * qi.d[d] + ym[5] * qs.d[d] + ym[6] * qg.d[d];
+#pragma unroll
+        for (int e = 0; e < X_COUNT; ++e)
+          if (e == at[d]) cot[e] = c;
+      }
+      if (pass == 0) {
+        tout = t.v;
+        if (vo[WF_T]) {
+          const float mv[7] = {0.f, q.v, qc.v, qr.v, qi.v, qs.v, qg.v};
+          for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = mv[m];
+        }
       }
     }
+    // prep: the cotangents through the temperature th pii and the Exner
+    // function
+    const float cpii = fmaf(cot[X_T], th, -ympten * (tout * rp) * rp);
+    b[WF_P][p] += cot[X_P] + cpii * (F(RCP) * pii / pfull);
+    b[WF_AL][p] -= cot[X_DEN] * (v[X_DEN] * v[X_DEN]);
   }
+  if (vo[WF_T]) {
+    const float mpten = tout / pii - th;
+    vo[WF_T][p] = tin + mpten;
+    vo[WF_H_DIABATIC][p] = mpten / dt;
+  }
+  b[WF_T][p] = quiet ? yt : yt + fmaf(cot[X_T], pii, -ympten);
+  b[WF_MOIST][n3 + p] = cot[X_Q];
+  b[WF_MOIST][2 * n3 + p] = cot[X_QC];
 #pragma unroll
-  for (int q = 0; q < kPointInputs; ++q)
-    if (in[q].id >= 0 && cot[q] != 0.f) atomicAdd(tc.adj(in[q].id, lane), cot[q] * in[q].s);
+  for (int m = 3; m < 7; ++m) b[WF_MOIST][m * n3 + p] = 0.f;
+  b[WF_H_DIABATIC][p] = 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (fall[q].id >= 0 && cot[X_RR + q] != 0.f) atomicAdd(tc.adj(fall[q].id, lane), cot[X_RR + q] * fall[q].s);
+}
+
+// the reverse sweep of the sedimentation's tapes: the inputs' cotangents into
+// the adjoints of entries [0, I_COUNT km)
+constexpr int kSweepBlock = 32, kSweepWindow = 16, kSweepRing = 64;
+__global__ void __launch_bounds__(kSweepBlock) k_mp_fall_rev(Grid g, TapeCtx tc, int c0, int nc, const int* used) {
+  __shared__ float acc[kSweepRing * kSweepBlock];
+  const int lane = blockIdx.x * blockDim.x + threadIdx.x;
+  if (lane >= nc) return;
+  const int n = used[c0 + lane];
+  if (n == 0 || n > tc.cap) return;
+  tape_sweep<kSweepWindow, kSweepRing, kSweepBlock>(tc, lane, I_COUNT * (g.nz - 1), n, acc);
+}
+
+// and from there through prep, one level per thread
+__global__ void __launch_bounds__(128) k_mp_fall_inputs(Grid g, S s, S b, Tv* ws, TapeCtx tc, int c0, int nc,
+                                                        const int* used) {
+  const int km = g.nz - 1;
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = (int)(x / nc), lane = (int)(x - (long long)k * nc);
+  if (k > km) return;
+  const int col = c0 + lane, n = used[col];
+  if (n == 0 || n > tc.cap) return;
+  ColPos cp;
+  col_pos(g, col, cp);
+  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
+  auto a = [&](int f, int kk) { return *tc.adj(f * km + kk, lane); };
+  const float below = k > 0 ? a(I_DELZ, k - 1) : 0.f;
+  if (k == km) {
+    b[WF_PH][p] += below / (float)G;
+    return;
+  }
+  const Base B = base_of(ws, lane, tc.stride, km + 1);
+  const float at = a(I_T, k), aden = a(I_DEN, k), adz = a(I_DELZ, k), den = B(B_DEN, k);
+  b[WF_T][p] += at * B(B_PII, k);
+  b[WF_P][p] += at * (B(B_T, k) * F(RCP) / (s[WF_P][p] + s[WF_PB][p]));
+  b[WF_AL][p] -= aden * (den * den);
+  b[WF_PH][p] += (below - adz) / (float)G;
+  b[WF_MOIST][3 * n3 + p] += a(I_QR, k);
+  b[WF_MOIST][4 * n3 + p] += a(I_QI, k);
+  b[WF_MOIST][5 * n3 + p] += a(I_QS, k);
+  b[WF_MOIST][6 * n3 + p] += a(I_QG, k);
 }
 
 // the reverse sweep of the tapes k_mp_tape left (same chunk and lanes):
 // the inputs' cotangents from the adjoints of entries [0, n_inputs)
-constexpr int kSweepBlock = 128, kSweepWindow = 16, kSweepRing = 64;
 __global__ void __launch_bounds__(kSweepBlock) k_mp_tape_rev(Grid g, S b, TapeCtx tc, int c0, int nc,
                                                              const int* used) {
   __shared__ float acc[kSweepRing * kSweepBlock];
@@ -1023,9 +1247,9 @@ __global__ void __launch_bounds__(64) k_mp_tangent(Grid g, S s, S yb, S b, float
 namespace {
 
 constexpr int kMpDirections = 8;
-// entries a column's tape may take per level by default (per time-split
-// loop of the whole column; of the column-coupled part in split mode), and
-// the memory the tapes of one chunk of columns may take
+// entries a column's tape may take per level by default (of the
+// sedimentation with one time-split loop, of the whole column per loop with
+// several), and the memory the tapes of one chunk of columns may take
 constexpr int kTapeEntriesPerLevel = 480, kTapeSplitPerLevel = 256;
 constexpr size_t kTapeChunkBytes = size_t(24) << 30;
 // the capacity set through set_microphysics_tape_capacity (0: default)
@@ -1044,8 +1268,6 @@ MpAdjWork mp_adj_work(const Grid& g) {
   MpAdjWork w;
   const int km = g.nz - 1;
   w.ncol = (g.ide - 1 - (g.ids + 1)) * (g.jde - 1 - (g.jds + 1));
-  // the tape holds the column-coupled part in split mode (one time-split
-  // loop), the whole column once per loop otherwise
   const int nloop = (int)fmaxf(g.dt / F(mp::DTCLDCR), 1.0f);
   const int per_level = nloop == 1 ? kTapeSplitPerLevel : kTapeEntriesPerLevel * nloop;
   w.cap = g_tape_capacity > 0 ? std::min(kTapeMaxEntries, g_tape_capacity)
@@ -1097,20 +1319,24 @@ int launch_physics_adj(const Grid& g, const S& s, const S& post, const S& b, flo
   tc.stride = w.width;
   tc.cap = w.cap;
   auto* cols = reinterpret_cast<Tv*>(work + w.cols);
-  // one time-split loop: the point processes are reversed per level
   const bool split = (int)fmaxf(dt / F(mp::DTCLDCR), 1.0f) == 1;
-  const int km = g.nz - 1;
   for (int c0 = 0; c0 < w.ncol; c0 += w.width) {
     const int nc = std::min(w.width, w.ncol - c0);
-    mpt::k_mp_tape<<<(nc + kTapeBlock - 1) / kTapeBlock, kTapeBlock, 0, st>>>(g, s, yb, b, dt, cols, tc, c0, nc, vo,
-                                                                               done, used, split);
+    const unsigned columns = (nc + kTapeBlock - 1) / kTapeBlock, sweeps = (nc + mpt::kSweepBlock - 1) / mpt::kSweepBlock;
     if (split) {
-      const long long nt = (long long)nc * km;
-      mpt::k_mp_points_adj<4><<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(g, yb, cols, tc, c0, nc, vo, done, used, dt);
-      ++n;
+      const unsigned levels = (unsigned)(((long long)nc * (g.nz - 1) + 127) / 128);
+      cudaMemsetAsync(used + c0, 0, nc * sizeof(int), st);
+      mpt::k_mp_levels<<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc.stride, c0, nc, vo, used);
+      mpt::k_mp_fall<<<columns, kTapeBlock, 0, st>>>(g, s, dt, cols, tc, c0, nc, done, used);
+      mpt::k_mp_levels_adj<4><<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, dt);
+      mpt::k_mp_fall_rev<<<sweeps, mpt::kSweepBlock, 0, st>>>(g, tc, c0, nc, used);
+      mpt::k_mp_fall_inputs<<<(unsigned)(((long long)nc * g.nz + 127) / 128), 128, 0, st>>>(g, s, b, cols, tc, c0, nc,
+                                                                                            used);
+      n += 5;
+      continue;
     }
-    mpt::k_mp_tape_rev<<<(nc + mpt::kSweepBlock - 1) / mpt::kSweepBlock, mpt::kSweepBlock, 0, st>>>(g, b, tc, c0, nc,
-                                                                                                    used);
+    mpt::k_mp_tape<<<columns, kTapeBlock, 0, st>>>(g, s, yb, b, dt, cols, tc, c0, nc, vo, done, used);
+    mpt::k_mp_tape_rev<<<sweeps, mpt::kSweepBlock, 0, st>>>(g, b, tc, c0, nc, used);
     n += 2;
   }
   // the columns whose tape outgrew the capacity, by tangent passes
