@@ -53,8 +53,7 @@
 //                        difference to it, dpn the vertical pressure average
 //                        of the two columns); v likewise in y.  The point
 //                        kernel gathers the 3-D cotangents from the u and v
-//                        points whose stencils hold the point (forming of
-//                        each only the factors that reach the point), the column
+//                        points whose stencils hold the point, the column
 //                        kernel sums the 2-D ones (muu, muv, mu, mudf) over
 //                        the levels.  The cotangents of u and v pass through
 //                        (du'/du = 1).
@@ -148,6 +147,11 @@ static void allow_smem(K kernel, size_t bytes) {
 }
 
 namespace {
+
+// x += v by a reduction at the memory side: a cotangent that the kernel only
+// adds to is not loaded (nor do the loads that follow wait for the store).
+// Each has one writer per kernel, so the order is fixed.
+__device__ __forceinline__ void add_to(float& x, float v) { atomicAdd(&x, v); }
 
 // dPhi/dq at stencil offset o = m - f of a 5th-order face (o in [-3, 2]),
 // Phi = (37(q0+qm1) - 8(qp1+qm2) + (qp2+qm3))/60 - s ((qp2-qm3) - 5(qp1-qm2) + 10(q0-qm1))/60
@@ -278,7 +282,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
       if (ord == 5) phi = flux5(Qv(p, -3, nx), Qv(p, -2, nx), Qv(p, -1, nx), Qv(p, 0, nx), Qv(p, 1, nx), Qv(p, 2, nx), r);
       else if (ord == 3) phi = flux3(Qv(p, -2, nx), Qv(p, -1, nx), Qv(p, 0, nx), Qv(p, 1, nx), r);
       else phi = 0.5f * (Qv(p, 0, nx) + Qv(p, -1, nx));
-      rvbar[p] += fb * phi;
+      add_to(rvbar[p], fb * phi);
     }
   }
   {  // x face f = i at (k, j)
@@ -293,7 +297,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
       if (ord == 5) phi = flux5(Qv(p, -3, 1), Qv(p, -2, 1), Qv(p, -1, 1), Qv(p, 0, 1), Qv(p, 1, 1), Qv(p, 2, 1), rs);
       else if (ord == 3) phi = flux3(Qv(p, -2, 1), Qv(p, -1, 1), Qv(p, 0, 1), Qv(p, 1, 1), rs);
       else phi = 0.5f * (Qv(p, 0, 1) + Qv(p, -1, 1));
-      rubar[p] += fb * phi;
+      add_to(rubar[p], fb * phi);
     }
   }
   {  // vertical face kf = k at (j, i)
@@ -308,7 +312,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
       if (ord == 5) phi = flux5(Qv(p, -3, st), Qv(p, -2, st), Qv(p, -1, st), Qv(p, 0, st), Qv(p, 1, st), Qv(p, 2, st), -r);
       else if (ord == 3) phi = flux3(Qv(p, -2, st), Qv(p, -1, st), Qv(p, 0, st), Qv(p, 1, st), -r);
       else phi = a.fnm[k] * Qv(p, 0, st) + a.fnp[k] * Qv(p, -1, st);
-      rombar[p] += fb * phi;
+      add_to(rombar[p], fb * phi);
     }
   }
 }
@@ -328,7 +332,7 @@ __global__ void k_advect_scalar_gather(Grid g, const float* Q, float* qbar) {
     if (i - o >= 0 && i - o < g.nx) aq += Q[(size_t)(1 * 6 + s) * n3 + (m - o)];
     if (k - o >= 0 && k - o < g.nz) aq += Q[(size_t)(2 * 6 + s) * n3 + (m - (long long)o * lev)];
   }
-  if (aq != 0.f) qbar[m] += aq;
+  if (aq != 0.f) add_to(qbar[m], aq);
 }
 
 // ------------------------------------------------------------ advance_uv
@@ -371,10 +375,10 @@ __device__ __forceinline__ float uv_dpn_coef(const Grid& g, const S& s, int kk, 
 // the factors of dp at an updated point of u (V = 0) or v (V = 1), the
 // cotangent ub of its new value and dpb = d L / d dp
 struct UvTerm {
-  float ub, dpb, A, B, Cf, C, D;
+  float ub, dpb, B, C;
 };
 
-template <bool kB = true, bool kD = true>
+template <bool kB>
 __device__ UvTerm uv_term(const Grid& g, const S& s, const S& b, float dts, int V, int k, int j, int i) {
   const size_t lev = (size_t)g.ny * g.nx;
   const size_t c = (size_t)j * g.nx + i, p = k * lev + c, no = V ? (size_t)g.nx : 1;
@@ -384,84 +388,154 @@ __device__ UvTerm uv_term(const Grid& g, const S& s, const S& b, float dts, int 
   const float* al = s[WF_AL];
   const float* pb = s[WF_PB];
   const float* php = s[WF_PHP];
-  const float* mu = s[WF_MU];
   const float r = V ? s[WF_MSFVY][c] / s[WF_MSFVX][c] : s[WF_MSFUX][c] / s[WF_MSFUY][c];
   const float rd = V ? g.rdy : g.rdx;
   UvTerm t;
   t.ub = b[V ? WF_V : WF_U][p];
   t.dpb = -dts * s[V ? WF_CQV : WF_CQU][p] * t.ub;
-  t.A = r * 0.5f * rd * s[V ? WF_MUV : WF_MUU][c];
   t.B = 0.f;
   if (kB)
     t.B = ((ph[p + lev] - ph[p + lev - no]) + (ph[p] - ph[p - no])) + (alt[p] + alt[p - no]) * (pp[p] - pp[p - no]) +
           (al[p] + al[p - no]) * (pb[p] - pb[p - no]);
-  t.Cf = r * rd;
-  t.C = t.Cf * (php[p] - php[p - no]);
-  t.D = 0.f;
-  if (kD)
-    t.D = s[WF_RDNW][k] * (uv_dpn(g, s, k + 1, c, c - no) - uv_dpn(g, s, k, c, c - no)) - 0.5f * (mu[c - no] + mu[c]);
+  t.C = r * rd * (php[p] - php[p - no]);
   return t;
 }
 
 }  // namespace
 
-__global__ void k_advance_uv_adj(Grid g, S s, S b, float dts) {
-  WRF_POINT_INDEX(g, k, j, i);
-  const int ktf = g.nz - 1, nx = g.nx;
-  const size_t lev = (size_t)g.ny * nx;
-  const size_t m = (size_t)k * lev + (size_t)j * nx + i;
-  if (k < ktf) {
-    if (uv_in(g, 0, j, i) || uv_spec(g, 0, j, i)) b[WF_RU_TEND][m] += dts * b[WF_U][m];
-    if (uv_in(g, 1, j, i) || uv_spec(g, 1, j, i)) b[WF_RV_TEND][m] += dts * b[WF_V][m];
+// A thread marches a chunk of levels of its column.  Four faces reach the
+// column (its own west and south, its east and north neighbours'), and a level
+// takes from the faces' levels k - 2 .. k + 1 only two sums over the faces: of
+// dpb A with sign (the phi differences of k - 1 and k) and of dpb C (the
+// pressure averages).  Each face's level is formed once as the march reaches
+// it and the sums are carried in registers, where a thread per point formed
+// sixteen face levels (their map-factor divisions included) and two more for
+// cqu and cqv: 372 us per launch at 240x240x41 and 61 us at 101x101x35, at a
+// memory floor of 50 and 8; 150 and 38 us now, with the
+// cotangents that it only adds to as reductions.
+constexpr int kUvChunk = 8;
+__global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float dts) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int nx = g.nx, ny = g.ny, ktf = g.nz - 1, lev = ny * nx;
+  if (i >= nx || j >= ny) return;
+  const int c = j * nx + i;
+  // the faces f = 2 V + e: P = the column itself (e = 0, sign +) or its
+  // neighbour (e = 1, sign -), Q = P's west (V = 0) or south (V = 1) column
+  bool on[4];
+  int cP[4], cQ[4];
+  float A[4], Cf[4], mm[4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const int V = f >> 1, e = f & 1, no = V ? nx : 1;
+    const int jP = j + V * e, iP = i + (1 - V) * e;
+    on[f] = jP < ny && iP < nx && uv_in(g, V, jP, iP);
+    cP[f] = c + e * no;
+    cQ[f] = cP[f] - no;
+    A[f] = Cf[f] = mm[f] = 0.f;
+    if (on[f]) {
+      const float r = V ? s[WF_MSFVY][cP[f]] / s[WF_MSFVX][cP[f]] : s[WF_MSFUX][cP[f]] / s[WF_MSFUY][cP[f]];
+      const float rd = V ? g.rdy : g.rdx;
+      A[f] = r * 0.5f * rd * s[V ? WF_MUV : WF_MUU][cP[f]];
+      Cf[f] = r * rd;
+      mm[f] = 0.5f * (s[WF_MU][cQ[f]] + s[WF_MU][cP[f]]);
+    }
   }
-  float aph = 0.f, aalt = 0.f, aal = 0.f, apb = 0.f, aphp = 0.f, ap = 0.f;
-  for (int V = 0; V < 2; ++V) {
-    const size_t no = V ? (size_t)nx : 1;
-    // the points P = (kP, j + V e, i + (1 - V) e), e = 0 (m is P's own
-    // column, sign +) or 1 (m is P's west / south neighbour, sign -)
-    for (int e = 0; e < 2; ++e) {
-      const int jP = j + V * e, iP = i + (1 - V) * e;
-      if (jP >= g.ny || iP >= nx || !uv_in(g, V, jP, iP)) continue;
-      const float sg = e == 0 ? 1.f : -1.f;
-      for (int kP = k - 2; kP <= k + 1; ++kP) {
-        if (kP < 0 || kP >= ktf) continue;
-        // B enters the gathered cotangents only through A (and the own
-        // point's cqu / cqv, below), D only at kP == k
-        const UvTerm t = kP == k ? uv_term<false, true>(g, s, b, dts, V, kP, jP, iP)
-                                 : uv_term<false, false>(g, s, b, dts, V, kP, jP, iP);
-        if (t.dpb == 0.f) continue;
-        const float Bb = t.dpb * t.A, Db = t.dpb * t.C;
-        const size_t P = (size_t)kP * lev + (size_t)jP * nx + iP;
-        if (kP == k || kP == k - 1) aph += sg * Bb;  // ph at kP and kP + 1
-        if (kP == k) {
-          aalt += Bb * (s[WF_P][P] - s[WF_P][P - no]);
-          aal += Bb * (s[WF_PB][P] - s[WF_PB][P - no]);
-          apb += sg * Bb * (s[WF_AL][P] + s[WF_AL][P - no]);
-          ap += sg * Bb * (s[WF_ALT][P] + s[WF_ALT][P - no]);
-          aphp += sg * t.dpb * t.Cf * t.D;
+  const bool tu = on[0] || uv_spec(g, 0, j, i), tv = on[2] || uv_spec(g, 1, j, i);
+  if (!(on[0] || on[1] || on[2] || on[3] || tu || tv)) return;
+  const float *php = s[WF_PHP], *pp = s[WF_P], *pb = s[WF_PB], *al = s[WF_AL], *alt = s[WF_ALT], *ph = s[WF_PH];
+  // dpb and C of the faces at level k, and the sums over the faces
+  struct Level {
+    float dpb[4], C[4], phi, dp;
+  };
+  auto level = [&](int k) {
+    Level v;
+    const bool in = k >= 0 && k < ktf;
+    v.phi = v.dp = 0.f;
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const int V = f >> 1;
+      v.dpb[f] = v.C[f] = 0.f;
+      if (in && on[f]) {
+        const int P = k * lev + cP[f];
+        v.dpb[f] = -dts * __ldg(&s[V ? WF_CQV : WF_CQU][P]) * __ldg(&b[V ? WF_V : WF_U][P]);
+        v.C[f] = Cf[f] * (__ldg(php + P) - __ldg(php + k * lev + cQ[f]));
+      }
+      v.phi += (f & 1 ? -1.f : 1.f) * (v.dpb[f] * A[f]);
+      v.dp += v.dpb[f] * v.C[f];
+    }
+    return v;
+  };
+  const int k0 = blockIdx.z * kUvChunk, k1 = min(k0 + kUvChunk, g.nz);
+  const float* rdnw = s[WF_RDNW];
+  const float *fnm = s[WF_FNM], *fnp = s[WF_FNP];
+  Level cur = level(k0 - 1);
+  float dp2 = level(k0 - 2).dp, dp1 = cur.dp, phi1 = cur.phi;
+  cur = level(k0);
+  // the sums of p over the faces' pairs at this level, and their averages
+  // dpn at the half level below it
+  float psum[4], dpn[4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    psum[f] = dpn[f] = 0.f;
+    if (on[f]) {
+      psum[f] = pp[k0 * lev + cP[f]] + pp[k0 * lev + cQ[f]];
+      dpn[f] = uv_dpn(g, s, k0, cP[f], cQ[f]);
+    }
+  }
+  for (int k = k0; k < k1; ++k) {
+    const int m = k * lev + c;
+    const Level next = level(k + 1);
+    float aph = cur.phi + phi1, aalt = 0.f, aal = 0.f, apb = 0.f, aphp = 0.f, ap = 0.f, cq[2] = {0.f, 0.f};
+    auto wt = [&](int kP) {
+      return kP < 0 || kP >= ktf ? 0.f : rdnw[kP] * (uv_dpn_coef(g, s, kP + 1, k) - uv_dpn_coef(g, s, kP, k));
+    };
+    ap = wt(k - 2) * dp2 + wt(k - 1) * dp1 + wt(k) * cur.dp + wt(k + 1) * next.dp;
+    if (k < ktf) {
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        if (!on[f]) continue;
+        const int V = f >> 1, P = k * lev + cP[f], Q = k * lev + cQ[f];
+        const float sg = f & 1 ? -1.f : 1.f, Bb = cur.dpb[f] * A[f];
+        const float up = __ldg(pp + P + lev) + __ldg(pp + Q + lev);
+        const float dn = k + 1 == ktf ? 0.f : 0.5f * (fnm[k + 1] * up + fnp[k + 1] * psum[f]);
+        const float D = rdnw[k] * (dn - dpn[f]) - mm[f];
+        psum[f] = up;
+        dpn[f] = dn;
+        const float pd = __ldg(pp + P) - __ldg(pp + Q), pbd = __ldg(pb + P) - __ldg(pb + Q);
+        const float als = __ldg(al + P) + __ldg(al + Q), alts = __ldg(alt + P) + __ldg(alt + Q);
+        aalt += Bb * pd;
+        aal += Bb * pbd;
+        apb += sg * Bb * als;
+        ap += sg * Bb * alts;
+        aphp += sg * cur.dpb[f] * Cf[f] * D;
+        if (!(f & 1)) {
+          const float B = ((__ldg(ph + P + lev) - __ldg(ph + Q + lev)) + (__ldg(ph + P) - __ldg(ph + Q))) + alts * pd +
+                          als * pbd;
+          cq[V] = -dts * (A[f] * B + cur.C[f] * D);
         }
-        // p through dpn(kP + 1) - dpn(kP) (both columns of the pair, sign +)
-        const float rw = s[WF_RDNW][kP] * Db;
-        ap += rw * (uv_dpn_coef(g, s, kP + 1, k) - uv_dpn_coef(g, s, kP, k));
+      }
+      if (tu) {
+        const float ub = __ldg(&b[WF_U][m]);
+        add_to(b[WF_RU_TEND][m], dts * ub);
+        if (on[0]) add_to(b[WF_CQU][m], cq[0] * ub);
+      }
+      if (tv) {
+        const float vb = __ldg(&b[WF_V][m]);
+        add_to(b[WF_RV_TEND][m], dts * vb);
+        if (on[2]) add_to(b[WF_CQV][m], cq[1] * vb);
       }
     }
+    if (aph != 0.f) add_to(b[WF_PH][m], aph);
+    if (aalt != 0.f) add_to(b[WF_ALT][m], aalt);
+    if (aal != 0.f) add_to(b[WF_AL][m], aal);
+    if (apb != 0.f) add_to(b[WF_PB][m], apb);
+    if (aphp != 0.f) add_to(b[WF_PHP][m], aphp);
+    if (ap != 0.f) add_to(b[WF_P][m], ap);
+    dp2 = dp1;
+    dp1 = cur.dp;
+    phi1 = cur.phi;
+    cur = next;
   }
-  if (k < ktf) {
-    if (uv_in(g, 0, j, i)) {
-      const UvTerm t = uv_term(g, s, b, dts, 0, k, j, i);
-      b[WF_CQU][m] += -dts * (t.A * t.B + t.C * t.D) * t.ub;
-    }
-    if (uv_in(g, 1, j, i)) {
-      const UvTerm t = uv_term(g, s, b, dts, 1, k, j, i);
-      b[WF_CQV][m] += -dts * (t.A * t.B + t.C * t.D) * t.ub;
-    }
-  }
-  if (aph != 0.f) b[WF_PH][m] += aph;
-  if (aalt != 0.f) b[WF_ALT][m] += aalt;
-  if (aal != 0.f) b[WF_AL][m] += aal;
-  if (apb != 0.f) b[WF_PB][m] += apb;
-  if (aphp != 0.f) b[WF_PHP][m] += aphp;
-  if (ap != 0.f) b[WF_P][m] += ap;
 }
 
 // the column sums by kColLevels level groups (threadIdx.y, levels ty,
@@ -486,8 +560,8 @@ __global__ void __launch_bounds__(32 * kColLevels) k_advance_uv_adj_col(Grid g, 
       const float em = V ? ev * s[WF_MSFVX_INV][cP] : eu / s[WF_MSFUY][cP];
 #pragma unroll 2
       for (int k = ty; k < ktf; k += kColLevels) {
-        const UvTerm t = e == 0 ? uv_term<true, false>(g, s, b, dts, V, k, jP, iP)
-                                : uv_term<false, false>(g, s, b, dts, V, k, jP, iP);
+        const UvTerm t = e == 0 ? uv_term<true>(g, s, b, dts, V, k, jP, iP)
+                                : uv_term<false>(g, s, b, dts, V, k, jP, iP);
         if (e == 0) {
           const float r = V ? s[WF_MSFVY][cP] / s[WF_MSFVX][cP] : s[WF_MSFUX][cP] / s[WF_MSFUY][cP];
           const float d = t.dpb * (r * 0.5f * (V ? g.rdy : g.rdx)) * t.B;
@@ -519,8 +593,9 @@ __global__ void __launch_bounds__(32 * kColLevels) k_advance_uv_adj_col(Grid g, 
 }
 
 int launch_advance_uv_adj(const Grid& g, const S& s, const S& b, float dts, cudaStream_t st) {
-  const dim3 b3(32, 4), b2(32, 8);
-  k_advance_uv_adj<<<point_grid(g, b3), b3, 0, st>>>(g, s, b, dts);
+  dim3 b3(32, 4), gr = point_grid(g, b3);
+  gr.z = (g.nz + kUvChunk - 1) / kUvChunk;
+  k_advance_uv_adj<<<gr, b3, 0, st>>>(g, s, b, dts);
   k_advance_uv_adj_col<<<dim3((g.nx + 31) / 32, g.ny), dim3(32, kColLevels), 0, st>>>(g, s, b, dts);
   return 2;
 }
@@ -1122,6 +1197,7 @@ size_t advance_w_adj_smem(const Grid& g) { return ((size_t)kAwArrays * g.nz * 32
 // the reference's order: t_2ave, wdwn, R, rhs, P and the explicit w x in
 // the column arrays, then the solve's two sweeps (y, z) on group 0, the
 // solve's coefficients staged first; ends with the block synchronised
+template <bool FIXED>
 struct AwLp {
   const Grid& g;
   const S& s;
@@ -1134,7 +1210,8 @@ struct AwLp {
   enum { T2A, WD, RR, RHS, PP, XX, YY, ZZ, ZB, YB, PB, RHSB };
   enum { CA = RHS, CAL = RHSB, CG = PB };
   __device__ float& A(int arr, int k) const { return sm[((size_t)arr * nz + k) * 32 + tx]; }
-  __device__ float F(int id, int k) const { return s[id][k * lev + c]; }
+  // FIXED: the kernel writes none of the state's fields
+  __device__ float F(int id, int k) const { return FIXED ? __ldg(&s[id][k * lev + c]) : s[id][k * lev + c]; }
   __device__ void forward() const {
     const float* rdnw = s[WF_RDNW];
     const float* rdn = s[WF_RDN];
@@ -1227,13 +1304,13 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
   const float minv = 1.0f / msfty;
   const float* rdnw = s[WF_RDNW];
   const float* rdn = s[WF_RDN];
-  const AwLp L{g, s, awsm, nz, ktf, tx, ty, on, lev, c, j, i, dts, ep1, em1, gf, t0, muave, muts, mut, msfty, minv};
+  const AwLp<true> L{g, s, awsm, nz, ktf, tx, ty, on, lev, c, j, i, dts, ep1, em1, gf, t0, muave, muts, mut, msfty, minv};
   auto A = [&](int arr, int k) -> float& { return L.A(arr, k); };
-  auto F = [&](int id, int k) { return s[id][k * lev + c]; };
+  auto F = [&](int id, int k) { return __ldg(&s[id][k * lev + c]); };
   auto B = [&](int id, int k) -> float& { return b[id][k * lev + c]; };
-  enum { T2A = AwLp::T2A, WD = AwLp::WD, RR = AwLp::RR, PP = AwLp::PP, XX = AwLp::XX, YY = AwLp::YY,
-         ZZ = AwLp::ZZ, ZB = AwLp::ZB, YB = AwLp::YB, PB = AwLp::PB, RHSB = AwLp::RHSB, CA = AwLp::CA,
-         CAL = AwLp::CAL, CG = AwLp::CG };
+  enum { T2A = AwLp<true>::T2A, WD = AwLp<true>::WD, RR = AwLp<true>::RR, PP = AwLp<true>::PP, XX = AwLp<true>::XX, YY = AwLp<true>::YY,
+         ZZ = AwLp<true>::ZZ, ZB = AwLp<true>::ZB, YB = AwLp<true>::YB, PB = AwLp<true>::PB, RHSB = AwLp<true>::RHSB, CA = AwLp<true>::CA,
+         CAL = AwLp<true>::CAL, CG = AwLp<true>::CG };
   L.forward();
   // ---- reverse
   const float dampmag = (float)((double)dts * 0.2), hpi = (float)(0.5 * 3.14159265359);
@@ -1251,9 +1328,9 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
       if (k == 0) A(ZB, 0) = B(WF_W, 0);
       if (k >= 1 && k <= ktf) {
         const float hk = (F(WF_PH_SAVE, k) + F(WF_PHB, k)) / gf;
-        float dk = 0.f;
+        float dk = 0.f, sn = 0.f, cn = 0.f;
         if (hk >= hbot) {
-          const float sn = sinf(hpi * (hk - hbot) / kAwHdepth);
+          sincosf(hpi * (hk - hbot) / kAwHdepth, &sn, &cn);
           dk = dampmag * (sn * sn);
         }
         const float ws = F(WF_W_SAVE, k), den = 1.0f + dk;
@@ -1262,12 +1339,11 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
         const float wfb = B(WF_W, k) + pbk * cph / muts;
         mutsb += -pbk * cph * wf / (muts * muts);
         A(ZB, k) = wfb / den;
-        B(WF_W_SAVE, k) += -wfb * dk * mut / den;
+        add_to(B(WF_W_SAVE, k), -wfb * dk * mut / den);
         mutb += -wfb * dk * ws / den;
         if (hk >= hbot) {
           const float db = wfb * (-mut * ws - wf) / den;
-          const float th = hpi * (hk - hbot) / kAwHdepth;
-          const float thb = db * dampmag * sinf(2.0f * th);
+          const float thb = db * dampmag * (2.0f * sn * cn);
           const float hkb = thb * hpi / kAwHdepth;
           hbotb += -hkb;
           ph1b[l] += hkb / gf;
@@ -1318,20 +1394,20 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
       }
       if (k >= 1) {  // the solve's coefficients
         const float ybk = A(YB, k), al = A(CAL, k);
-        if (k <= ktf - 1) B(WF_GAMMA, k) += -A(ZZ, k + 1) * A(WD, k);
-        B(WF_A, k) += -A(YY, k - 1) * al * ybk;
-        B(WF_ALPHA, k) += (A(XX, k) - A(CA, k) * A(YY, k - 1)) * ybk;
+        if (k <= ktf - 1) add_to(B(WF_GAMMA, k), -A(ZZ, k + 1) * A(WD, k));
+        add_to(B(WF_A, k), -A(YY, k - 1) * al * ybk);
+        add_to(B(WF_ALPHA, k), (A(XX, k) - A(CA, k) * A(YY, k - 1)) * ybk);
       }
       float c2ab = 0.f, altb = 0.f, pbk = 0.f, t2ab = 0.f;
       if (k >= 1 && k < ktf) {  // the level's own terms
         const float x_b = A(ZB, k);
         if (x_b != 0.f) {
           wib[l] += x_b;
-          B(WF_RW_TEND, k) += dts * x_b;
+          add_to(B(WF_RW_TEND, k), dts * x_b);
           const float X1 = F(WF_C2A, k) * rdnw[k] / mut * A(PP, k);
           const float X2 = F(WF_C2A, k - 1) * rdnw[k - 1] / mut * A(PP, k - 1);
           const float C1 = minv * F(WF_CQW, k) * 0.5f * dts * gf * rdn[k];
-          B(WF_CQW, k) += x_b * minv * 0.5f * dts * gf * rdn[k] * (X1 - X2);
+          add_to(B(WF_CQW, k), x_b * minv * 0.5f * dts * gf * rdn[k] * (X1 - X2));
           const float X1b = x_b * C1, X2b = -x_b * C1;
           c2ab += X1b * rdnw[k] / mut * A(PP, k);
           mutb += -X1b * X1 / mut;
@@ -1360,7 +1436,7 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
       if (k == ktf) {  // the top level's own terms
         const float x_b = A(ZB, k), rm = rdnw[k - 1];
         wib[l] += x_b;
-        B(WF_RW_TEND, k) += dts * x_b;
+        add_to(B(WF_RW_TEND, k), dts * x_b);
         const float Ct = minv * (-0.5f * dts * gf / mut * (rm * rm) * 2.0f);
         const float term1 = Ct * F(WF_C2A, k - 1) * A(PP, k - 1);
         mutb += -x_b * term1 / mut;
@@ -1376,8 +1452,8 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
         altb += Bt * 2.0f * rm * F(WF_C2A, k) * A(T2A, k);
         t2ab += Bt * 2.0f * rm * F(WF_C2A, k) * F(WF_ALT, k);
       }
-      if (c2ab != 0.f) B(WF_C2A, k) += c2ab;
-      if (altb != 0.f) B(WF_ALT, k) += altb;
+      if (c2ab != 0.f) add_to(B(WF_C2A, k), c2ab);
+      if (altb != 0.f) add_to(B(WF_ALT, k), altb);
       if (k < ktf) {
         A(PB, k) = pbk;
         // t_2ave(k) = (0.5 ((1+e) t_2 + (1-e) t_2ave) + muave t0) / (muts (t0 + t_1))
@@ -1386,8 +1462,8 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
         const float ttb = T / Dm;
         muaveb += T * t0 / Dm;
         mutsb += -T * A(T2A, k) / muts;
-        B(WF_T_SAVE, k) += -T * A(T2A, k) / (t0 + t1);
-        B(WF_T, k) += ttb * 0.5f * ep1;
+        add_to(B(WF_T_SAVE, k), -T * A(T2A, k) / (t0 + t1));
+        add_to(B(WF_T, k), ttb * 0.5f * ep1);
         B(WF_T_2SAVE, k) = ttb * 0.5f * em1;
       }
     }
@@ -1413,7 +1489,7 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
         pb += rhsb;
         const float Rb = rhsb * msfty / mut;
         mutb += -rhsb * msfty * A(RR, k) / (mut * mut);
-        B(WF_PH_TEND, k) += dts * Rb;
+        add_to(B(WF_PH_TEND, k), dts * Rb);
         wib[l] += dts * 0.5f * gf * em1 * Rb;
       }
       A(RHSB, k) = rhsb;
@@ -1458,9 +1534,9 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
           phbb[l] += -dphb;
         }
       }
-      if (wwb != 0.f) B(WF_WW, k) += wwb;
-      B(WF_PH_SAVE, k) += ph1b[l];
-      B(WF_PHB, k) += phbb[l];
+      if (wwb != 0.f) add_to(B(WF_WW, k), wwb);
+      add_to(B(WF_PH_SAVE, k), ph1b[l]);
+      add_to(B(WF_PHB, k), phbb[l]);
       B(WF_PH, k) = pbin[l];
       B(WF_W, k) = wib[l];  // w(0) is replaced by the lower boundary value: wib = 0 there
     }
@@ -1476,9 +1552,9 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_adj_lp(Grid g, S s
       m1 += red[(1 * kAwGroups + y) * 32 + tx];
       m2 += red[(2 * kAwGroups + y) * 32 + tx];
     }
-    b[WF_MUT][c] += m0;
-    b[WF_MUTS][c] += m1;
-    b[WF_MUAVE][c] += m2;
+    add_to(b[WF_MUT][c], m0);
+    add_to(b[WF_MUTS][c], m1);
+    add_to(b[WF_MUAVE][c], m2);
     work[c] = A(ZB, 0);
   }
 }
@@ -1497,7 +1573,7 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_lp(Grid g, S s, fl
   const float gf = (float)G, t0 = (float)T0;
   float muave = 0.f, muts = 1.f, mut = 1.f, msfty = 1.f;
   if (on) muave = s[WF_MUAVE][c], muts = s[WF_MUTS][c], mut = s[WF_MUT][c], msfty = s[WF_MSFTY][c];
-  const AwLp L{g, s, awsm, nz, ktf, tx, ty, on, lev, c, j, i, dts, ep1, em1, gf, t0, muave, muts, mut, msfty,
+  const AwLp<false> L{g, s, awsm, nz, ktf, tx, ty, on, lev, c, j, i, dts, ep1, em1, gf, t0, muave, muts, mut, msfty,
                1.0f / msfty};
   L.forward();
   if (!on) return;
@@ -1507,9 +1583,9 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_lp(Grid g, S s, fl
   for (int l = 0; l < kAwLevels; ++l) {
     const int k = ty + kAwGroups * l;
     if (k > ktf) continue;
-    if (k < ktf) s[WF_T_2SAVE][k * lev + c] = L.A(AwLp::T2A, k);
+    if (k < ktf) s[WF_T_2SAVE][k * lev + c] = L.A(AwLp<false>::T2A, k);
     if (k == 0) {
-      s[WF_W][c] = L.A(AwLp::ZZ, 0);
+      s[WF_W][c] = L.A(AwLp<false>::ZZ, 0);
       continue;
     }
     const float hk = (L.F(WF_PH_SAVE, k) + L.F(WF_PHB, k)) / gf;
@@ -1518,8 +1594,8 @@ __global__ void __launch_bounds__(32 * kAwGroups) k_advance_w_lp(Grid g, S s, fl
       const float sn = sinf(hpi * (hk - hbot) / kAwHdepth);
       dw = dampmag * (sn * sn);
     }
-    const float wf = (L.A(AwLp::ZZ, k) - dw * mut * L.F(WF_W_SAVE, k)) / (1.0f + dw);
-    const float rhs = L.F(WF_PH, k) + msfty * L.A(AwLp::RR, k) / mut;
+    const float wf = (L.A(AwLp<false>::ZZ, k) - dw * mut * L.F(WF_W_SAVE, k)) / (1.0f + dw);
+    const float rhs = L.F(WF_PH, k) + msfty * L.A(AwLp<false>::RR, k) / mut;
     s[WF_W][k * lev + c] = wf;
     s[WF_PH][k * lev + c] = rhs + msfty * 0.5f * dts * gf * ep1 * wf / muts;
   }
@@ -2224,7 +2300,7 @@ __global__ void k_advect_mom_gather(Grid g, const float* Q, const float* R, floa
       if (f >= 0 && f < (long long)n3) aq += Q[(size_t)(D * 6 + s) * n3 + (size_t)f];
     }
   }
-  if (aq != 0.f) qbar[m] += aq;
+  if (aq != 0.f) add_to(qbar[m], aq);
   float ar[3] = {0.f, 0.f, 0.f};
 #pragma unroll
   for (int D = 0; D < 3; ++D)
