@@ -1679,7 +1679,7 @@ __global__ void k_relax_field(Grid g, S s, RelaxShape r, const float* field, flo
   if (k >= r.nk) return;
   const int nx = g.nx, ny = g.ny;
   float* o = tend + ((size_t)k * ny + j) * nx + i;
-  relax_point(g, s, 0, k, j, i, r.ibe, r.jbe, r.nk,
+  relax_point(g, s, 0, k, j, i, r.ibe, r.jbe,
               [&](int kk, int jj, int ii) { return field[((size_t)kk * ny + jj) * nx + ii]; }, dtbc, o);
 }
 

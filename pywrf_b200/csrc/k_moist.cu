@@ -160,29 +160,44 @@ __global__ void k_bdy_final(Grid g, S s, int ring) {
   const size_t p = k * lev + c;
   const float dtbc = s[WF_DSCAL][DS_DTBC];
   const int its = g.ids, jts = g.jds;
-  // value for one stagger: y rows first, then x columns (which overwrite corners)
-  auto put = [&](float* f, int bx, const float* mu, const float* msf, int ibe, int jbe, int itf, int jtf, int ktf) {
-    if (k >= ktf) return;
-    float val = 0.f;
-    bool hit = false;
-    auto ybv = [&](int id, int ii) { return s[id][((size_t)k * 5) * nx + ii]; };
-    auto xbv = [&](int id, int jj) { return s[id][((size_t)k * ny + jj) * 5]; };
-    if (i >= its && i < ibe) {
-      if (j == jts) { val = ybv(bx + 2, i) + dtbc * ybv(bx + 6, i); hit = true; }
-      if (j == jtf - 1) { val = ybv(bx + 3, i) + dtbc * ybv(bx + 7, i); hit = true; }
-    }
-    if (j >= jts && j < jbe) {
-      if (i == its) { val = xbv(bx + 0, j) + dtbc * xbv(bx + 4, j); hit = true; }
-      if (i == itf - 1) { val = xbv(bx + 1, j) + dtbc * xbv(bx + 5, j); hit = true; }
-    }
-    if (!hit) return;
-    f[p] = (msf ? msf[c] : 1.0f) * val / mu[c];
+  // value for one stagger: y rows first, then x columns (which overwrite
+  // corners); all five fields' values first, then the stores (which would hold
+  // back the next field's loads)
+  struct Put {
+    bool hit;
+    float val;
   };
-  put(s[WF_U], WF_U_BXS, s[WF_MUUS], s[WF_MSFUY], g.ide, g.jde - 1, g.ide, g.jde - 1, nz - 1);
-  put(s[WF_V], WF_V_BXS, s[WF_MUVS], s[WF_MSFVX], g.ide - 1, g.jde, g.ide - 1, g.jde, nz - 1);
-  put(s[WF_T], WF_T_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz - 1);
-  put(s[WF_PH], WF_PH_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz);
-  put(s[WF_MOIST] + n3, WF_QV_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz - 1);
+  auto get = [&](int bx, const float* mu, const float* msf, int ibe, int jbe, int itf, int jtf, int ktf) {
+    Put r{false, 0.f};
+    const float *bv = nullptr, *bt = nullptr;
+    size_t q = ((size_t)k * 5) * nx + i;
+    if (k < ktf) {
+      if (i >= its && i < ibe) {
+        if (j == jts) bv = s[bx + 2], bt = s[bx + 6];
+        if (j == jtf - 1) bv = s[bx + 3], bt = s[bx + 7];
+      }
+      if (j >= jts && j < jbe && (i == its || i == itf - 1)) {
+        q = ((size_t)k * ny + j) * 5;
+        if (i == its) bv = s[bx + 0], bt = s[bx + 4];
+        if (i == itf - 1) bv = s[bx + 1], bt = s[bx + 5];
+      }
+    }
+    if (bv) {
+      r.hit = true;
+      r.val = (msf ? msf[c] : 1.0f) * (bv[q] + dtbc * bt[q]) / mu[c];
+    }
+    return r;
+  };
+  const Put u = get(WF_U_BXS, s[WF_MUUS], s[WF_MSFUY], g.ide, g.jde - 1, g.ide, g.jde - 1, nz - 1);
+  const Put v = get(WF_V_BXS, s[WF_MUVS], s[WF_MSFVX], g.ide - 1, g.jde, g.ide - 1, g.jde, nz - 1);
+  const Put t = get(WF_T_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz - 1);
+  const Put ph = get(WF_PH_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz);
+  const Put qv = get(WF_QV_BXS, s[WF_MUTS], nullptr, g.ide - 1, g.jde - 1, g.ide - 1, g.jde - 1, nz - 1);
+  if (u.hit) s[WF_U][p] = u.val;
+  if (v.hit) s[WF_V][p] = v.val;
+  if (t.hit) s[WF_T][p] = t.val;
+  if (ph.hit) s[WF_PH][p] = ph.val;
+  if (qv.hit) s[WF_MOIST][n3 + p] = qv.val;
 }
 
 __global__ void k_w_surface(Grid g, S s) {

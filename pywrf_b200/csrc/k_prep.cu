@@ -167,48 +167,53 @@ __global__ void __launch_bounds__(kWwTX * kWwKT) k_ww_cp(Grid g, S s) {
     for (int k = 1 + tk; k < ktf; k += kWwKT) ww[k * lev + c] = sww[k][tx];
 }
 
-// calc_ww_cp with one thread per mass column (32 x 4 columns per block): the
-// column's divergences stay in registers (the level loop is unrolled to the
-// 64-level limit and predicated), the column sum and the upward scan run in
-// the reference's order; neighbouring threads' columns make every level's
-// loads and stores coalesced.  Same operations as k_ww_cp (the divisions by
-// the map factors in their correctly rounded reciprocal form).
-__global__ void __launch_bounds__(128) k_ww_cp_col(Grid g, S s) {
-  const int i = g.ids + blockIdx.x * 32 + threadIdx.x, j = g.jds + blockIdx.y * 4 + threadIdx.y;
-  if (i >= g.ide - 1 || j >= g.jde - 1) return;
-  const int ktf = g.nz - 1;
-  const int c = g.i2(j, i), ce = c + 1, cn = c + g.nx;
+// calc_ww_cp by a warp's 32 columns and 8 level groups: the same steps as
+// k_ww_cp with the divisions by the map factors in their correctly rounded
+// reciprocal form, rows of whole sectors and the column's own scan in shared
+// memory.  The one-thread-per-column form that it replaces waited on a memory
+// round trip every few levels: 16 -> 5.6 us per launch at 28x28x16, 27 ->
+// 9.4 at 131x131x35, 30 -> 23 at 240x240x41.
+constexpr int kWcTX = 32, kWcKT = 8;
+__global__ void __launch_bounds__(kWcTX * kWcKT) k_ww_cp_tile(Grid g, S s, int i0) {
+  __shared__ float sdv[kMaxNz][kWcTX];
+  const int tx = threadIdx.x % kWcTX, tk = threadIdx.x / kWcTX;
+  const int i = i0 + blockIdx.x * kWcTX + tx, j = g.jds + blockIdx.y;
+  const bool col = i >= g.ids && i < g.ide - 1;
+  const int ktf = g.nz - 1, lev = g.ny * g.nx;
+  const int c = col ? g.i2(j, i) : g.i2(j, g.ids), ce = c + 1, cn = c + g.nx;
   const float* u = s[WF_U];
   const float* v = s[WF_V];
   const float* dnw = s[WF_DNW];
   const float* c1h = s[WF_C1H];
-  const size_t lev = (size_t)g.ny * g.nx;
   const float muu0 = s[WF_MUU][c], muu1 = s[WF_MUU][ce], mfu0 = s[WF_MSFUY][c], mfu1 = s[WF_MSFUY][ce];
   const float muv0 = s[WF_MUV][c], muv1 = s[WF_MUV][cn], mfv0 = s[WF_MSFVX_INV][c], mfv1 = s[WF_MSFVX_INV][cn];
   const float r_mfu0 = __frcp_rn(mfu0), r_mfu1 = __frcp_rn(mfu1);
   const float msftx = s[WF_MSFTX][c];
   const float rdx = g.rdx, rdy = g.rdy;
-  float sdv[kMaxNz];
-  float dmdt = 0.f;
-#pragma unroll
-  for (int k = 0; k < kMaxNz; ++k) {
-    if (k < ktf) {
-      const size_t p = k * lev + c;
-      const float fu1 = divc(muu1 * __ldg(&u[p + 1]), mfu1, r_mfu1), fu0 = divc(muu0 * __ldg(&u[p]), mfu0, r_mfu0);
-      const float fv1 = muv1 * __ldg(&v[p + g.nx]) * mfv1, fv0 = muv0 * __ldg(&v[p]) * mfv0;
-      sdv[k] = (msftx * __ldg(&dnw[k])) * (rdx * (fu1 - fu0) + rdy * (fv1 - fv0));
-      dmdt = dmdt + sdv[k];
-    }
-  }
   float* ww = s[WF_WW];
-  float wk = ww[c];
-#pragma unroll
-  for (int k = 0; k < kMaxNz - 1; ++k) {
-    if (k < ktf - 1) {
-      wk = wk - (__ldg(&dnw[k]) * __ldg(&c1h[k])) * dmdt - sdv[k];
-      ww[(k + 1) * lev + c] = wk;
+  float wk = tk == 0 ? ww[c] : 0.f;
+#pragma unroll 4
+  for (int k = tk; k < ktf; k += kWcKT) {
+    const int p = k * lev + c;
+    const float fu1 = divc(muu1 * __ldg(&u[p + 1]), mfu1, r_mfu1), fu0 = divc(muu0 * __ldg(&u[p]), mfu0, r_mfu0);
+    const float fv1 = muv1 * __ldg(&v[p + g.nx]) * mfv1, fv0 = muv0 * __ldg(&v[p]) * mfv0;
+    sdv[k][tx] = (msftx * __ldg(&dnw[k])) * (rdx * (fu1 - fu0) + rdy * (fv1 - fv0));
+  }
+  __syncthreads();
+  if (tk == 0) {
+    float dmdt = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < ktf; ++k) dmdt = dmdt + sdv[k][tx];
+#pragma unroll 8
+    for (int k = 0; k < ktf - 1; ++k) {
+      wk = wk - (__ldg(&dnw[k]) * __ldg(&c1h[k])) * dmdt - sdv[k][tx];
+      sdv[k][tx] = wk;
     }
   }
+  __syncthreads();
+  if (!col) return;
+#pragma unroll 4
+  for (int k = tk; k < ktf - 1; k += kWcKT) ww[(k + 1) * lev + c] = sdv[k][tx];
 }
 
 __global__ void k_diff_metrics(Grid g, S s) {
@@ -484,7 +489,6 @@ __global__ void k_relax(Grid g, S s, int ring) {
   if (!relax_index(g, ring, k, j, i)) return;
   const float dtbc = s[WF_DSCAL][DS_DTBC];
   const int nz = g.nz;
-  const size_t lev = (size_t)g.ny * g.nx;
   const int p = g.i3(k, j, i);
   const float* ru = s[WF_RU];
   const float* rv = s[WF_RV];
@@ -493,27 +497,46 @@ __global__ void k_relax(Grid g, S s, int ring) {
   const float* mut = s[WF_MUT];
   const int nx = g.nx;
   auto idx = [&](int kk, int jj, int ii) { return (size_t)(kk * g.ny + jj) * nx + ii; };
-  if (k < nz - 1) {
-    float* o = s[WF_U_SAVE] + p;
-    relax_point(g, s, WF_U_BXS, k, j, i, g.ide, g.jde - 1, nz, [&](int kk, int jj, int ii) { return ru[idx(kk, jj, ii)]; }, dtbc, o);
-    o = s[WF_V_SAVE] + p;
-    relax_point(g, s, WF_V_BXS, k, j, i, g.ide - 1, g.jde, nz, [&](int kk, int jj, int ii) { return rv[idx(kk, jj, ii)]; }, dtbc, o);
-    o = s[WF_T_SAVE] + p;
-    relax_point(g, s, WF_T_BXS, k, j, i, g.ide - 1, g.jde - 1, nz,
-                [&](int kk, int jj, int ii) { return t[idx(kk, jj, ii)] * mut[(size_t)jj * nx + ii]; }, dtbc, o);
+  // every field's terms first, then the updates (a store would hold back the
+  // next field's loads): 20 -> 9 us at 28x28x16, 24 -> 12 at
+  // 240x240x41
+  const bool half = k < nz - 1;
+  RelaxSite ru_at = relax_site(g, j, i, g.ide, g.jde - 1), rv_at = relax_site(g, j, i, g.ide - 1, g.jde);
+  const RelaxSite at = relax_site(g, j, i, g.ide - 1, g.jde - 1);
+  const bool du = half && ru_at.side >= 0, dv = half && rv_at.side >= 0, dt = half && at.side >= 0, dp = at.side >= 0;
+  const bool dmu = k == 0 && dp;
+  float *const ou = s[WF_U_SAVE] + p, *const ov = s[WF_V_SAVE] + p, *const ot = s[WF_T_SAVE] + p;
+  float *const op = s[WF_PH_SAVE] + p, *const om = s[WF_MU_TEND] + g.i2(j, i);
+  const float* mu = s[WF_MU];
+  RelaxTerms tu{}, tv{}, tt{}, tp{}, tm{};
+  float vu = 0.f, vv = 0.f, vt = 0.f, vp = 0.f, vm = 0.f;
+  if (du) {
+    tu = relax_terms(g, s, WF_U_BXS, k, j, i, ru_at, [&](int kk, int jj, int ii) { return ru[idx(kk, jj, ii)]; }, dtbc);
+    vu = *ou;
   }
-  {
-    float* o = s[WF_PH_SAVE] + p;
-    relax_point(g, s, WF_PH_BXS, k, j, i, g.ide - 1, g.jde - 1, nz,
-                [&](int kk, int jj, int ii) { return ph[idx(kk, jj, ii)] * mut[(size_t)jj * nx + ii]; }, dtbc, o);
+  if (dv) {
+    tv = relax_terms(g, s, WF_V_BXS, k, j, i, rv_at, [&](int kk, int jj, int ii) { return rv[idx(kk, jj, ii)]; }, dtbc);
+    vv = *ov;
   }
-  if (k == 0) {
-    const float* mu = s[WF_MU];
-    float* o = s[WF_MU_TEND] + g.i2(j, i);
-    relax_point(g, s, WF_MU_BXS, 0, j, i, g.ide - 1, g.jde - 1, 1,
-                [&](int kk, int jj, int ii) { (void)kk; return mu[(size_t)jj * nx + ii]; }, dtbc, o);
+  if (dt) {
+    tt = relax_terms(g, s, WF_T_BXS, k, j, i, at,
+                     [&](int kk, int jj, int ii) { return t[idx(kk, jj, ii)] * mut[(size_t)jj * nx + ii]; }, dtbc);
+    vt = *ot;
   }
-  (void)lev;
+  if (dp) {
+    tp = relax_terms(g, s, WF_PH_BXS, k, j, i, at,
+                     [&](int kk, int jj, int ii) { return ph[idx(kk, jj, ii)] * mut[(size_t)jj * nx + ii]; }, dtbc);
+    vp = *op;
+  }
+  if (dmu) {
+    tm = relax_terms(g, s, WF_MU_BXS, 0, j, i, at, [&](int, int jj, int ii) { return mu[(size_t)jj * nx + ii]; }, dtbc);
+    vm = *om;
+  }
+  if (du) *ou = relaxed(vu, ru_at, tu);
+  if (dv) *ov = relaxed(vv, rv_at, tv);
+  if (dt) *ot = relaxed(vt, at, tt);
+  if (dp) *op = relaxed(vp, at, tp);
+  if (dmu) *om = relaxed(vm, at, tm);
 }
 
 // relaxation + specified tendency of qv at the first stage (relax_bdy_scalar,
@@ -534,7 +557,7 @@ __global__ void k_relax_qv(Grid g, S s, int ring) {
     if (jj < g.jds || jj >= g.jde - 1 || ii < g.ids || ii >= g.ide - 1) return 0.f;
     return qv[(size_t)(kk * g.ny + jj) * nx + ii] * mut[(size_t)jj * nx + ii];
   };
-  relax_point(g, s, WF_QV_BXS, k, j, i, ibe, jbe, g.nz, rq, dtbc, tend + p);
+  relax_point(g, s, WF_QV_BXS, k, j, i, ibe, jbe, rq, dtbc, tend + p);
   // specified row: the boundary tendency replaces the tendency (applied after
   // the relaxation, on disjoint points)
   const float* txs = s[WF_QV_BTXS];
@@ -560,8 +583,8 @@ int launch_prep(const Grid& g, const S& s, cudaStream_t st) {
   k_rk_prep2d<<<col_grid(g, b2), b2, 0, st>>>(g, s);
   k_rk_prep3d<<<point_grid(g, b3), b3, 0, st>>>(g, s);
   if (kernel_form() == WRF_FORM_FAST) {
-    const dim3 bc(32, 4);
-    k_ww_cp_col<<<dim3((g.ide - 1 - g.ids + 31) / 32, (g.jde - 1 - g.jds + 3) / 4), bc, 0, st>>>(g, s);
+    const int i0 = g.nx % 8 == 0 ? g.ids / 8 * 8 : g.ids;  // blocks start on a sector when the rows do
+    k_ww_cp_tile<<<dim3((g.ide - 1 - i0 + kWcTX - 1) / kWcTX, g.jde - 1 - g.jds), kWcTX * kWcKT, 0, st>>>(g, s, i0);
   } else {
     k_ww_cp<<<dim3((g.ide - 1 - g.ids + kWwTX - 1) / kWwTX, g.jde - 1 - g.jds), kWwTX * kWwKT, 0, st>>>(g, s);
   }
