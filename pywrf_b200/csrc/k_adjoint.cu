@@ -15,9 +15,9 @@
 //   Fbar(f)  = a(cell above f) tbar(cell above) - a(cell below f) tbar(cell below)
 //   qbar(m) += sum over faces f whose stencil holds m of Fbar(f) r(f) dPhi_f/dq(m)
 //   rbar(f) += Fbar(f) Phi(f)
-// The faces pass forms each face once (its rbar, and its field terms stored
-// by stencil offset in 18 slot arrays of caller work); the gather pass sums,
-// per point, the slots that address it in a fixed order.  Each output
+// The faces pass forms each face once (its rbar, and Fbar r with the
+// upwind sign in six arrays of caller work); the gather pass sums, per point, over the faces whose
+// stencils hold it in a fixed order.  Each output
 // element is written by one thread, so results do not depend on scheduling;
 // tend's own cotangent is tbar unchanged (the caller passes it through).
 //
@@ -239,30 +239,28 @@ struct ScalarFaces {
   }
 };
 
-// one face's contributions Fbar r dPhi/dq(f + o) to the slots o + 3 of
-// direction D (ord 5: o in [-3, 2], 3: [-2, 1], 2: the two-point average,
-// 1: the fnm / fnp average of the vertical faces next to the ends)
-__device__ __forceinline__ void scalar_slots(float* Q, size_t n3, int D, size_t p, int ord, float fbr, float s,
-                                             float c0, float cm1) {
-#pragma unroll
-  for (int o = -3; o <= 2; ++o) {
-    float w = 0.f;
-    if (ord == 5) w = w5(o, s);
-    else if (ord == 3) w = w3(o, s);
-    else if (ord == 2) w = (o == 0 || o == -1) ? 0.5f : 0.f;
-    else if (ord == 1) w = o == 0 ? c0 : (o == -1 ? cm1 : 0.f);
-    Q[(size_t)(D * 6 + o + 3) * n3 + p] = fbr * w;
-  }
+// A face's dPhi/dq(f + o) is w5 or w3 of the upwind sign s by its order, or the
+// average with weights c0 (o = 0) and cm1 (o = -1): the faces pass leaves Fbar
+// r and s, the gather forms the weights.
+__device__ __forceinline__ void scalar_face(float* Q, size_t n3, int D, size_t p, float fbr, float s) {
+  Q[(size_t)(2 * D) * n3 + p] = fbr;
+  Q[(size_t)(2 * D + 1) * n3 + p] = s;
+}
+__device__ __forceinline__ float scalar_term(int ord, int o, float fbr, float s, float c0, float cm1) {
+  if (ord == 5) return fbr * w5(o, s);
+  if (ord == 3) return fbr * w3(o, s);
+  return fbr * (o == 0 ? c0 : (o == -1 ? cm1 : 0.f));
 }
 
 }  // namespace
 
 // Pass 1 of advect_scalar's reverse: one thread per point p, taken as the y
 // face jf = j, the x face f = i and the vertical face kf = k.  Each face's
-// cotangent Fbar (from the cells either side), velocity r and upwind sign
-// give its contributions to the field at its stencil offsets (slots, as in
-// the momentum reverse) and its own velocity cotangent rbar = Fbar Phi,
-// which only this thread writes.
+// cotangent Fbar (from the cells either side) gives Fbar r, kept for pass 2
+// with the upwind sign, and the face's own velocity cotangent rbar = Fbar Phi,
+// which only this thread writes: six arrays between the passes.
+// With the six products of each face stored instead, eighteen arrays were
+// written and read back, 75 and 35 us at 240x240x41; 51 and 44 now.
 __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, float* Q, float* rubar, float* rvbar,
                                       float* rombar) {
   WRF_POINT_INDEX(g, k, j, i);
@@ -276,7 +274,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
     const int ord = horder(j, jds, jde);
     const float fb = ord ? F.fby(k, j, i) : 0.f;
     const float r = a.rv[p];
-    scalar_slots(Q, n3, 0, p, fb != 0.f ? ord : 0, fb * r, sgnf(r), 0.f, 0.f);
+    scalar_face(Q, n3, 0, p, fb * r, sgnf(r));
     if (fb != 0.f) {
       float phi;
       if (ord == 5) phi = flux5(Qv(p, -3, nx), Qv(p, -2, nx), Qv(p, -1, nx), Qv(p, 0, nx), Qv(p, 1, nx), Qv(p, 2, nx), r);
@@ -291,7 +289,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
     const size_t row = (size_t)k * lev + (size_t)j * nx;
     const float r = a.ru[p];
     const float rs = (i == ide - 3 && ord) ? a.ru[row + ide - 2] : r;  // the reference's sign source of that face
-    scalar_slots(Q, n3, 1, p, fb != 0.f ? ord : 0, fb * r, sgnf(rs), 0.f, 0.f);
+    scalar_face(Q, n3, 1, p, fb * r, sgnf(rs));
     if (fb != 0.f) {
       float phi;
       if (ord == 5) phi = flux5(Qv(p, -3, 1), Qv(p, -2, 1), Qv(p, -1, 1), Qv(p, 0, 1), Qv(p, 1, 1), Qv(p, 2, 1), rs);
@@ -304,8 +302,7 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
     const int ord = vorder(k, ktf);
     const float fb = ord ? F.fbz(k, j, i) : 0.f;
     const float r = a.rom[p];
-    scalar_slots(Q, n3, 2, p, fb != 0.f ? ord : 0, fb * r, sgnf(-r), ord == 1 ? a.fnm[k] : 0.f,
-                 ord == 1 ? a.fnp[k] : 0.f);
+    scalar_face(Q, n3, 2, p, fb * r, sgnf(-r));
     if (fb != 0.f) {
       const int st = (int)lev;
       float phi;
@@ -318,19 +315,35 @@ __global__ void k_advect_scalar_faces(Grid g, AdvArgs0 a, const float* tbar, flo
 }
 
 // Pass 2: the field cotangent of each point, summed in a fixed order over
-// the slots of the faces whose stencils hold it (faces on the point's own
-// line in each direction)
-__global__ void k_advect_scalar_gather(Grid g, const float* Q, float* qbar) {
+// the faces whose stencils hold it (on the point's own line in each direction)
+__global__ void k_advect_scalar_gather(Grid g, AdvArgs0 a, const float* __restrict__ Q, float* qbar) {
   WRF_POINT_INDEX(g, k, j, i);
-  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3();
-  const size_t m = (size_t)k * lev + (size_t)j * g.nx + i;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, ktf = nz - 1;
+  const int lev = ny * nx;
+  const size_t n3 = g.n3();
+  const size_t m = (size_t)k * lev + (size_t)j * nx + i;
+  const float *qy = Q + m, *qx = Q + 2 * n3 + m, *qz = Q + 4 * n3 + m;
   float aq = 0.f;
+  // faces j - 2 .. j + 3 and so on: of order 5 away from the sides
+  if (j >= g.jds + 5 && j < g.jde - 6 && i >= g.ids + 5 && i < g.ide - 6 && k >= 5 && k < ktf - 5) {
 #pragma unroll
-  for (int s = 0; s < 6; ++s) {
-    const int o = s - 3;
-    if (j - o >= 0 && j - o < g.ny) aq += Q[(size_t)(0 * 6 + s) * n3 + (m - (long long)o * g.nx)];
-    if (i - o >= 0 && i - o < g.nx) aq += Q[(size_t)(1 * 6 + s) * n3 + (m - o)];
-    if (k - o >= 0 && k - o < g.nz) aq += Q[(size_t)(2 * 6 + s) * n3 + (m - (long long)o * lev)];
+    for (int o = -3; o <= 2; ++o) {
+      aq += scalar_term(5, o, qy[-o * nx], qy[n3 - o * nx], 0.f, 0.f);
+      aq += scalar_term(5, o, qx[-o], qx[n3 - o], 0.f, 0.f);
+      aq += scalar_term(5, o, qz[-o * lev], qz[n3 - o * lev], 0.f, 0.f);
+    }
+  } else {
+#pragma unroll
+    for (int o = -3; o <= 2; ++o) {
+      const int jf = j - o, f = i - o, kf = k - o;
+      if (jf >= 0 && jf < ny)
+        aq += scalar_term(horder(jf, g.jds, g.jde), o, qy[-o * nx], qy[n3 - o * nx], 0.5f, 0.5f);
+      if (f >= 0 && f < nx) aq += scalar_term(horder(f, g.ids, g.ide), o, qx[-o], qx[n3 - o], 0.5f, 0.5f);
+      if (kf >= 0 && kf < nz) {
+        const int ord = vorder(kf, ktf);
+        aq += scalar_term(ord, o, qz[-o * lev], qz[n3 - o * lev], ord ? a.fnm[kf] : 0.f, ord ? a.fnp[kf] : 0.f);
+      }
+    }
   }
   if (aq != 0.f) add_to(qbar[m], aq);
 }
@@ -1138,7 +1151,7 @@ int launch_advance_mu_t(const Grid& g, const S& s, float dts, cudaStream_t st) {
 
 int launch_advance_mu_t_adj(const Grid& g, const S& s, const S& b, float dts, int ref_no_grad, float* work,
                             cudaStream_t st) {
-  const dim3 b2(32, 4), b3(32, 4);
+  const dim3 b3(32, 4);
   const size_t col = (size_t)g.nz * kMutTX * sizeof(float);
   k_advance_mu_t_adj_dv<<<mut_grid(g, 0), dim3(kMutTX, kMutKT), col, st>>>(g, s, b, dts, ref_no_grad, work);
   k_advance_mu_t_adj_pt<<<point_grid(g, b3), b3, 0, st>>>(g, s, b, dts, work);
@@ -2337,7 +2350,7 @@ int launch_advect_mom_adj(const Grid& g, int component, const float* q, const fl
   return 2;
 }
 
-size_t advect_scalar_adj_work_floats(const Grid& g) { return (size_t)18 * g.n3(); }
+size_t advect_scalar_adj_work_floats(const Grid& g) { return (size_t)6 * g.n3(); }
 
 int launch_advect_scalar_adj(const Grid& g, const float* q, const float* ru, const float* rv, const float* rom,
                              const float* msftx, const float* fnm, const float* fnp, const float* rdnw,
@@ -2346,7 +2359,7 @@ int launch_advect_scalar_adj(const Grid& g, const float* q, const float* ru, con
   const dim3 b3(32, 4);
   AdvArgs0 a{q, ru, rv, rom, msftx, fnm, fnp, rdnw};
   k_advect_scalar_faces<<<point_grid(g, b3), b3, 0, st>>>(g, a, tbar, work, rubar, rvbar, rombar);
-  k_advect_scalar_gather<<<point_grid(g, b3), b3, 0, st>>>(g, work, qbar);
+  k_advect_scalar_gather<<<point_grid(g, b3), b3, 0, st>>>(g, a, work, qbar);
   return 2;
 }
 
