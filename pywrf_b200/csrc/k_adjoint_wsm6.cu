@@ -47,16 +47,25 @@ struct Col {
   T* base;
   int ncol, kst;
   __device__ __forceinline__ T& operator()(int a, int k) const { return base[((size_t)a * kst + k) * ncol]; }
+  __device__ __forceinline__ const T& temp(int k) const;
+  __device__ __forceinline__ const T& den(int k) const;
+  __device__ __forceinline__ const T& delz(int k) const;
+  __device__ __forceinline__ const T& denfac(int k) const;
 };
 
 enum {
   A_TIN, A_TH, A_PII, A_T, A_Q, A_QC, A_QI, A_QR, A_QS, A_QG, A_DEN, A_P, A_DELZ, A_CPM, A_XL, A_DENFAC, A_QS0,
   A_QS1, A_RH0, A_RH1, A_XNI, A_R1, A_R2, A_R3, A_W1, A_W2, A_ZI, A_WI, A_ZA, A_DZA, A_QA, A_QA2, A_WD, A_WWW,
-  A_SR3, A_SRS, A_COUNT,
-  // with one time-split loop: the fallen cloud ice, and (float arrays in
-  // their slots) the level's temperature, Exner function, density and depth
-  A_RI = A_SR3, B_T = A_TIN, B_PII = A_TH, B_DEN = A_PII, B_DELZ = A_CPM
+  A_SR3, A_SRS, A_COUNT
 };
+template <class T>
+__device__ __forceinline__ const T& Col<T>::temp(int k) const { return (*this)(A_T, k); }
+template <class T>
+__device__ __forceinline__ const T& Col<T>::den(int k) const { return (*this)(A_DEN, k); }
+template <class T>
+__device__ __forceinline__ const T& Col<T>::delz(int k) const { return (*this)(A_DELZ, k); }
+template <class T>
+__device__ __forceinline__ const T& Col<T>::denfac(int k) const { return (*this)(A_DENFAC, k); }
 
 template <class T>
 __device__ __forceinline__ T cst(float x) {
@@ -168,8 +177,8 @@ __device__ __forceinline__ T venfac(const T& p, const T& t, const T& den) {
 
 // interface fall speeds: 3rd-order interpolation of the cell speeds (www),
 // the ww == 0 fallback and the downward CFL limiter (wrf_physics.py:1269-1293)
-template <class T>
-__device__ void fall_interfaces(const Col<T>& C, int km, float dt) {
+template <class T, class C_>
+__device__ void fall_interfaces(const C_& C, int km, float dt) {
   const float fa1 = 9.0f / 16.0f, fa2 = 1.0f / 16.0f;
   C(A_WI, 0) = C(A_WWW, 0);
   C(A_WI, 1) = 0.5f * (C(A_WWW, 1) + C(A_WWW, 0));
@@ -180,7 +189,7 @@ __device__ void fall_interfaces(const Col<T>& C, int km, float dt) {
   for (int k = 1; k < km; ++k)
     if (val(C(A_WWW, k)) == 0.f) C(A_WI, k) = C(A_WWW, k - 1);
   for (int k = km - 1; k >= 0; --k) {
-    const T dz = C(A_DELZ, k);
+    const T dz = C.delz(k);
     const T decfl = (C(A_WI, k + 1) - C(A_WI, k)) * dt / dz;
     if (val(decfl) > 0.05f) C(A_WI, k) = C(A_WI, k + 1) - 0.05f * dz / dt;
   }
@@ -192,8 +201,8 @@ __device__ void fall_interfaces(const Col<T>& C, int km, float dt) {
 // overlap is not positive contributes the constant 0 (value and
 // derivatives), so the pairs are screened on the values first: only the
 // few overlapping departure cells of a level enter the dual arithmetic.
-template <class T>
-__device__ void remap(const Col<T>& C, int km, int qa, int out) {
+template <class T, class C_>
+__device__ void remap(const C_& C, int km, int qa, int out) {
   float za[kMaxNz + 1];
   for (int k = 0; k <= km; ++k) za[k] = val(C(A_ZA, k));
   for (int k = 0; k < km; ++k) {
@@ -209,7 +218,7 @@ __device__ void remap(const Col<T>& C, int km, int qa, int out) {
       const T ov = vmax(0.0f, vmin(zhi, ahi) - vmax(zlo, alo));
       acc = acc + C(qa, ka) * ov;
     }
-    C(out, k) = acc / C(A_DELZ, k);
+    C(out, k) = acc / C.delz(k);
   }
 }
 
@@ -218,8 +227,8 @@ __device__ void remap(const Col<T>& C, int km, int qa, int out) {
 // mass-weighted speed): the cell speeds are in A_W1, the masses (den q) in
 // r1 (and r2), replaced by the sedimented masses.  (The surface flux feeds
 // the precipitation accumulators only, which are not differentiated.)
-template <class T>
-__device__ void nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float dt, int iter) {
+template <class T, class C_>
+__device__ void nislfv(const C_& C, int km, int kind, int r1, int r2, float dt, int iter) {
   float allold = 0.f;
   for (int k = 0; k < km; ++k) allold = allold + val(C(r1, k));
   if (kind == 1)
@@ -233,36 +242,36 @@ __device__ void nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float 
     return;
   }
   C(A_ZI, 0) = cst<T>(0.f);
-  for (int k = 0; k < km; ++k) C(A_ZI, k + 1) = C(A_ZI, k) + C(A_DELZ, k);
+  for (int k = 0; k < km; ++k) C(A_ZI, k + 1) = C(A_ZI, k) + C.delz(k);
   for (int k = 0; k < km; ++k) {
     C(A_WD, k) = C(A_W1, k);
     C(A_WWW, k) = C(A_W1, k);
   }
   const int npass = iter >= 1 ? 2 : 1;
   for (int n = 1; n <= npass; ++n) {
-    fall_interfaces(C, km, dt);
+    fall_interfaces<T>(C, km, dt);
     for (int k = 0; k <= km; ++k) C(A_ZA, k) = C(A_ZI, k) - C(A_WI, k) * dt;
     for (int k = 0; k < km; ++k) C(A_DZA, k) = C(A_ZA, k + 1) - C(A_ZA, k);
     C(A_DZA, km) = C(A_ZI, km) - C(A_ZA, km);
     for (int k = 0; k < km; ++k) {
-      C(A_QA, k) = C(r1, k) * C(A_DELZ, k) / C(A_DZA, k);
-      if (kind == 1) C(A_QA2, k) = C(r2, k) * C(A_DELZ, k) / C(A_DZA, k);
+      C(A_QA, k) = C(r1, k) * C.delz(k) / C(A_DZA, k);
+      if (kind == 1) C(A_QA2, k) = C(r2, k) * C.delz(k) / C(A_DZA, k);
     }
     C(A_QA, km) = cst<T>(0.f);
-    C(A_QA2, km) = cst<T>(0.f);
+    if (kind == 1) C(A_QA2, km) = cst<T>(0.f);
     if (n <= iter) {
       for (int k = 0; k < km; ++k) {
-        const T den = C(A_DEN, k), denfac = C(A_DENFAC, k);
+        const T den = C.den(k), denfac = C.denfac(k);
         const T qr = C(A_QA, k) / den;
         T wa;
         if (kind == 1) {
           const T qr2 = C(A_QA2, k) / den;
-          const T wa1 = vt_of(1, qr, den, denfac, C(A_T, k));
-          const T wa2 = vt_of(2, qr2, den, denfac, C(A_T, k));
+          const T wa1 = vt_of(1, qr, den, denfac, C.temp(k));
+          const T wa2 = vt_of(2, qr2, den, denfac, C.temp(k));
           const T tmp = vmax(qr + qr2, 1.0e-15f);
           wa = val(tmp) > 1.0e-15f ? (wa1 * qr + wa2 * qr2) / tmp : cst<T>(0.f);
         } else {
-          wa = vt_of(0, qr, den, denfac, C(A_T, k));
+          wa = vt_of(0, qr, den, denfac, C.temp(k));
         }
         C(A_WWW, k) = 0.5f * (C(A_WD, k) + wa);
       }
@@ -271,7 +280,7 @@ __device__ void nislfv(const Col<T>& C, int km, int kind, int r1, int r2, float 
   for (int sp = 0; sp < (kind == 1 ? 2 : 1); ++sp) {
     const int qa = sp == 0 ? A_QA : A_QA2, r = sp == 0 ? r1 : r2;
     C(qa, km - 1) = cst<T>(0.f);
-    remap(C, km, qa, r);
+    remap<T>(C, km, qa, r);
   }
 }
 
@@ -619,9 +628,9 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
       C(A_R2, k) = snow ? den * qs : cst<T>(0.f);
       C(A_R3, k) = snow ? den * qg : cst<T>(0.f);
     }
-    nislfv(C, km, 0, A_R1, -1, dtcld, 1);
+    nislfv<T>(C, km, 0, A_R1, -1, dtcld, 1);
     for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_W2, k);
-    nislfv(C, km, 1, A_R2, A_R3, dtcld, 1);
+    nislfv<T>(C, km, 1, A_R2, A_R3, dtcld, 1);
     for (int k = 0; k < km; ++k) {
       const T den = C(A_DEN, k), p = C(A_P, k), cpm = C(A_CPM, k);
       T qr = vmax(C(A_R1, k) / den, 0.0f), qs = vmax(C(A_R2, k) / den, 0.0f), qg = vmax(C(A_R3, k) / den, 0.0f);
@@ -644,7 +653,7 @@ __device__ void wsm6_column(const Col<T>& C, int km, float delt, bool skip_dead 
       }
       C(A_R1, k) = ice ? den * qi : cst<T>(0.f);
     }
-    nislfv(C, km, 2, A_R1, -1, dtcld, 0);
+    nislfv<T>(C, km, 2, A_R1, -1, dtcld, 0);
     for (int k = 0; k < km; ++k) {
       T t = C(A_T, k), q = C(A_Q, k), qc = C(A_QC, k), qr = C(A_QR, k), qs = C(A_QS, k), qg = C(A_QG, k);
       const T den = C(A_DEN, k);
@@ -791,8 +800,7 @@ __device__ __forceinline__ void put_input_cot(const Grid& g, const S& b, int c2,
 // tape outgrew the capacity.
 __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, float dt, Tv* ws, TapeCtx tc,
                                                         int c0, int nc, S vo, int* done, int* used) {
-  if (threadIdx.x == 0) g_tape = tc;
-  __syncthreads();
+  tape_open(tc);
   const int lane = tape_lane(), col = c0 + lane;
   ColPos cp;
   if (lane >= nc || !col_pos(g, col, cp)) return;
@@ -859,26 +867,65 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_tape(Grid g, S s, S yb, S b, 
 
 // the level's values that the kernels below share (float arrays in the slots
 // of the column arrays)
+enum { B_T, B_PII, B_DEN, B_DELZ, B_COUNT };
 struct Base {
   float* base;
   int ncol, kst;
   __device__ __forceinline__ float& operator()(int a, int k) const {
-    return base[(size_t)a * kst * ncol * (sizeof(Tv) / sizeof(float)) + (size_t)k * ncol];
+    return base[((size_t)a * kst + k) * ncol];
   }
 };
 __device__ __forceinline__ Base base_of(Tv* ws, int lane, int stride, int kst) {
   return Base{reinterpret_cast<float*>(ws) + lane, stride, kst};
 }
 
-// the falling species that a column holds at some level
-enum { FALL_RAIN = 1, FALL_SNOW = 2, FALL_ICE = 4 };
+// The three falls -- rain, snow with graupel, cloud ice -- read the level's
+// values only, so each is taped by a thread of its own, on a tape of its own
+// (a share of the column's capacity) over column arrays of its own: A_R1,
+// A_R2 the masses, A_W2 the density factor, the rest as in nislfv.  Its inputs
+// are density and depth, then the species' and, for snow, the temperature.
+enum { FALL_RAIN, FALL_SNOW, FALL_ICE, FALLS };
+enum { I_DEN, I_DELZ, I_Q, I_Q2, I_T };
+constexpr int kFallArrays = A_WWW - A_R1 + 1;
+constexpr int kFallSlots = FALLS * kFallArrays + (B_COUNT + 2) / 3;  // arrays of Tv
+__host__ __device__ constexpr int fall_inputs(int f) { return f == FALL_SNOW ? 5 : 3; }
+// entries per level: at most 45, 82 and 26 where each level overlaps two
+// departure cells, and as much again for those that overlap more
+__host__ __device__ constexpr int fall_share(int f) { return f == FALL_RAIN ? 75 : (f == FALL_SNOW ? 138 : 53); }
+__device__ __forceinline__ TapeCtx fall_tape(const TapeCtx& tc, int f) {
+  constexpr int all = fall_share(0) + fall_share(1) + fall_share(2);
+  auto part = [&](int shares) { return (int)((long long)tc.cap * shares / all); };
+  const int c0 = f == FALL_RAIN ? 0 : part(f == FALL_SNOW ? fall_share(0) : fall_share(0) + fall_share(1));
+  const int c1 = f == FALL_RAIN ? part(fall_share(0)) : (f == FALL_SNOW ? part(fall_share(0) + fall_share(1)) : tc.cap);
+  return TapeCtx{tc.rec + (size_t)c0 * tc.stride, tc.stride, c1 - c0};
+}
+
+struct FallCol {
+  Tv* base;  // array A_R1
+  int ncol, kst, km;
+  Base B;
+  __device__ __forceinline__ Tv& operator()(int a, int k) const {
+    return base[((size_t)(a - A_R1) * kst + k) * ncol];
+  }
+  __device__ __forceinline__ Tv in(int f, int k, float v) const { return Tv{v, f * km + k, 1.f}; }
+  __device__ __forceinline__ Tv den(int k) const { return in(I_DEN, k, B(B_DEN, k)); }
+  __device__ __forceinline__ Tv delz(int k) const { return in(I_DELZ, k, B(B_DELZ, k)); }
+  __device__ __forceinline__ Tv temp(int k) const { return in(I_T, k, B(B_T, k)); }
+  __device__ __forceinline__ const Tv& denfac(int k) const { return (*this)(A_W2, k); }
+};
+__device__ __forceinline__ FallCol fall_col(Tv* ws, int f, int lane, int stride, int km) {
+  const size_t array = (size_t)(km + 1) * stride;
+  return FallCol{ws + ((B_COUNT + 2) / 3 + f * kFallArrays) * array + lane, stride, km + 1, km,
+                 base_of(ws, lane, stride, km + 1)};
+}
 
 // moist_physics_prep_em of one level per thread (neighbouring threads take
-// neighbouring columns); flags[col] (zero on entry) collects the species that
-// fall.  Columns outside WSM6's block pass t and q through and set
+// neighbouring columns); used[f * ncol + col] (zero on entry) becomes 1
+// where fall f has mass, done[col] 1, or 0 where the tapes are too small for any
+// column.  Columns outside WSM6's block pass t and q through and set
 // h_diabatic to zero.
-__global__ void __launch_bounds__(128) k_mp_levels(Grid g, S s, S yb, S b, Tv* ws, int stride, int c0, int nc, S vo,
-                                                   int* flags) {
+__global__ void __launch_bounds__(128) k_mp_levels(Grid g, S s, S yb, S b, Tv* ws, TapeCtx tc, int c0, int nc, S vo,
+                                                   int* done, int* used, int ncol) {
   const int km = g.nz - 1;
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(x / nc), lane = (int)(x - (long long)k * nc);
@@ -887,6 +934,7 @@ __global__ void __launch_bounds__(128) k_mp_levels(Grid g, S s, S yb, S b, Tv* w
   ColPos cp;
   col_pos(g, col, cp);
   const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
+  if (k == 0) done[col] = !cp.run || tc.cap >= mp_inputs(g);
   if (!cp.run) {
     b[WF_T][p] = yb[WF_T][p];
     for (int m = 1; m < 7; ++m) b[WF_MOIST][m * n3 + p] = yb[WF_MOIST][m * n3 + p];
@@ -898,92 +946,79 @@ __global__ void __launch_bounds__(128) k_mp_levels(Grid g, S s, S yb, S b, Tv* w
     }
     return;
   }
-  const Base B = base_of(ws, lane, stride, km + 1);
+  const Base B = base_of(ws, lane, tc.stride, km + 1);
   const float pii = wpow((s[WF_P][p] + s[WF_PB][p]) / (float)P0, F(RCP));
   B(B_PII, k) = pii;
   B(B_T, k) = (s[WF_T][p] + (float)T0) * pii;
   B(B_DEN, k) = 1.0f / (s[WF_AL][p] + s[WF_ALB][p]);
   B(B_DELZ, k) = (s[WF_PH][p + lev] + s[WF_PHB][p + lev]) / (float)G - (s[WF_PH][p] + s[WF_PHB][p]) / (float)G;
   const float* q = s[WF_MOIST];
-  const int f = (q[3 * n3 + p] > 0.f ? FALL_RAIN : 0) | (q[5 * n3 + p] > 0.f || q[6 * n3 + p] > 0.f ? FALL_SNOW : 0) |
-                (q[4 * n3 + p] > 0.f ? FALL_ICE : 0);
-  if (f) atomicOr(&flags[col], f);
+  if (q[3 * n3 + p] > 0.f) used[FALL_RAIN * ncol + col] = 1;
+  if (q[5 * n3 + p] > 0.f || q[6 * n3 + p] > 0.f) used[FALL_SNOW * ncol + col] = 1;
+  if (q[4 * n3 + p] > 0.f) used[FALL_ICE * ncol + col] = 1;
 }
 
-// the inputs of a column's sedimentation tape, km levels each
-enum { I_T, I_DEN, I_DELZ, I_QR, I_QI, I_QS, I_QG, I_COUNT };
-
 // The sedimentation of the columns that hold falling species, taped: one
-// thread per column, the species' fallen masses (den q; zero for a species
-// that the column does not hold) left in A_R1 (rain), A_R2 (snow), A_R3
-// (graupel) and A_RI.  used[col] holds the column's flags on entry and
-// receives the entries its tape took, 0 without a tape; done[col] whether
-// the column's cotangents will be written by the kernels that follow: not
-// when the tape outgrew the capacity.  The rest of the column's taped code
-// (saturation ratios, melting) went to the per-level tangents: a third of
-// the entries, and none at all in columns where nothing falls.
+// thread per column and fall (blockIdx.y), the fallen masses (den q) left in
+// A_R1 and A_R2 of the fall's arrays.  used receives the entries each tape
+// took, 0 without a tape; done[col] becomes 0 where one outgrew its capacity.
+// A column's chain of levels is bound by its own latencies: the three falls
+// side by side take 1.1 and 0.6 ms (tape and sweep) at 101x101x35 where one
+// after another they took 2.0 and 1.1, and 2.1 and 1.2 against 3.8 and 1.4 at
+// 240x240x41.
 __global__ void __launch_bounds__(kTapeBlock) k_mp_fall(Grid g, S s, float dt, Tv* ws, TapeCtx tc, int c0, int nc,
-                                                        int* done, int* used) {
-  if (threadIdx.x == 0) g_tape = tc;
-  __syncthreads();
-  const int lane = tape_lane(), col = c0 + lane;
+                                                        int* done, int* used, int ncol) {
+  const int f = blockIdx.y;
+  const TapeCtx tf = fall_tape(tc, f);
+  tape_open(tf);
+  const int lane = tape_lane(), col = c0 + lane, km = g.nz - 1;
   ColPos cp;
   if (lane >= nc || !col_pos(g, col, cp)) return;
-  const int flags = used[col], km = g.nz - 1;
-  used[col] = 0;
-  const bool room = tc.cap >= mp_inputs(g);
-  done[col] = room || !cp.run;
-  if (!cp.run || !flags || !room) return;
+  int& entries = used[f * ncol + col];
+  if (!cp.run || !entries) return;
+  if (tc.cap < mp_inputs(g)) {
+    entries = 0;
+    return;
+  }
   const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3();
-  const bool rain = flags & FALL_RAIN, snow = flags & FALL_SNOW, ice = flags & FALL_ICE;
-  const Col<Tv> C{ws + lane, tc.stride, km + 1};
-  const Base B = base_of(ws, lane, tc.stride, km + 1);
+  const FallCol C = fall_col(ws, f, lane, tc.stride, km);
   const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
   const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
-  tape_reserve(I_COUNT * km);
-  auto in = [&](int f, int k, float v) { return Tv{v, f * km + k, 1.f}; };
+  tape_reserve(fall_inputs(f) * km);
+  const float* q = s[WF_MOIST] + cp.c2;
   const Tv none = cst<Tv>(0.f);
-  for (int k = 0; k < km; ++k) {
-    const size_t p = k * lev + cp.c2;
-    const float* q = s[WF_MOIST] + p;
-    const Tv t = in(I_T, k, B(B_T, k)), den = in(I_DEN, k, B(B_DEN, k));
-    const Tv qr = vmax(in(I_QR, k, q[3 * n3]), 0.0f), qi = vmax(in(I_QI, k, q[4 * n3]), 0.0f);
-    const Tv qs = vmax(in(I_QS, k, q[5 * n3]), 0.0f), qg = vmax(in(I_QG, k, q[6 * n3]), 0.0f);
-    C(A_T, k) = t;
-    C(A_DEN, k) = den;
-    C(A_DELZ, k) = in(I_DELZ, k, B(B_DELZ, k));
-    const Tv denfac = rain || snow ? vsqrt(1.0f / den * F(DEN0)) : none;
-    C(A_DENFAC, k) = denfac;
-    C(A_W1, k) = rain ? vt_of(0, qr, den, denfac, t) : none;
-    const Tv qsum = vmax(qs + qg, 1.0e-15f);
-    C(A_W2, k) = snow && val(qsum) > 1.0e-15f
-                     ? (vt_of(1, qs, den, denfac, t) * qs + vt_of(2, qg, den, denfac, t) * qg) / qsum
-                     : none;
-    C(A_R1, k) = rain ? den * qr : none;
-    C(A_R2, k) = snow ? den * qs : none;
-    C(A_R3, k) = snow ? den * qg : none;
-    C(A_RI, k) = ice ? den * qi : none;
-    // cloud ice's speed (of this level alone) waits in A_XNI
-    Tv wi = none;
-    if (val(qi) > 0.f) {
-      const Tv xni = vmin(vmax(5.387e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
-      const Tv wt = vmax(vmin(F(DICON) * vsqrt(den * qi / xni), F(DIMAX)), 1.0e-25f);
-      wi = 1.49e4f * vexp(vlog(wt) * 1.31f);
+  for (int k = 0; k < km; ++k, q += lev) {
+    const Tv den = C.den(k), denfac = f == FALL_ICE ? none : vsqrt(1.0f / den * F(DEN0));
+    if (f != FALL_ICE) C(A_W2, k) = denfac;
+    if (f == FALL_RAIN) {
+      const Tv qr = vmax(C.in(I_Q, k, q[3 * n3]), 0.0f);
+      C(A_W1, k) = vt_of(0, qr, den, denfac, none);
+      C(A_R1, k) = den * qr;
+    } else if (f == FALL_SNOW) {
+      const Tv t = C.temp(k), qs = vmax(C.in(I_Q, k, q[5 * n3]), 0.0f), qg = vmax(C.in(I_Q2, k, q[6 * n3]), 0.0f);
+      const Tv qsum = vmax(qs + qg, 1.0e-15f);
+      C(A_W1, k) = val(qsum) > 1.0e-15f
+                       ? (vt_of(1, qs, den, denfac, t) * qs + vt_of(2, qg, den, denfac, t) * qg) / qsum
+                       : none;
+      C(A_R1, k) = den * qs;
+      C(A_R2, k) = den * qg;
+    } else {
+      const Tv qi = vmax(C.in(I_Q, k, q[4 * n3]), 0.0f);
+      Tv w = none;
+      if (val(qi) > 0.f) {
+        const Tv xni = vmin(vmax(5.387e7f * vpow(den * vmax(qi, F(QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+        const Tv wt = vmax(vmin(F(DICON) * vsqrt(den * qi / xni), F(DIMAX)), 1.0e-25f);
+        w = 1.49e4f * vexp(vlog(wt) * 1.31f);
+      }
+      C(A_W1, k) = w;
+      C(A_R1, k) = den * qi;
     }
-    C(A_XNI, k) = wi;
   }
-  if (rain) nislfv(C, km, 0, A_R1, -1, dtcld, 1);
-  if (snow) {
-    for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_W2, k);
-    nislfv(C, km, 1, A_R2, A_R3, dtcld, 1);
-  }
-  if (ice) {
-    for (int k = 0; k < km; ++k) C(A_W1, k) = C(A_XNI, k);
-    nislfv(C, km, 2, A_RI, -1, dtcld, 0);
-  }
+  // kinds 0, 1 and 2 as the falls; cloud ice takes no second pass
+  nislfv<Tv>(C, km, f, A_R1, f == FALL_SNOW ? A_R2 : -1, dtcld, f == FALL_ICE ? 0 : 1);
   const int n = g_tape_n[threadIdx.x];
-  used[col] = n;
-  if (n > tc.cap) done[col] = 0;
+  entries = n;
+  if (n > tf.cap) done[col] = 0;
 }
 
 // All but the sedimentation of one level, reversed by forward-mode tangents:
@@ -1004,7 +1039,7 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_fall(Grid g, S s, float dt, T
 enum { X_T, X_Q, X_QC, X_P, X_DEN, X_RR, X_RS, X_RG, X_RI, X_COUNT };
 template <int N>
 __global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, Tv* ws, TapeCtx tc, int c0, int nc,
-                                                       S vo, const int* done, const int* used, float dt) {
+                                                       S vo, const int* done, const int* used, int ncol, float dt) {
   const int km = g.nz - 1;
   const long long xt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(xt / nc), lane = (int)(xt - (long long)k * nc);
@@ -1025,13 +1060,14 @@ __global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, T
   Tv fall[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) fall[q] = cst<Tv>(0.f);
-  if (used[col] > 0) {
-    const Col<Tv> C{ws + lane, tc.stride, km + 1};
-    fall[0] = C(A_R1, k);
-    fall[1] = C(A_R2, k);
-    fall[2] = C(A_R3, k);
-    fall[3] = C(A_RI, k);
+  // (X_RR, X_RS, X_RG, X_RI)
+  if (used[FALL_RAIN * ncol + col]) fall[0] = fall_col(ws, FALL_RAIN, lane, tc.stride, km)(A_R1, k);
+  if (used[FALL_SNOW * ncol + col]) {
+    const FallCol C = fall_col(ws, FALL_SNOW, lane, tc.stride, km);
+    fall[1] = C(A_R1, k);
+    fall[2] = C(A_R2, k);
   }
+  if (used[FALL_ICE * ncol + col]) fall[3] = fall_col(ws, FALL_ICE, lane, tc.stride, km)(A_R1, k);
 #pragma unroll
   for (int q = 0; q < 4; ++q) v[X_RR + q] = fall[q].v;
   const float yt = yb[WF_T][p];
@@ -1136,49 +1172,62 @@ __global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, T
   b[WF_H_DIABATIC][p] = 0.f;
 #pragma unroll
   for (int q = 0; q < 4; ++q)
-    if (fall[q].id >= 0 && cot[X_RR + q] != 0.f) atomicAdd(tc.adj(fall[q].id, lane), cot[X_RR + q] * fall[q].s);
+    if (fall[q].id >= 0 && cot[X_RR + q] != 0.f)
+      atomicAdd(fall_tape(tc, q == 0 ? FALL_RAIN : (q == 3 ? FALL_ICE : FALL_SNOW)).adj(fall[q].id, lane),
+                cot[X_RR + q] * fall[q].s);
 }
 
 // the reverse sweep of the sedimentation's tapes: the inputs' cotangents into
-// the adjoints of entries [0, I_COUNT km)
+// the adjoints of the first entries
 constexpr int kSweepBlock = 32, kSweepWindow = 16, kSweepRing = 64;
-__global__ void __launch_bounds__(kSweepBlock) k_mp_fall_rev(Grid g, TapeCtx tc, int c0, int nc, const int* used) {
+__global__ void __launch_bounds__(kSweepBlock) k_mp_fall_rev(Grid g, TapeCtx tc, int c0, int nc, const int* done,
+                                                             const int* used, int ncol) {
   __shared__ float acc[kSweepRing * kSweepBlock];
-  const int lane = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
   if (lane >= nc) return;
-  const int n = used[c0 + lane];
-  if (n == 0 || n > tc.cap) return;
-  tape_sweep<kSweepWindow, kSweepRing, kSweepBlock>(tc, lane, I_COUNT * (g.nz - 1), n, acc);
+  const int n = used[f * ncol + c0 + lane];
+  if (n == 0 || !done[c0 + lane]) return;
+  tape_sweep<kSweepWindow, kSweepRing, kSweepBlock>(fall_tape(tc, f), lane, fall_inputs(f) * (g.nz - 1), n, acc);
 }
 
 // and from there through prep, one level per thread
 __global__ void __launch_bounds__(128) k_mp_fall_inputs(Grid g, S s, S b, Tv* ws, TapeCtx tc, int c0, int nc,
-                                                        const int* used) {
+                                                        const int* done, const int* used, int ncol) {
   const int km = g.nz - 1;
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(x / nc), lane = (int)(x - (long long)k * nc);
   if (k > km) return;
-  const int col = c0 + lane, n = used[col];
-  if (n == 0 || n > tc.cap) return;
+  const int col = c0 + lane;
   ColPos cp;
   col_pos(g, col, cp);
+  if (!cp.run || !done[col]) return;
   const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
-  auto a = [&](int f, int kk) { return *tc.adj(f * km + kk, lane); };
-  const float below = k > 0 ? a(I_DELZ, k - 1) : 0.f;
-  if (k == km) {
-    b[WF_PH][p] += below / (float)G;
-    return;
+  float below = 0.f, at = 0.f, aden = 0.f, adz = 0.f;
+  bool any = false;
+#pragma unroll
+  for (int f = 0; f < FALLS; ++f) {
+    if (!used[f * ncol + col]) continue;
+    any = true;
+    const TapeCtx tf = fall_tape(tc, f);
+    auto a = [&](int in, int kk) { return *tf.adj(in * km + kk, lane); };
+    if (k > 0) below += a(I_DELZ, k - 1);
+    if (k == km) continue;
+    aden += a(I_DEN, k);
+    adz += a(I_DELZ, k);
+    b[WF_MOIST][(f == FALL_RAIN ? 3 : (f == FALL_SNOW ? 5 : 4)) * n3 + p] += a(I_Q, k);
+    if (f == FALL_SNOW) {
+      b[WF_MOIST][6 * n3 + p] += a(I_Q2, k);
+      at += a(I_T, k);
+    }
   }
+  if (!any) return;
+  b[WF_PH][p] += (below - adz) / (float)G;
+  if (k == km) return;
   const Base B = base_of(ws, lane, tc.stride, km + 1);
-  const float at = a(I_T, k), aden = a(I_DEN, k), adz = a(I_DELZ, k), den = B(B_DEN, k);
+  const float den = B(B_DEN, k);
   b[WF_T][p] += at * B(B_PII, k);
   b[WF_P][p] += at * (B(B_T, k) * F(RCP) / (s[WF_P][p] + s[WF_PB][p]));
   b[WF_AL][p] -= aden * (den * den);
-  b[WF_PH][p] += (below - adz) / (float)G;
-  b[WF_MOIST][3 * n3 + p] += a(I_QR, k);
-  b[WF_MOIST][4 * n3 + p] += a(I_QI, k);
-  b[WF_MOIST][5 * n3 + p] += a(I_QS, k);
-  b[WF_MOIST][6 * n3 + p] += a(I_QG, k);
 }
 
 // the reverse sweep of the tapes k_mp_tape left (same chunk and lanes):
@@ -1256,7 +1305,7 @@ constexpr size_t kTapeChunkBytes = size_t(24) << 30;
 int g_tape_capacity = 0;
 
 // the adjoint's workspace, in floats: the outputs' cotangents (9 n3), the
-// per-column done flags and tape sizes, then one region shared by the
+// per-column done flags and the tapes' sizes, then one region shared by the
 // chunk's tapes and column arrays and (afterwards) the tangent passes'
 // column arrays
 struct MpAdjWork {
@@ -1272,17 +1321,18 @@ MpAdjWork mp_adj_work(const Grid& g) {
   const int per_level = nloop == 1 ? kTapeSplitPerLevel : kTapeEntriesPerLevel * nloop;
   w.cap = g_tape_capacity > 0 ? std::min(kTapeMaxEntries, g_tape_capacity)
                               : std::min(kTapeMaxEntries, per_level * km + mpt::mp_inputs(g));
-  const size_t per_col = (size_t)w.cap * 16 + (size_t)mpt::A_COUNT * (km + 1) * sizeof(Tv);
+  const int arrays = std::max<int>(mpt::A_COUNT, mpt::kFallSlots);
+  const size_t per_col = (size_t)w.cap * 16 + (size_t)arrays * (km + 1) * sizeof(Tv);
   const size_t fit = std::max<size_t>(64, kTapeChunkBytes / per_col / 64 * 64);
   w.width = (int)std::min<size_t>(fit, ((size_t)w.ncol + 63) / 64 * 64);
   w.done = 9 * g.n3();
   w.used = w.done + w.ncol;
-  w.region = (w.used + w.ncol + 3) / 4 * 4;
+  w.region = (w.used + (size_t)mpt::FALLS * w.ncol + 3) / 4 * 4;
   w.tangent = (size_t)mpt::A_COUNT * g.nz * w.ncol * (kMpDirections + 1);
   const size_t ent = (size_t)w.cap * w.width;
   w.rec = w.region;
   w.cols = w.rec + 4 * ent;
-  const size_t tape = 4 * ent + sizeof(Tv) / sizeof(float) * (size_t)mpt::A_COUNT * (km + 1) * w.width;
+  const size_t tape = 4 * ent + sizeof(Tv) / sizeof(float) * (size_t)arrays * (km + 1) * w.width;
   w.total = w.region + std::max(w.tangent, tape);
   return w;
 }
@@ -1325,13 +1375,14 @@ int launch_physics_adj(const Grid& g, const S& s, const S& post, const S& b, flo
     const unsigned columns = (nc + kTapeBlock - 1) / kTapeBlock, sweeps = (nc + mpt::kSweepBlock - 1) / mpt::kSweepBlock;
     if (split) {
       const unsigned levels = (unsigned)(((long long)nc * (g.nz - 1) + 127) / 128);
-      cudaMemsetAsync(used + c0, 0, nc * sizeof(int), st);
-      mpt::k_mp_levels<<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc.stride, c0, nc, vo, used);
-      mpt::k_mp_fall<<<columns, kTapeBlock, 0, st>>>(g, s, dt, cols, tc, c0, nc, done, used);
-      mpt::k_mp_levels_adj<4><<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, dt);
-      mpt::k_mp_fall_rev<<<sweeps, mpt::kSweepBlock, 0, st>>>(g, tc, c0, nc, used);
-      mpt::k_mp_fall_inputs<<<(unsigned)(((long long)nc * g.nz + 127) / 128), 128, 0, st>>>(g, s, b, cols, tc, c0, nc,
-                                                                                            used);
+      const dim3 falls(columns, mpt::FALLS), fsweeps(sweeps, mpt::FALLS);
+      const unsigned ends = (unsigned)(((long long)nc * g.nz + 127) / 128);
+      if (c0 == 0) cudaMemsetAsync(used, 0, mpt::FALLS * w.ncol * sizeof(int), st);
+      mpt::k_mp_levels<<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, w.ncol);
+      mpt::k_mp_fall<<<falls, kTapeBlock, 0, st>>>(g, s, dt, cols, tc, c0, nc, done, used, w.ncol);
+      mpt::k_mp_levels_adj<4><<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, w.ncol, dt);
+      mpt::k_mp_fall_rev<<<fsweeps, mpt::kSweepBlock, 0, st>>>(g, tc, c0, nc, done, used, w.ncol);
+      mpt::k_mp_fall_inputs<<<ends, 128, 0, st>>>(g, s, b, cols, tc, c0, nc, done, used, w.ncol);
       n += 5;
       continue;
     }

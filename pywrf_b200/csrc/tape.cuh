@@ -21,7 +21,7 @@
 // each (0xffff for none), the two partials, and the entry's adjoint (zeroed
 // when the entry is recorded) -- written by one vector store and read back
 // by one vector load.  The per-thread entry count sits in shared memory
-// (blocks of at most kTapeBlock threads) beside the launch's tape context.
+// (blocks of at most kTapeBlock threads) beside the address of its tape.
 // Entries past the capacity are counted but not stored; the caller
 // compares the count with the capacity and treats such a thread's tape as
 // unusable.
@@ -48,8 +48,9 @@ struct TapeCtx {
   }
 };
 
-// the block's tape context and the per-thread entry counts
-__shared__ TapeCtx g_tape;
+// the block's tape capacity, and per thread its tape and the entry count
+__shared__ int g_tape_cap;
+__shared__ TapeRec* g_tape_rec[kTapeBlock];
 __shared__ int g_tape_n[kTapeBlock];
 
 // a taped value: v the value, id the entry it is a multiple of (-1: a
@@ -63,13 +64,21 @@ struct Tv {
 
 __device__ __forceinline__ int tape_lane() { return blockIdx.x * blockDim.x + threadIdx.x; }
 
+// the calling thread's tape (every thread of the block)
+__device__ __forceinline__ void tape_open(const TapeCtx& tc) {
+  if (threadIdx.x == 0) g_tape_cap = tc.cap;
+  g_tape_rec[threadIdx.x] = tc.at(0, tape_lane());
+  g_tape_n[threadIdx.x] = 0;
+  __syncthreads();
+}
+
 __device__ __forceinline__ int tape_rec(int a, int b, float da, float db) {
   if (a < 0 && b < 0) return -1;  // constant operands: a constant
   const int t = threadIdx.x;
   const int n = g_tape_n[t];
   g_tape_n[t] = n + 1;
-  if (n < g_tape.cap)
-    *g_tape.at(n, tape_lane()) =
+  if (n < g_tape_cap)
+    g_tape_rec[t][n] =
         make_uint4((unsigned)(a & 0xffff) | ((unsigned)(b & 0xffff) << 16), __float_as_uint(da), __float_as_uint(db), 0u);
   return n;
 }
@@ -78,8 +87,8 @@ __device__ __forceinline__ int tape_rec(int a, int b, float da, float db) {
 // taped code): Tv{value, index, 1} with index < n then names input index
 __device__ __forceinline__ void tape_reserve(int n) {
   const int t = threadIdx.x;
-  const int m = n < g_tape.cap ? n : g_tape.cap;
-  for (int k = 0; k < m; ++k) *g_tape.at(k, tape_lane()) = make_uint4(0xffffffffu, 0u, 0u, 0u);
+  const int m = n < g_tape_cap ? n : g_tape_cap;
+  for (int k = 0; k < m; ++k) g_tape_rec[t][k] = make_uint4(0xffffffffu, 0u, 0u, 0u);
   g_tape_n[t] = n;
 }
 
