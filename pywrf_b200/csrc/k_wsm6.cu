@@ -37,6 +37,16 @@ __device__ __forceinline__ float n0sfac_of(float t) {
 // warp whose lanes all lie outside branches around them.  What is taken is
 // the same expression either way.
 
+// the slope a = (num / (q den))^(-1/4) and its power bv: a call of its own,
+// because the two powers, expanded at every species and level slot of the
+// sedimentation kernel, made its code outgrow the instruction caches: 471 -> 318 us per launch at
+// 240x240x41 and 40 -> 28 us at 28x28x16 with the calls below
+struct SlopePowers { float a, rb; };
+__device__ __noinline__ SlopePowers slope_powers(float num, float qden, float bv) {
+  const float a = 1.0f / wpow(num / qden, 0.25f);
+  return SlopePowers{a, wpow(a, bv)};
+}
+
 // slope_wsm6 (wrf_physics.py:2048-2104); the rain caps serve all species
 __device__ __forceinline__ void slope_point(float q0, float q1, float q2, float den, float denfac, float t, Slope& o) {
   const float be[3] = {F(mp::BVTR), F(mp::BVTS), F(mp::BVTG)};
@@ -50,9 +60,10 @@ __device__ __forceinline__ void slope_point(float q0, float q1, float q2, float 
     o.r3[m] = F(mp::RSLOPER3MAX);
     if (!(qq[m] <= F(mp::QCRMIN))) {
       const float num = m == 0 ? F(mp::PIDN0R) : m == 1 ? F(mp::PIDN0S) * n0sfac_of(t) : F(mp::PIDN0G);
-      const float a = 1.0f / wpow(num / (qq[m] * den), 0.25f);
+      const SlopePowers sp = slope_powers(num, qq[m] * den, be[m]);
+      const float a = sp.a;
       o.rs[m] = a;
-      o.rb[m] = wpow(a, be[m]);
+      o.rb[m] = sp.rb;
       o.r2[m] = a * a;
       o.r3[m] = a * a * a;
     }
@@ -64,19 +75,19 @@ __device__ __forceinline__ void slope_point(float q0, float q1, float q2, float 
 // terminal velocities alone (wrf_physics.py:1988-2046)
 __device__ __forceinline__ float vt_rain(float qr, float den, float denfac) {
   float rb = F(mp::RSLOPERBMAX);
-  if (!(qr <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0R) / (qr * den), 0.25f), F(mp::BVTR));
+  if (!(qr <= F(mp::QCRMIN))) rb = slope_powers(F(mp::PIDN0R), qr * den, F(mp::BVTR)).rb;
   const float v = F(mp::PVTR) * rb * denfac;
   return qr <= 0.f ? 0.f : v;
 }
 __device__ __forceinline__ float vt_snow(float qs, float den, float denfac, float t) {
   float rb = F(mp::RSLOPERBMAX);
-  if (!(qs <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0S) * n0sfac_of(t) / (qs * den), 0.25f), F(mp::BVTS));
+  if (!(qs <= F(mp::QCRMIN))) rb = slope_powers(F(mp::PIDN0S) * n0sfac_of(t), qs * den, F(mp::BVTS)).rb;
   const float v = F(mp::PVTS) * rb * denfac;
   return qs <= 0.f ? 0.f : v;
 }
 __device__ __forceinline__ float vt_graup(float qg, float den, float denfac) {
   float rb = F(mp::RSLOPERBMAX);
-  if (!(qg <= F(mp::QCRMIN))) rb = wpow(1.0f / wpow(F(mp::PIDN0G) / (qg * den), 0.25f), F(mp::BVTG));
+  if (!(qg <= F(mp::QCRMIN))) rb = slope_powers(F(mp::PIDN0G), qg * den, F(mp::BVTG)).rb;
   const float v = F(mp::PVTG) * rb * denfac;
   return qg <= 0.f ? 0.f : v;
 }
@@ -691,6 +702,43 @@ __device__ void nislfv6_w(const Seg<SEG, NS>& g, const float (&den)[NS], const f
   __syncwarp();
 }
 
+// melting of snow, then graupel, of one point (wrf_physics.py:415-470): a call
+// of its own for its size, as slope_powers is
+struct Melted { float t, qr, qs, qg; };
+__device__ __noinline__ Melted melt_point(float t, float qr, float qs, float qg, float den, float denfac, float p,
+                                          float cpm, float dtcld) {
+  const float t0c = F(mp::T0C), xlf = F(mp::XLF0);
+  Slope sl;
+  slope_point(qr, qs, qg, den, denfac, t, sl);
+  const float work2 = venfac(p, t, den);
+  if (qs > 0.f) {
+    const float n0sfac = n0sfac_of(t);
+    const float coeres = sl.r2[1] * sqrtf(sl.rs[1] * sl.rb[1]);
+    float psmlt = xka(t, den) / xlf * (t0c - t) * F(mp::PI) / 2.0f * n0sfac *
+                  (F(mp::PRECS1) * sl.r2[1] + F(mp::PRECS2) * work2 * coeres) / den;
+    psmlt = fminf(fmaxf(psmlt * dtcld / 1.0f, -qs / 1.0f), 0.0f);
+    qs = qs + psmlt;
+    qr = qr - psmlt;
+    t = t + xlf / cpm * psmlt;
+  }
+  if (qg > 0.f) {
+    const float coeres = sl.r2[2] * sqrtf(sl.rs[2] * sl.rb[2]);
+    float pgmlt = xka(t, den) / xlf * (t0c - t) * (F(mp::PRECG1) * sl.r2[2] + F(mp::PRECG2) * work2 * coeres) / den;
+    pgmlt = fminf(fmaxf(pgmlt * dtcld / 1.0f, -qg / 1.0f), 0.0f);
+    qg = qg + pgmlt;
+    qr = qr - pgmlt;
+    t = t + xlf / cpm * pgmlt;
+  }
+  return Melted{t, qr, qs, qg};
+}
+
+// cloud ice's fall speed (wrf_physics.py:470-480)
+__device__ __noinline__ float ice_speed(float qi, float den) {
+  const float xni = fminf(fmaxf(5.387e7f * wpow(den * fmaxf(qi, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
+  const float wt = fmaxf(fminf(F(mp::DICON) * sqrtf(den * qi / xni), F(mp::DIMAX)), 1.0e-25f);
+  return 1.49e4f * wexp(wlog(wt) * 1.31f);
+}
+
 // the column state a segment carries through the scheme
 template <int NS>
 struct WCol {
@@ -769,62 +817,53 @@ __device__ void wsm6_column_w(const Seg<SEG, NS>& g, WCol<NS>& c, float delt, Pr
         rq2[s] = c.den[s] * c.qr1[s];
         rq3[s] = c.den[s] * c.qr2[s];
       }
-      // sedimentation of rain, then of snow + graupel
-      const float delq1 = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 1, sc);
+      // sedimentation of rain and of cloud ice (which reads nothing that rain,
+      // snow or melting change): one copy of the code, run twice
+      float delq1 = 0.f, delqi = 0.f;
+#pragma unroll 1
+      for (int f = 0; f < 2; ++f) {
+        const bool ice = f == 1;
+        if (ice) {
+#pragma unroll
+          for (int s = 0; s < NS; ++s) {
+            ww[s] = c.qc1[s] <= 0.f ? 0.f : ice_speed(c.qc1[s], c.den[s]);
+            rq[s] = c.den[s] * c.qc1[s];
+          }
+        }
+        const float d = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, ice ? 0 : 1, sc);
+        if (ice) delqi = d;
+        else delq1 = d;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+          const float q = fmaxf(rq[s] / c.den[s], 0.0f);
+          if (ice) c.qc1[s] = q;
+          else c.qr0[s] = q;
+        }
+      }
+      // sedimentation of snow + graupel
       float delq2, delq3;
       nislfv6_w<SEG, NS>(g, c.den, denfac, c.t, c.delz, ww2, rq2, rq3, dtcld, 1, sc, &delq2, &delq3);
       const float fall0 = delq1 / dz0 / dtcld, fall1 = delq2 / dz0 / dtcld, fall2 = delq3 / dz0 / dtcld;
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
         const float den = c.den[s];
-        c.qr0[s] = fmaxf(rq[s] / den, 0.0f);
         c.qr1[s] = fmaxf(rq2[s] / den, 0.0f);
         c.qr2[s] = fmaxf(rq3[s] / den, 0.0f);
         qr0s[s] = c.qr0[s];
-        // melting of snow, then graupel
-        float t = c.t[s];
-        const bool cond = t > t0c;
-        const bool melt = cond && (c.qr1[s] > 0.f || c.qr2[s] > 0.f);
-        Slope sl;
-        if (kPoint || melt) slope_point(c.qr0[s], c.qr1[s], c.qr2[s], den, denfac[s], t, sl);
         if constexpr (kPoint) {
+          Slope sl;
+          slope_point(c.qr0[s], c.qr1[s], c.qr2[s], den, denfac[s], c.t[s], sl);
           rs0[s] = sl.rs[0];
           r30[s] = sl.r3[0];
         }
-        const float work2 = melt ? venfac(c.p[s], t, den) : 0.f;
-        const float xlf = F(mp::XLF0);
-        if (c.qr1[s] > 0.f && cond) {
-          const float n0sfac = n0sfac_of(t);
-          const float coeres = sl.r2[1] * sqrtf(sl.rs[1] * sl.rb[1]);
-          float psmlt = xka(t, den) / xlf * (t0c - t) * F(mp::PI) / 2.0f * n0sfac *
-                        (F(mp::PRECS1) * sl.r2[1] + F(mp::PRECS2) * work2 * coeres) / den;
-          psmlt = fminf(fmaxf(psmlt * dtcld / 1.0f, -c.qr1[s] / 1.0f), 0.0f);
-          c.qr1[s] = c.qr1[s] + psmlt;
-          c.qr0[s] = c.qr0[s] - psmlt;
-          t = t + xlf / cpm[s] * psmlt;
+        if (c.t[s] > t0c && (c.qr1[s] > 0.f || c.qr2[s] > 0.f)) {
+          const Melted o = melt_point(c.t[s], c.qr0[s], c.qr1[s], c.qr2[s], den, denfac[s], c.p[s], cpm[s], dtcld);
+          c.t[s] = o.t;
+          c.qr0[s] = o.qr;
+          c.qr1[s] = o.qs;
+          c.qr2[s] = o.qg;
         }
-        if (c.qr2[s] > 0.f && cond) {
-          const float coeres = sl.r2[2] * sqrtf(sl.rs[2] * sl.rb[2]);
-          float pgmlt = xka(t, den) / xlf * (t0c - t) * (F(mp::PRECG1) * sl.r2[2] + F(mp::PRECG2) * work2 * coeres) / den;
-          pgmlt = fminf(fmaxf(pgmlt * dtcld / 1.0f, -c.qr2[s] / 1.0f), 0.0f);
-          c.qr2[s] = c.qr2[s] + pgmlt;
-          c.qr0[s] = c.qr0[s] - pgmlt;
-          t = t + xlf / cpm[s] * pgmlt;
-        }
-        c.t[s] = t;
-        // cloud-ice fall speed (ice number from the loop-start ice)
-        const float qi = c.qc1[s];
-        ww[s] = 0.f;
-        if (!(qi <= 0.f)) {
-          const float xni = fminf(fmaxf(5.387e7f * wpow(den * fmaxf(qi, F(mp::QMIN)), 0.75f), 1.0e3f), 1.0e6f);
-          const float wt = fmaxf(fminf(F(mp::DICON) * sqrtf(den * qi / xni), F(mp::DIMAX)), 1.0e-25f);
-          ww[s] = 1.49e4f * wexp(wlog(wt) * 1.31f);
-        }
-        rq[s] = den * qi;
       }
-      const float delqi = nislfv_w<SEG, NS>(g, c.den, denfac, c.delz, ww, rq, dtcld, 0, sc);
-#pragma unroll
-      for (int s = 0; s < NS; ++s) c.qc1[s] = fmaxf(rq[s] / c.den[s], 0.0f);
       const float fallc = delqi / dz0 / dtcld;
       const float fallsum = fall0 + fall1 + fall2 + fallc;
       const float fallsum_qsi = fall1 + fallc;
@@ -1092,7 +1131,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_wsm6(Grid g, Wsm6Args a
 // list[16], each j * nx + i of a column of the scheme's block): the WSM6
 // fallback of the surrogate microphysics for the columns its gate rejected.
 template <int SEG, int NS, bool kList = false>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_wsm6_sed(Grid g, S s, float dt, const int* list = nullptr) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) k_wsm6_sed(Grid g, S s, float dt, const int* list = nullptr) {
   constexpr int SPW = 32 / SEG, SPB = kWarpsPerBlock * SPW;
   __shared__ SegScratch<SEG, NS> scratch[SPB];
   if constexpr (kList) {
@@ -1270,7 +1309,7 @@ static __device__ __align__(256) float g_wsm6_scratch[2 * kNoAllocMaxPoints];
 // rain after the sedimentation), qr / qi / qs / qg after the sedimentation
 // and melting, and the precipitation
 template <int SEG, int NS>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_wsm6_sed_args(Grid g, Wsm6Args a, float delt, float* scr_t,
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3) k_wsm6_sed_args(Grid g, Wsm6Args a, float delt, float* scr_t,
                                                                        float* scr_qr0s) {
   constexpr int SPW = 32 / SEG, SPB = kWarpsPerBlock * SPW;
   __shared__ SegScratch<SEG, NS> scratch[SPB];
