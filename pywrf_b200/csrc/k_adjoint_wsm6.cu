@@ -1035,81 +1035,150 @@ __global__ void __launch_bounds__(kTapeBlock) k_mp_fall(Grid g, S s, float dt, T
 // passes (nine at most, where the saturation ratios, slopes and heat
 // capacities as inputs of their own made eighteen), and a level with nothing
 // to condense, freeze or fall runs it not at all: its derivatives are the
-// identity.
+// identity.  A warp runs every branch that one of its points takes, so a block
+// first sorts its points: the quiet ones are done on the spot, those with
+// precipitation are listed from the front, the others from the back, and the
+// evaluations run down the list.  The code is larger than the instruction
+// caches, and three directions at a time keep it smallest for its use: 2.5 ms
+// at 240x240x41 with three, 3.1 with two, 3.2 with four, 3.1 with six; 4.5
+// unsorted with four.
 enum { X_T, X_Q, X_QC, X_P, X_DEN, X_RR, X_RS, X_RG, X_RI, X_COUNT };
-template <int N>
-__global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, Tv* ws, TapeCtx tc, int c0, int nc,
-                                                       S vo, const int* done, const int* used, int ncol, float dt) {
+constexpr int kLvBlock = 128;
+template <int N, int kLvPoints>  // directions, points per thread
+__global__ void __launch_bounds__(kLvBlock) k_mp_levels_adj(Grid g, S s, S yb, S b, Tv* ws, TapeCtx tc, int c0, int nc,
+                                                            S vo, const int* done, const int* used, int ncol, float dt) {
+  __shared__ int list[kLvBlock * kLvPoints], nfront, nback;
   const int km = g.nz - 1;
-  const long long xt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = (int)(xt / nc), lane = (int)(xt - (long long)k * nc);
-  if (k >= km) return;
-  const int col = c0 + lane;
-  ColPos cp;
-  col_pos(g, col, cp);
-  if (!cp.run || !done[col]) return;
-  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3(), p = k * lev + cp.c2;
-  const Base B = base_of(ws, lane, tc.stride, km + 1);
-  const float pfull = s[WF_P][p] + s[WF_PB][p], tin = s[WF_T][p], pii = B(B_PII, k);
-  float v[X_COUNT];
-  v[X_T] = B(B_T, k);
-  v[X_Q] = s[WF_MOIST][n3 + p];
-  v[X_QC] = s[WF_MOIST][2 * n3 + p];
-  v[X_P] = pfull;
-  v[X_DEN] = B(B_DEN, k);
-  Tv fall[4];
+  const size_t lev = (size_t)g.ny * g.nx, n3 = g.n3();
+  const long long x0 = (long long)blockIdx.x * (kLvBlock * kLvPoints);
+  if (threadIdx.x == 0) nfront = nback = 0;
+  __syncthreads();
+  // a point's place and inputs
+  struct Point {
+    int k, lane, col;
+    size_t p;
+    float v[X_COUNT], tin, pii;
+    Tv fall[4];
+  };
+  auto point = [&](int e, Point& o) {
+    const long long x = x0 + e;
+    o.k = (int)(x / nc);
+    o.lane = (int)(x - (long long)o.k * nc);
+    if (o.k >= km) return false;
+    o.col = c0 + o.lane;
+    ColPos cp;
+    col_pos(g, o.col, cp);
+    if (!cp.run || !done[o.col]) return false;
+    const size_t p = o.p = o.k * lev + cp.c2;
+    const Base B = base_of(ws, o.lane, tc.stride, km + 1);
+    o.tin = s[WF_T][p];
+    o.pii = B(B_PII, o.k);
+    o.v[X_T] = B(B_T, o.k);
+    o.v[X_Q] = s[WF_MOIST][n3 + p];
+    o.v[X_QC] = s[WF_MOIST][2 * n3 + p];
+    o.v[X_P] = s[WF_P][p] + s[WF_PB][p];
+    o.v[X_DEN] = B(B_DEN, o.k);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) fall[q] = cst<Tv>(0.f);
-  // (X_RR, X_RS, X_RG, X_RI)
-  if (used[FALL_RAIN * ncol + col]) fall[0] = fall_col(ws, FALL_RAIN, lane, tc.stride, km)(A_R1, k);
-  if (used[FALL_SNOW * ncol + col]) {
-    const FallCol C = fall_col(ws, FALL_SNOW, lane, tc.stride, km);
-    fall[1] = C(A_R1, k);
-    fall[2] = C(A_R2, k);
-  }
-  if (used[FALL_ICE * ncol + col]) fall[3] = fall_col(ws, FALL_ICE, lane, tc.stride, km)(A_R1, k);
+    for (int q = 0; q < 4; ++q) o.fall[q] = cst<Tv>(0.f);
+    // (X_RR, X_RS, X_RG, X_RI)
+    if (used[FALL_RAIN * ncol + o.col]) o.fall[0] = fall_col(ws, FALL_RAIN, o.lane, tc.stride, km)(A_R1, o.k);
+    if (used[FALL_SNOW * ncol + o.col]) {
+      const FallCol C = fall_col(ws, FALL_SNOW, o.lane, tc.stride, km);
+      o.fall[1] = C(A_R1, o.k);
+      o.fall[2] = C(A_R2, o.k);
+    }
+    if (used[FALL_ICE * ncol + o.col]) o.fall[3] = fall_col(ws, FALL_ICE, o.lane, tc.stride, km)(A_R1, o.k);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) v[X_RR + q] = fall[q].v;
-  const float yt = yb[WF_T][p];
-  float ym[7];
+    for (int q = 0; q < 4; ++q) o.v[X_RR + q] = o.fall[q].v;
+    return true;
+  };
+  // the fallen masses' cotangents into the tapes
+  auto to_tape = [&](const Point& o, const float* cot) {
 #pragma unroll
-  for (int m = 1; m < 7; ++m) ym[m] = yb[WF_MOIST][m * n3 + p];
-  const float th = tin + (float)T0, rp = 1.0f / pii;
+    for (int q = 0; q < 4; ++q)
+      if (o.fall[q].id >= 0 && cot[X_RR + q] != 0.f)
+        atomicAdd(fall_tape(tc, q == 0 ? FALL_RAIN : (q == 3 ? FALL_ICE : FALL_SNOW)).adj(o.fall[q].id, o.lane),
+                  cot[X_RR + q] * o.fall[q].s);
+  };
   // moist_physics_finish_em: mpten = t / pii - th is added to theta and
   // gives h_diabatic = mpten / dt
-  const float ympten = yt + yb[WF_H_DIABATIC][p] / dt;
-  float qs0, qs1;
-  fpvs(v[X_T], pfull, qs0, qs1);
-  const float qm = vmax(v[X_Q], F(QMIN));
+  auto theta_out = [&](const Point& o, float tout) {
+    const float mpten = tout / o.pii - (o.tin + (float)T0);
+    vo[WF_T][o.p] = o.tin + mpten;
+    vo[WF_H_DIABATIC][o.p] = mpten / dt;
+  };
   // no hydrometeors, no condensation; no nucleation of ice
-  const bool dry = v[X_QC] <= 0.f && v[X_RR] == 0.f && v[X_RS] == 0.f && v[X_RG] == 0.f && v[X_RI] == 0.f;
-  const bool no_ice = qm <= qs1 || v[X_T] >= F(T0C);
-  const bool quiet = dry && no_ice && qm < qs0;
-  float cot[X_COUNT];
-#pragma unroll
-  for (int q = 0; q < X_COUNT; ++q) cot[q] = 0.f;
-  float tout = v[X_T];
-  if (quiet) {
-    cot[X_Q] = ym[1];
+  auto is_dry = [](const float* v) {
+    return v[X_QC] <= 0.f && v[X_RR] == 0.f && v[X_RS] == 0.f && v[X_RG] == 0.f && v[X_RI] == 0.f;
+  };
+  bool own = false;  // (one point a thread) the evaluation is this thread's
+#pragma unroll 1
+  for (int e = threadIdx.x; e < kLvBlock * kLvPoints; e += kLvBlock) {
+    Point o;
+    if (!point(e, o)) continue;
+    const float* v = o.v;
+    float qs0, qs1;
+    fpvs(v[X_T], v[X_P], qs0, qs1);
+    const float qm = vmax(v[X_Q], F(QMIN));
+    if (!(is_dry(v) && (qm <= qs1 || v[X_T] >= F(T0C)) && qm < qs0)) {
+      if (kLvPoints == 1) {
+        own = true;
+      } else {
+        const bool precip = v[X_RR] > 0.f || v[X_RS] > 0.f || v[X_RG] > 0.f;
+        list[precip ? atomicAdd(&nfront, 1) : kLvBlock * kLvPoints - 1 - atomicAdd(&nback, 1)] = e;
+      }
+      continue;
+    }
+    const size_t p = o.p;
+    float cot[X_COUNT];
     const float rden = 1.0f / v[X_DEN];
-    cot[X_RR] = ym[3] * rden;
-    cot[X_RS] = ym[5] * rden;
-    cot[X_RG] = ym[6] * rden;
+    cot[X_RR] = yb[WF_MOIST][3 * n3 + p] * rden;
+    cot[X_RS] = yb[WF_MOIST][5 * n3 + p] * rden;
+    cot[X_RG] = yb[WF_MOIST][6 * n3 + p] * rden;
+    cot[X_RI] = 0.f;
     if (vo[WF_T]) {
+      theta_out(o, v[X_T]);
       vo[WF_MOIST][n3 + p] = v[X_Q];
       for (int m = 2; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = 0.f;
     }
-  } else {
-    // the time-split loop's step (one loop: dt itself up to the split step)
-    const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
-    const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
+    b[WF_T][p] = yb[WF_T][p];
+    b[WF_MOIST][n3 + p] = yb[WF_MOIST][n3 + p];
+#pragma unroll
+    for (int m = 2; m < 7; ++m) b[WF_MOIST][m * n3 + p] = 0.f;
+    b[WF_H_DIABATIC][p] = 0.f;
+    to_tape(o, cot);
+  }
+  if (kLvPoints > 1) __syncthreads();
+  // the time-split loop's step (one loop: dt itself up to the split step)
+  const float loops = fmaxf(dt / F(DTCLDCR), 1.0f);
+  const float dtcld = dt <= F(DTCLDCR) ? dt : dt / loops;
+  const int front = nfront, gap = (front + 31) / 32 * 32, all = kLvPoints > 1 ? gap + nback : (own ? kLvBlock : 0);
+#pragma unroll 1
+  for (int e = threadIdx.x; e < all; e += kLvBlock) {
+    if (kLvPoints > 1 && e >= front && e < gap) continue;
+    Point o;
+    point(kLvPoints == 1 ? e : list[e < front ? e : kLvBlock * kLvPoints - 1 - (e - gap)], o);
+    const float* v = o.v;
+    const size_t p = o.p;
+    float ym[7];
+#pragma unroll
+    for (int m = 1; m < 7; ++m) ym[m] = yb[WF_MOIST][m * n3 + p];
+    const float yt = yb[WF_T][p], ympten = yt + yb[WF_H_DIABATIC][p] / dt;
+    const float th = o.tin + (float)T0, rp = 1.0f / o.pii;
+    float cot[X_COUNT];
+#pragma unroll
+    for (int q = 0; q < X_COUNT; ++q) cot[q] = 0.f;
+    float tout = v[X_T];
     using D = Dual<N>;
     int seeds = 1 << X_T | 1 << X_Q | 1 << X_P;
     if (!(v[X_QC] < 0.f)) seeds |= 1 << X_QC;
-    if (!(dry && no_ice)) seeds |= 1 << X_DEN;
+    float qs0, qs1;
+    fpvs(v[X_T], v[X_P], qs0, qs1);
+    const float qm = vmax(v[X_Q], F(QMIN));
+    if (!(is_dry(v) && (qm <= qs1 || v[X_T] >= F(T0C)))) seeds |= 1 << X_DEN;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (fall[q].id >= 0) seeds |= 1 << (X_RR + q);
+      if (o.fall[q].id >= 0) seeds |= 1 << (X_RR + q);
 #pragma unroll 1
     for (int pass = 0; seeds; ++pass) {
       int at[N];  // the inputs seeded in this pass
@@ -1148,6 +1217,7 @@ __global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, T
       if (pass == 0) {
         tout = t.v;
         if (vo[WF_T]) {
+          theta_out(o, tout);
           const float mv[7] = {0.f, q.v, qc.v, qr.v, qi.v, qs.v, qg.v};
           for (int m = 1; m < 7; ++m) vo[WF_MOIST][m * n3 + p] = mv[m];
         }
@@ -1156,25 +1226,16 @@ __global__ void __launch_bounds__(128) k_mp_levels_adj(Grid g, S s, S yb, S b, T
     // prep: the cotangents through the temperature th pii and the Exner
     // function
     const float cpii = fmaf(cot[X_T], th, -ympten * (tout * rp) * rp);
-    b[WF_P][p] += cot[X_P] + cpii * (F(RCP) * pii / pfull);
+    b[WF_P][p] += cot[X_P] + cpii * (F(RCP) * o.pii / v[X_P]);
     b[WF_AL][p] -= cot[X_DEN] * (v[X_DEN] * v[X_DEN]);
-  }
-  if (vo[WF_T]) {
-    const float mpten = tout / pii - th;
-    vo[WF_T][p] = tin + mpten;
-    vo[WF_H_DIABATIC][p] = mpten / dt;
-  }
-  b[WF_T][p] = quiet ? yt : yt + fmaf(cot[X_T], pii, -ympten);
-  b[WF_MOIST][n3 + p] = cot[X_Q];
-  b[WF_MOIST][2 * n3 + p] = cot[X_QC];
+    b[WF_T][p] = yt + fmaf(cot[X_T], o.pii, -ympten);
+    b[WF_MOIST][n3 + p] = cot[X_Q];
+    b[WF_MOIST][2 * n3 + p] = cot[X_QC];
 #pragma unroll
-  for (int m = 3; m < 7; ++m) b[WF_MOIST][m * n3 + p] = 0.f;
-  b[WF_H_DIABATIC][p] = 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (fall[q].id >= 0 && cot[X_RR + q] != 0.f)
-      atomicAdd(fall_tape(tc, q == 0 ? FALL_RAIN : (q == 3 ? FALL_ICE : FALL_SNOW)).adj(fall[q].id, lane),
-                cot[X_RR + q] * fall[q].s);
+    for (int m = 3; m < 7; ++m) b[WF_MOIST][m * n3 + p] = 0.f;
+    b[WF_H_DIABATIC][p] = 0.f;
+    to_tape(o, cot);
+  }
 }
 
 // the reverse sweep of the sedimentation's tapes: the inputs' cotangents into
@@ -1380,7 +1441,13 @@ int launch_physics_adj(const Grid& g, const S& s, const S& post, const S& b, flo
       if (c0 == 0) cudaMemsetAsync(used, 0, mpt::FALLS * w.ncol * sizeof(int), st);
       mpt::k_mp_levels<<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, w.ncol);
       mpt::k_mp_fall<<<falls, kTapeBlock, 0, st>>>(g, s, dt, cols, tc, c0, nc, done, used, w.ncol);
-      mpt::k_mp_levels_adj<4><<<levels, 128, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, w.ncol, dt);
+      // sorting pays where it leaves enough blocks to even out (two per SM at
+      // a time); elsewhere a thread runs its own point: 2.5 ms sorted, 3.4 not,
+      // at 240x240x41 (4062 blocks of sorted points); 0.53 and 0.38 at 101x101x35
+      // (527)
+      const bool deep = levels >= 4 * 148 * 2 * 8;
+      const unsigned sorted = deep ? (levels + 3) / 4 : levels;
+      (deep ? mpt::k_mp_levels_adj<3, 4> : mpt::k_mp_levels_adj<3, 1>)<<<sorted, mpt::kLvBlock, 0, st>>>(g, s, yb, b, cols, tc, c0, nc, vo, done, used, w.ncol, dt);
       mpt::k_mp_fall_rev<<<fsweeps, mpt::kSweepBlock, 0, st>>>(g, tc, c0, nc, done, used, w.ncol);
       mpt::k_mp_fall_inputs<<<ends, 128, 0, st>>>(g, s, b, cols, tc, c0, nc, done, used, w.ncol);
       n += 5;
