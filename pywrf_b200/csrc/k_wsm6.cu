@@ -129,6 +129,14 @@ __device__ void wsm6_point(float& t, float& q, float& qc0, float& qc1, float& qr
                            const float qs0, const float qs1, const float rs0pre, const float r30pre,
                            const float dtcld) {
   const float t0c = F(mp::T0C);
+  // A point without hydrometeors that neither condenses nor nucleates ice
+  // keeps what it has: every rate below is an exact zero (qs0 and qs1 are
+  // those of t).  @QU@
+  const float qm = fmaxf(q, F(mp::QMIN));
+  if (qc0 == 0.f && qc1 == 0.f && qr0 == 0.f && qr1 == 0.f && qr2 == 0.f && qm < qs0 && (qm <= qs1 || t >= t0c)) {
+    qc0 = qc1 = qr0 = qr1 = qr2 = 0.f;
+    return;
+  }
   const float rh0 = fmaxf(q / qs0, F(mp::QMIN));
   const float rh1 = fmaxf(q / qs1, F(mp::QMIN));
   // instantaneous melting / freezing (one supcol for all four)
