@@ -156,8 +156,19 @@ __device__ __forceinline__ void store_row16_bf16(__nv_bfloat16* dst, const float
 // partial-sum index of a split reduction, 0 otherwise)
 __device__ __forceinline__ void epilogue16(const GemmEpi& e, float (&v)[16], int m, int n, int split) {
   if (e.bias && split == 0) {  // (once over the partial sums of a split reduction)
+    if ((reinterpret_cast<uintptr_t>(e.bias) & 15u) == 0) {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) v[t] += __ldg(&e.bias[n + t]);
+      for (int t = 0; t < 16; t += 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(e.bias + n + t));
+        v[t] += q.x;
+        v[t + 1] += q.y;
+        v[t + 2] += q.z;
+        v[t + 3] += q.w;
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < 16; ++t) v[t] += __ldg(&e.bias[n + t]);
+    }
   }
   switch (e.kind) {
     case EPI_F32: {
