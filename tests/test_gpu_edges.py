@@ -1,0 +1,314 @@
+"""Kernels and dispatch branches at the sizes where they can go wrong: tile
+and warp remainders, the smallest and largest depths, rows that are and are
+not whole 16-byte words."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from pywrf_b200 import _native as N
+from pywrf_b200 import adjoint as A
+from pywrf_b200 import synthetic
+from pywrf_b200.config import Grid
+from pywrf_b200.solver import Integrator
+from pywrf_b200.state import DeviceState, make_cgrid
+
+pytestmark = pytest.mark.gpu
+
+
+def _cg(nx, ny, nz, dt=45.0):
+    return make_cgrid(Grid.make(nx, ny, nz, 9000.0, 9000.0, dt),
+                      {"cf1": 0.0, "cf2": 0.0, "cf3": 0.0, "cfn": 0.0, "cfn1": 0.0})
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("n,nz", [(316, 12), (317, 17)], ids=["316x12", "317x17"])
+def test_marching_acoustic_columns_equal_the_tiled_form_bitwise(n, nz):
+    """Domains wide enough for the one-thread-per-column acoustic kernel
+    against the point forms (which keep the tiled kernel), every field."""
+    spec = synthetic.CaseSpec(n=n, nz=nz, nsteps=1, bdy_tend_amp=1.0e-4, seed=5)
+    g = synthetic.grid_for(spec)
+    inputs, bdy = synthetic.build(spec)
+    states = []
+    for form in (N.WRF_FORM_FAST, N.WRF_FORM_POINT):
+        prev = N.lib().wrf_set_kernel_form(form)
+        try:
+            st = DeviceState.from_inputs(g, inputs, bdy, device="cuda")
+            it = Integrator(st)
+            it.run(1, graph=False)
+            torch.cuda.synchronize()
+            assert it.status()["wait_timeouts"] == 0
+        finally:
+            N.lib().wrf_set_kernel_form(prev)
+        states.append(st)
+    fast, point = states
+    bad = [k for k in fast.names if not torch.equal(fast[k].view(torch.int32), point[k].view(torch.int32))]
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("ncol,nz", [(1, 3), (33, 12), (1000, 41), (31, 64)])
+def test_implicit_w_solve_and_its_reverse(ncol, nz):
+    """The column solve and its transposed solve against float64 loops.  The
+    coefficients are those of a diagonally dominant system (|a alpha|, |gamma|
+    < 1/2), whose rounding stays within a few ulp per level: 64 levels of
+    half an ulp each way and twice that for the reverse, 1e-5 of the norm."""
+    gen = torch.Generator(device="cuda").manual_seed(ncol + nz)
+    x, a, al, ga, cot = (torch.randn(nz, ncol, generator=gen, device="cuda") for _ in range(5))
+    a, al, ga = 0.3 * torch.tanh(a), 1.0 + 0.2 * torch.tanh(al), 0.3 * torch.tanh(ga)
+    args = [v.clone().requires_grad_(True) for v in (x, a, al, ga)]
+    w = A.vsolve_w(*args)
+    grads = torch.autograd.grad(w, args, grad_outputs=cot)
+    ref = [v.double().cpu().requires_grad_(True) for v in (x, a, al, ga)]
+    y = [ref[0][0]]
+    for k in range(1, nz):
+        y.append((ref[0][k] - ref[1][k] * y[k - 1]) * ref[2][k])
+    z = list(y)
+    for k in range(nz - 2, 0, -1):
+        z[k] = y[k] - ref[3][k] * z[k + 1]
+    z = torch.stack(z)
+    want = (z.detach(),) + torch.autograd.grad(z, ref, grad_outputs=cot.double().cpu())
+    for got, exact in zip((w.detach(),) + grads, want):
+        err = (got.double().cpu() - exact).norm() / exact.norm().clamp_min(1e-30)
+        assert float(err) < 1e-5
+
+
+@pytest.mark.parametrize("nx,ny,nz,dt", [(24, 25, 12, 45.0), (41, 30, 48, 150.0), (37, 24, 64, 45.0),
+                                         (24, 24, 20, 250.0)])
+def test_wsm6_with_caller_scratch_equals_the_fused_kernel_bitwise(nx, ny, nz, dt):
+    """Columns that hold nothing, one species, or all of them side by side."""
+    gen = torch.Generator(device="cuda").manual_seed(nx * nz)
+    rnd = lambda *s: torch.rand(*s, generator=gen, device="cuda")  # noqa: E731
+    k = torch.linspace(0.0, 1.0, nz, device="cuda")[:, None, None]
+    p = 1.0e5 * torch.exp(-1.6 * k) * (1.0 + 0.001 * rnd(nz, ny, nx))
+    pii = (p / 1.0e5) ** 0.2857143
+    th = 295.0 + 45.0 * k + rnd(nz, ny, nx)
+    f = dict(th=th, qv=0.012 * torch.exp(-5.0 * k) * (0.7 + 0.6 * rnd(nz, ny, nx)))
+    for i, q in enumerate(("qc", "qr", "qi", "qs", "qg")):
+        col = (rnd(ny, nx) < 0.4).float() * (rnd(nz, ny, nx) < 0.5).float()
+        f[q] = 1.0e-3 * col * rnd(nz, ny, nx) ** 4 - (1.0e-9 if i == 0 else 0.0)
+    f |= dict(rho=p / (287.0 * th * pii), pii=pii, p=p, dz=200.0 + 400.0 * k.expand(nz, ny, nx))
+    f = {a: b.contiguous() for a, b in f.items()}
+    cg, L = _cg(nx, ny, nz, dt), N.lib()
+    n = ctypes.c_size_t(0)
+    N.check(L.wrf_wsm6_work_floats(ctypes.byref(cg), dt, ctypes.byref(n)), "work")
+    assert (n.value == 0) == (dt >= 240.0)
+    outs = []
+    for split in (False, True):
+        d = {a: b.clone() for a, b in f.items()}
+        flat = [torch.zeros(ny, nx, device="cuda") for _ in range(7)]
+        args = [ctypes.byref(cg)] + [_p(d[a]) for a in d] + [ctypes.c_float(dt)] + [_p(v) for v in flat]
+        if split:
+            work = torch.full((max(n.value, 1),), float("nan"), device="cuda")
+            N.check(L.wrf_wsm6_work(*args, _p(work), n.value, _stream()), "wrf_wsm6_work")
+        else:
+            N.check(L.wrf_wsm6(*args, _stream()), "wrf_wsm6")
+        torch.cuda.synchronize()
+        outs.append(list(d.values()) + flat)
+    assert float(outs[0][11].max()) > 0.0  # it rained
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    if n.value:
+        rc = L.wrf_wsm6_work(*args, _p(work), n.value - 1, _stream())
+        assert rc == N.WRF_EINVAL
+
+
+LETTERS = "uvwtpdefUVxyZ"
+
+
+@pytest.mark.parametrize("nx,ny", [(24, 24), (32, 27), (45, 30), (61, 38), (132, 70)])
+def test_batched_halos_and_their_adjoint(nx, ny):
+    """One launch for a batch of fields against the in-place copies of each
+    (bitwise), and the adjoint against the transposed copy (dot products of
+    integers, exact in float64)."""
+    nz = 12
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    num = lambda *s: torch.randint(-8, 9, s, generator=gen, device="cuda").float()  # noqa: E731
+    fields = [num(nz, ny, nx) for _ in LETTERS] + [num(7, nz, ny, nx)] + [num(ny, nx) for _ in "tuv"]
+    letters = LETTERS + "M" + "tuv"
+    leaves = [f.clone().requires_grad_(True) for f in fields]
+    outs = A.halos(leaves, letters)
+    for f, v, o in zip(fields, letters, outs):
+        if v == "Z":
+            want = A.zero_grad_w(f)
+        elif v == "M":
+            want = torch.stack([f[0]] + [A.halo(f[m], "p") for m in range(1, 7)])
+        else:
+            want = A.halo(f, v)
+        assert torch.equal(o.detach(), want), v
+    cots = [num(*f.shape) for f in fields]
+    grads = torch.autograd.grad(outs, leaves, grad_outputs=cots)
+    for f, v, o, c, gr in zip(fields, letters, outs, cots, grads):
+        assert float((o.detach().double() * c).sum()) == float((f.double() * gr).sum()), v
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 7), (3, 256), (5, 264), (6, 2560), (130, 8192), (2, 8190)])
+def test_row_sums_of_bf16_rows(rows, cols):
+    """Row sums against float64 (float32 partial sums of at most 64 terms and
+    two trees of eight levels: 80 roundings of half an ulp of the row's
+    absolute sum)."""
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    a = torch.randn(rows, cols, generator=gen, device="cuda").to(torch.bfloat16)
+    out = torch.empty(rows, device="cuda")
+    N.check(N.lib().wrf_rowsum_bf16(_p(a), rows, cols, _p(out), _stream()), "rowsum")
+    want = a.double().sum(1)
+    assert bool(((out.double() - want).abs() <= 80 * 6e-8 * a.double().abs().sum(1)).all())
+
+
+@pytest.mark.parametrize("r,c", [(64, 62), (33, 40), (1, 5), (130, 258)])
+def test_transpose_and_adam_tiles(r, c):
+    """The transposed bf16 copy (both element widths) and one Adam step of a
+    batch of two matrices, one of them without copies, against float64 (a
+    handful of float32 roundings of the update, 1e-6 of its size)."""
+    gen = torch.Generator(device="cuda").manual_seed(r)
+    a = torch.randn(r, c, generator=gen, device="cuda").to(torch.bfloat16)
+    out = torch.empty(c, r, dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().wrf_transpose_bf16(_p(a), r, c, _p(out), _stream()), "transpose")
+    assert torch.equal(out, a.t())
+    w, m, v = (torch.randn(r, c, generator=gen, device="cuda") for _ in range(3))
+    v = v.abs()
+    gp = torch.randn(3, r, c, generator=gen, device="cuda")
+    bias, bm, bv, bg = torch.randn(4, c, generator=gen, device="cuda")
+    bv = bv.abs()
+    wb, wtb = torch.empty_like(a), torch.empty_like(out)
+    lr, b1, b2, eps = (ctypes.c_float(q).value for q in (1e-2, 0.9, 0.999, 1e-8))  # as the entry takes them
+    exact = []
+    for x, y, z, g in ((w, m, v, gp.double().sum(0)), (bias, bm, bv, bg.double())):
+        mm, vv = b1 * y.double() + (1 - b1) * g, b2 * z.double() + (1 - b2) * g * g
+        step = (mm / (1 - b1 ** 3)) / ((vv / (1 - b2 ** 3)).sqrt() + eps)
+        exact.append(x.double() - lr * step)
+    items = (N.WrfAdamItemC * 2)(
+        N.WrfAdamItemC(w.data_ptr(), gp.data_ptr(), m.data_ptr(), v.data_ptr(), wb.data_ptr(), wtb.data_ptr(), r * c,
+                       3, r, c, 0.0),
+        N.WrfAdamItemC(bias.data_ptr(), bg.data_ptr(), bm.data_ptr(), bv.data_ptr(), None, None, c, 1, 1, c, 0.0))
+    N.check(N.lib().wrf_adam_batch(2, items, lr, b1, b2, eps, 3, _stream()), "adam")
+    for got, want in zip((w, bias), exact):
+        assert float((got.double() - want).abs().max()) <= 1e-6 * float(want.abs().max()) + 1e-6
+    assert torch.equal(wb, w.to(torch.bfloat16)) and torch.equal(wtb, w.to(torch.bfloat16).t())
+
+
+@pytest.mark.parametrize("n,nz", [(28, 12), (37, 20), (64, 33)])
+def test_horizontal_diffusion_of_every_stagger(n, nz):
+    """The stand-alone diffusion of each variable against its reverse: both
+    are bilinear, <D(f), c> = <f, D^T c> (float32 products summed in float64:
+    1e-5 of the sum of their sizes)."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    data = {k: 1.0 + 0.1 * torch.rand(n, n, generator=gen, device="cuda") for k in A.HDIFF_DATA}
+    mut, xk = 9.0e4 + 100.0 * rnd(n, n), 1.0e3 * (1.0 + 0.1 * rnd(nz, n, n))
+    for var in "uvwm":
+        f, c = rnd(nz, n, n).requires_grad_(True), rnd(nz, n, n)
+        out = A.horizontal_diffusion(var, f, torch.zeros_like(f), mut, xk, data, 1 / 9000.0, 1 / 9000.0)
+        (g,) = torch.autograd.grad(out, f, grad_outputs=c)
+        lhs, rhs = (out.detach().double() * c).sum(), (f.detach().double() * g).sum()
+        size = (out.detach().double() * c).abs().sum()
+        assert float(size) > 0 and abs(float(lhs - rhs)) <= 1e-5 * float(size), var
+
+
+
+
+@pytest.mark.parametrize("n,nz", [(24, 12), (37, 16), (64, 17), (33, 41)])
+def test_advance_uv_reverse_at_the_ends_of_its_level_chunks(n, nz):
+    """The pressure-gradient part A B + C D is homogeneous in its factors: of
+    degree one in (muu, muv, php), of (ph, alt, al) in B, of (p, mu) in D and
+    of (alt p, al pb) pairwise, so by Euler's identity the products of the
+    values and their cotangents agree in four ways (float32 terms of some ten
+    roundings summed in float64: 1e-5 of the sum of their sizes)."""
+    gen = torch.Generator(device="cuda").manual_seed(n * nz)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    two_d = {"mu", "muu", "muv", "mudf"}
+    x = {k: rnd(*((n, n) if k in two_d else (nz, n, n))).requires_grad_(True) for k in A.UV_INPUTS}
+    data = {k: (rnd(nz) if k in ("fnm", "fnp", "rdnw") else 1.0 + 0.1 * rnd(n, n)) for k in A.UV_DATA}
+    u, v = A.advance_uv(x, data, 9.0, 0.01, 2.0, -1.5, 0.5, 1 / 9000.0, 1 / 9000.0)
+    grads = torch.autograd.grad((u, v), list(x.values()), grad_outputs=[rnd(nz, n, n), rnd(nz, n, n)])
+    prod = {k: (x[k].detach().double() * gk) for k, gk in zip(x, grads)}
+
+    def agree(left, right):
+        a, b = (sum(prod[k].sum() for k in side) for side in (left, right))
+        size = sum(prod[k].abs().sum() for k in left + right)
+        assert float(size) > 0 and abs(float(a - b)) <= 1e-5 * float(size), (left, right)
+
+    agree(("cqu", "cqv"), ("muu", "muv", "php"))
+    agree(("muu", "muv"), ("ph", "alt", "al"))
+    agree(("p", "mu"), ("alt", "php"))
+    agree(("pb",), ("al",))
+
+
+@pytest.mark.parametrize("n,nz", [(24, 12), (41, 15), (50, 40)])
+def test_advect_scalar_reverse_is_its_transpose(n, nz):
+    """The advection is linear in the field, and in the fluxes for fixed
+    signs: <A q, c> = <q, A^T c> = the fluxes' products (1e-5 of the sum of
+    the sizes)."""
+    gen = torch.Generator(device="cuda").manual_seed(n + nz)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    q, ru, rv, rom = (rnd(nz, n, n).requires_grad_(True) for _ in range(4))
+    c = rnd(nz, n, n)
+    out = A.advect_scalar(q, torch.zeros_like(c), ru, rv, rom, 1.0 + 0.1 * rnd(n, n), rnd(nz), rnd(nz), rnd(nz),
+                          1 / 9000.0, 1 / 9000.0)
+    grads = torch.autograd.grad(out, (q, ru, rv, rom), grad_outputs=c)
+    prods = [a.detach().double() * b for a, b in zip((out, q, ru, rv, rom), (c,) + grads)]
+    lhs, field, fluxes = prods[0].sum(), prods[1].sum(), sum(p.sum() for p in prods[2:])
+    size = float(prods[0].abs().sum() + prods[1].abs().sum() + sum(p.abs().sum() for p in prods[2:]))
+    assert size > 0 and abs(float(lhs - field)) <= 1e-5 * size and abs(float(lhs - fluxes)) <= 1e-5 * size
+
+
+@pytest.mark.parametrize("n", [300, 61], ids=["sorted", "own"])
+def test_microphysics_reverse_by_levels_against_the_tangents(n):
+    """Domains on either side of the line from which a block sorts its points
+    before their tangents: the column, sedimentation tapes and all, against
+    forward-mode tangents of the whole column (the tape capacity at 1), to the
+    float32 summation order that the small case is held to (relative L2 1e-5)."""
+    from test_gpu_adjoint import MP_OUT, _microphysics_state_before_step2
+
+    g, snap = _microphysics_state_before_step2()
+    pick = 6 + np.arange(n) % 16
+
+    def wide(v):
+        v = np.asarray(v, np.float32)
+        if v.ndim >= 2 and v.shape[-2:] == (g.ny, g.nx):
+            v = v[..., pick[:, None], pick[None, :]]
+        return torch.tensor(np.ascontiguousarray(v), device="cuda")
+
+    st = {k: wide(snap[k]) for k in A._Microphysics.fields}
+    data = {k: wide(snap[k]) for k in A._Microphysics.data}
+    st["t"] += 0.2 * torch.sin(torch.arange(st["t"].numel(), device="cuda").view_as(st["t"]).float())
+    dt = float(g.dt)
+    out = A.microphysics(st, data, dt, g.rdx, g.rdy)
+    cg = A.scalar_grid(st["t"].shape, g.rdx, g.rdy)
+    cg.dt = dt
+    tab = A._table({**st, **data})
+    post = A._table({**st, **data, **{k: out[k].detach() for k in ("t", "moist", "al", "p")}})
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    seeds = {k: torch.randn(st[k].shape, generator=gen, device="cuda") for k in MP_OUT}
+
+    def reverse(capacity):
+        prev = ctypes.c_int(-1)
+        N.check(N.lib().wrf_set_microphysics_tape_capacity(capacity, ctypes.byref(prev)), "capacity")
+        try:
+            bars = {k: torch.zeros_like(st[k]) for k in ("t", "moist", "al", "p", "ph", "mu", "muts", "h_diabatic")}
+            bars.update({k: torch.zeros_like(st["t"]) for k in ("alb", "pb")})
+            for k in MP_OUT:
+                bars[k].copy_(seeds[k])
+            words = ctypes.c_size_t(0)
+            N.check(N.lib().wrf_microphysics_adj_work(ctypes.byref(cg), ctypes.byref(words)), "work")
+            work = torch.empty(int(words.value), dtype=torch.float32, device="cuda")
+            N.check(N.lib().wrf_microphysics_adj(ctypes.byref(cg), tab, post, A._table(bars), _p(work), words, None,
+                                                 _stream()), "adj")
+            torch.cuda.synchronize()
+            return bars
+        finally:
+            N.check(N.lib().wrf_set_microphysics_tape_capacity(prev.value, None), "restore")
+
+    taped, tangents = reverse(0), reverse(1)
+    for k in ("t", "moist", "al", "p", "ph"):
+        a, b = taped[k].double(), tangents[k].double()
+        assert float((a - b).norm()) <= 1e-5 * float(b.norm()), k
+    assert float(taped["moist"][3].abs().max()) > 0.0
