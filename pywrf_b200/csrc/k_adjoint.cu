@@ -2030,48 +2030,40 @@ namespace {
 // the linear forms of one face flux F = V Phi: Phi = sum qc[n] q[qi[n]],
 // V = sum rc[n] r[ri[n]] (r: ru for x faces, rv for y faces, rom for z faces)
 struct FaceLin {
-  int nq = 0, nr = 0;
-  size_t qi[6];
-  float qc[6];
-  size_t ri[2];
-  float rc[2];
+  float w[6];   // dPhi/dq at stencil offsets -3 .. 2 along D, [lo, hi] of them in use
+  int lo, hi;
+  float c0, c1; // V = c0 r(p - r0 d) + c1 r(p - (r0 + 1) d), d the component's own stride
+  int r0;
 };
 
 struct MomAdjArgs {
   const float *q, *ru, *rv, *rom, *msf, *msf2, *fzm, *fzp, *rdz;
 };
 
-__device__ __forceinline__ size_t off(size_t b, int o, size_t st) {
-  return (size_t)((long long)b + (long long)o * (long long)st);
+__device__ __forceinline__ void put5(FaceLin& L, float s) {
+  L.lo = 0;
+  L.hi = 5;
+#pragma unroll
+  for (int o = -3; o <= 2; ++o) L.w[o + 3] = w5(o, s);
 }
-__device__ __forceinline__ void put5(FaceLin& L, size_t b, size_t st, float s) {
-  L.nq = 6;
-  for (int o = -3; o <= 2; ++o) {
-    L.qi[o + 3] = off(b, o, st);
-    L.qc[o + 3] = w5(o, s);
-  }
+__device__ __forceinline__ void put3(FaceLin& L, float s) {
+  L.lo = 1;
+  L.hi = 4;
+#pragma unroll
+  for (int o = -2; o <= 1; ++o) L.w[o + 3] = w3(o, s);
 }
-__device__ __forceinline__ void put3(FaceLin& L, size_t b, size_t st, float s) {
-  L.nq = 4;
-  for (int o = -2; o <= 1; ++o) {
-    L.qi[o + 2] = off(b, o, st);
-    L.qc[o + 2] = w3(o, s);
-  }
+// c0 q(p) + cm q(p - st)
+__device__ __forceinline__ void put2(FaceLin& L, float c0, float cm) {
+  L.lo = 2;
+  L.hi = 3;
+  L.w[2] = cm;
+  L.w[3] = c0;
 }
-__device__ __forceinline__ void put2(FaceLin& L, size_t i0, float c0, size_t i1, float c1) {
-  L.nq = 2;
-  L.qi[0] = i0;
-  L.qc[0] = c0;
-  L.qi[1] = i1;
-  L.qc[1] = c1;
-}
-// V = c0 r[i0] + c1 r[i1], returned
-__device__ __forceinline__ float putr(FaceLin& L, const float* r, size_t i0, float c0, size_t i1, float c1) {
-  L.nr = 2;
-  L.ri[0] = i0;
-  L.rc[0] = c0;
-  L.ri[1] = i1;
-  L.rc[1] = c1;
+// V, returned (r0: the first of its two points)
+__device__ __forceinline__ float putr(FaceLin& L, const float* r, size_t i0, float c0, size_t i1, float c1, int r0 = 0) {
+  L.c0 = c0;
+  L.c1 = c1;
+  L.r0 = r0;
   return c0 * r[i0] + c1 * r[i1];
 }
 
@@ -2079,78 +2071,76 @@ __device__ __forceinline__ float putr(FaceLin& L, const float* r, size_t i0, flo
 // i or k along D.  Returns false where the forward has no flux.  The cases
 // and their order are those of fqy_u .. vf_w (k_tend.cu).
 template <int C, int D>
-__device__ bool face_lin(const Grid& g, const MomAdjArgs& a, int k, int j, int i, FaceLin& L) {
+__device__ bool face_lin(const Grid& g, const MomAdjArgs& a, int k, int j, int i, FaceLin& L, float& v) {
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde, ktf = g.nz - 1, nx = g.nx;
   const size_t lev = (size_t)g.ny * nx;
   const size_t p = (size_t)k * lev + (size_t)j * nx + i;
   const float* q = a.q;
   if (D == 0) {  // y faces, rv
     const int jf = j;
-    float v;
     if (C == 0) {
       v = putr(L, a.rv, p, 0.5f, p - 1, 0.5f);
-      if (jf >= jds + 3 && jf < jde - 3) put5(L, p, nx, sgnf(v));
-      else if (jf == jds + 1) put2(L, p, 0.5f, p - nx, 0.5f);
-      else if (jf == jds + 2) put3(L, p, nx, sgnf(v));
-      else if (jf == jde - 2) put2(L, p, 0.5f, p - nx, 0.5f);
-      else if (jf == jde - 3) put3(L, p, nx, 1.0f);  // the reference's sign source there is 0
+      if (jf >= jds + 3 && jf < jde - 3) put5(L, sgnf(v));
+      else if (jf == jds + 1) put2(L, 0.5f, 0.5f);
+      else if (jf == jds + 2) put3(L, sgnf(v));
+      else if (jf == jde - 2) put2(L, 0.5f, 0.5f);
+      else if (jf == jde - 3) put3(L, 1.0f);  // the reference's sign source there is 0
       else return false;
     } else if (C == 1) {
       v = putr(L, a.rv, p, 0.5f, p - nx, 0.5f);
-      if (jf >= jds + 3 && jf < jde - 2) put5(L, p, nx, sgnf(v));
+      if (jf >= jds + 3 && jf < jde - 2) put5(L, sgnf(v));
       else if (jf == jds + 1) {
-        if (q[p] < 0.f) put2(L, p, 1.0f, p - nx, 0.0f);
-        else put2(L, p, 0.5f, p - nx, 0.5f);
-      } else if (jf == jds + 2) put3(L, p, nx, sgnf(v));
+        if (q[p] < 0.f) put2(L, 1.0f, 0.0f);
+        else put2(L, 0.5f, 0.5f);
+      } else if (jf == jds + 2) put3(L, sgnf(v));
       else if (jf == jde - 1) {
-        if (q[p - nx] > 0.f) put2(L, p - nx, 1.0f, p, 0.0f);
-        else put2(L, p - nx, 0.5f, p, 0.5f);
-      } else if (jf == jde - 2) put3(L, p, nx, sgnf(v));
+        if (q[p - nx] > 0.f) put2(L, 0.0f, 1.0f);
+        else put2(L, 0.5f, 0.5f);
+      } else if (jf == jde - 2) put3(L, sgnf(v));
       else return false;
     } else {
       if (k < 1) return false;
       v = k < ktf ? putr(L, a.rv, p, a.fzm[k], p - lev, a.fzp[k])
-                  : putr(L, a.rv, p - lev, 2.0f - a.fzm[ktf - 1], p - 2 * lev, -a.fzp[ktf - 1]);
-      if (jf >= jds + 3 && jf < jde - 3) put5(L, p, nx, sgnf(v));
-      else if (jf == jds + 1) put2(L, p, 0.5f, p - nx, 0.5f);
-      else if (jf == jds + 2) put3(L, p, nx, sgnf(v));
-      else if (jf == jde - 2) put2(L, p, 0.5f, p - nx, 0.5f);
-      else if (jf == jde - 3) put3(L, p, nx, sgnf(v));
+                  : putr(L, a.rv, p - lev, 2.0f - a.fzm[ktf - 1], p - 2 * lev, -a.fzp[ktf - 1], 1);
+      if (jf >= jds + 3 && jf < jde - 3) put5(L, sgnf(v));
+      else if (jf == jds + 1) put2(L, 0.5f, 0.5f);
+      else if (jf == jds + 2) put3(L, sgnf(v));
+      else if (jf == jde - 2) put2(L, 0.5f, 0.5f);
+      else if (jf == jde - 3) put3(L, sgnf(v));
       else return false;
     }
     return true;
   } else if (D == 1) {  // x faces, ru
     const int f = i;
-    float v;
     if (C == 0) {
       v = putr(L, a.ru, p, 0.5f, p - 1, 0.5f);
-      if (f >= ids + 3 && f < ide - 2) put5(L, p, 1, sgnf(v));
+      if (f >= ids + 3 && f < ide - 2) put5(L, sgnf(v));
       else if (f == ids + 1) {
-        if (q[p] < 0.f) put2(L, p, 1.0f, p - 1, 0.0f);
-        else put2(L, p, 0.5f, p - 1, 0.5f);
-      } else if (f == ids + 2) put3(L, p, 1, sgnf(v));
+        if (q[p] < 0.f) put2(L, 1.0f, 0.0f);
+        else put2(L, 0.5f, 0.5f);
+      } else if (f == ids + 2) put3(L, sgnf(v));
       else if (f == ide - 1) {
-        if (q[p - 1] > 0.f) put2(L, p - 1, 1.0f, p, 0.0f);
-        else put2(L, p - 1, 0.5f, p, 0.5f);
-      } else if (f == ide - 2) put3(L, p, 1, sgnf(v));
+        if (q[p - 1] > 0.f) put2(L, 0.0f, 1.0f);
+        else put2(L, 0.5f, 0.5f);
+      } else if (f == ide - 2) put3(L, sgnf(v));
       else return false;
     } else if (C == 1) {
       v = putr(L, a.ru, p, 0.5f, p - nx, 0.5f);
-      if (f >= ids + 3 && f < ide - 3) put5(L, p, 1, sgnf(v));
-      else if (f == ids + 1) put2(L, p, 0.5f, p - 1, 0.5f);
-      else if (f == ids + 2) put3(L, p, 1, sgnf(v));
-      else if (f == ide - 2) put2(L, p, 0.5f, p - 1, 0.5f);
-      else if (f == ide - 3) put3(L, p, 1, sgnf(v));
+      if (f >= ids + 3 && f < ide - 3) put5(L, sgnf(v));
+      else if (f == ids + 1) put2(L, 0.5f, 0.5f);
+      else if (f == ids + 2) put3(L, sgnf(v));
+      else if (f == ide - 2) put2(L, 0.5f, 0.5f);
+      else if (f == ide - 3) put3(L, sgnf(v));
       else return false;
     } else {
       if (k < 1) return false;
       v = k < ktf ? putr(L, a.ru, p, a.fzm[k], p - lev, a.fzp[k])
-                  : putr(L, a.ru, p - lev, 2.0f - a.fzm[ktf - 1], p - 2 * lev, -a.fzp[ktf - 1]);
-      if (f >= ids + 3 && f < ide - 3) put5(L, p, 1, sgnf(v));
-      else if (f == ids + 1) put2(L, p, 0.5f, p - 1, 0.5f);
-      else if (f == ids + 2) put3(L, p, 1, sgnf(v));
-      else if (f == ide - 2) put2(L, p, 0.5f, p - 1, 0.5f);
-      else if (f == ide - 3) put3(L, p, 1, sgnf(v));
+                  : putr(L, a.ru, p - lev, 2.0f - a.fzm[ktf - 1], p - 2 * lev, -a.fzp[ktf - 1], 1);
+      if (f >= ids + 3 && f < ide - 3) put5(L, sgnf(v));
+      else if (f == ids + 1) put2(L, 0.5f, 0.5f);
+      else if (f == ids + 2) put3(L, sgnf(v));
+      else if (f == ide - 2) put2(L, 0.5f, 0.5f);
+      else if (f == ide - 3) put3(L, sgnf(v));
       else return false;
     }
     return true;
@@ -2159,20 +2149,20 @@ __device__ bool face_lin(const Grid& g, const MomAdjArgs& a, int k, int j, int i
     if (kf < 1) return false;
     if (C == 0 || C == 1) {
       const size_t nb = C == 0 ? 1 : (size_t)nx;  // the second rom point: i-1 (u) or j-1 (v)
-      const float v = putr(L, a.rom, p, 0.5f, p - nb, 0.5f);
-      if (kf >= 3 && kf < ktf - 2) put5(L, p, lev, sgnf(-v));
-      else if (kf == 1) put2(L, p, a.fzm[kf], p - lev, a.fzp[kf]);
-      else if (kf == 2) put3(L, p, lev, sgnf(-v));
-      else if (kf == ktf - 2) put3(L, p, lev, C == 0 ? sgnf(-v) : sgnf(v));
-      else if (kf == ktf - 1) put2(L, p, a.fzm[kf], p - lev, a.fzp[kf]);
+      v = putr(L, a.rom, p, 0.5f, p - nb, 0.5f);
+      if (kf >= 3 && kf < ktf - 2) put5(L, sgnf(-v));
+      else if (kf == 1) put2(L, a.fzm[kf], a.fzp[kf]);
+      else if (kf == 2) put3(L, sgnf(-v));
+      else if (kf == ktf - 2) put3(L, C == 0 ? sgnf(-v) : sgnf(v));
+      else if (kf == ktf - 1) put2(L, a.fzm[kf], a.fzp[kf]);
       else return false;
     } else {
-      const float v = putr(L, a.rom, p, 0.5f, p - lev, 0.5f);
-      if (kf >= 3 && kf < ktf - 1) put5(L, p, lev, sgnf(-v));
-      else if (kf == 1) put2(L, p, 0.5f, p - lev, 0.5f);
-      else if (kf == 2) put3(L, p, lev, sgnf(-v));
-      else if (kf == ktf - 1) put3(L, p, lev, sgnf(v));
-      else if (kf == ktf) put2(L, p, 0.5f, p - lev, 0.5f);
+      v = putr(L, a.rom, p, 0.5f, p - lev, 0.5f);
+      if (kf >= 3 && kf < ktf - 1) put5(L, sgnf(-v));
+      else if (kf == 1) put2(L, 0.5f, 0.5f);
+      else if (kf == 2) put3(L, sgnf(-v));
+      else if (kf == ktf - 1) put3(L, sgnf(v));
+      else if (kf == ktf) put2(L, 0.5f, 0.5f);
       else return false;
     }
     return true;
@@ -2233,13 +2223,10 @@ __device__ float fbar(const Grid& g, const MomAdjArgs& a, const float* tbar, int
 // per distance d of the component's velocity forms: d in {0, 1} for u,
 // {0, nx} for v, {0, lev, 2 lev} for w).  Pass 2 gathers each point's
 // cotangents from the slots that address it, in a fixed order (one writer
-// per output element, no atomics).
-template <int C>
-__device__ __forceinline__ int r_slot(size_t d, size_t nx, size_t lev) {
-  if (C == 0) return (int)d;
-  if (C == 1) return d == 0 ? 0 : 1;
-  return d == 0 ? 0 : (d == lev ? 1 : 2);
-}
+// per output element).  A face's weights are kept by slot: found again from
+// the points' addresses (a 64-bit division each) they were most of the
+// instructions of pass 1, 218 us per component at 240x240x41; 67 to 83
+// now.
 template <int C>
 __device__ __forceinline__ size_t r_dist(int s, size_t nx, size_t lev) {
   if (C == 0) return (size_t)s;
@@ -2258,23 +2245,20 @@ __device__ __forceinline__ void face_pass(const Grid& g, const MomAdjArgs& a, co
   float q6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, r3[3] = {0.f, 0.f, 0.f};
   const float fb = fbar<C, D>(g, a, tbar, k, j, i);
   FaceLin L;
-  if (fb != 0.f && face_lin<C, D>(g, a, k, j, i, L)) {
-    const float* r = D == 0 ? a.rv : D == 1 ? a.ru : a.rom;
-    const long long st = D == 0 ? (long long)nx : D == 1 ? 1 : (long long)lev;
-    float v = 0.f, phi = 0.f;
-    for (int n = 0; n < L.nr; ++n) v += L.rc[n] * r[L.ri[n]];
-    for (int n = 0; n < L.nq; ++n) phi += L.qc[n] * a.q[L.qi[n]];
+  float v = 0.f;
+  if (fb != 0.f && face_lin<C, D>(g, a, k, j, i, L, v)) {
+    const float* q = a.q + p;
+    const int st = D == 0 ? (int)nx : D == 1 ? 1 : (int)lev;
+    float phi = 0.f;
+#pragma unroll
+    for (int s = 0; s < 6; ++s)
+      if (s >= L.lo && s <= L.hi) phi += L.w[s] * q[(s - 3) * st];
     const float gv = fb * v, gp = fb * phi;
-    for (int n = 0; n < L.nq; ++n) {
-      const int slot = (int)(((long long)L.qi[n] - (long long)p) / st) + 3;
 #pragma unroll
-      for (int s = 0; s < 6; ++s) q6[s] += slot == s ? gv * L.qc[n] : 0.f;
-    }
-    for (int n = 0; n < L.nr; ++n) {
-      const int slot = r_slot<C>(p - L.ri[n], nx, lev);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) r3[s] += slot == s ? gp * L.rc[n] : 0.f;
-    }
+    for (int s = 0; s < 6; ++s) q6[s] = s >= L.lo && s <= L.hi ? gv * L.w[s] : 0.f;
+    r3[0] = L.r0 == 0 ? gp * L.c0 : 0.f;
+    r3[1] = gp * (L.r0 == 0 ? L.c1 : L.c0);
+    r3[2] = L.r0 == 0 ? 0.f : gp * L.c1;
   }
 #pragma unroll
   for (int s = 0; s < 6; ++s) Q[(size_t)(D * 6 + s) * n3 + p] = q6[s];
