@@ -1317,9 +1317,9 @@ __global__ void __launch_bounds__(32 * kAwGroups, 3) k_advance_w_adj_lp(Grid g, 
   auto A = [&](int arr, int k) -> float& { return L.A(arr, k); };
   auto F = [&](int id, int k) { return __ldg(&s[id][k * lev + c]); };
   auto B = [&](int id, int k) -> float& { return b[id][k * lev + c]; };
-  enum { T2A = AwLp<true>::T2A, WD = AwLp<true>::WD, RR = AwLp<true>::RR, PP = AwLp<true>::PP, XX = AwLp<true>::XX, YY = AwLp<true>::YY,
-         ZZ = AwLp<true>::ZZ, ZB = AwLp<true>::ZB, YB = AwLp<true>::YB, PB = AwLp<true>::PB, RHSB = AwLp<true>::RHSB, CA = AwLp<true>::CA,
-         CAL = AwLp<true>::CAL, CG = AwLp<true>::CG };
+  using Lp = AwLp<true>;
+  enum { T2A = Lp::T2A, WD = Lp::WD, RR = Lp::RR, PP = Lp::PP, XX = Lp::XX, YY = Lp::YY, ZZ = Lp::ZZ, ZB = Lp::ZB,
+         YB = Lp::YB, PB = Lp::PB, RHSB = Lp::RHSB, CA = Lp::CA, CAL = Lp::CAL, CG = Lp::CG };
   // ask L2 for what the later phases load (no registers, and the phases find
   // their operands in L2 instead of waiting on DRAM one after another: 343 -> 319
   // us per launch at 240x240x41)
