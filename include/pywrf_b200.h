@@ -361,16 +361,20 @@ int wrf_microphysics_adj_work(const WrfGrid* g, size_t* floats);
  * those of the inputs, while ph, mu, muts, alb and pb accumulate.  The
  * equation of state is reversed exactly; prep + WSM6 + finish by reverse
  * mode over a per-column restatement of the scheme (the derivative of the
- * branch taken): each column runs once on taped scalars and one reverse
- * sweep of its tape gives its inputs' cotangents; a column whose tape
- * outgrows the capacity takes forward-mode tangents of the same
- * restatement instead.  values (optional: t, moist, h_diabatic) receives
- * that restatement's own outputs, for checking it against the forward. */
+ * branch taken): with one time-split loop the sedimentation of each column
+ * runs once on taped scalars, reversed by one sweep of the tape, and all else
+ * takes forward-mode tangents per level; with several the whole column is
+ * taped.  A column whose tape outgrows the capacity takes forward-mode
+ * tangents of the whole restatement instead.  values (optional: t, moist,
+ * h_diabatic) receives that restatement's own outputs, for checking it against
+ * the forward. */
 int wrf_microphysics_adj(const WrfGrid* g, const WrfState* s, const WrfState* post, const WrfState* sbar,
                          float* work, size_t work_floats, const WrfState* values, void* stream);
 /* The tape capacity of wrf_microphysics_adj in entries per column, for the
- * whole library (0 restores the default, 480 entries per level plus the
- * inputs, at most 65535); *previous (optional) receives the setting it
+ * whole library (0 restores the default, 256 entries per level with one
+ * time-split loop, 480 per level and loop with several, plus the inputs, at
+ * most 65535; with one loop rain, snow with graupel, and ice share it 75 : 138 :
+ * 53); *previous (optional) receives the setting it
  * replaces.  A capacity below the column's input count sends every column
  * to the tangents.  Call wrf_microphysics_adj_work again after changing
  * it. */
