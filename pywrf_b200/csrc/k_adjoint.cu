@@ -419,9 +419,10 @@ __device__ UvTerm uv_term(const Grid& g, const S& s, const S& b, float dts, int 
 // it and the sums are carried in registers, where a thread per point formed
 // sixteen face levels (their map-factor divisions included) and two more for
 // cqu and cqv: 372 us per launch at 240x240x41 and 61 us at 101x101x35, at a
-// memory floor of 50 and 8; 150 and 38 us now, with the
+// memory floor of 50 and 8; 125 and 28 us now, with the
 // cotangents that it only adds to as reductions.
-constexpr int kUvChunk = 8;
+// At most eight levels a chunk, of equal length, fewer where that leaves SMs
+// short of blocks.
 __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float dts) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = g.nx, ny = g.ny, ktf = g.nz - 1, lev = ny * nx;
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
     }
     return v;
   };
-  const int k0 = blockIdx.z * kUvChunk, k1 = min(k0 + kUvChunk, g.nz);
+  const int k0 = blockIdx.z * g.nz / gridDim.z, k1 = (blockIdx.z + 1) * g.nz / gridDim.z;
   const float* rdnw = s[WF_RDNW];
   const float *fnm = s[WF_FNM], *fnp = s[WF_FNP];
   Level cur = level(k0 - 1);
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(32 * kColLevels) k_advance_uv_adj_col(Grid g, 
 
 int launch_advance_uv_adj(const Grid& g, const S& s, const S& b, float dts, cudaStream_t st) {
   dim3 b3(32, 4), gr = point_grid(g, b3);
-  gr.z = (g.nz + kUvChunk - 1) / kUvChunk;
+  gr.z = level_chunks(g.nz, gr.x * gr.y, 8, 6);
   k_advance_uv_adj<<<gr, b3, 0, st>>>(g, s, b, dts);
   k_advance_uv_adj_col<<<dim3((g.nx + 31) / 32, g.ny), dim3(32, kColLevels), 0, st>>>(g, s, b, dts);
   return 2;
