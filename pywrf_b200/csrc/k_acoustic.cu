@@ -231,17 +231,17 @@ static void run_coef_w(const Grid& g, const S& s, float dts, cudaStream_t st) {
 }
 
 // advance_uv for rows that are no multiple of 16 bytes (and the cross-check of
-// the tensor-map form below): a thread marches kUvLevels levels of its column,
+// the tensor-map form below): a thread marches LZ levels of its column,
 // its ph, p and vertical averages carried in registers and its map factors,
 // with their divisions, formed once.  A thread per point loaded two and a half
 // times as much and waited for it in two rounds, the second behind u's store:
-// 19.7 -> 14.6 us per launch at 131x131x35.
-constexpr int kUvLevels = 4;
+// 19.7 -> 12.4 us per launch at 131x131x35, 14.3 -> 10.1 at 101x101x35.
+template <int LZ>
 __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx;
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde;
-  const int k0 = blockIdx.z * kUvLevels, k1 = min(k0 + kUvLevels, ktf);
+  const int k0 = blockIdx.z * LZ, k1 = min(k0 + LZ, ktf);
   if (i >= nx || j >= g.ny) return;
   // updated points, and the specified rows (spec_bdyupdate)
   const bool uin = j >= jds + 1 && j < jde - 2 && i >= ids + 1 && i < ide - 1;
@@ -1633,8 +1633,14 @@ int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st) {
   }
   const dim3 b3(32, 4);
   dim3 gr = point_grid(g, b3);
-  gr.z = (g.nz - 1 + kUvLevels - 1) / kUvLevels;
-  k_advance_uv<<<gr, b3, 0, st>>>(g, s, dts);
+  // short chunks while the grid is about one wave (ten blocks fit an SM): with
+  // two, three and four levels 10.1, 11.7 and 14.2 us at 101x101x35, 16.4, 12.4
+  // and 14.6 at 131x131x35
+  const int ktf = g.nz - 1;
+  const bool two = (long long)gr.x * gr.y * ((ktf + 1) / 2) <= 148 * 12;
+  gr.z = two ? (ktf + 1) / 2 : (ktf + 2) / 3;
+  if (two) k_advance_uv<2><<<gr, b3, 0, st>>>(g, s, dts);
+  else k_advance_uv<3><<<gr, b3, 0, st>>>(g, s, dts);
   return 1;
 }
 
