@@ -135,10 +135,14 @@
 
 namespace wrf {
 
-// dynamic shared memory above 48 KB has to be allowed kernel by kernel
+// A block's shared memory above 48 KB has to be allowed kernel by kernel: the
+// limit is on the sum of the dynamic part and the kernel's own arrays (at most
+// kOwnSmem here), which reaches it at 64 levels before the dynamic part alone.
+constexpr size_t kOwnSmem = 4 * 1024;
 template <typename K>
 static void allow_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes + kOwnSmem > 48 * 1024)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 namespace {

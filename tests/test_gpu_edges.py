@@ -312,3 +312,85 @@ def test_microphysics_reverse_by_levels_against_the_tangents(n):
         a, b = taped[k].double(), tangents[k].double()
         assert float((a - b).norm()) <= 1e-5 * float(b.norm()), k
     assert float(taped["moist"][3].abs().max()) > 0.0
+
+
+def _column_operator(name, x, data, sc):
+    """The operator's outputs on CUDA tensors, in the order of its fixture's
+    cotangents."""
+    rd = (1.0 / sc["dx"], 1.0 / sc["dy"])
+    if name == "coefw":
+        return A.coef_w(x["mut"], x["cqw"], x["c2a"], data["rdn"], data["rdnw"], sc["dts"], epssm=sc["epssm"])
+    if name == "prho":
+        return A.calc_p_rho(x, data["rdnw"], sc["smdiv"], 1, *rd)
+    if name == "mut":
+        out = A.advance_mu_t(x, data, sc["dts"], sc["epssm"], *rd)
+        return [out[k] for k in A.MUT_OUTPUTS]
+    out = A.advance_w(x, data, sc["dts"], sc["epssm"], sc["cf1"], sc["cf2"], sc["cf3"], *rd)
+    return [out[k] for k in A.AW_OUTPUTS]
+
+
+def _column_oracle(name, g, x, data, sc):
+    from oracle import dynamics as OD
+
+    x = {k: v.copy() for k, v in x.items()}
+    if name == "coefw":
+        out = [np.zeros_like(x["cqw"]) for _ in range(3)]
+        OD.calc_coef_w(g, *out, x["mut"], x["cqw"], data["rdn"], data["rdnw"], x["c2a"], sc["dts"], sc["epssm"])
+        return out
+    if name == "prho":
+        pm1 = OD.calc_p_rho(g, *[x[k] for k in A.PRHO_INPUTS], data["rdnw"], sc["smdiv"], 1)
+        return [x["al"], x["p"], pm1]
+    names, outs = (A._MUT_FIELD, A.MUT_OUTPUTS) if name == "mut" else (A._AW_FIELD, A.AW_OUTPUTS)
+    st = {names.get(k, k): v for k, v in x.items()} | data
+    if name == "mut":
+        OD.advance_mu_t(g, st, sc["dts"], sc["epssm"], 1)
+    else:
+        OD.advance_w(g, st, sc["dts"], sc["epssm"], sc["cf1"], sc["cf2"], sc["cf3"])
+    return [st[names.get(k, k)] for k in outs]
+
+
+@pytest.mark.parametrize("name,inputs,data", [("coefw", ("mut", "cqw", "c2a"), ("rdn", "rdnw")),
+                                              ("prho", A.PRHO_INPUTS, ("rdnw",)),
+                                              ("mut", A.MUT_INPUTS, A.MUT_DATA), ("advw", A.AW_INPUTS, A.AW_DATA)],
+                         ids=["coef_w", "calc_p_rho", "advance_mu_t", "advance_w"])
+def test_column_reverses_at_the_greatest_depth(name, inputs, data):
+    """64 levels, the deepest accepted column and so the largest shared
+    memory: the operator against the float64 oracle on its fixture's profiles
+    stretched over the column, and the reverse's derivative along one random
+    direction per input against the oracle's central differences (the
+    fixtures' tolerance, of the gradient's size: a sum of 64 levels' terms in
+    float32)."""
+    from helpers import load_npz, rel_l2
+
+    z, nz = load_npz(f"{name}_adj_ref64.npz"), 64
+    sc = {k: float(z[k]) for k in ("dts", "epssm", "smdiv", "cf1", "cf2", "cf3") if k in z}
+    g = synthetic.grid_for(synthetic.CaseSpec(n=24, nz=nz))
+    sc |= {"dx": g.dx, "dy": g.dy}
+
+    def deep(v):
+        if v.ndim == 2:
+            return v.astype(np.float32)
+        at = np.linspace(0.0, v.shape[0] - 1.0, nz)
+        lo = np.minimum(at.astype(int), v.shape[0] - 2)
+        w = (at - lo).reshape((nz,) + (1,) * (v.ndim - 1))
+        return ((1.0 - w) * v[lo] + w * v[lo + 1]).astype(np.float32)
+
+    x, dd = {k: deep(z[k]) for k in inputs}, {k: deep(z[k]) for k in data}
+    xg = {k: torch.tensor(v, device="cuda").requires_grad_(True) for k, v in x.items()}
+    outs = _column_operator(name, xg, {k: torch.tensor(v, device="cuda") for k, v in dd.items()}, sc)
+    x64, d64 = ({k: v.astype(np.float64) for k, v in q.items()} for q in (x, dd))
+    want = _column_oracle(name, g, x64, d64, sc)
+    rng = np.random.default_rng(64)
+    cots = [rng.standard_normal(o.shape).astype(np.float32) for o in want]
+    for o, ref in zip(outs, want):
+        assert rel_l2(o.detach().cpu().numpy(), ref) < 1e-5
+    grads = torch.autograd.grad(outs, list(xg.values()), grad_outputs=[torch.tensor(c, device="cuda") for c in cots])
+
+    def loss(v):
+        return sum(float((o * c).sum()) for o, c in zip(_column_oracle(name, g, v, d64, sc), cots))
+
+    for k, gk in zip(inputs, grads):
+        gr, d = gk.double().cpu().numpy(), rng.standard_normal(x64[k].shape)
+        eps = float(z[f"fd_eps_{k}"]) if f"fd_eps_{k}" in z else 1e-4 * float(np.abs(x64[k]).max())
+        fd = (loss({**x64, k: x64[k] + eps * d}) - loss({**x64, k: x64[k] - eps * d})) / (2.0 * eps)
+        assert abs(float((gr * d).sum()) - fd) <= 2e-4 * float(np.sqrt((gr * gr).sum())) + 1e-9, k
