@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kCwTX* kCwKT) k_coef_w(Grid g, S s, float dts,
   const int i = i0 + blockIdx.x * kCwTX + tx, j = g.jds + blockIdx.y;
   const bool col = i >= g.ids && i < g.ide - 1;
   const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
-  const int lev = g.ny * g.nx;
+  const size_t lev = g.n2();
   const double cofd = (0.5 * (double)dts * G * (1.0 + (double)g.epssm)) * (0.5 * (double)dts * G * (1.0 + (double)g.epssm));
   const float cof = (float)cofd, cofm2 = (float)(-2.0 * cofd), cof2 = (float)(2.0 * cofd);
   const float* cqw = s[WF_CQW];
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kCwTX* kCwKT) k_coef_w(Grid g, S s, float dts,
   const float mm = mut * mut, r_mm = __frcp_rn(mm);
 #pragma unroll 4
   for (int k = 1 + tk; k < nz - 1; k += kCwKT) {
-    const int p = k * lev + c;
+    const size_t p = k * lev + c;
     const float cw = __ldg(&cqw[p]), c2k = __ldg(&c2a[p]), c2m = __ldg(&c2a[p - lev]);
     const float rk = __ldg(&rdn[k]), rwk = __ldg(&rdnw[k]), rwm = __ldg(&rdnw[k - 1]);
     sa[k * kCwTX] = k >= 2 ? divc(-cw * cof * rk * rwm * c2m, mm, r_mm) : 0.f;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kCwTX* kCwKT) k_coef_w(Grid g, S s, float dts,
   if (!col) return;
 #pragma unroll 4
   for (int k = tk; k < nz; k += kCwKT) {
-    const int p = k * lev + c;
+    const size_t p = k * lev + c;
     if (k > 0) {
       a[p] = sa[k * kCwTX];
       alpha[p] = sb[k * kCwTX];
@@ -239,7 +239,8 @@ static void run_coef_w(const Grid& g, const S& s, float dts, cudaStream_t st) {
 template <int LZ>
 __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx;
+  const int nz = g.nz, ktf = nz - 1, nx = g.nx;
+  const size_t lev = g.n2();
   const int ids = g.ids, ide = g.ide, jds = g.jds, jde = g.jde;
   const int k0 = blockIdx.z * LZ, k1 = min(k0 + LZ, ktf);
   if (i >= nx || j >= g.ny) return;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
     dpn_v = dpn0(k0, so);
   }
   for (int k = k0; k < k1; ++k) {
-    const int o = k * lev, q = o + c;
+    const size_t o = k * lev, q = o + c;
     const float rdk = __ldg(&s[WF_RDNW][k]);
     const bool top = k + 1 == ktf;
     const float fm1 = top ? 0.f : __ldg(fnm + k + 1), fp1 = top ? 0.f : __ldg(fnp + k + 1);
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
     if (us) un = U[q] + dts * __ldg(&s[WF_RU_TEND][q]);
     if (vs) vn = V[q] + dts * __ldg(&s[WF_RV_TEND][q]);
     if (uin) {
-      const int n = o + w;
+      const size_t n = o + w;
       const float hn = __ldg(ph + n + lev), pn = __ldg(pp + n + lev);
       const float up = top ? 0.f : 0.5f * (fm1 * (pu + pn) + fp1 * (p_c + p_w));
       float dp = cu * (((hu - hn) + (ph_c - ph_w)) + (altc + __ldg(alt + n)) * (p_c - p_w) +
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
       dpn_u = up;
     }
     if (vin) {
-      const int n = o + so;
+      const size_t n = o + so;
       const float hn = __ldg(ph + n + lev), pn = __ldg(pp + n + lev);
       const float up = top ? 0.f : 0.5f * (fm1 * (pu + pn) + fp1 * (p_c + p_s));
       float dp = cv * (((hu - hn) + (ph_c - ph_s)) + (altc + __ldg(alt + n)) * (p_c - p_s) +

@@ -429,7 +429,8 @@ __device__ UvTerm uv_term(const Grid& g, const S& s, const S& b, float dts, int 
 // short of blocks.
 __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float dts) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int nx = g.nx, ny = g.ny, ktf = g.nz - 1, lev = ny * nx;
+  const int nx = g.nx, ny = g.ny, ktf = g.nz - 1;
+  const size_t lev = g.n2();
   if (i >= nx || j >= ny) return;
   const int c = j * nx + i;
   // the faces f = 2 V + e: P = the column itself (e = 0, sign +) or its
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
       const int V = f >> 1;
       v.dpb[f] = v.C[f] = 0.f;
       if (in && on[f]) {
-        const int P = k * lev + cP[f];
+        const size_t P = k * lev + cP[f];
         v.dpb[f] = -dts * __ldg(&s[V ? WF_CQV : WF_CQU][P]) * __ldg(&b[V ? WF_V : WF_U][P]);
         v.C[f] = Cf[f] * (__ldg(php + P) - __ldg(php + k * lev + cQ[f]));
       }
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
     }
   }
   for (int k = k0; k < k1; ++k) {
-    const int m = k * lev + c;
+    const size_t m = k * lev + c;
     const Level next = level(k + 1);
     float aph = cur.phi + phi1, aalt = 0.f, aal = 0.f, apb = 0.f, aphp = 0.f, ap = 0.f, cq[2] = {0.f, 0.f};
     auto wt = [&](int kP) {
@@ -507,7 +508,8 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         if (!on[f]) continue;
-        const int V = f >> 1, P = k * lev + cP[f], Q = k * lev + cQ[f];
+        const int V = f >> 1;
+        const size_t P = k * lev + cP[f], Q = k * lev + cQ[f];
         const float sg = f & 1 ? -1.f : 1.f, Bb = cur.dpb[f] * A[f];
         const float up = __ldg(pp + P + lev) + __ldg(pp + Q + lev);
         const float dn = k + 1 == ktf ? 0.f : 0.5f * (fnm[k + 1] * up + fnp[k + 1] * psum[f]);
@@ -665,7 +667,8 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
   const int tx = threadIdx.x, ty = threadIdx.y, nz = g.nz;
   const int i = blockIdx.x * 32 + tx, j = blockIdx.y;
   const bool col = i < g.nx, on = col && prho_in(g, 0, j, i);
-  const int lev = g.ny * g.nx, c = g.i2(j, col ? i : 0);
+  const size_t lev = g.n2();
+  const int c = g.i2(j, col ? i : 0);
   const float mut = on ? __ldg(&s[WF_MUTS][c]) : 1.f, mu = on ? __ldg(&s[WF_MU][c]) : 0.f;
   const float r_mut = __frcp_rn(mut), ninv = -1.0f / mut;
   const float* rdnw = s[WF_RDNW];
@@ -675,7 +678,8 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
     float alt[kBatch], t1[kBatch], t2[kBatch], c2[kBatch], dph[kBatch], Pb[kBatch], Mb[kBatch], Ab[kBatch];
 #pragma unroll
     for (int q = 0; q < kBatch; ++q) {
-      const int k = k0 + q * kColLevels, p = k * lev + c;
+      const int k = k0 + q * kColLevels;
+      const size_t p = k * lev + c;
       const bool in = on && k < nz - 1;
       Pb[q] = Mb[q] = Ab[q] = alt[q] = t1[q] = t2[q] = c2[q] = dph[q] = 0.f;
       if (in || (step == 0 && k < nz)) {
@@ -693,7 +697,8 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
     }
 #pragma unroll
     for (int q = 0; q < kBatch; ++q) {
-      const int k = k0 + q * kColLevels, p = k * lev + c;
+      const int k = k0 + q * kColLevels;
+      const size_t p = k * lev + c;
       if (k >= nz) break;
       if (!(on && k < nz - 1)) {
         if (step == 0) {
@@ -792,7 +797,7 @@ struct MutDiv {
     r_mfup = __frcp_rn(mfup);
     r_mfu0 = __frcp_rn(mfu0);
   }
-  __device__ __forceinline__ float at(const Grid& g, const S& s, int p) const {
+  __device__ __forceinline__ float at(const Grid& g, const S& s, size_t p) const {
     const int nx = g.nx;
     const float* u = s[WF_U];
     const float* v = s[WF_V];
@@ -832,9 +837,9 @@ __device__ __forceinline__ void mut_scan(const Grid& g, const S& s, bool in, int
 
 // the cotangents of wdtn(k), k in [1, ktf), and of ww'(k), k in [0, ktf), of
 // one level (p: the point, dm = dts msfty)
-__device__ __forceinline__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dm, int k, int p, float& wdb,
+__device__ __forceinline__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dm, int k, size_t p, float& wdb,
                                            float& wwb) {
-  const int lev = g.ny * g.nx;
+  const size_t lev = g.n2();
   const float* t1 = s[WF_T_SAVE];
   const float* rdnw = s[WF_RDNW];
   wdb = 0.f;
@@ -856,7 +861,8 @@ __device__ __forceinline__ float mut_mu_bar(const Grid& g, const S& b, size_t c)
 
 __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, float dts) {
   extern __shared__ float mut_smem[];
-  const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx;
+  const int nz = g.nz, ktf = nz - 1, nx = g.nx;
+  const size_t lev = g.n2();
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
@@ -903,7 +909,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
     for (int q = 0; q < 4; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       tk_[q] = s[WF_T][p];
       tt[q] = s[WF_T_TEND][p];
       const float tc = __ldg(t1 + p);
@@ -917,7 +923,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
     for (int q = 0; q < 4; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       s[WF_WW][p] = sw[k * kMutTX];
       s[WF_T_2SAVE][p] = tk_[q];
       const float t1v = tk_[q] + msfty * dts * tt[q];
@@ -929,7 +935,8 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
 __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, S s, S b, float dts, int ref_no_grad,
                                                                         float* work) {
   extern __shared__ float mut_smem[];
-  const int ktf = g.nz - 1, nx = g.nx, lev = g.ny * nx;
+  const int ktf = g.nz - 1, nx = g.nx;
+  const size_t lev = g.n2();
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
@@ -1010,7 +1017,8 @@ __global__ void k_advance_mu_t_adj_pt(Grid g, S s, S b, float dts, const float* 
 __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g, S s, S b, float dts, int ref_no_grad,
                                                                          const float* work) {
   extern __shared__ float mut_smem[];
-  const int nz = g.nz, ktf = nz - 1, nx = g.nx, lev = g.ny * nx, n = nz * kMutTX;
+  const int nz = g.nz, ktf = nz - 1, nx = g.nx, n = nz * kMutTX;
+  const size_t lev = g.n2();
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   // muu, muv: the u / v terms of the divergence at this column
@@ -1028,7 +1036,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     const float mfu = s[WF_MSFUY][c], r_mfu = __frcp_rn(mfu), mvi = s[WF_MSFVX_INV][c];
 #pragma unroll 4
     for (int k = tk; k < ktf; k += kMutKT) {
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       const float wo = in ? __ldg(work + p) : 0.f;
       float ub = 0.f, vb = 0.f;
       if (w) ub += mw * rdx * __ldg(work + p - 1);
@@ -1044,7 +1052,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     const float dm = dts * s[WF_MSFTY][c];
 #pragma unroll 2
     for (int k = tk; k < ktf; k += kMutKT) {
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       sdv[k * kMutTX] = d.at(g, s, p);
       float wdb, wwb;
       mut_ww_bar(g, s, b, dm, k, p, wdb, wwb);
@@ -1098,7 +1106,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     for (int q = 0; q < 2; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       w1b[q] = b[WF_WW1][p];
       tb[q] = b[WF_T][p];
       tt[q] = b[WF_T_TEND][p];
@@ -1111,7 +1119,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     for (int q = 0; q < 2; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const int p = k * lev + c;
+      const size_t p = k * lev + c;
       b[WF_WW1][p] = w1b[q] - swb[k * kMutTX];
       b[WF_WW][p] = k >= 1 ? 0.f : sws[threadIdx.x];
       b[WF_T_TEND][p] = tt[q] + msfty * dts * tb[q];
@@ -1927,7 +1935,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   const int i = i0 + blockIdx.x * kVsTX + tx, j = g.jds + blockIdx.y;
   const bool col = i >= g.ids && i < g.ide - 1;
   const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
-  const int lev = g.ny * g.nx;
+  const size_t lev = g.n2();
   const int n = nz * kVsTX;
   float* const sa = vs_smem + tx;                                // a
   float *const sb = sa + n, *const sc = sa + 2 * n;              // b (then the level's own c2a term), c
@@ -1941,7 +1949,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   const float lid = g.top_lid ? 0.f : 1.f;
 #pragma unroll 4
   for (int k = 1 + tk; k < nz; k += kVsKT) {
-    const int p = k * lev + c;
+    const size_t p = k * lev + c;
     st[k * kVsTX] = alphabar[p];
     if (k == nz - 1) continue;
     sg[k * kVsTX] = gammabar[p];
@@ -1991,7 +1999,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   __syncthreads();
 #pragma unroll 4
   for (int k = 1 + tk; k < nz - 1; k += kVsKT) {
-    const int p = k * lev + c;
+    const size_t p = k * lev + c;
     const float cw = cqw[p], c2k = c2a[p], c2m = c2a[p - lev];
     const float rk = rdn[k], rwk = rdnw[k], rwm = rdnw[k - 1];
     const float ak = sa[k * kVsTX], bk = sb[k * kVsTX], ck = sc[k * kVsTX], al = sl[k * kVsTX];

@@ -140,15 +140,16 @@ struct DiffPoint {
 
 template <int VAR>
 __device__ __forceinline__ void diff_point(const Grid& g, const S& s, const float* __restrict__ f,
-                                           const float* __restrict__ base, const float* __restrict__ K, int c, int p,
+                                           const float* __restrict__ base, const float* __restrict__ K, int c, size_t p,
                                            const Coef (&cf)[4], DiffPoint& o) {
-  const int nx = g.nx, lev = g.ny * nx;
+  const int nx = g.nx;
+  const size_t lev = g.n2();
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     float ks = 0.f;
 #pragma unroll
     for (int q = 0; q < visc_points(VAR, e); ++q)
-      ks = ks + __ldg(K + p + cf[e].kk[q] * lev + cf[e].kj[q] * nx + cf[e].ki[q]);
+      ks = ks + __ldg(K + p + ((long long)cf[e].kk[q] * (long long)lev + cf[e].kj[q] * nx + cf[e].ki[q]));
     o.kavg[e] = cf[e].wk * ks;
     // a mass-point scalar's viscosity average multiplies before the mass average
     o.kx[e] = VAR == DV_M ? cf[e].ratio * o.kavg[e] * cf[e].mavg * cf[e].rd
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(128) k_hdiff_op(Grid g, S s, const float* __re
 #pragma unroll 2
   for (int k = z0; k < z0 + kHdiffLevels && k < g.nz; ++k) {
     if (!diff_region(g, var, k, j, i)) continue;
-    const int p = k * g.ny * g.nx + c;
+    const size_t p = k * g.n2() + c;
     DiffPoint o;
     diff_point<VAR>(g, s, f, base, K, c, p, cf, o);
     tend[p] = tend[p] + (o.mr[0] * (o.kx[1] * o.d[1] - o.kx[0] * o.d[0]) + o.mr[1] * (o.kx[3] * o.d[3] - o.kx[2] * o.d[2]));
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(128) k_hdiff_op_adj(Grid g, S s, const float* 
     const float T = tbar[p];
     if (T == 0.f) continue;
     DiffPoint o;
-    diff_point<VAR>(g, s, f, base, K, c, (int)p, cf, o);
+    diff_point<VAR>(g, s, f, base, K, c, p, cf, o);
     // d/d(differences): +-mr * k..
     const float gx0 = -o.mr[0] * o.kx[0] * T, gx1 = o.mr[0] * o.kx[1] * T;
     const float gy0 = -o.mr[1] * o.kx[2] * T, gy1 = o.mr[1] * o.kx[3] * T;
