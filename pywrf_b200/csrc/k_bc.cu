@@ -45,8 +45,14 @@ __device__ __forceinline__ void zero_grad_w_level(const Grid& g, float* w, int k
 }
 
 // one block per (level, field); with b.zgw set, the blocks of the extra row
-// f == b.n apply zero_grad_bdy(w) (w is never one of the batch's fields);
-// shared memory: 2 (ny + nx) floats
+// f == b.n apply zero_grad_bdy(w) (w is never one of the batch's fields).
+// STAGED holds the sources in shared memory, 2 (ny + nx) floats; where those
+// pass the 48 KB that every launch may have (nx + ny above 6144), the two sides
+// run one after the other: at that length the second round trip is a small part
+// of the sides' own time (one field of 41 levels, staged below the line and not
+// above it: 24 and 24 us at 24 x 6130, 44 and 30 at 6130 x 24, 36 and 32 at
+// 3075 x 3075).
+template <bool STAGED>
 __global__ void __launch_bounds__(256) k_bc(Grid g, BcBatch b) {
   extern __shared__ float bc_smem[];
   const int k = blockIdx.x, f = blockIdx.y;
@@ -68,6 +74,27 @@ __global__ void __launch_bounds__(256) k_bc(Grid g, BcBatch b) {
   // field staggered in neither direction that copies it) takes their source
   const int c1 = ide + it.istag;
   const int ys = it.vstag ? jde - 1 : jde - 2;
+  if constexpr (!STAGED) {
+    for (int j = max(rhi0, 0) + threadIdx.x; j < min(r1, ny); j += blockDim.x) {
+      float* row = d + (size_t)j * nx;
+      const float lo = row[ids], hi = row[xs];
+#pragma unroll
+      for (int q = 1; q <= 3; ++q) {
+        if (j >= r0) row[ids - q] = lo;
+        row[xs + q] = hi;
+      }
+    }
+    __syncthreads();
+    for (int i = ids + threadIdx.x; i < c1; i += blockDim.x) {
+      const float lo = d[(size_t)jds * nx + i], hi = d[(size_t)ys * nx + i];
+#pragma unroll
+      for (int q = 1; q <= 3; ++q) {
+        d[(size_t)(jds - q) * nx + i] = lo;
+        d[(size_t)(ys + q) * nx + i] = hi;
+      }
+    }
+    return;
+  }
   for (int j = max(rhi0, 0) + threadIdx.x; j < min(r1, ny); j += blockDim.x) {
     const float* row = d + (size_t)j * nx;
     xlo[j] = row[ids];
@@ -134,9 +161,10 @@ int launch_bc(const Grid& g, const BcBatch& b, cudaStream_t st) {
   if (b.n == 0 && !b.zgw) return 0;
   int kmax = b.zgw ? g.nz : 1;
   for (int f = 0; f < b.n; ++f) kmax = b.item[f].k_end > kmax ? b.item[f].k_end : kmax;
-  const size_t smem = 2 * (size_t)(g.nx + g.ny) * sizeof(float);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_bc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_bc<<<dim3(kmax, b.n + (b.zgw ? 1 : 0)), 256, smem, st>>>(g, b);
+  const size_t smem = 2 * ((size_t)g.nx + g.ny) * sizeof(float);
+  const dim3 gr(kmax, b.n + (b.zgw ? 1 : 0));
+  if (smem <= 48 * 1024) k_bc<true><<<gr, 256, smem, st>>>(g, b);
+  else k_bc<false><<<gr, 256, 0, st>>>(g, b);
   return 1;
 }
 

@@ -394,3 +394,17 @@ def test_column_reverses_at_the_greatest_depth(name, inputs, data):
         eps = float(z[f"fd_eps_{k}"]) if f"fd_eps_{k}" in z else 1e-4 * float(np.abs(x64[k]).max())
         fd = (loss({**x64, k: x64[k] + eps * d}) - loss({**x64, k: x64[k] - eps * d})) / (2.0 * eps)
         assert abs(float((gr * d).sum()) - fd) <= 2e-4 * float(np.sqrt((gr * gr).sum())) + 1e-9, k
+
+
+@pytest.mark.parametrize("nx,ny", [(6120, 24), (6121, 24), (24, 6122), (30000, 24), (24, 30001)])
+def test_halo_copies_of_long_rows_and_columns(nx, ny):
+    """Either side of the length whose edges fit the halo kernel's shared
+    memory, and past the largest a block can have: the in-place copies against
+    the gathered ones, every stagger, bitwise."""
+    nz = 12
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    fields = [torch.rand(nz, ny, nx, generator=gen, device="cuda") for _ in LETTERS]
+    fields += [torch.rand(ny, nx, generator=gen, device="cuda") for _ in "tuv"]
+    letters = LETTERS + "tuv"
+    for f, v, want in zip(fields, letters, A.halos(fields, letters)):
+        assert torch.equal(A.zero_grad_w(f) if v == "Z" else A.halo(f, v), want), v
