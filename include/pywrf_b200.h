@@ -45,7 +45,7 @@ extern "C" {
 /* status words (WF_STATUS) */
 #define WRF_ST_NAN_P 0        /* NaN points met in the diagnosed p (summed over RK stages) */
 #define WRF_ST_STEP 1         /* completed steps (device step counter) */
-#define WRF_ST_WAIT 2         /* thread blocks whose bounded wait on a tile load ran out (tiled advection) */
+#define WRF_ST_WAIT 2         /* thread blocks whose bounded wait on a tile load ran out (tensor-map kernels) */
 
 /* the persistent state of one integration, in table order */
 #define WRF_FIELD_TABLE(X) \
@@ -537,6 +537,18 @@ int wrf_wsm6_noalloc(const WrfGrid* g, float* th, float* qv, float* qc, float* q
                      float* qg, const float* rho, const float* pii, const float* p, const float* dz8w,
                      float delt, float* rainnc, float* rainncv, float* snownc, float* snowncv,
                      float* graupelnc, float* graupelncv, float* sr, void* stream);
+
+/* The tensor-map kernels (tiled advection, forces, advance_uv) wait for their
+ * tile loads with a bound of about two seconds.  A block whose wait runs out
+ * stores NaN to the outputs it leaves and adds 1 to the table's
+ * WRF_ST_WAIT word; a table without status words (the stand-alone operators
+ * take one) has the NaN alone.  This runs such a kernel with every wait taken
+ * as run out, so that a caller can check its own handling: op 0 the forces of
+ * wrf_forces, 1 the advection of wrf_advect_moist, 2 wrf_advect_momentum's of
+ * u, v and w (ru_tend, rv_tend, rw_tend; fluxes ru, rv, ww), 3 wrf_advance_uv,
+ * on the fields of the table.  WRF_EINVAL where they have no tensor-map form
+ * (rows of whole 16-byte words, 16-byte aligned arrays, WRF_FORM_FAST). */
+int wrf_expired_waits(const WrfGrid* g, const WrfState* s, int op, void* stream);
 
 /* copies the 16 device status words to host memory (synchronises the stream) */
 int wrf_status_read(const WrfState* s, void* stream, int* out16);

@@ -230,6 +230,8 @@ def lib() -> ctypes.CDLL:
     L.wrf_wsm6_work.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 11 + [ctypes.c_float] + [vp] * 8 + [ctypes.c_size_t, vp]
     L.wrf_wsm6_noalloc.restype = ip
     L.wrf_wsm6_noalloc.argtypes = [ctypes.POINTER(WrfGridC)] + [vp] * 11 + [ctypes.c_float] + [vp] * 7 + [vp]
+    L.wrf_expired_waits.restype = ip
+    L.wrf_expired_waits.argtypes = [ctypes.POINTER(WrfGridC), vp, ip, vp]
     L.wrf_status_read.restype = ip
     L.wrf_status_read.argtypes = [vp, vp, ctypes.POINTER(ctypes.c_int)]
     L.wrf_last_launch_count.restype = ip

@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(128) k_advance_uv(Grid g, S s, float dts) {
 // vertical pressure averages dpn(k) come from the level below in registers
 // (each is the same operation on the same operands as in k_advance_uv), and
 // the thread's own u, v, tendencies and cq are loaded a level ahead.  Every
-// wait on a box is bounded; a block whose wait runs out stops, drains its
-// copies and adds 1 to STATUS[WRF_ST_WAIT].
+// wait on a box is bounded; a block whose wait runs out fills the levels it
+// leaves with NaN, drains its copies and adds 1 to STATUS[WRF_ST_WAIT].
 constexpr int kUvTX = 32, kUvTY = 8, kUvBW = 40, kUvBH = kUvTY + 1;
 constexpr int kUvNB = 6;                 // boxes per level: alt al pb php (k), ph p (k+1)
 constexpr int kUvSlot = 384;             // floats per box slot (1536 B >= 40 x 9 x 4)
@@ -359,7 +359,7 @@ static_assert(kUvBW * kUvBH <= kUvSlot && (kUvOSlot * 4) % 128 == 0, "ring slots
 struct UvTmaArgs {
   CUtensorMap alt, al, pb, php, ph, pp;
   CUtensorMap own[kUvNO];  // u, ru_tend, v, rv_tend, cqu, cqv
-  int nchunk;
+  int nchunk, expired;     // expired: every wait counts as run out
 };
 
 __global__ void __launch_bounds__(kUvTX * kUvTY, 4) k_advance_uv_tma(Grid g, S s, float dts,
@@ -459,9 +459,9 @@ __global__ void __launch_bounds__(kUvTX * kUvTY, 4) k_advance_uv_tma(Grid g, S s
   }
   const int oA = (ty + 1) * kUvBW + om + tx;
   const int oO = ty * kUvOW + oo + tx;  // (j, i) in an own-value box
-  int kstop = k1, slot = 0;
+  int kstop = a.expired ? k0 : k1, slot = 0;
   uint32_t par = 0;
-  for (int k = k0; k < k1; ++k) {
+  for (int k = a.expired ? k1 : k0; k < k1; ++k) {
     const float rdk = __ldg(&rdnw[k]);
     const float fm1 = k + 1 < nz - 1 ? __ldg(&fnm[k + 1]) : 0.f, fp1 = k + 1 < nz - 1 ? __ldg(&fnp[k + 1]) : 0.f;
     const bool ok = tma::mbar_wait_bounded(&bar[slot], par, kUvWaitCycles);
@@ -529,7 +529,14 @@ __global__ void __launch_bounds__(kUvTX * kUvTY, 4) k_advance_uv_tma(Grid g, S s
       par ^= 1u;
     }
   }
-  if (kstop < k1 && tid == 0) {
+  if (kstop == k1) return;
+#pragma unroll 1
+  for (int k = kstop; k < k1; ++k) {
+    const size_t p = (size_t)k * lev + c;
+    if (wu) U[p] = tma::unfinished();
+    if (wv) V[p] = tma::unfinished();
+  }
+  if (tid == 0) {
     for (int k = kstop; k <= hi; ++k)
       tma::mbar_wait_bounded(&bar[(k - k0) % kUvRing], ((k - k0) / kUvRing) & 1, kUvWaitCycles);
     if (s[WF_STATUS]) atomicAdd(reinterpret_cast<int*>(s[WF_STATUS]) + WRF_ST_WAIT, 1);
@@ -1613,7 +1620,7 @@ int launch_coef_w(const Grid& g, const float* mut, const float* cqw, const float
   return 1;
 }
 
-int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st) {
+int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st, bool expired) {
   if (kernel_form() == WRF_FORM_FAST && g.nx % 4 == 0 && g.nz >= 4) {
     UvTmaArgs a{};
     const char* err = nullptr;
@@ -1627,11 +1634,13 @@ int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st) {
     if (ok) {
       const int bx = (g.ide + 1 - g.ids + kUvTX - 1) / kUvTX, by = (g.jde - g.jds + kUvTY - 1) / kUvTY;
       a.nchunk = level_chunks(g.nz - 1, bx * by, kUvKCH, 4);
+      a.expired = expired;
       const dim3 gr(bx, by, a.nchunk);
       k_advance_uv_tma<<<gr, dim3(kUvTX, kUvTY), 0, st>>>(g, s, dts, a);
       return 1;
     }
   }
+  if (expired) return 0;
   const dim3 b3(32, 4);
   dim3 gr = point_grid(g, b3);
   // short chunks while the grid is about one wave (ten blocks fit an SM): with

@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(kAdvTX * kAdvTY) k_advect_tiled(Grid g, S s, A
 // its order are those of the cp.async form above.
 //
 // Every wait on a tile is bounded (~2 s); a block whose wait runs out stops,
-// waits (bounded) for the copies it issued, adds 1 to STATUS[WRF_ST_WAIT]
-// and returns.
+// fills the levels it leaves with NaN, waits (bounded) for the copies it
+// issued, adds 1 to STATUS[WRF_ST_WAIT] and returns.
 constexpr int kTTX = 32, kTTY = 8;
 constexpr int kQW = 44, kQH = kTTY + 6;        // scalar box
 constexpr int kAW = 40, kAH = kTTY + 1;        // per-level box
@@ -270,6 +270,7 @@ struct AdvTmaArgs {
   const float* romg;              // rom, for the chunk's bottom face
   int qw0, tw0;                   // array index of the first scalar in q / tend
   int ngroup, nchunk;
+  int expired;                    // every wait counts as run out
 };
 
 template <int NSP, bool ACCUM>
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(kTTX * kTTY, WRF_ADV_MINB) k_advect_tma(Grid g
     }
     fbot[m] = zface(ktf, fnm, fnp, win[m], k0, k0, rbot);
   }
-  int kstop = k1;  // the level at which a bounded wait ran out (k1: none did)
+  int kstop = a.expired ? k0 : k1;  // the level at which a bounded wait ran out (k1: none did)
   // ring slots and phase parities of levels k and k+3 (scalars) and k (the rest)
   int qs = 0, q3s = 3 % kTRing, as = 0;
   uint32_t qp = 0, q3p = 3 / kTRing, ap = 0;
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(kTTX * kTTY, WRF_ADV_MINB) k_advect_tma(Grid g
   float* tb[NSP];
 #pragma unroll
   for (int m = 0; m < NSP; ++m) tb[m] = a.tout[grp * NSP + m] + (size_t)k0 * lev + c;
-  for (int k = k0; k < k1; ++k) {
+  for (int k = a.expired ? k1 : k0; k < k1; ++k) {
     const float rdk = __ldg(&rdnw[k]);
     bool ok = tma::mbar_wait_bounded(&sm.qbar[qs], qp, kAdvWaitCycles);
     ok = ok && tma::mbar_wait_bounded(&sm.abar[as], ap, kAdvWaitCycles);
@@ -484,7 +485,15 @@ __global__ void __launch_bounds__(kTTX * kTTY, WRF_ADV_MINB) k_advect_tma(Grid g
     next(q3s, q3p, kTRing);
     next(as, ap, kARing);
   }
-  if (kstop < k1 && tid == 0) {
+  if (kstop == k1) return;
+#pragma unroll 1
+  for (int k = kstop; k < k1; ++k)
+#pragma unroll
+    for (int m = 0; m < NSP; ++m) {
+      if ((cell && k < ktf) || (!ACCUM && zreg)) *tb[m] = tma::unfinished();
+      tb[m] += lev;
+    }
+  if (tid == 0) {
     // let the copies still in flight land before the block's shared memory
     // goes (levels below kstop were all consumed)
     for (int k = kstop; k <= q_hi; ++k)
@@ -575,6 +584,7 @@ struct MomTmaArgs {
   float* tout[3];
   const float* romg;
   int nchunk, comp0;  // blockIdx.z = (component - comp0) * nchunk + chunk
+  int expired;        // every wait counts as run out
 };
 
 // per-level boxes: u, v: ru(k) rv(k) rom(k+1) tend(k); w: ru(k) ru(k-1) rv(k)
@@ -706,7 +716,7 @@ __device__ __forceinline__ void advect_mom_block(const Grid& g, const S& s, cons
       fbot = zface_w(ktf, win, k0, k0, rprev, rb);
     }
   }
-  int kstop = k1;
+  int kstop = a.expired ? k0 : k1;
   int qs = 0, q3s = 3 % kTRing, as = 0;
   uint32_t qp = 0, q3p = 3 / kTRing, ap = 0;
   auto next = [](int& slot, uint32_t& par, int ring) {
@@ -720,7 +730,7 @@ __device__ __forceinline__ void advect_mom_block(const Grid& g, const S& s, cons
   const int offC = offX + 3;                  // the cell
   const int oA = (ty + 1) * kMW + om + tx;    // (j, i) in a per-level box; -1: i-1, -kMW: j-1
   float* tb = a.tout[C] + (size_t)k0 * lev + c;
-  for (int k = k0; k < k1; ++k) {
+  for (int k = a.expired ? k1 : k0; k < k1; ++k) {
     const float rdk = __ldg(&rdz[C == 2 && k == ktf ? ktf - 1 : k]);
     bool ok = tma::mbar_wait_bounded(&qbar[qs], qp, kAdvWaitCycles);
     ok = ok && tma::mbar_wait_bounded(&abar[as], ap, kAdvWaitCycles);
@@ -840,7 +850,11 @@ __device__ __forceinline__ void advect_mom_block(const Grid& g, const S& s, cons
     next(q3s, q3p, kTRing);
     next(as, ap, kARing);
   }
-  if (kstop < k1 && tid == 0) {
+  if (kstop == k1) return;
+#pragma unroll 1
+  for (int k = kstop; k < k1; ++k, tb += lev)
+    if (cell) *tb = tma::unfinished();
+  if (tid == 0) {
     for (int k = kstop; k <= q_hi; ++k)
       tma::mbar_wait_bounded(&qbar[(k - k0) % kTRing], ((k - k0) / kTRing) & 1, kAdvWaitCycles);
     for (int k = kstop; k <= a_hi; ++k)
@@ -885,7 +899,7 @@ bool aux_maps(AdvTmaArgs& a, const Grid& g, const float* ru, const float* rv, co
 // advection of the momentum components comp0 .. comp0+ncomp-1 (0 u, 1 v,
 // 2 w) into ru_tend / rv_tend / rw_tend (TMA form); returns 0 (nothing
 // launched) when the arrays do not allow tensor maps
-int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaStream_t st) {
+int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaStream_t st, bool expired) {
   if (!tma_form(g) || g.nz < 4 || comp0 < 0 || ncomp < 1 || comp0 + ncomp > 3) return 0;
   MomTmaArgs a{};
   const char* err = nullptr;
@@ -903,6 +917,7 @@ int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaS
     return 0;
   a.romg = s[WF_WW];
   a.comp0 = comp0;
+  a.expired = expired;
   const int bx = (g.ide - g.ids + kTTX - 1) / kTTX, by = (g.jde - g.jds + kTTY - 1) / kTTY;
   a.nchunk = level_chunks(g.nz - 1, bx * by * ncomp, kMomKCH, 4);
   const dim3 gr(bx, by, ncomp * a.nchunk);
@@ -910,7 +925,7 @@ int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaS
   return 1;
 }
 
-int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st) {
+int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st, bool expired) {
   const size_t n3 = g.n3();
   if (tma_form(g)) {
     AdvTmaArgs a{};
@@ -926,11 +941,13 @@ int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st) {
       a.qw0 = 1;
       a.tw0 = 1;
       a.ngroup = 3;
+      a.expired = expired;
       const dim3 gr = tma_grid(g, 3, &a.nchunk);
       k_advect_tma<2, false><<<gr, dim3(kTTX, kTTY), 0, st>>>(g, s, a);
       return 1;
     }
   }
+  if (expired) return 0;
   AdvArgs a;
   for (int m = 0; m < 6; ++m) {
     a.q[m] = s[WF_MOIST] + (m + 1) * n3;

@@ -12,8 +12,8 @@
 // uses (u, v, ru, rv at the two points each formula takes, the column's p)
 // and the vertical averages wdwn(k) and dpn(k) are carried up the column in
 // registers; the thread's own tendencies and coefficients are loaded a level
-// ahead.  Every wait is bounded; a block whose wait runs out drains its copies
-// and adds 1 to STATUS[WRF_ST_WAIT].
+// ahead.  Every wait is bounded; a block whose wait runs out fills the levels
+// it leaves with NaN, drains its copies and adds 1 to STATUS[WRF_ST_WAIT].
 #include "kernels.cuh"
 #include "tma.cuh"
 
@@ -36,7 +36,7 @@ static_assert((kFQSlot * 4) % 128 == 0 && (kFMSlot * 4) % 128 == 0, "slots keep 
 struct ForcesTmaArgs {
   CUtensorMap ph, phb;
   CUtensorMap m[kFNM];
-  int nchunk;
+  int nchunk, expired;  // expired: every wait counts as run out
 };
 
 // 45 (a[1] - a[-1]) - 9 (a[2] - a[-2]) + (a[3] - a[-3]) with stride st
@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
   own(k0, cur);
   const int oA = (ty + 1) * kFMW + om + tx;  // (j, i) in an M box
   const int oQ = (ty + 3) * kFQW + oq + 3 + tx;  // (j, i) in a ph / phb box
-  int kstop = k1, r0 = 0, r1 = 1 % kFRing;
+  int kstop = a.expired ? k0 : k1, r0 = 0, r1 = 1 % kFRing;
   uint32_t p0 = 0, p1 = 1 / kFRing;
-  for (int k = k0; k < k1; ++k) {
+  for (int k = a.expired ? k1 : k0; k < k1; ++k) {
     Own nxt{};
     if (k + 1 < k1) own(k + 1, nxt);
     bool ok = tma::mbar_wait_bounded(&bar[r0], p0, kFWaitCycles);
@@ -418,7 +418,20 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
     }
     if (r1 == 0) p1 ^= 1u;
   }
-  if (kstop < k1 && tid == 0) {
+  if (kstop == k1) return;
+#pragma unroll 1
+  for (int k = kstop; k < k1; ++k) {
+    const size_t p = (size_t)k * lev + c;
+    const float nan = tma::unfinished();
+    if (mass && k >= 1) s[WF_PH_TEND][p] = nan;
+    if (uc && k < ktf) s[WF_RU_TEND][p] = nan;
+    if (vc && k < ktf) s[WF_RV_TEND][p] = nan;
+    if (mass && k >= 1 && k < nz - 1) {
+      s[WF_RW_TEND][p] = s[WF_CQW][p] = nan;
+      if (k == nz - 2) s[WF_RW_TEND][p + lev] = nan;
+    }
+  }
+  if (tid == 0) {
     for (int L = kstop; L <= hi; ++L)
       tma::mbar_wait_bounded(&bar[(L - k0) % kFRing], ((L - k0) / kFRing) & 1, kFWaitCycles);
     if (s[WF_STATUS]) atomicAdd(reinterpret_cast<int*>(s[WF_STATUS]) + WRF_ST_WAIT, 1);
@@ -429,7 +442,7 @@ __global__ void __launch_bounds__(kFTX * kFTY, WRF_FORCES_MINB) k_forces_tma(Gri
 
 // k_forces in its tensor-map form; returns 0 (nothing launched) when the
 // arrays do not allow tensor maps or the point form is selected
-int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st) {
+int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st, bool expired) {
   if (kernel_form() != WRF_FORM_FAST || g.nx % 4 != 0 || g.nz < 4) return 0;
   ForcesTmaArgs a{};
   const char* err = nullptr;
@@ -441,6 +454,7 @@ int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st) {
     if (!tma::encode_f32_4d(&a.m[e], s[f[e]], g.nx, g.ny, g.nz, 1, kFMW, kFMH, &err)) return 0;
   const int bx = (g.ide - g.ids + kFTX - 1) / kFTX, by = (g.jde - g.jds + kFTY - 1) / kFTY;
   a.nchunk = level_chunks(g.nz, bx * by, kFKCH, 2);
+  a.expired = expired;
   const size_t dyn = (size_t)kFRing * kFSlot * sizeof(float) + 128;
   if (cudaFuncSetAttribute(k_forces_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess) return 0;
   const dim3 gr(bx, by, a.nchunk);

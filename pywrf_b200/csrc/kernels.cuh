@@ -32,8 +32,9 @@ int launch_relax_qv(const Grid& g, const S& s, cudaStream_t st);
 int launch_advect_forces(const Grid& g, const S& s, cudaStream_t st);
 // k_forces in its tiled tensor-map form (k_forces_tma.cu); 0 (nothing
 // launched) when nx is not a multiple of 4, a map is refused or the point form
-// is selected
-int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st);
+// is selected.  Here and below, expired: every wait of the tensor-map kernel
+// counts as run out
+int launch_forces_tma(const Grid& g, const S& s, cudaStream_t st, bool expired = false);
 // the tendency terms selected by a mask (1 rhs_ph, 2 pressure gradient,
 // 4 pg_buoy_w, 8 coriolis, 16 curvature) with the point kernel (k_tend.cu),
 // and their adjoint (k_adjoint_forces.cu)
@@ -80,12 +81,12 @@ int launch_addtend(const Grid& g, const S& s, int rk_step, cudaStream_t st);
 int launch_advect_moist(const Grid& g, const S& s, cudaStream_t st);
 // tiled scalar advection (k_advect_tiled.cu): the six moisture species with
 // ru_m / rv_m / ww_m into advect_tend, theta with ru / rv / ww into t_tend
-int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st);
+int launch_advect_moist_tiled(const Grid& g, const S& s, cudaStream_t st, bool expired = false);
 int launch_advect_theta_tiled(const Grid& g, const S& s, cudaStream_t st);
 // advect_u / advect_v / advect_w of the components comp0 .. comp0+ncomp-1
 // (0 u, 1 v, 2 w) in one tiled TMA launch (k_advect_tiled.cu); 0 (nothing
 // launched) when nx is not a multiple of 4 or a map is refused
-int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaStream_t st);
+int launch_advect_mom_tma(const Grid& g, const S& s, int comp0, int ncomp, cudaStream_t st, bool expired = false);
 // the same with one thread per point (k_tend.cu), components as a bit mask
 int launch_advect_mom_point(const Grid& g, const S& s, int comps, cudaStream_t st);
 // stand-alone advect_scalar (k_tend.cu)
@@ -139,7 +140,7 @@ int launch_coef_w(const Grid& g, const float* mut, const float* cqw, const float
 
 // acoustic steps (k_acoustic.cu)
 int launch_small_step_prep(const Grid& g, const S& s, int rk_step, float dts, cudaStream_t st);
-int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st);
+int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st, bool expired = false);
 int launch_acoustic_col(const Grid& g, const S& s, float dts, int iteration, int nsub, cudaStream_t st);
 int launch_small_step_finish(const Grid& g, const S& s, float dts, int nsub, int rk_step, cudaStream_t st);
 // small_step_prep without the calc_p_rho / calc_coef_w that follow it in the

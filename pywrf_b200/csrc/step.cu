@@ -780,6 +780,36 @@ int wrf_forces_adj(const WrfGrid* gin, const WrfState* sin, const WrfState* sbar
   return check_launch("forces_adj");
 }
 
+int wrf_expired_waits(const WrfGrid* gin, const WrfState* sin, int op, void* stream) {
+  Grid g;
+  int rc = make_grid(gin, g);
+  if (rc) return rc;
+  constexpr int moist[] = {WF_MOIST, WF_ADVECT_TEND, WF_RU_M, WF_RV_M, WF_WW_M, WF_MSFTX, WF_FNM, WF_FNP, WF_RDNW};
+  constexpr int mom[] = {WF_U, WF_V, WF_W, WF_RU_TEND, WF_RV_TEND, WF_RW_TEND, WF_RU, WF_RV, WF_WW, WF_MSFUX,
+                         WF_MSFVX, WF_MSFVY, WF_MSFTX, WF_FNM, WF_FNP, WF_RDN, WF_RDNW};
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  S s;
+  int launched = 0;
+  cudaGetLastError();
+  if (op == 0) {
+    if ((rc = state_of(sin, kForcesOperands, sizeof(kForcesOperands) / sizeof(int), s))) return rc;
+    launched = launch_forces_tma(g, s, st, true);
+  } else if (op == 1) {
+    if ((rc = state_of(sin, moist, sizeof(moist) / sizeof(int), s))) return rc;
+    launched = launch_advect_moist_tiled(g, s, st, true);
+  } else if (op == 2) {
+    if ((rc = state_of(sin, mom, sizeof(mom) / sizeof(int), s))) return rc;
+    launched = launch_advect_mom_tma(g, s, 0, 3, st, true);
+  } else if (op == 3) {
+    if ((rc = state_of(sin, kUvOperands, sizeof(kUvOperands) / sizeof(int), s))) return rc;
+    launched = launch_advance_uv(g, s, 1.f, st, true);
+  } else {
+    return fail(WRF_EINVAL, "expired_waits: op is 0 .. 3");
+  }
+  if (!launched) return fail(WRF_EINVAL, "expired_waits: these arrays have no tensor-map form");
+  return check_launch("expired_waits");
+}
+
 int wrf_sumflux(const WrfGrid* gin, const WrfState* sin, int iteration, int nsub, void* stream) {
   Grid g;
   int rc = make_grid(gin, g);

@@ -54,6 +54,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* b, uint32_t parity, 
   }
 }
 
+// what a block whose bounded wait ran out stores for the levels it leaves: a
+// table without status words has nothing else to tell its caller by, and an old
+// value would pass for a result
+__device__ __forceinline__ float unfinished() { return __int_as_float(0x7fffffff); }
+
 // box of a 4-D tensor map (x fastest) at integer coordinates into shared
 // memory; completion is signalled on bar with the box's byte count
 __device__ __forceinline__ void load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {

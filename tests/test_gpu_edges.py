@@ -408,3 +408,65 @@ def test_halo_copies_of_long_rows_and_columns(nx, ny):
     letters = LETTERS + "tuv"
     for f, v, want in zip(fields, letters, A.halos(fields, letters)):
         assert torch.equal(A.zero_grad_w(f) if v == "Z" else A.halo(f, v), want), v
+
+
+@pytest.mark.parametrize("op,outputs", [(0, ("ph_tend", "ru_tend", "rv_tend", "rw_tend", "cqw")), (1, ("advect_tend",)),
+                                        (2, ("ru_tend", "rv_tend", "rw_tend")), (3, ("u", "v"))],
+                         ids=["forces", "advect_moist", "advect_momentum", "advance_uv"])
+@pytest.mark.parametrize("counted", [True, False], ids=["status", "no_status"])
+def test_waits_that_ran_out_leave_no_plausible_result(op, outputs, counted):
+    """A tensor-map kernel whose waits on its tiles ran out: NaN at every point
+    that the kernel updates otherwise, the rest untouched, with and without
+    the status words that count the blocks; the context stays usable."""
+    n, nz = 40, 14
+    cg, L = A.scalar_grid((nz, n, n), 1 / 9000.0, 1 / 9000.0), N.lib()
+    gen = torch.Generator(device="cuda").manual_seed(op)
+    three = set(A.FORCES_INPUTS) | set(A.UV_INPUTS) | {"ru_m", "rv_m", "ww_m", "rw_tend"}
+    three -= {"mu", "muu", "muv", "mudf", "mut", "mub"}
+    rnd = lambda *s: 1.0 + torch.rand(*s, generator=gen, device="cuda")  # noqa: E731
+    st = {k: rnd(nz, n, n) for k in three} | {k: rnd(7, nz, n, n) for k in ("moist", "advect_tend")}
+    st |= {k: rnd(n, n) for k in ("mu", "muu", "muv", "mudf", "mut", "mub", *A.FORCES_DATA, *A.UV_DATA)}
+    st |= {k: rnd(nz) for k in ("fnm", "fnp", "rdn", "rdnw")}
+    status = torch.zeros(16, dtype=torch.int32, device="cuda")
+
+    def run(expired):
+        d = {k: v.clone() for k, v in st.items()}
+        tab = A._table(d)
+        if counted:
+            tab[N.field_names().index("status")] = status.data_ptr()
+        by, s = ctypes.byref(cg), _stream()
+        if expired:
+            rc = L.wrf_expired_waits(by, tab, op, s)
+        elif op == 0:
+            rc = L.wrf_forces(by, tab, 31, s)
+        elif op == 1:
+            rc = L.wrf_advect_moist(by, *[_p(d[k]) for k in ("moist", "advect_tend", "ru_m", "rv_m", "ww_m", "msftx",
+                                                              "fnm", "fnp", "rdnw")], s)
+        elif op == 2:
+            rc = 0
+            for c, (q, t, m) in enumerate((("u", "ru_tend", "msfux"), ("v", "rv_tend", "msfvy"),
+                                           ("w", "rw_tend", "msftx"))):
+                rc |= L.wrf_advect_momentum(by, c, *[_p(d[k]) for k in (q, t, "ru", "rv", "ww", m, "msfvx", "fnm", "fnp",
+                                                                        "rdn" if c == 2 else "rdnw")], 0, s)
+        else:
+            rc = L.wrf_advance_uv(by, tab, 1.0, s)
+        N.check(rc, "operator")
+        torch.cuda.synchronize()
+        return d
+
+    good, left = run(False), run(True)
+    assert int(status[N.WRF_ST_WAIT]) > 0 if counted else int(status.abs().sum()) == 0
+    for k in good:
+        if k not in outputs:
+            assert torch.equal(left[k], st[k]), k
+            continue
+        assert bool(torch.isfinite(good[k]).all())
+        updated = good[k] != st[k]
+        assert bool(updated.any()) and bool(left[k][updated].isnan().all()), k
+        same = ~left[k].isnan()
+        assert torch.equal(left[k][same], st[k][same]), k
+    prev = L.wrf_set_kernel_form(N.WRF_FORM_POINT)
+    try:
+        assert L.wrf_expired_waits(ctypes.byref(cg), A._table(st), op, _stream()) == N.WRF_EINVAL
+    finally:
+        L.wrf_set_kernel_form(prev)
