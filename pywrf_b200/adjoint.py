@@ -1113,34 +1113,39 @@ class _Bars(dict):
 
 class _ChainOp:
     """One operator of a chain: ``reads`` are the state names its reverse
-    needs (their values on entry are kept), ``writes`` those it replaces.
-    ``forward(cg, st, out, stream)`` fills ``out`` (copies of the written
+    needs (their values on entry are kept), ``writes`` those it replaces and
+    ``const`` the constant arrays that both directions use.
+    ``forward(cg, st, out, const, stream)`` fills ``out`` (copies of the written
     fields, updated in place; with ``fresh``, uninitialised) and
-    ``backward(cg, saved, bars, stream)`` turns the written names' cotangents
-    into those of the values on entry and adds the rest."""
-    fresh = False
+    ``backward(cg, saved, bars, const, stream)`` turns the written names'
+    cotangents into those of the values on entry and adds the rest.  The chain
+    saves what the reverse uses with its other tensors (an array changed in
+    between raises, saved-tensor hooks see it, a checkpoint drops it), so
+    ``backward`` holds no tensor itself."""
 
-    def __init__(self, reads, writes, forward, backward, fresh=False, fill=None):
+    def __init__(self, reads, writes, forward, backward, const=None, fresh=False, fill=None):
         self.reads, self.writes, self.forward, self.backward = tuple(reads), tuple(writes), forward, backward
-        self.fresh, self.fill = fresh, fill
+        self.const, self.fresh, self.fill = dict(const or {}), fresh, fill
 
 
 def _rc(rc, name):
     N.check(rc, name)
 
 
-def _table_chain_op(op, data: dict):
-    """A chain operator from a state-table operator (see :class:`_TableOp`)."""
-    const = {k: data[k] for k in op.data}
+def _table_chain_op(op, data: dict, held=()):
+    """A chain operator from a state-table operator (see :class:`_TableOp`);
+    ``held`` names those of its constants that are fields of the chain's state
+    (which receive no cotangent)."""
+    reads = op.fields + tuple(held)
 
-    def fwd(cg, st, out, stream):
-        _rc(op.fwd(cg, _table({**const, **{k: st[k] for k in op.fields}, **out}), stream), op.name)
+    def fwd(cg, st, out, const, stream):
+        _rc(op.fwd(cg, _table({**const, **{k: st[k] for k in reads}, **out}), stream), op.name)
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         likes = {k: saved[k] for k in op.fields}
-        _rc(op.adj(cg, _table({**const, **likes}), _table(bars.need(likes)), stream), op.name + "_adj")
+        _rc(op.adj(cg, _table({**const, **saved}), _table(bars.need(likes)), stream), op.name + "_adj")
 
-    return _ChainOp(op.fields, op.outputs, fwd, bwd)
+    return _ChainOp(reads, op.outputs, fwd, bwd, {k: data[k] for k in op.data if k not in held})
 
 
 class _CallOp:
@@ -1161,20 +1166,21 @@ class _Chain(torch.autograd.Function):
         _cuda_only(*tensors)
         st = {k: v.detach() for k, v in zip(names, tensors)}
         kept = {}     # id of a kept tensor -> its place among the saved ones
-        saved, places = [], []
+        saved, steps = [], []
         own = set()   # ids of this chain's tensors that nothing has kept
+
+        def keep(v):
+            if id(v) not in kept:
+                kept[id(v)] = len(saved)
+                saved.append(v.detach() if v.requires_grad else v)
+                own.discard(id(v))
+            return kept[id(v)]
+
         with _on(tensors[0]):
             stream = _stream(tensors[0])
             for op in ops:
-                at = []
-                for k in op.reads:
-                    v = st[k]
-                    if id(v) not in kept:
-                        kept[id(v)] = len(saved)
-                        saved.append(v)
-                        own.discard(id(v))
-                    at.append(kept[id(v)])
-                places.append(at)
+                steps.append((op.backward, [(k, keep(st[k])) for k in op.reads],
+                              [(k, keep(v)) for k, v in op.const.items()]))
                 out = {}
                 for k in op.writes:
                     if op.fresh:
@@ -1184,12 +1190,12 @@ class _Chain(torch.autograd.Function):
                         out[k] = st[k]
                     else:
                         out[k] = st[k].clone()
-                op.forward(cg, st, out, stream)
+                op.forward(cg, st, out, op.const, stream)
                 for k, v in out.items():
                     st[k] = v
                     own.add(id(v))
         ctx.save_for_backward(*saved)
-        ctx.ops, ctx.cg, ctx.names, ctx.outs, ctx.places = ops, cg, names, outs, places
+        ctx.steps, ctx.cg, ctx.names, ctx.outs = steps, cg, names, outs
         ctx.device = tensors[0].get_device()
         return tuple(st[k] for k in outs)
 
@@ -1202,8 +1208,8 @@ class _Chain(torch.autograd.Function):
                 bars[k] = gk.contiguous().clone()
         with torch.cuda.device(ctx.device):
             stream = torch.cuda.current_stream(ctx.device).cuda_stream
-            for op, at in zip(reversed(ctx.ops), reversed(ctx.places)):
-                op.backward(ctx.cg, {k: saved[q] for k, q in zip(op.reads, at)}, bars, stream)
+            for backward, reads, const in reversed(ctx.steps):
+                backward(ctx.cg, {k: saved[q] for k, q in reads}, bars, {k: saved[q] for k, q in const}, stream)
         need = ctx.needs_input_grad[4:]
         return (None, None, None, None) + tuple(bars.get(k) if w else None for k, w in zip(ctx.names, need))
 
@@ -1223,10 +1229,10 @@ def _run_chain(ops, cg, st: dict) -> dict:
 
 def _zero_op(name, like):
     """``name`` starts from zero (shaped like the state field ``like``)."""
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         out[name].zero_()
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         bars.pop(name, None)
 
     return _ChainOp((), (name,), fwd, bwd, fresh=True, fill=like)
@@ -1234,10 +1240,10 @@ def _zero_op(name, like):
 
 def _halo_op(names, letters):
     """The halo copies of ``names`` (:class:`Halos`), out of place."""
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         Halos._call("wrf_halo_copy", cg, letters, [st[k] for k in names], [out[k] for k in names])
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         some = [q for q, k in enumerate(names) if bars.get(k) is not None]
         if some:
             gs = [bars[names[q]] for q in some]
@@ -1249,11 +1255,11 @@ def _halo_op(names, letters):
 
 
 def _spec_update_op(field, tend, dt, var):
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         _rc(N.lib().wrf_spec_bdyupdate(ctypes.byref(cg), _ptr(out[field]), _ptr(st[tend]), dt, var.encode(), stream),
             "wrf_spec_bdyupdate")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(field) is not None:
             b = bars.need({tend: saved[tend]})
             _rc(N.lib().wrf_spec_bdyupdate_adj(ctypes.byref(cg), _ptr(bars[field]), _ptr(b[tend]), dt, var.encode(),
@@ -1263,11 +1269,11 @@ def _spec_update_op(field, tend, dt, var):
 
 
 def _spec_tend_op(tend, bt: dict, var):
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         _rc(N.lib().wrf_spec_bdytend(ctypes.byref(cg), _ptr(out[tend]), _ptr(bt["txs"]), _ptr(bt["txe"]),
                                      _ptr(bt["tys"]), _ptr(bt["tye"]), var.encode(), stream), "wrf_spec_bdytend")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(tend) is not None:
             _rc(N.lib().wrf_spec_bdytend_adj(ctypes.byref(cg), _ptr(bars[tend]), var.encode(), stream),
                 "wrf_spec_bdytend_adj")
@@ -1280,12 +1286,12 @@ def _relax_op(field, tend, bdy: dict, var, dtbc):
     level of it."""
     arrays = [bdy[k] for k in BDY_NAMES]
 
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         arr = (ctypes.c_void_p * 8)(*[_ptr(v) for v in arrays])
         _rc(N.lib().wrf_relax_bdytend(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), arr, var.encode(),
                                       float(dtbc), stream), "wrf_relax_bdytend")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(tend) is not None:
             b = bars.need({field: saved[field]})
             _rc(N.lib().wrf_relax_bdytend_adj(ctypes.byref(cg), _ptr(bars[tend]), _ptr(b[field]), var.encode(),
@@ -1295,12 +1301,12 @@ def _relax_op(field, tend, bdy: dict, var, dtbc):
 
 
 def _mass_weight_op(field, mass, out_name, nk):
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         out[out_name].zero_()
         _rc(N.lib().wrf_mass_weight(ctypes.byref(cg), _ptr(st[field]), _ptr(st[mass]), _ptr(out[out_name]), nk,
                                     stream), "wrf_mass_weight")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         gk = bars.pop(out_name, None)
         if gk is not None:
             b = bars.need(saved)
@@ -1317,127 +1323,131 @@ def _advect_work(cg, name, like):
 
 
 def _advect_momentum_op(component, field, tend, data: dict):
-    msf = data[("msfux", "msfvy", "msftx")[component]]
-    msf2 = data["msfvx"] if component == 1 else None
-    rdz = data["rdn" if component == 2 else "rdnw"]
-    fnm, fnp = data["fnm"], data["fnp"]
+    msf = ("msfux", "msfvy", "msftx")[component]
+    msf2 = "msfvx" if component == 1 else None
+    names = (msf, msf2, "fnm", "fnp", "rdn" if component == 2 else "rdnw")
 
-    def fwd(cg, st, out, stream):
-        m2 = None if msf2 is None else _ptr(msf2)
+    def pointers(const):
+        return [None if k is None else _ptr(const[k]) for k in names]
+
+    def fwd(cg, st, out, const, stream):
         _rc(N.lib().wrf_advect_momentum(ctypes.byref(cg), component, _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
-                                        _ptr(st["rv"]), _ptr(st["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
-                                        _ptr(rdz), 0, stream), "wrf_advect_momentum")
+                                        _ptr(st["rv"]), _ptr(st["ww"]), *pointers(const), 0, stream),
+            "wrf_advect_momentum")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
-        m2 = None if msf2 is None else _ptr(msf2)
         work, n = _advect_work(cg, "wrf_advect_momentum_adj_work", saved[field])
         _rc(N.lib().wrf_advect_momentum_adj(ctypes.byref(cg), component, _ptr(saved[field]), _ptr(saved["ru"]),
-                                            _ptr(saved["rv"]), _ptr(saved["ww"]), _ptr(msf), m2, _ptr(fnm), _ptr(fnp),
-                                            _ptr(rdz), _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
-                                            _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n, stream),
+                                            _ptr(saved["rv"]), _ptr(saved["ww"]), *pointers(const), _ptr(bars[tend]),
+                                            _ptr(b[field]), _ptr(b["ru"]), _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work),
+                                            n, stream),
             "wrf_advect_momentum_adj")
 
-    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd)
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, {k: data[k] for k in names if k})
+
+
+ADVECT_DATA = ("msftx", "fnm", "fnp", "rdnw")
 
 
 def _advect_scalar_op(field, tend, data: dict):
-    const = [data[k] for k in ("msftx", "fnm", "fnp", "rdnw")]
-
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         _rc(N.lib().wrf_advect_scalar(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
-                                      _ptr(st["rv"]), _ptr(st["ww"]), *map(_ptr, const), stream), "wrf_advect_scalar")
+                                      _ptr(st["rv"]), _ptr(st["ww"]), *[_ptr(const[k]) for k in ADVECT_DATA], stream),
+            "wrf_advect_scalar")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
         work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved[field])
         _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved[field]), _ptr(saved["ru"]), _ptr(saved["rv"]),
-                                          _ptr(saved["ww"]), *map(_ptr, const), _ptr(bars[tend]), _ptr(b[field]), _ptr(b["ru"]),
-                                          _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n, stream),
-            "wrf_advect_scalar_adj")
+                                          _ptr(saved["ww"]), *[_ptr(const[k]) for k in ADVECT_DATA], _ptr(bars[tend]),
+                                          _ptr(b[field]), _ptr(b["ru"]), _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n,
+                                          stream), "wrf_advect_scalar_adj")
 
-    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd)
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, {k: data[k] for k in ADVECT_DATA})
 
 
 def _advect_moist_op(data: dict):
     """advect_tend = the advection of qv .. qg (slots 1..6) by the averaged
     fluxes, zero outside the advected points (pywrf/wrf_dynamics.py:
     3982-4051)."""
-    const = [data[k] for k in ("msftx", "fnm", "fnp", "rdnw")]
     fluxes = ("ru_m", "rv_m", "ww_m")
 
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         out["advect_tend"].zero_()
         _rc(N.lib().wrf_advect_moist(ctypes.byref(cg), _ptr(st["moist"]), _ptr(out["advect_tend"]),
-                                     *[_ptr(st[k]) for k in fluxes], *map(_ptr, const), stream), "wrf_advect_moist")
+                                     *[_ptr(st[k]) for k in fluxes], *[_ptr(const[k]) for k in ADVECT_DATA], stream),
+            "wrf_advect_moist")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         gk = bars.pop("advect_tend", None)
         if gk is None:
             return
         b = bars.need(saved)
         work, n = _advect_work(cg, "wrf_advect_scalar_adj_work", saved["ru_m"])
+        maps = [_ptr(const[k]) for k in ADVECT_DATA]
         for m in range(1, 7):
             _rc(N.lib().wrf_advect_scalar_adj(ctypes.byref(cg), _ptr(saved["moist"][m]),
-                                              *[_ptr(saved[k]) for k in fluxes], *map(_ptr, const), _ptr(gk[m]),
+                                              *[_ptr(saved[k]) for k in fluxes], *maps, _ptr(gk[m]),
                                               _ptr(b["moist"][m]), *[_ptr(b[k]) for k in fluxes], _ptr(work), n,
                                               stream), "wrf_advect_scalar_adj")
 
-    return _ChainOp(("moist",) + fluxes, ("advect_tend",), fwd, bwd, fresh=True, fill="moist")
+    return _ChainOp(("moist",) + fluxes, ("advect_tend",), fwd, bwd, {k: data[k] for k in ADVECT_DATA},
+                    fresh=True, fill="moist")
 
 
 def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
     """tend += horizontal_diffusion(field); ``field`` "moist": its six
     species into the slots of ``tend``."""
-    const = {k: data[k] for k in HDIFF_DATA}
-
     def each(v):
         return [v[m] for m in range(1, 7)] if v.dim() == 4 else [v]
 
-    def fwd(cg, st, out, stream):
-        tab, bp = _table(const), None if base is None else _ptr(base)
+    def fwd(cg, st, out, const, stream):
+        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), _ptr(const["base"]) if "base" in const else None
         for f, o in zip(each(st[field]), each(out[tend])):
             _rc(N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp, _ptr(st[mass]),
                                                  _ptr(st[visc]), _ptr(o), stream), "wrf_horizontal_diffusion")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
-        tab, bp = _table(const), None if base is None else _ptr(base)
+        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), _ptr(const["base"]) if "base" in const else None
         for f, gk, fb in zip(each(saved[field]), each(bars[tend]), each(b[field])):
             _rc(N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp,
                                                      _ptr(saved[mass]), _ptr(saved[visc]), _ptr(gk), _ptr(fb),
                                                      _ptr(b[mass]), _ptr(b[visc]), stream),
                 "wrf_horizontal_diffusion_adj")
 
-    return _ChainOp((field, mass, visc), (tend,), fwd, bwd)
+    return _ChainOp((field, mass, visc), (tend,), fwd, bwd,
+                    {k: data[k] for k in HDIFF_DATA} | ({} if base is None else {"base": base}))
 
 
 def _coef_w_op(dts, data: dict):
     names = ("a", "alpha", "gamma")
 
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         for k in names:
             out[k].zero_()
         _rc(N.lib().wrf_coef_w(ctypes.byref(cg), _ptr(st["mut"]), _ptr(st["cqw"]), _ptr(st["c2a"]),
-                               _ptr(data["rdn"]), _ptr(data["rdnw"]), float(dts), *[_ptr(out[k]) for k in names],
+                               _ptr(const["rdn"]), _ptr(const["rdnw"]), float(dts), *[_ptr(out[k]) for k in names],
                                stream), "wrf_coef_w")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         gs = bars.need({k: saved["cqw"] for k in names})
         b = bars.need(saved)
         _rc(N.lib().wrf_coef_w_adj(ctypes.byref(cg), _ptr(saved["mut"]), _ptr(saved["cqw"]), _ptr(saved["c2a"]),
-                                   _ptr(data["rdn"]), _ptr(data["rdnw"]), float(dts), *[_ptr(gs[k]) for k in names],
+                                   _ptr(const["rdn"]), _ptr(const["rdnw"]), float(dts), *[_ptr(gs[k]) for k in names],
                                    _ptr(b["mut"]), _ptr(b["cqw"]), _ptr(b["c2a"]), stream), "wrf_coef_w_adj")
         for k in names:
             del bars[k]
 
-    return _ChainOp(("mut", "cqw", "c2a"), names, fwd, bwd, fresh=True, fill="cqw")
+    return _ChainOp(("mut", "cqw", "c2a"), names, fwd, bwd, {k: data[k] for k in ("rdn", "rdnw")}, fresh=True,
+                    fill="cqw")
 
 
 def _substep_ops(data: dict, iteration: int, nsub: int, dts: float) -> list:
@@ -1887,9 +1897,8 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
     if rk_step == 1:
         ops.append(_diffusion_op("m", "moist", "moist_tend", "muts", "xkhh", data))
         ops += _relax_qv_ops(st["u"].shape[0], bt["q"], dtbc)
-    # the averaged fluxes enter flow_dep_bdy by their sign alone: data
-    dd = {"msfty": data["msfty"], "ru_m": st["ru_m"].detach(), "rv_m": st["rv_m"].detach(), "rdnw": data["rdnw"]}
-    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk, st["u"]), dd))
+    # (the averaged fluxes enter flow_dep_bdy by their sign alone)
+    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk, st["u"]), data, held=("ru_m", "rv_m")))
     if rk_step < 3:
         ops.append(_halo_op(("u", "v", "w", "t", "ph", "mu", "moist"), "UVwpwtM"))
     return _run_chain(ops, cg, st)
@@ -1901,7 +1910,7 @@ def _relax_qv_ops(nz: int, bdy: dict, dtbc: float) -> list:
     L, by = N.lib(), ctypes.byref
     arrays = [bdy[k] for k in BDY_NAMES]
 
-    def fwd(cg, st, out, stream):
+    def fwd(cg, st, out, const, stream):
         arr = (ctypes.c_void_p * 8)(*[_ptr(v) for v in arrays])
         tend = out["moist_tend"][1]
         mass = torch.zeros_like(tend)
@@ -1911,7 +1920,7 @@ def _relax_qv_ops(nz: int, bdy: dict, dtbc: float) -> list:
         _rc(L.wrf_spec_bdytend(by(cg), _ptr(tend), *[_ptr(bdy[k]) for k in ("txs", "txe", "tys", "tye")], b"t",
                                stream), "wrf_spec_bdytend")
 
-    def bwd(cg, saved, bars, stream):
+    def bwd(cg, saved, bars, const, stream):
         if bars.get("moist_tend") is None:
             return
         b, gk = bars.need(saved), bars["moist_tend"][1]

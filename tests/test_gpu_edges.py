@@ -470,3 +470,60 @@ def test_waits_that_ran_out_leave_no_plausible_result(op, outputs, counted):
         assert L.wrf_expired_waits(ctypes.byref(cg), A._table(st), op, _stream()) == N.WRF_EINVAL
     finally:
         L.wrf_set_kernel_form(prev)
+
+
+def _chain_case():
+    """A small moist state, its constants and boundary arrays, and the
+    scalars of a step."""
+    spec = synthetic.CaseSpec(n=28, nz=16, dt=45.0, soundsteps=4, bdy_tend_amp=1.0e-4, seed=11)
+    inputs, bdy = synthetic.build(spec)
+    g = synthetic.grid_for(spec)
+    st = DeviceState.from_inputs(g, inputs, bdy, device="cuda")
+    names = dict.fromkeys(A.RK_STATE + ("u_1", "w_1", "ph_1", "mu_1", "t_1", "v_1"))
+    state = {k: st[k].clone() for k in names}
+    data = {k: st[k].clone() for k in dict.fromkeys(A.STEP_DATA + ("alb", "pb", "phb", "rdnw"))}
+    keys = (("bxs", "xs"), ("bxe", "xe"), ("bys", "ys"), ("bye", "ye"), ("btxs", "txs"), ("btxe", "txe"), ("btys", "tys"),
+            ("btye", "tye"))
+    bd = {f: {key: st[f"{f}_{n}"].clone() for n, key in keys} for f in ("u", "v", "ph", "t", "mu", "qv")}
+    sc = dict(epssm=g.epssm, emdiv=g.emdiv, smdiv=g.smdiv, rdx=g.rdx, rdy=g.rdy, **st.scal)
+    return g, state, data, bd, sc
+
+
+def _first_stage(state, data, bd, sc):
+    bt = {"u": bd["u"], "v": bd["v"], "h": bd["ph"], "t": bd["t"], "m": bd["mu"], "q": bd["qv"]}
+    return A.rk_stage(state, data, bt, 1, 1, 15.0, 15.0, dtbc=45.0, **sc)
+
+
+@pytest.mark.parametrize("name", ["msftx", "msfty", "msfux", "msfuy", "msfvx", "msfvx_inv", "msfvy", "fnm", "rdn", "rdnw",
+                                  "dnw", "t_init"])
+def test_a_constant_changed_before_the_reverse_is_refused(name):
+    """The reverse of an RK stage reads its constant arrays again: one changed
+    in place since the forward raises, as a changed state field does."""
+    _, state, data, bd, sc = _chain_case()
+    state["t"].requires_grad_(True)
+    out = _first_stage(state, data, bd, sc)
+    data[name].mul_(1.01)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        (out["t"].sum() + out["moist"].sum()).backward()
+
+
+def test_all_that_a_stage_reverses_with_passes_the_saved_tensor_hooks():
+    """Saved-tensor hooks that copy: with every array of the caller overwritten
+    after the forward, the copies alone give the same gradients (sums by
+    atomics in some order: 1e-5 of the norm)."""
+    grads = []
+    for hooked in (False, True):
+        _, state, data, bd, sc = _chain_case()
+        leaves = [state[k].requires_grad_(True) for k in ("u", "t", "ph", "mu", "moist")]
+        if hooked:
+            with torch.autograd.graph.saved_tensors_hooks(lambda v: v.detach().clone(), lambda v: v):
+                out = _first_stage(state, data, bd, sc)
+            with torch.no_grad():
+                for v in [*state.values(), *data.values(), *[b for d in bd.values() for b in d.values()]]:
+                    v.fill_(float("nan"))
+        else:
+            out = _first_stage(state, data, bd, sc)
+        grads.append(torch.autograd.grad([out[k] for k in ("u", "w", "t", "p", "moist")], leaves,
+                                         grad_outputs=[torch.ones_like(out[k]) for k in ("u", "w", "t", "p", "moist")]))
+    for a, b in zip(*grads):
+        assert float(a.norm()) > 0.0 and float((a - b).norm()) <= 1e-5 * float(a.norm())
