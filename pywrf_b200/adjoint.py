@@ -1050,7 +1050,16 @@ def acoustic_substep(st: dict, data: dict, iteration: int, nsub: int, dts: float
     is a hand-written reverse kernel, and the chain keeps only the operators'
     inputs."""
     cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3)
-    return _run_chain(_substep_ops({**data, "_like3": st["ww"]}, iteration, nsub, dts), cg, st)
+    return _run_chain(_substep_ops(data, iteration, nsub, dts), cg, st)
+
+
+def _scratch_like(cg, per_point: int = 0, per_column: int = 0) -> torch.Tensor:
+    """Uninitialised float32 scratch of the grid's size on the current device
+    and stream.  An operator takes its scratch when it runs: one that belongs to
+    an operator object stays with the graph's node, where a checkpoint cannot
+    drop it."""
+    n2 = cg.ny * cg.nx
+    return torch.empty((per_point * cg.nz + per_column) * n2, dtype=torch.float32, device="cuda")
 
 
 class _TableOp(torch.autograd.Function):
@@ -1059,7 +1068,8 @@ class _TableOp(torch.autograd.Function):
     them), its constant arrays (``op.data``), and runs the forward
     (``op.fwd(cg, table, stream)``) and the reverse product
     (``op.adj(cg, table, bar_table, stream)``, which rewrites the outputs'
-    cotangents to the inputs' and accumulates the rest)."""
+    cotangents to the inputs' and accumulates the rest; or ``op.reverse`` on
+    the named tensors themselves).  ``op`` holds no tensor."""
 
     @staticmethod
     def forward(ctx, op, cg, *tensors):
@@ -1085,7 +1095,11 @@ class _TableOp(torch.autograd.Function):
         bars = _bars(named, op.fields, dict(zip(op.outputs, gouts)))
         stream = _stream(saved[0])
         with _on(saved[0]):
-            N.check(op.adj(ctx.cg, _table(named), _table(bars), stream), op.name + "_adj")
+            if hasattr(op, "reverse"):
+                rc = op.reverse(ctx.cg, named, bars, stream)
+            else:
+                rc = op.adj(ctx.cg, _table(named), _table(bars), stream)
+            N.check(rc, op.name + "_adj")
         return (None, None) + tuple(bars[k] for k in op.fields) + (None,) * len(op.data)
 
 
@@ -1456,21 +1470,18 @@ def _substep_ops(data: dict, iteration: int, nsub: int, dts: float) -> list:
     by = ctypes.byref
     field = lambda names, ren: tuple(ren.get(k, k) for k in names)  # noqa: E731
 
-    def work_like(tab_adj, like):
-        return lambda cg, tab, btab, stream: tab_adj(cg, tab, btab, torch.empty_like(like), stream)
+    def with_work(tab_adj, **size):
+        return lambda cg, tab, btab, stream: tab_adj(cg, tab, btab, _ptr(_scratch_like(cg, **size)), stream)
 
-    ws3 = data["_like3"]
     uv = _CallOp("wrf_advance_uv", UV_INPUTS, ("u", "v"), UV_DATA,
                  lambda cg, tab, s: L.wrf_advance_uv(by(cg), tab, dts, s),
                  lambda cg, tab, b, s: L.wrf_advance_uv_adj(by(cg), tab, b, dts, s))
     mt = _CallOp("wrf_advance_mu_t", field(MUT_INPUTS, _MUT_FIELD), field(MUT_OUTPUTS, _MUT_FIELD), MUT_DATA,
                  lambda cg, tab, s: L.wrf_advance_mu_t(by(cg), tab, dts, s),
-                 work_like(lambda cg, tab, b, w, s: L.wrf_advance_mu_t_adj(by(cg), tab, b, dts, 0, _ptr(w), s),
-                           ws3))
+                 with_work(lambda cg, tab, b, w, s: L.wrf_advance_mu_t_adj(by(cg), tab, b, dts, 0, w, s), per_point=1))
     aw = _CallOp("wrf_advance_w", field(AW_INPUTS, _AW_FIELD), field(AW_OUTPUTS, _AW_FIELD), AW_DATA,
                  lambda cg, tab, s: L.wrf_advance_w(by(cg), tab, dts, s),
-                 work_like(lambda cg, tab, b, w, s: L.wrf_advance_w_adj(by(cg), tab, b, dts, _ptr(w), s),
-                           data["msftx"]))
+                 with_work(lambda cg, tab, b, w, s: L.wrf_advance_w_adj(by(cg), tab, b, dts, w, s), per_column=1))
     sf = _CallOp("wrf_sumflux", SF_INPUTS, SF_INPUTS[:3], SF_DATA,
                  lambda cg, tab, s: L.wrf_sumflux(by(cg), tab, iteration, nsub, s),
                  lambda cg, tab, b, s: L.wrf_sumflux_adj(by(cg), tab, b, iteration, nsub, s))
@@ -1509,16 +1520,15 @@ class _SmallStepPrep:
                "t", "t_1", "t_save", "w", "w_1", "w_save", "ph", "ph_1", "ph_save", "ww1", "c2a")
     data = ("msfuy", "msfvx_inv", "msfty")
 
-    def __init__(self, rk_step, ny, nx, device):
+    def __init__(self, rk_step):
         self.rk_step = rk_step
-        self.work = torch.empty(3 * ny * nx, dtype=torch.float32, device=device)
 
     def fwd(self, cg, tab, stream):
         return N.lib().wrf_small_step_prep(ctypes.byref(cg), tab, self.rk_step, stream)
 
     def adj(self, cg, tab, btab, stream):
-        return N.lib().wrf_small_step_prep_adj(ctypes.byref(cg), tab, btab, self.rk_step,
-                                               ctypes.c_void_p(self.work.data_ptr()), stream)
+        work = _scratch_like(cg, per_column=3)
+        return N.lib().wrf_small_step_prep_adj(ctypes.byref(cg), tab, btab, self.rk_step, _ptr(work), stream)
 
 
 class _SmallStepFinish:
@@ -1528,23 +1538,22 @@ class _SmallStepFinish:
     outputs = ("u", "v", "w", "ph", "ww", "t", "mu", "muus", "muvs")
     data = ("msfuy", "msfvx", "msfty")
 
-    def __init__(self, dts, nsub, rk_step, ny, nx, device):
+    def __init__(self, dts, nsub, rk_step):
         self.dts, self.nsub, self.rk_step = dts, nsub, rk_step
-        self.work = torch.empty(2 * ny * nx, dtype=torch.float32, device=device)
 
     def fwd(self, cg, tab, stream):
         return N.lib().wrf_small_step_finish(ctypes.byref(cg), tab, self.dts, self.nsub, self.rk_step, stream)
 
     def adj(self, cg, tab, btab, stream):
+        work = _scratch_like(cg, per_column=2)
         return N.lib().wrf_small_step_finish_adj(ctypes.byref(cg), tab, btab, self.dts, self.nsub, self.rk_step,
-                                                 ctypes.c_void_p(self.work.data_ptr()), stream)
+                                                 _ptr(work), stream)
 
 
 def small_step_prep(st: dict, data: dict, rk_step: int, rdx, rdy) -> dict:
     """Differentiable small_step_prep (pywrf/wrf_dynamics.py:3152-3266):
     returns ``st`` with the fields it updates replaced."""
-    nz, ny, nx = st["u"].shape
-    op = _SmallStepPrep(rk_step, ny, nx, st["u"].device)
+    op = _SmallStepPrep(rk_step)
     cg = scalar_grid(st["u"].shape, rdx, rdy)
     outs = _TableOp.apply(op, cg, *[st[k] for k in op.fields], *[data[k] for k in op.data])
     return {**st, **dict(zip(op.outputs, outs))}
@@ -1554,8 +1563,7 @@ def small_step_finish(st: dict, data: dict, dts: float, nsub: int, rk_step: int,
     """Differentiable calc_mu_uv_1 + small_step_finish
     (pywrf/wrf_dynamics.py:3844-3930): returns ``st`` with the fields they
     update replaced."""
-    nz, ny, nx = st["u"].shape
-    op = _SmallStepFinish(dts, nsub, rk_step, ny, nx, st["u"].device)
+    op = _SmallStepFinish(dts, nsub, rk_step)
     cg = scalar_grid(st["u"].shape, rdx, rdy)
     outs = _TableOp.apply(op, cg, *[st[k] for k in op.fields], *[data[k] for k in op.data])
     return {**st, **dict(zip(op.outputs, outs))}
@@ -1580,18 +1588,16 @@ def acoustic_stage(st: dict, data: dict, rk_step: int, nsub: int, dts: float, *,
     returns the state after the stage."""
     cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3,
                      top_lid=int(bool(top_lid)))
-    return _run_chain(_acoustic_ops(st, data, rk_step, nsub, dts), cg, st)
+    return _run_chain(_acoustic_ops(data, rk_step, nsub, dts), cg, st)
 
 
-def _acoustic_ops(st: dict, data: dict, rk_step: int, nsub: int, dts: float) -> list:
+def _acoustic_ops(data: dict, rk_step: int, nsub: int, dts: float) -> list:
     """The operators of :func:`acoustic_stage`."""
-    nz, ny, nx = st["u"].shape
-    dev = st["u"].device
-    ops = [_table_chain_op(_SmallStepPrep(rk_step, ny, nx, dev), data), _p_rho_op(data, 0), _coef_w_op(dts, data),
+    ops = [_table_chain_op(_SmallStepPrep(rk_step), data), _p_rho_op(data, 0), _coef_w_op(dts, data),
            _halo_op(("ru_tend", "rv_tend", "ph", "al", "p", "t_1", "t_save", "mu_1", "mu", "mudf"), "uvwppttttt")]
     for it in range(1, nsub + 1):
-        ops += _substep_ops({**data, "_like3": st["ww"]}, it, nsub, dts)
-    ops.append(_table_chain_op(_SmallStepFinish(dts, nsub, rk_step, ny, nx, dev), data))
+        ops += _substep_ops(data, it, nsub, dts)
+    ops.append(_table_chain_op(_SmallStepFinish(dts, nsub, rk_step), data))
     if rk_step == 3:
         ops.append(_halo_op(("ru_m", "rv_m", "ww_m", "mut", "muts"), "uvwtt"))
     return ops
@@ -1758,25 +1764,20 @@ class _EddyViscosity:
     data = ("phb", "msfux", "msfuy", "msfvx", "msfvy", "msftx", "msfty", "fnm", "fnp", "dn", "dnw")
     scratch = ("rdzw", "zx", "zy", "defor11", "defor22", "defor12")
 
-    def __init__(self, like):
-        n3 = like.numel()
-        self.buf = torch.empty(len(self.scratch) * n3, dtype=torch.float32, device=like.device)
-        self.views = [self.buf[q * n3:(q + 1) * n3] for q in range(len(self.scratch))]
-        self.work = torch.empty(6 * n3, dtype=torch.float32, device=like.device)
-
-    def _scratch(self, tab):
-        names = N.field_names()
-        for k, v in zip(self.scratch, self.views):
-            tab[names.index(k)] = v.data_ptr()
+    def _metrics(self, cg, tab):
+        """The metrics and deformations, which each direction forms anew."""
+        buf, names, n3 = _scratch_like(cg, per_point=len(self.scratch)), N.field_names(), cg.nz * cg.ny * cg.nx
+        for q, k in enumerate(self.scratch):
+            tab[names.index(k)] = buf.data_ptr() + 4 * q * n3
+        return buf
 
     def fwd(self, cg, tab, stream):
-        self._scratch(tab)
+        buf = self._metrics(cg, tab)  # noqa: F841 (held through the call)
         return N.lib().wrf_eddy_viscosity(ctypes.byref(cg), tab, stream)
 
     def adj(self, cg, tab, btab, stream):
-        self._scratch(tab)
-        return N.lib().wrf_eddy_viscosity_adj(ctypes.byref(cg), tab, btab, ctypes.c_void_p(self.work.data_ptr()),
-                                              stream)
+        buf, work = self._metrics(cg, tab), _scratch_like(cg, per_point=6)  # noqa: F841
+        return N.lib().wrf_eddy_viscosity_adj(ctypes.byref(cg), tab, btab, _ptr(work), stream)
 
 
 def eddy_viscosity(st: dict, data: dict, rdx, rdy, cf1: float, cf2: float, cf3: float):
@@ -1784,7 +1785,7 @@ def eddy_viscosity(st: dict, data: dict, rdx, rdy, cf1: float, cf2: float, cf3: 
     cal_deform_and_div, calculate_km_kh: pywrf/wrf_dynamics.py:491-995) from
     u, v and ph; returns (xkmh, xkhh).  ``st`` also maps the incoming xkmh
     and xkhh (which survive outside the formula's region)."""
-    op = _EddyViscosity(st["u"])
+    op = _EddyViscosity()
     cg = scalar_grid(st["u"].shape, rdx, rdy)
     cg.cf1, cg.cf2, cg.cf3 = float(cf1), float(cf2), float(cf3)
     return _TableOp.apply(op, cg, *[st[k] for k in op.fields], *[data[k] for k in op.data])
@@ -1841,7 +1842,7 @@ def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts:
     if rk_step == 1:
         tendf = ("ru_tendf", "rv_tendf", "rw_tendf", "ph_tendf", "t_tendf", "mu_tendf", "moist_tend")
         ops += [_zero_op(k, k) for k in tendf]
-        ops += [_table_chain_op(_EddyViscosity(st["u"]), data), _halo_op(("xkmh", "xkhh"), "tt")]
+        ops += [_table_chain_op(_EddyViscosity(), data), _halo_op(("xkmh", "xkhh"), "tt")]
     ops += [_zero_op(k, k) for k in zeros]
     ops += [_advect_momentum_op(0, "u", "ru_tend", data), _advect_momentum_op(1, "v", "rv_tend", data),
             _advect_momentum_op(2, "w", "rw_tend", data), _advect_scalar_op("t", "t_tend", data)]
@@ -1856,7 +1857,7 @@ def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts:
         s["t_tend"] = s["t_tend"] + theta_bias
     ops = [_spec_tend_op(k, bt[var], var) for k, var in (("ru_tend", "u"), ("rv_tend", "v"), ("ph_tend", "h"),
                                                          ("t_tend", "t"), ("mu_tend", "m"))]
-    return _run_chain(ops + _acoustic_ops(s, data, rk_step, nsub, dts), cg, s)
+    return _run_chain(ops + _acoustic_ops(data, rk_step, nsub, dts), cg, s)
 
 
 class _MoistUpdate:
@@ -1866,19 +1867,18 @@ class _MoistUpdate:
     outputs = ("moist", "moist_old", "al", "p")
     data = ("msfty", "ru_m", "rv_m", "rdnw")
 
-    def __init__(self, rk_step, dt_rk, like):
+    def __init__(self, rk_step, dt_rk):
         self.rk_step, self.dt_rk = rk_step, float(dt_rk)
-        self.work = torch.empty(like.numel(), dtype=torch.float32, device=like.device)
-        self.status = torch.zeros(16, dtype=torch.int32, device=like.device)
 
     def fwd(self, cg, tab, stream):
-        tab[N.field_names().index("status")] = self.status.data_ptr()
+        status = torch.empty(16, dtype=torch.int32, device="cuda")  # counts NaN points for nobody
+        tab[N.field_names().index("status")] = status.data_ptr()
         return N.lib().wrf_moist_update(ctypes.byref(cg), tab, self.rk_step, self.dt_rk, stream)
 
     def adj(self, cg, tab, btab, stream):
-        tab[N.field_names().index("status")] = self.status.data_ptr()
-        return N.lib().wrf_moist_update_adj(ctypes.byref(cg), tab, btab, self.rk_step, self.dt_rk,
-                                            ctypes.c_void_p(self.work.data_ptr()), stream)
+        work = _scratch_like(cg, per_point=1)
+        tab[N.field_names().index("status")] = work.data_ptr()  # the reverse counts nothing
+        return N.lib().wrf_moist_update_adj(ctypes.byref(cg), tab, btab, self.rk_step, self.dt_rk, _ptr(work), stream)
 
 
 def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: dict | None = None,
@@ -1898,7 +1898,7 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
         ops.append(_diffusion_op("m", "moist", "moist_tend", "muts", "xkhh", data))
         ops += _relax_qv_ops(st["u"].shape[0], bt["q"], dtbc)
     # (the averaged fluxes enter flow_dep_bdy by their sign alone)
-    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk, st["u"]), data, held=("ru_m", "rv_m")))
+    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk), data, held=("ru_m", "rv_m")))
     if rk_step < 3:
         ops.append(_halo_op(("u", "v", "w", "t", "ph", "mu", "moist"), "UVwpwtM"))
     return _run_chain(ops, cg, st)
@@ -2008,45 +2008,38 @@ class _Microphysics:
     scratch3 = ("qv_diabatic", "qc_diabatic", "wsm_t", "wsm_qr0s")
     scratch2 = ("rainnc", "rainncv", "snownc", "snowncv", "graupelnc", "graupelncv", "sr")
 
-    def __init__(self, like):
-        nz, ny, nx = like.shape
-        dev = like.device
-        self.s3 = {k: torch.zeros(nz, ny, nx, dtype=torch.float32, device=dev) for k in self.scratch3}
-        self.s2 = {k: torch.zeros(ny, nx, dtype=torch.float32, device=dev) for k in self.scratch2}
-        self.dbar = {k: torch.zeros(nz, ny, nx, dtype=torch.float32, device=dev) for k in ("alb", "pb")}
-
-    def _scratch(self, tab):
-        names = N.field_names()
-        for k, v in {**self.s3, **self.s2}.items():
-            tab[names.index(k)] = v.data_ptr()
+    def _scratch(self, cg, tab):
+        """The diagnostics and accumulators the block writes, in ``tab``."""
+        names, n2, n3 = N.field_names(), cg.ny * cg.nx, cg.nz * cg.ny * cg.nx
+        buf = _scratch_like(cg, per_point=len(self.scratch3), per_column=len(self.scratch2))
+        for q, k in enumerate(self.scratch3):
+            tab[names.index(k)] = buf.data_ptr() + 4 * q * n3
+        for q, k in enumerate(self.scratch2):
+            tab[names.index(k)] = buf.data_ptr() + 4 * (len(self.scratch3) * n3 + q * n2)
+        return buf
 
     def fwd(self, cg, tab, stream):
-        self._scratch(tab)
+        buf = self._scratch(cg, tab)  # noqa: F841 (held through the call)
         return N.lib().wrf_microphysics_op(ctypes.byref(cg), tab, stream)
 
-    def adj(self, cg, tab, btab, stream):
-        names = N.field_names()
+    def reverse(self, cg, named, bars, stream):
         # the state after the block, recomputed from clones of the inputs it
         # updates (the other fields are the same tensors)
-        ptab = (ctypes.c_void_p * len(names))()
-        for q in range(len(names)):
-            ptab[q] = tab[q]
-        clones = {k: self._saved[k].detach().clone() for k in self.outputs}
-        for k, v in clones.items():
-            ptab[names.index(k)] = v.data_ptr()
-        self._scratch(ptab)
+        post = {k: named[k].clone() for k in self.outputs}
+        ptab = _table({**named, **post})
+        buf = self._scratch(cg, ptab)  # noqa: F841
         rc = N.lib().wrf_microphysics_op(ctypes.byref(cg), ptab, stream)
         if rc:
             return rc
-        for k, v in self.dbar.items():
-            btab[names.index(k)] = v.data_ptr()
+        # the base state's cotangents, which the block accumulates and nobody takes
+        dropped = dict(zip(("alb", "pb"), _zeros(named["t"], named["t"])))
         n = ctypes.c_size_t(0)
         rc = N.lib().wrf_microphysics_adj_work(ctypes.byref(cg), ctypes.byref(n))
         if rc:
             return rc
-        work = torch.empty(int(n.value), dtype=torch.float32, device=clones["t"].device)
-        return N.lib().wrf_microphysics_adj(ctypes.byref(cg), tab, ptab, btab, ctypes.c_void_p(work.data_ptr()), n,
-                                            None, stream)
+        work = torch.empty(int(n.value), dtype=torch.float32, device=named["t"].device)
+        return N.lib().wrf_microphysics_adj(ctypes.byref(cg), _table(named), ptab, _table({**bars, **dropped}),
+                                            _ptr(work), n, None, stream)
 
 
 def microphysics(st: dict, data: dict, dt: float, rdx, rdy) -> dict:
@@ -2057,10 +2050,9 @@ def microphysics(st: dict, data: dict, dt: float, rdx, rdy) -> dict:
     taped scalars and one reverse sweep of its tape gives its inputs'
     cotangents (forward-mode tangents for a column whose tape outgrows the
     capacity)."""
-    op = _Microphysics(st["t"])
+    op = _Microphysics()
     cg = scalar_grid(st["t"].shape, rdx, rdy)
     cg.dt = float(dt)
-    op._saved = {k: st[k] for k in op.outputs}
     outs = _TableOp.apply(op, cg, *[st[k] for k in op.fields], *[data[k] for k in op.data])
     return {**st, **dict(zip(op.outputs, outs))}
 

@@ -527,3 +527,28 @@ def test_all_that_a_stage_reverses_with_passes_the_saved_tensor_hooks():
                                          grad_outputs=[torch.ones_like(out[k]) for k in ("u", "w", "t", "p", "moist")]))
     for a, b in zip(*grads):
         assert float(a.norm()) > 0.0 and float((a - b).norm()) <= 1e-5 * float(a.norm())
+
+
+def test_a_checkpointed_rollout_holds_one_state_per_step():
+    """What the forward of a checkpointed rollout leaves allocated: the states
+    at the segments' starts, and no operator's scratch or intermediates (one
+    percent of a state per step for the small arrays of the step's end)."""
+    g, state, data, bd, sc = _chain_case()
+    names = tuple(state)
+
+    def one(*xs):
+        out = A.step(dict(zip(names, xs)), data, bd, 45.0, dt=45.0, soundsteps=4,
+                     microphysics=lambda q: A.microphysics(q, data, 45.0, g.rdx, g.rdy), **sc)
+        return tuple(out[k] for k in names)
+
+    def held(n):
+        xs = tuple(state[k].clone().requires_grad_(k == "t") for k in names)
+        before = torch.cuda.memory_allocated()
+        out = A.rollout(one, xs, n)
+        torch.cuda.synchronize()
+        return torch.cuda.memory_allocated() - before, out
+
+    held(1)
+    size = sum(v.numel() * 4 for v in state.values())
+    first, last = held(1)[0], held(4)[0]
+    assert last - first <= 3 * 1.01 * size + 4096 * len(names), (first / size, last / size)
