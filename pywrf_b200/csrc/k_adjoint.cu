@@ -130,6 +130,7 @@
 //                        forward recurrence alpha(k) = 1 / (b(k) - a(k)
 //                        gamma(k-1)), gamma(k) = c(k) alpha(k) is recomputed
 //                        into local arrays and run backwards.
+#include <limits.h>
 #include "kernels.cuh"
 #include "relax.cuh"
 
@@ -430,7 +431,7 @@ __device__ UvTerm uv_term(const Grid& g, const S& s, const S& b, float dts, int 
 __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float dts) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = g.nx, ny = g.ny, ktf = g.nz - 1;
-  const size_t lev = g.n2();
+  const unsigned lev = (unsigned)g.ny * g.nx;
   if (i >= nx || j >= ny) return;
   const int c = j * nx + i;
   // the faces f = 2 V + e: P = the column itself (e = 0, sign +) or its
@@ -470,9 +471,9 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
       const int V = f >> 1;
       v.dpb[f] = v.C[f] = 0.f;
       if (in && on[f]) {
-        const size_t P = k * lev + cP[f];
+        const size_t P = (size_t)k * lev + cP[f];
         v.dpb[f] = -dts * __ldg(&s[V ? WF_CQV : WF_CQU][P]) * __ldg(&b[V ? WF_V : WF_U][P]);
-        v.C[f] = Cf[f] * (__ldg(php + P) - __ldg(php + k * lev + cQ[f]));
+        v.C[f] = Cf[f] * (__ldg(php + P) - __ldg(php + (size_t)k * lev + cQ[f]));
       }
       v.phi += (f & 1 ? -1.f : 1.f) * (v.dpb[f] * A[f]);
       v.dp += v.dpb[f] * v.C[f];
@@ -492,12 +493,12 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
   for (int f = 0; f < 4; ++f) {
     psum[f] = dpn[f] = 0.f;
     if (on[f]) {
-      psum[f] = pp[k0 * lev + cP[f]] + pp[k0 * lev + cQ[f]];
+      psum[f] = pp[(size_t)k0 * lev + cP[f]] + pp[(size_t)k0 * lev + cQ[f]];
       dpn[f] = uv_dpn(g, s, k0, cP[f], cQ[f]);
     }
   }
   for (int k = k0; k < k1; ++k) {
-    const size_t m = k * lev + c;
+    const size_t m = (size_t)k * lev + c;
     const Level next = level(k + 1);
     float aph = cur.phi + phi1, aalt = 0.f, aal = 0.f, apb = 0.f, aphp = 0.f, ap = 0.f, cq[2] = {0.f, 0.f};
     auto wt = [&](int kP) {
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(128) k_advance_uv_adj(Grid g, S s, S b, float 
       for (int f = 0; f < 4; ++f) {
         if (!on[f]) continue;
         const int V = f >> 1;
-        const size_t P = k * lev + cP[f], Q = k * lev + cQ[f];
+        const size_t P = (size_t)k * lev + cP[f], Q = (size_t)k * lev + cQ[f];
         const float sg = f & 1 ? -1.f : 1.f, Bb = cur.dpb[f] * A[f];
         const float up = __ldg(pp + P + lev) + __ldg(pp + Q + lev);
         const float dn = k + 1 == ktf ? 0.f : 0.5f * (fnm[k + 1] * up + fnp[k + 1] * psum[f]);
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
   const int tx = threadIdx.x, ty = threadIdx.y, nz = g.nz;
   const int i = blockIdx.x * 32 + tx, j = blockIdx.y;
   const bool col = i < g.nx, on = col && prho_in(g, 0, j, i);
-  const size_t lev = g.n2();
+  const unsigned lev = (unsigned)g.ny * g.nx;
   const int c = g.i2(j, col ? i : 0);
   const float mut = on ? __ldg(&s[WF_MUTS][c]) : 1.f, mu = on ? __ldg(&s[WF_MU][c]) : 0.f;
   const float r_mut = __frcp_rn(mut), ninv = -1.0f / mut;
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
 #pragma unroll
     for (int q = 0; q < kBatch; ++q) {
       const int k = k0 + q * kColLevels;
-      const size_t p = k * lev + c;
+      const size_t p = (size_t)k * lev + c;
       const bool in = on && k < nz - 1;
       Pb[q] = Mb[q] = Ab[q] = alt[q] = t1[q] = t2[q] = c2[q] = dph[q] = 0.f;
       if (in || (step == 0 && k < nz)) {
@@ -698,7 +699,7 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
 #pragma unroll
     for (int q = 0; q < kBatch; ++q) {
       const int k = k0 + q * kColLevels;
-      const size_t p = k * lev + c;
+      const size_t p = (size_t)k * lev + c;
       if (k >= nz) break;
       if (!(on && k < nz - 1)) {
         if (step == 0) {
@@ -735,7 +736,7 @@ __global__ void __launch_bounds__(32 * kColLevels) k_calc_p_rho_adj(Grid g, S s,
     float aph = 0.f;
     if (k < nz - 1) aph += pr_ab[k * 32 + tx];
     if (k >= 1) aph -= pr_ab[(k - 1) * 32 + tx];
-    if (aph != 0.f) add_to(b[WF_PH][k * lev + c], aph);
+    if (aph != 0.f) add_to(b[WF_PH][(size_t)k * lev + c], aph);
   }
   if (ty != 0) return;
   amu = amut = 0.f;
@@ -797,7 +798,8 @@ struct MutDiv {
     r_mfup = __frcp_rn(mfup);
     r_mfu0 = __frcp_rn(mfu0);
   }
-  __device__ __forceinline__ float at(const Grid& g, const S& s, size_t p) const {
+  template <typename Ix>
+  __device__ __forceinline__ float at(const Grid& g, const S& s, Ix p) const {
     const int nx = g.nx;
     const float* u = s[WF_U];
     const float* v = s[WF_V];
@@ -837,9 +839,10 @@ __device__ __forceinline__ void mut_scan(const Grid& g, const S& s, bool in, int
 
 // the cotangents of wdtn(k), k in [1, ktf), and of ww'(k), k in [0, ktf), of
 // one level (p: the point, dm = dts msfty)
-__device__ __forceinline__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dm, int k, size_t p, float& wdb,
+template <typename Ix>
+__device__ __forceinline__ void mut_ww_bar(const Grid& g, const S& s, const S& b, float dm, int k, Ix p, float& wdb,
                                            float& wwb) {
-  const size_t lev = g.n2();
+  const Ix lev = (Ix)g.ny * g.nx;
   const float* t1 = s[WF_T_SAVE];
   const float* rdnw = s[WF_RDNW];
   wdb = 0.f;
@@ -862,7 +865,7 @@ __device__ __forceinline__ float mut_mu_bar(const Grid& g, const S& b, size_t c)
 __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, float dts) {
   extern __shared__ float mut_smem[];
   const int nz = g.nz, ktf = nz - 1, nx = g.nx;
-  const size_t lev = g.n2();
+  const unsigned lev = (unsigned)g.ny * g.nx;
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
@@ -872,7 +875,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
   if (in) {
     const MutDiv d(g, s, c);
 #pragma unroll 4
-    for (int k = tk; k < ktf; k += kMutKT) sdv[k * kMutTX] = d.at(g, s, k * lev + c);
+    for (int k = tk; k < ktf; k += kMutKT) sdv[k * kMutTX] = d.at(g, s, (size_t)k * lev + c);
   }
   __syncthreads();
   if (in && tk == 0) {
@@ -892,7 +895,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
   mut_scan(g, s, in, c, sdm[threadIdx.x], sdv, sw);
   if (in) {
 #pragma unroll 4
-    for (int k = tk; k < ktf; k += kMutKT) sw[k * kMutTX] = sw[k * kMutTX] - __ldg(s[WF_WW1] + k * lev + c);
+    for (int k = tk; k < ktf; k += kMutKT) sw[k * kMutTX] = sw[k * kMutTX] - __ldg(s[WF_WW1] + (size_t)k * lev + c);
   }
   __syncthreads();
   if (!in) return;
@@ -909,7 +912,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
     for (int q = 0; q < 4; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const size_t p = k * lev + c;
+      const size_t p = (size_t)k * lev + c;
       tk_[q] = s[WF_T][p];
       tt[q] = s[WF_T_TEND][p];
       const float tc = __ldg(t1 + p);
@@ -923,7 +926,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
     for (int q = 0; q < 4; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const size_t p = k * lev + c;
+      const size_t p = (size_t)k * lev + c;
       s[WF_WW][p] = sw[k * kMutTX];
       s[WF_T_2SAVE][p] = tk_[q];
       const float t1v = tk_[q] + msfty * dts * tt[q];
@@ -936,7 +939,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, 
                                                                         float* work) {
   extern __shared__ float mut_smem[];
   const int ktf = g.nz - 1, nx = g.nx;
-  const size_t lev = g.n2();
+  const unsigned lev = (unsigned)g.ny * g.nx;
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
@@ -947,7 +950,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, 
 #pragma unroll 4
     for (int k = 1 + tk; k < ktf; k += kMutKT) {
       float wdb, wwb;
-      mut_ww_bar(g, s, b, dm, k, k * lev + c, wdb, wwb);
+      mut_ww_bar(g, s, b, dm, k, (size_t)k * lev + c, wdb, wwb);
       swb[k * kMutTX] = wwb;
     }
   }
@@ -969,7 +972,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, 
   const float dmdtb = sdm[threadIdx.x];
 #pragma unroll 4
   for (int k = tk; k < ktf; k += kMutKT)
-    work[k * lev + c] = (k <= ktf - 2 ? swb[(k + 1) * kMutTX] : 0.f) + __ldg(s[WF_DNW] + k) * dmdtb;
+    work[(size_t)k * lev + c] = (k <= ktf - 2 ? swb[(k + 1) * kMutTX] : 0.f) + __ldg(s[WF_DNW] + k) * dmdtb;
 }
 
 __global__ void k_advance_mu_t_adj_pt(Grid g, S s, S b, float dts, const float* work) {
@@ -1014,11 +1017,15 @@ __global__ void k_advance_mu_t_adj_pt(Grid g, S s, S b, float dts, const float* 
 }
 
 // (b[WF_T] is rewritten here, so this runs after the two passes above)
+// Ix: the type of a point's offset.  Two dozen addresses from 64-bit offsets take
+// 80 registers where 32-bit ones take 48, and three blocks an SM instead of five:
+// 94 against 67 us per launch at 240x240x41.
+template <typename Ix>
 __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g, S s, S b, float dts, int ref_no_grad,
                                                                          const float* work) {
   extern __shared__ float mut_smem[];
   const int nz = g.nz, ktf = nz - 1, nx = g.nx, n = nz * kMutTX;
-  const size_t lev = g.n2();
+  const Ix lev = (Ix)g.ny * g.nx;
   const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   // muu, muv: the u / v terms of the divergence at this column
@@ -1036,7 +1043,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     const float mfu = s[WF_MSFUY][c], r_mfu = __frcp_rn(mfu), mvi = s[WF_MSFVX_INV][c];
 #pragma unroll 4
     for (int k = tk; k < ktf; k += kMutKT) {
-      const size_t p = k * lev + c;
+      const Ix p = k * lev + c;
       const float wo = in ? __ldg(work + p) : 0.f;
       float ub = 0.f, vb = 0.f;
       if (w) ub += mw * rdx * __ldg(work + p - 1);
@@ -1052,7 +1059,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     const float dm = dts * s[WF_MSFTY][c];
 #pragma unroll 2
     for (int k = tk; k < ktf; k += kMutKT) {
-      const size_t p = k * lev + c;
+      const Ix p = k * lev + c;
       sdv[k * kMutTX] = d.at(g, s, p);
       float wdb, wwb;
       mut_ww_bar(g, s, b, dm, k, p, wdb, wwb);
@@ -1106,7 +1113,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     for (int q = 0; q < 2; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const size_t p = k * lev + c;
+      const Ix p = k * lev + c;
       w1b[q] = b[WF_WW1][p];
       tb[q] = b[WF_T][p];
       tt[q] = b[WF_T_TEND][p];
@@ -1119,7 +1126,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
     for (int q = 0; q < 2; ++q) {
       const int k = kb + q * kMutKT;
       if (k >= ktf) continue;
-      const size_t p = k * lev + c;
+      const Ix p = k * lev + c;
       b[WF_WW1][p] = w1b[q] - swb[k * kMutTX];
       b[WF_WW][p] = k >= 1 ? 0.f : sws[threadIdx.x];
       b[WF_T_TEND][p] = tt[q] + msfty * dts * tb[q];
@@ -1164,8 +1171,9 @@ int launch_advance_mu_t_adj(const Grid& g, const S& s, const S& b, float dts, in
   const size_t col = (size_t)g.nz * kMutTX * sizeof(float);
   k_advance_mu_t_adj_dv<<<mut_grid(g, 0), dim3(kMutTX, kMutKT), col, st>>>(g, s, b, dts, ref_no_grad, work);
   k_advance_mu_t_adj_pt<<<point_grid(g, b3), b3, 0, st>>>(g, s, b, dts, work);
-  allow_smem(k_advance_mu_t_adj_col, 6 * col);
-  k_advance_mu_t_adj_col<<<mut_grid(g, 1), dim3(kMutTX, kMutKT), 6 * col, st>>>(g, s, b, dts, ref_no_grad, work);
+  const auto columns = g.n3() <= INT_MAX ? k_advance_mu_t_adj_col<int> : k_advance_mu_t_adj_col<size_t>;
+  allow_smem(columns, 6 * col);
+  columns<<<mut_grid(g, 1), dim3(kMutTX, kMutKT), 6 * col, st>>>(g, s, b, dts, ref_no_grad, work);
   return 3;
 }
 
@@ -1935,7 +1943,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   const int i = i0 + blockIdx.x * kVsTX + tx, j = g.jds + blockIdx.y;
   const bool col = i >= g.ids && i < g.ide - 1;
   const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
-  const size_t lev = g.n2();
+  const unsigned lev = (unsigned)g.ny * g.nx;
   const int n = nz * kVsTX;
   float* const sa = vs_smem + tx;                                // a
   float *const sb = sa + n, *const sc = sa + 2 * n;              // b (then the level's own c2a term), c
@@ -1949,7 +1957,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   const float lid = g.top_lid ? 0.f : 1.f;
 #pragma unroll 4
   for (int k = 1 + tk; k < nz; k += kVsKT) {
-    const size_t p = k * lev + c;
+    const size_t p = (size_t)k * lev + c;
     st[k * kVsTX] = alphabar[p];
     if (k == nz - 1) continue;
     sg[k * kVsTX] = gammabar[p];
@@ -1961,8 +1969,8 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   }
   float c2t = 0.f, atopb = 0.f;
   if (tk == 0) {
-    c2t = c2a[(nz - 2) * lev + c];
-    atopb = abar[(nz - 1) * lev + c];
+    c2t = c2a[(size_t)(nz - 2) * lev + c];
+    atopb = abar[(size_t)(nz - 1) * lev + c];
   }
   __syncthreads();
   float mmb = 0.f, c2tb = 0.f;
@@ -1999,7 +2007,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   __syncthreads();
 #pragma unroll 4
   for (int k = 1 + tk; k < nz - 1; k += kVsKT) {
-    const size_t p = k * lev + c;
+    const size_t p = (size_t)k * lev + c;
     const float cw = cqw[p], c2k = c2a[p], c2m = c2a[p - lev];
     const float rk = rdn[k], rwk = rdnw[k], rwm = rdnw[k - 1];
     const float ak = sa[k * kVsTX], bk = sb[k * kVsTX], ck = sc[k * kVsTX], al = sl[k * kVsTX];
@@ -2029,7 +2037,7 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
     float v = k == 0 ? 0.f : sb[k * kVsTX];
     v += k == nz - 2 ? 0.f : st[(k + 1) * kVsTX];
     if (k == nz - 2) v += sb[(nz - 1) * kVsTX];
-    c2abar[k * lev + c] += v;
+    c2abar[(size_t)k * lev + c] += v;
   }
   if (tk == 0) {
 #pragma unroll 8

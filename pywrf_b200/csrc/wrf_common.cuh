@@ -42,8 +42,8 @@ struct Grid {
   __host__ __device__ __forceinline__ int i3(int k, int j, int i) const { return (k * ny + j) * nx + i; }
   __host__ __device__ __forceinline__ int i2(int j, int i) const { return j * nx + i; }
   __host__ __device__ __forceinline__ size_t n3() const { return (size_t)nz * ny * nx; }
-  // (the stand-alone operators take fields of more than 2^31 points: the
-  // offset of a level is formed from this, in 64 bits)
+  // (the stand-alone operators take fields of more than 2^31 points, so they
+  // form the offset of a level in 64 bits)
   __host__ __device__ __forceinline__ size_t n2() const { return (size_t)ny * nx; }
 };
 
