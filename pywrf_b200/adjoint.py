@@ -252,6 +252,11 @@ def _zeros(*likes):
     return out
 
 
+def _packed_like(t: torch.Tensor) -> torch.Tensor:
+    """An uninitialised tensor like ``t``, its points without gaps."""
+    return torch.empty_like(t, memory_format=torch.contiguous_format)
+
+
 def _packed(t: torch.Tensor) -> tuple:
     """The strides of ``t``'s shape without gaps."""
     if t.is_contiguous():
@@ -623,17 +628,17 @@ class Halos(torch.autograd.Function):
     """The halo copies of several fields in one launch each way: ``scal`` =
     (vars, rdx, rdy), one letter of ``vars`` per tensor: a stagger letter of
     :func:`halo`, 'Z' for zero_grad_bdy of w, or for a [7, nz, ny, nx]
-    moisture array 'M' (slots 1..6 as 'p', slot 0 copied)."""
+    moisture array 'M' (slots 1..6 as 'p', slot 0 copied; each slot's points
+    lie together, the slots need not)."""
 
     @staticmethod
     def _call(name, cg, letters, ins, outs):
         pi, po, vs, td = [], [], [], []
         for var, a, b in zip(letters, ins, outs):
             if var == "M":
-                step = a.numel() // 7 * 4
                 for m in range(1, 7):
-                    pi.append(a.data_ptr() + m * step)
-                    po.append(b.data_ptr() + m * step)
+                    pi.append(a.data_ptr() + 4 * m * a.stride(0))
+                    po.append(b.data_ptr() + 4 * m * b.stride(0))
                     vs.append("p")
                     td.append(0)
                 b[0].copy_(a[0])
@@ -652,17 +657,18 @@ class Halos(torch.autograd.Function):
     @staticmethod
     def forward(ctx, scal, *fields):
         ctx.set_materialize_grads(False)
-        _cuda_only(*fields)
         letters = str(scal[0])
         if len(letters) != len(fields):
             raise ValueError("one letter per field")
+        for var, f in zip(letters, fields):
+            _cuda_only(*(f.unbind() if var == "M" else (f,)))
         shape = next((f.shape[-3:] for f in fields if f.dim() > 2), (12,) + tuple(fields[0].shape[-2:]))
         for var, f in zip(letters, fields):
             want = shape[1:] if f.dim() == 2 else ((7,) + tuple(shape) if var == "M" else shape)
             if tuple(f.shape) != tuple(want):
                 raise ValueError(f"halos: a field of shape {tuple(f.shape)} where {tuple(want)} is expected")
         cg = scalar_grid(shape, float(scal[1]), float(scal[2]))
-        outs = tuple(torch.empty_like(f) for f in fields)
+        outs = tuple(_packed_like(f) for f in fields)
         Halos._call("wrf_halo_copy", cg, letters, [f.detach() for f in fields], outs)
         ctx.cg, ctx.letters = cg, letters
         return outs
@@ -1058,8 +1064,8 @@ def _scratch_like(cg, per_point: int = 0, per_column: int = 0) -> torch.Tensor:
     and stream.  An operator takes its scratch when it runs: one that belongs to
     an operator object stays with the graph's node, where a checkpoint cannot
     drop it."""
-    n2 = cg.ny * cg.nx
-    return torch.empty((per_point * cg.nz + per_column) * n2, dtype=torch.float32, device="cuda")
+    return torch.empty((per_point * cg.nz + per_column) * cg.ny * cg.nx, dtype=torch.float32,
+                       device=torch.cuda.current_device())
 
 
 class _TableOp(torch.autograd.Function):
@@ -1171,45 +1177,52 @@ class _CallOp:
 
 
 class _Chain(torch.autograd.Function):
-    """The operators ``ops`` in order on the state fields ``names``; returns
-    the final values of ``outs``."""
+    """The operators ``ops`` in order on the state fields ``names`` (each
+    with what is used of it, see :func:`_run_chain`); returns the final values
+    of ``outs``."""
 
     @staticmethod
     def forward(ctx, ops, cg, names, outs, *tensors):
         ctx.set_materialize_grads(False)
-        _cuda_only(*tensors)
+        for use, v in zip(names.values(), tensors):
+            if use == _COPY and v.dim() == 4:  # taken slot by slot
+                _cuda_only(*v.unbind())
+            elif use != _LIKE:
+                _ptr(v)
         st = {k: v.detach() for k, v in zip(names, tensors)}
         kept = {}     # id of a kept tensor -> its place among the saved ones
         saved, steps = [], []
         own = set()   # ids of this chain's tensors that nothing has kept
 
-        def keep(v):
-            if id(v) not in kept:
-                kept[id(v)] = len(saved)
-                saved.append(v.detach() if v.requires_grad else v)
-                own.discard(id(v))
-            return kept[id(v)]
+        def places(values):
+            at = []
+            for k, v in values:
+                q = kept.get(id(v))
+                if q is None:
+                    q = kept[id(v)] = len(saved)
+                    saved.append(v.detach() if v.requires_grad else v)
+                    own.discard(id(v))
+                at.append((k, q))
+            return at
 
         with _on(tensors[0]):
             stream = _stream(tensors[0])
             for op in ops:
-                steps.append((op.backward, [(k, keep(st[k])) for k in op.reads],
-                              [(k, keep(v)) for k, v in op.const.items()]))
+                steps.append((op.backward, places([(k, st[k]) for k in op.reads]), places(op.const.items())))
                 out = {}
                 for k in op.writes:
                     if op.fresh:
-                        like = st[op.fill or k]
-                        out[k] = torch.empty_like(like)
+                        out[k] = _packed_like(st[op.fill or k])
                     elif id(st[k]) in own:
                         out[k] = st[k]
                     else:
-                        out[k] = st[k].clone()
+                        out[k] = st[k].clone(memory_format=torch.contiguous_format)
                 op.forward(cg, st, out, op.const, stream)
                 for k, v in out.items():
                     st[k] = v
                     own.add(id(v))
         ctx.save_for_backward(*saved)
-        ctx.steps, ctx.cg, ctx.names, ctx.outs = steps, cg, names, outs
+        ctx.steps, ctx.cg, ctx.names, ctx.outs = steps, cg, tuple(names), outs
         ctx.device = tensors[0].get_device()
         return tuple(st[k] for k in outs)
 
@@ -1228,16 +1241,29 @@ class _Chain(torch.autograd.Function):
         return (None, None, None, None) + tuple(bars.get(k) if w else None for k, w in zip(ctx.names, need))
 
 
+# what a chain uses of a field it is given: its shape, an updated copy of it, or
+# its values
+_LIKE, _COPY, _READ = range(3)
+
+
 def _run_chain(ops, cg, st: dict) -> dict:
     """``st`` after the chain: the fields the operators write replaced."""
     names, made = {}, set()
+
+    def uses(keys, use):
+        for k in keys:
+            if k not in made and names.get(k, -1) < use:
+                names[k] = use
+
     for op in ops:
-        for k in op.reads + ((op.fill,) if op.fill else op.writes):
-            if k not in made:
-                names[k] = None
+        uses(op.reads, _READ)
+        if op.fill:
+            uses((op.fill,), _LIKE)
+        else:
+            uses(op.writes, _READ if op.fresh else _COPY)
         made.update(op.writes)
     outs = tuple(k for k in dict.fromkeys(k for op in ops for k in op.writes) if not k.startswith("_"))
-    new = _Chain.apply(tuple(ops), cg, tuple(names), outs, *[st[k] for k in names])
+    new = _Chain.apply(tuple(ops), cg, names, outs, *[st[k] for k in names])
     return {**st, **dict(zip(outs, new))}
 
 
@@ -1766,9 +1792,9 @@ class _EddyViscosity:
 
     def _metrics(self, cg, tab):
         """The metrics and deformations, which each direction forms anew."""
-        buf, names, n3 = _scratch_like(cg, per_point=len(self.scratch)), N.field_names(), cg.nz * cg.ny * cg.nx
+        buf, at, n3 = _scratch_like(cg, per_point=len(self.scratch)), _field_index(), cg.nz * cg.ny * cg.nx
         for q, k in enumerate(self.scratch):
-            tab[names.index(k)] = buf.data_ptr() + 4 * q * n3
+            tab[at[k]] = buf.data_ptr() + 4 * q * n3
         return buf
 
     def fwd(self, cg, tab, stream):
@@ -1871,13 +1897,13 @@ class _MoistUpdate:
         self.rk_step, self.dt_rk = rk_step, float(dt_rk)
 
     def fwd(self, cg, tab, stream):
-        status = torch.empty(16, dtype=torch.int32, device="cuda")  # counts NaN points for nobody
-        tab[N.field_names().index("status")] = status.data_ptr()
+        status = _scratch_like(cg, per_column=1)  # counts NaN points for nobody
+        tab[_field_index()["status"]] = status.data_ptr()
         return N.lib().wrf_moist_update(ctypes.byref(cg), tab, self.rk_step, self.dt_rk, stream)
 
     def adj(self, cg, tab, btab, stream):
         work = _scratch_like(cg, per_point=1)
-        tab[N.field_names().index("status")] = work.data_ptr()  # the reverse counts nothing
+        tab[_field_index()["status"]] = work.data_ptr()  # the reverse counts nothing
         return N.lib().wrf_moist_update_adj(ctypes.byref(cg), tab, btab, self.rk_step, self.dt_rk, _ptr(work), stream)
 
 
@@ -2010,12 +2036,12 @@ class _Microphysics:
 
     def _scratch(self, cg, tab):
         """The diagnostics and accumulators the block writes, in ``tab``."""
-        names, n2, n3 = N.field_names(), cg.ny * cg.nx, cg.nz * cg.ny * cg.nx
+        at, n2, n3 = _field_index(), cg.ny * cg.nx, cg.nz * cg.ny * cg.nx
         buf = _scratch_like(cg, per_point=len(self.scratch3), per_column=len(self.scratch2))
         for q, k in enumerate(self.scratch3):
-            tab[names.index(k)] = buf.data_ptr() + 4 * q * n3
+            tab[at[k]] = buf.data_ptr() + 4 * q * n3
         for q, k in enumerate(self.scratch2):
-            tab[names.index(k)] = buf.data_ptr() + 4 * (len(self.scratch3) * n3 + q * n2)
+            tab[at[k]] = buf.data_ptr() + 4 * (len(self.scratch3) * n3 + q * n2)
         return buf
 
     def fwd(self, cg, tab, stream):

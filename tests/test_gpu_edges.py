@@ -552,3 +552,38 @@ def test_a_checkpointed_rollout_holds_one_state_per_step():
     size = sum(v.numel() * 4 for v in state.values())
     first, last = held(1)[0], held(4)[0]
     assert last - first <= 3 * 1.01 * size + 4096 * len(names), (first / size, last / size)
+
+
+def test_arrays_with_gaps_where_only_their_slots_or_shapes_are_used():
+    """Species that lie together slot by slot in a larger array (step_end's
+    moist, the first stage's moist_tend) and tendencies whose shape alone is
+    read: the same values as from packed arrays; where an operator reads the
+    whole array, or a slot has gaps of its own, it is refused."""
+    g, state, data, bd, sc = _chain_case()
+    bt = {"u": bd["u"], "v": bd["v"], "h": bd["ph"], "t": bd["t"], "m": bd["mu"], "q": bd["qv"]}
+
+    def slots(v):
+        big = torch.full((2 * v.shape[0],) + tuple(v.shape[1:]), 7.0, device="cuda")
+        big[::2] = v
+        return big[::2]
+
+    def inner(v):
+        return torch.full(tuple(v.shape[:-1]) + (2 * v.shape[-1],), 7.0, device="cuda")[..., :v.shape[-1]].copy_(v)
+
+    def end(s):
+        return A.step_end(s, data, bd, 45.0, cf1=sc["cf1"], cf2=sc["cf2"], cf3=sc["cf3"], rdx=g.rdx, rdy=g.rdy)
+
+    def moist(s, rk=1):
+        return A.moist_stage(s, data, rk, 15.0, g.rdx, g.rdy, bt, 45.0)
+
+    def dynamics(s):
+        return A.dynamics_stage(s, data, bt, 2, 2, 9.0, **sc)
+
+    for run, name, gaps in ((end, "moist", slots), (moist, "moist_tend", slots), (dynamics, "ru_tend", inner)):
+        want, got = run(state), run({**state, name: gaps(state[name])})
+        for k in want:
+            assert torch.equal(want[k].view(torch.int32), got[k].contiguous().view(torch.int32)), (name, k)
+    for run, name, gaps in ((end, "moist", inner), (moist, "moist_tend", inner), (moist, "moist", slots),
+                            (lambda s: moist(s, 2), "moist_tend", slots), (dynamics, "u", inner)):
+        with pytest.raises(TypeError):
+            run({**state, name: gaps(state[name])})
