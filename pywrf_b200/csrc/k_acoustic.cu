@@ -1643,9 +1643,14 @@ int launch_advance_uv(const Grid& g, const S& s, float dts, cudaStream_t st, boo
   if (expired) return 0;
   const dim3 b3(32, 4);
   dim3 gr = point_grid(g, b3);
-  // short chunks while the grid is about one wave (ten blocks fit an SM): with
-  // two, three and four levels 10.1, 11.7 and 14.2 us at 101x101x35, 16.4, 12.4
-  // and 14.6 at 131x131x35
+  // two levels a thread while that leaves at most 12 blocks an SM (ten fit at a
+  // time; the frame's return at once), where a thread's own chain is the time;
+  // three from there on.  Two and three levels, us per launch with the operands
+  // in L2 / in DRAM: 8.5 / 14.3 and 8.5 / 16.4 at 91x91x35 (8 blocks an SM), 9.0 /
+  // 14.3 and 10.5 / 18.4 at 101x101x35 (11.9), 10.5 / 20.5 and 10.5 / 18.4 at
+  // 107x107x35 (12.4), 11.2 / 20.5 and 10.5 / 18.4 at 91x91x61 (14), 11.8 / 20.5
+  // and 10.5 / 18.4 at 121x121x35 (14.2), 12.6 / 20.5 and 10.5 / 18.4 at
+  // 131x131x35 (19)
   const int ktf = g.nz - 1;
   const bool two = (long long)gr.x * gr.y * ((ktf + 1) / 2) <= 148 * 12;
   gr.z = two ? (ktf + 1) / 2 : (ktf + 2) / 3;
