@@ -146,7 +146,19 @@ static void allow_smem(K kernel, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Blocks of 32 columns, row after row in one dimension of the grid (the second
+// takes no more than 65535 rows): nb blocks a row, and a block's place
+static unsigned row_blocks(int nb, int rows) { return (unsigned)nb * (unsigned)rows; }
+
 namespace {
+
+struct RowBlock {
+  int x, row;
+  __device__ __forceinline__ explicit RowBlock(int nb) {
+    row = blockIdx.x / nb;
+    x = blockIdx.x - row * nb;
+  }
+};
 
 // x += v by a reduction at the memory side: a cotangent that the kernel only
 // adds to is not loaded (nor do the loads that follow wait for the store).
@@ -780,6 +792,7 @@ __device__ __forceinline__ bool mut_in(const Grid& g, int j, int i) {
 // column passes of the reverse) at 240x240x41 and hardly less at 101x101x35,
 // a memory round trip every few levels.
 constexpr int kMutTX = 32, kMutKT = 8;
+__host__ __device__ inline int mut_blocks(const Grid& g) { return (g.ide - 1 + kMutTX - 1) / kMutTX; }
 
 // dvdxi of a column's levels, its two-dimensional factors loaded once
 struct MutDiv {
@@ -866,7 +879,8 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t(Grid g, S s, fl
   extern __shared__ float mut_smem[];
   const int nz = g.nz, ktf = nz - 1, nx = g.nx;
   const unsigned lev = (unsigned)g.ny * g.nx;
-  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const RowBlock rb(mut_blocks(g));
+  const int i = rb.x * kMutTX + threadIdx.x, j = g.jds + 1 + rb.row, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
   float* const sdv = mut_smem + threadIdx.x;
@@ -940,7 +954,8 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_dv(Grid g, 
   extern __shared__ float mut_smem[];
   const int ktf = g.nz - 1, nx = g.nx;
   const unsigned lev = (unsigned)g.ny * g.nx;
-  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const RowBlock rb(mut_blocks(g));
+  const int i = rb.x * kMutTX + threadIdx.x, j = g.jds + 1 + rb.row, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   const int c = in ? j * nx + i : 0;
   float* const swb = mut_smem + threadIdx.x;  // wwb, then qb one level down
@@ -1026,7 +1041,8 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
   extern __shared__ float mut_smem[];
   const int nz = g.nz, ktf = nz - 1, nx = g.nx, n = nz * kMutTX;
   const Ix lev = (Ix)g.ny * g.nx;
-  const int i = blockIdx.x * kMutTX + threadIdx.x, j = g.jds + 1 + blockIdx.y, tk = threadIdx.y;
+  const RowBlock rb(mut_blocks(g));
+  const int i = rb.x * kMutTX + threadIdx.x, j = g.jds + 1 + rb.row, tk = threadIdx.y;
   const bool in = mut_in(g, j, i);
   // muu, muv: the u / v terms of the divergence at this column
   const bool w = i >= 1 && mut_in(g, j, i - 1), sth = mut_in(g, j - 1, i), any = w || in || sth;
@@ -1156,9 +1172,7 @@ __global__ void __launch_bounds__(kMutTX* kMutKT) k_advance_mu_t_adj_col(Grid g,
 }
 
 // the rows of the updated columns (more: those above them, which muv's cotangent reaches)
-static dim3 mut_grid(const Grid& g, int more) {
-  return dim3((g.ide - 1 + kMutTX - 1) / kMutTX, g.jde - 3 - g.jds + more);
-}
+static unsigned mut_grid(const Grid& g, int more) { return row_blocks(mut_blocks(g), g.jde - 3 - g.jds + more); }
 
 int launch_advance_mu_t(const Grid& g, const S& s, float dts, cudaStream_t st) {
   k_advance_mu_t<<<mut_grid(g, 0), dim3(kMutTX, kMutKT), 2 * (size_t)g.nz * kMutTX * sizeof(float), st>>>(g, s, dts);
@@ -1940,7 +1954,8 @@ __global__ void __launch_bounds__(kVsTX* kVsKT) k_coef_w_adj(
   extern __shared__ float vs_smem[];
   const int nz = g.nz;
   const int tx = threadIdx.x % kVsTX, tk = threadIdx.x / kVsTX;
-  const int i = i0 + blockIdx.x * kVsTX + tx, j = g.jds + blockIdx.y;
+  const RowBlock rb((g.ide - 1 - i0 + kVsTX - 1) / kVsTX);
+  const int i = i0 + rb.x * kVsTX + tx, j = g.jds + rb.row;
   const bool col = i >= g.ids && i < g.ide - 1;
   const int c = col ? g.i2(j, i) : g.i2(j, g.ids);
   const unsigned lev = (unsigned)g.ny * g.nx;
@@ -2052,7 +2067,7 @@ int launch_coef_w_adj(const Grid& g, const float* mut, const float* cqw, const f
   const int i0 = g.nx % 8 == 0 ? g.ids / 8 * 8 : g.ids;
   const size_t smem = 7 * (size_t)g.nz * kVsTX * sizeof(float);
   allow_smem(k_coef_w_adj, smem);
-  k_coef_w_adj<<<dim3((g.ide - 1 - i0 + kVsTX - 1) / kVsTX, g.jde - 1 - g.jds), kVsTX * kVsKT, smem, st>>>(
+  k_coef_w_adj<<<row_blocks((g.ide - 1 - i0 + kVsTX - 1) / kVsTX, g.jde - 1 - g.jds), kVsTX * kVsKT, smem, st>>>(
       g, mut, cqw, c2a, rdn, rdnw, dts, abar, alphabar, gammabar, mutbar, cqwbar, c2abar, i0);
   return 1;
 }

@@ -587,3 +587,47 @@ def test_arrays_with_gaps_where_only_their_slots_or_shapes_are_used():
                             (lambda s: moist(s, 2), "moist_tend", slots), (dynamics, "u", inner)):
         with pytest.raises(TypeError):
             run({**state, name: gaps(state[name])})
+
+
+@pytest.mark.parametrize("name", ["advance_mu_t", "coef_w_adj"])
+def test_column_tiles_on_more_rows_than_a_grid_dimension(name):
+    """70000 rows (a grid's second dimension takes 65535): the last inner rows
+    against the same rows as a domain of their own, bitwise (nothing sums over
+    rows)."""
+    nz, nx, rows, crop = 12, 24, 70000, 64
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    fld = {True: {}, False: {}}
+
+    def field(k, two_d):
+        if k not in fld[two_d]:
+            fld[two_d][k] = 1.0 + 0.1 * torch.rand(*((rows, nx) if two_d else (nz, rows, nx)), generator=gen, device="cuda")
+        return fld[two_d][k]
+
+    prof = {k: torch.linspace(0.9, 1.1, nz, device="cuda") for k in ("fnm", "fnp", "rdn", "rdnw", "dnw")}
+
+    def run(cut):
+        def get(k, two_d=False):
+            v = field(k, two_d)
+            return (v[..., rows - crop:, :] if cut else v).clone()
+
+        ny = crop if cut else rows
+        if name == "coef_w_adj":
+            cg = A.scalar_grid((nz, ny, nx), 1 / 9000.0, 1 / 9000.0)
+            out = [torch.zeros(ny, nx, device="cuda")] + [torch.zeros(nz, ny, nx, device="cuda") for _ in range(2)]
+            ops = [get("mut", True), get("cqw"), get("c2a"), prof["rdn"], prof["rdnw"]]
+            cots = [get(k) for k in ("ca", "calpha", "cgamma")]
+            N.check(N.lib().wrf_coef_w_adj(ctypes.byref(cg), *map(_p, ops), 0.01, *map(_p, cots), *map(_p, out),
+                                           _stream()), "coef_w_adj")
+        else:
+            two = {"mu", "mut", "muave", "muts", "muu", "muv", "mudf", "mu_tend"}
+            x = {k: get(k, k in two).requires_grad_(True) for k in A.MUT_INPUTS}
+            data = {k: prof[k] if k in prof else get(k, True) for k in A.MUT_DATA}
+            res = A.advance_mu_t(x, data, 0.1, 0.1, 1 / 9000.0, 1 / 9000.0)
+            out = [v.detach() for v in res.values()]
+            out += torch.autograd.grad(list(res.values()), list(x.values()),
+                                       grad_outputs=[get("cot_" + k, k in two) for k in res])
+        torch.cuda.synchronize()
+        return [v[..., ny - 32:ny - 12, :].clone() for v in out]
+
+    for a, b in zip(run(True), run(False)):
+        assert float(a.abs().max()) > 0.0 and torch.equal(a, b)
