@@ -631,3 +631,63 @@ def test_column_tiles_on_more_rows_than_a_grid_dimension(name):
 
     for a, b in zip(run(True), run(False)):
         assert float(a.abs().max()) > 0.0 and torch.equal(a, b)
+
+
+def test_marching_acoustic_columns_from_a_sector_and_deep():
+    """Rows of whole sectors, whose blocks start left of the first column, and
+    the depth the marching kernel was made for."""
+    test_marching_acoustic_columns_equal_the_tiled_form_bitwise(320, 61)
+
+
+@pytest.mark.parametrize("n,nz,rk", [(64, 17, 1), (140, 41, 1), (140, 41, 2), (130, 38, 1)])
+def test_tendency_accumulation_at_both_depths_per_thread(n, nz, rk):
+    """The step's fused accumulation, at one level a thread and (from 606208
+    points on) at four with a remainder, against the stand-alone accumulation
+    and the specified rows on the fields the step had before it, bitwise (its
+    divisions are correctly rounded)."""
+    spec = synthetic.CaseSpec(n=n, nz=nz, nsteps=1, bdy_tend_amp=1.0e-4, seed=n)
+    g = synthetic.grid_for(spec)
+    inputs, bdy = synthetic.build(spec)
+    st = DeviceState.from_inputs(g, inputs, bdy, device="cuda")
+    before, after = {}, {}
+
+    def probe(name):
+        if name == ("s1.diff" if rk == 1 else f"s{rk}.forces"):
+            before.update({k: st[k].clone() for k in A._Addtend.fields})
+        if name == f"s{rk}.tend":
+            after.update({k: st[k].clone() for k in A._Addtend.outputs})
+
+    Integrator(st).step(probe)
+    torch.cuda.synchronize()
+    want = A.addtend(before, {k: st[k] for k in A._Addtend.data}, rk, g.rdx, g.rdy)
+    for k, var, f in (("ru_tend", "u", "u"), ("rv_tend", "v", "v"), ("ph_tend", "h", "ph"), ("t_tend", "t", "t"),
+                      ("mu_tend", "m", "mu")):
+        bt = {key: st[f"{f}_{b}"] for b, key in (("btxs", "txs"), ("btxe", "txe"), ("btys", "tys"), ("btye", "tye"))}
+        want[k] = A.spec_bdytend(want[k], bt, var, g.rdx, g.rdy)
+    for k in A._Addtend.outputs:
+        assert torch.equal(after[k], want[k]), k
+    assert float(after["ru_tend"].abs().max()) > 0.0
+
+
+def test_a_chain_whose_names_share_a_tensor():
+    """One tensor under two names of the state: its gradient is the sum of
+    those of two equal tensors (sums by atomics in some order: 1e-5 of the
+    norm)."""
+    pairs = (("u", "u_1"), ("t", "t_1"), ("mu", "mu_1"))
+    got = []
+    for shared in (True, False):
+        _, state, data, bd, sc = _chain_case()
+        state["t"] += 0.1 * torch.sin(torch.arange(state["t"].numel(), device="cuda").view_as(state["t"]).float())
+        leaves = []
+        for a, b in pairs:
+            state[a].requires_grad_(True)
+            state[b] = state[a] if shared else state[a].detach().clone().requires_grad_(True)
+            leaves += [state[a]] if shared else [state[a], state[b]]
+        out = _first_stage(state, data, bd, sc)
+        names = ("u", "w", "t", "p", "t_1", "mu_1")
+        grads = torch.autograd.grad([out[k] for k in names], leaves,
+                                    grad_outputs=[torch.cos(torch.arange(out[k].numel(), device="cuda").view_as(out[k])
+                                                            .float()) for k in names])
+        got.append(grads if shared else [a + b for a, b in zip(grads[::2], grads[1::2])])
+    for a, b in zip(*got):
+        assert float(a.norm()) > 0.0 and float((a - b).norm()) <= 1e-5 * float(a.norm())
