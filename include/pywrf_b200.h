@@ -254,7 +254,6 @@ int wrf_halo(const WrfGrid* g, float* field, char var, int two_d, void* stream);
 /* Its adjoint: the cotangent of the copied field is added (+=) into in_bar,
  * the cotangent of the field before the copies (a separate array). */
 int wrf_halo_adj(const WrfGrid* g, const float* field_bar, float* in_bar, char var, int two_d, void* stream);
-/* wrf_boundary.py:358-400 zero_grad_bdy of w (all levels), in place. */
 /* out[f] = the halo copies of in[f] (stagger letter vars[f], two_d[f] as for
  * wrf_halo; 'Z': zero_grad_bdy of w) for a batch of n fields, out of place,
  * and the adjoint (in_bar[f] written, not accumulated); every out array is
@@ -269,6 +268,7 @@ int wrf_halo_copy_adj(const WrfGrid* g, int n, const float* const* out_bar, floa
 int wrf_advect_moist(const WrfGrid* g, const float* moist, float* advect_tend, const float* ru, const float* rv,
                      const float* rom, const float* msftx, const float* fzm, const float* fzp, const float* rdzw,
                      void* stream);
+/* wrf_boundary.py:358-400 zero_grad_bdy of w (all levels), in place. */
 int wrf_zero_grad_w(const WrfGrid* g, float* w, void* stream);
 /* Its adjoint: w_bar is added (+=) into in_bar (a separate array). */
 int wrf_zero_grad_w_adj(const WrfGrid* g, const float* w_bar, float* in_bar, void* stream);

@@ -54,7 +54,8 @@ operators keeps no tape of the forward's intermediates.
 * :func:`addtend`, :class:`SpecBdytend`, the moisture update
   (rk_update_scalar, flow_dep_bdy, calc_p_rho_phi), :func:`microphysics`
   (moist_physics_prep_em, WSM6, moist_physics_finish_em, calc_p_rho_phi;
-  WSM6's reverse in reverse mode over a per-column tape of a restatement) and
+  WSM6's sedimentation in reverse mode over tapes of a restatement, the rest
+  of it per level by forward-mode tangents) and
   :func:`step_end` (halo copies, spec_bdy_final, set_w_surface).
 * Composed in the reference's order: :func:`acoustic_substep`,
   :func:`acoustic_stage`, :func:`dynamics_stage`, :func:`moist_stage`,
@@ -2071,11 +2072,12 @@ class _Microphysics:
 def microphysics(st: dict, data: dict, dt: float, rdx, rdy) -> dict:
     """Differentiable microphysics of the step (pywrf/solver.py:1714-1766):
     returns ``st`` with t, moist, al, p and h_diabatic replaced.  Its reverse
-    is the equation of state's exact reverse, then prep + WSM6 + finish in
-    reverse mode: each column of a restatement of the scheme runs once on
-    taped scalars and one reverse sweep of its tape gives its inputs'
-    cotangents (forward-mode tangents for a column whose tape outgrows the
-    capacity)."""
+    is the equation of state's exact reverse, then that of prep + WSM6 + finish
+    over a restatement of the scheme.  With one time-split loop (dt up to 240 s)
+    the falls of a column run once on taped scalars, reversed by one sweep of
+    their tapes, and all else takes forward-mode tangents per level; with several
+    loops the whole column is taped.  A column whose tape outgrows the capacity
+    takes tangents of the whole restatement."""
     op = _Microphysics()
     cg = scalar_grid(st["t"].shape, rdx, rdy)
     cg.dt = float(dt)

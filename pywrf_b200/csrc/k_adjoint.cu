@@ -16,10 +16,10 @@
 //   qbar(m) += sum over faces f whose stencil holds m of Fbar(f) r(f) dPhi_f/dq(m)
 //   rbar(f) += Fbar(f) Phi(f)
 // The faces pass forms each face once (its rbar, and Fbar r with the
-// upwind sign in six arrays of caller work); the gather pass sums, per point, over the faces whose
-// stencils hold it in a fixed order.  Each output
-// element is written by one thread, so results do not depend on scheduling;
-// tend's own cotangent is tbar unchanged (the caller passes it through).
+// upwind sign in six arrays of caller work); the gather pass sums, per point,
+// over the faces whose stencils hold it in a fixed order.  Each output element
+// is written by one thread, so results do not depend on scheduling; tend's own
+// cotangent is tbar unchanged (the caller passes it through).
 //
 //   k_advect_mom_faces<C> + k_advect_mom_gather<C>
 //                        adjoint of advect_u (C = 0, wrf_dynamics.py:1112-1331),
@@ -85,7 +85,8 @@
 //                        reference's autograd sees it (computed under
 //                        torch.no_grad(): each passes its cotangent to the
 //                        input of the same name and nothing to dmdt, mut or
-//                        mu_tend).
+//                        mu_tend).  All but (2) are 32-column blocks with
+//                        the scans in shared memory.
 //
 //   k_advance_w_lp / k_advance_w_adj_lp / k_advance_w_adj_bc  advance_w
 //                        (wrf_dynamics.py:3641-3796) on the columns [ids+1,
@@ -121,15 +122,18 @@
 //                        a, alpha, gamma of calc_coef_w:
 //   y(0) = x(0);  y(k) = (x(k) - a(k) y(k-1)) alpha(k),  k = 1..nz-1
 //   w(nz-1) = y(nz-1);  w(k) = y(k) - gamma(k) w(k+1),  k = nz-2..1;  w(0) = y(0)
-//                        The reverse sweep runs the two recurrences backwards
-//                        (one thread per column; the column's y and w are
-//                        recomputed into local arrays).
+//                        The reverse runs the two recurrences backwards.  A
+//                        block brings its 32 columns into shared memory over
+//                        eight level groups, one warp recomputes y and w while
+//                        another runs the reversed sweeps, and the products
+//                        of the levels follow in parallel.
 //
 //   k_coef_w_adj         adjoint of calc_coef_w (wrf_dynamics.py:3316-3388)
 //                        with respect to cqw, c2a and mut: the column's
 //                        forward recurrence alpha(k) = 1 / (b(k) - a(k)
 //                        gamma(k-1)), gamma(k) = c(k) alpha(k) is recomputed
-//                        into local arrays and run backwards.
+//                        in shared memory and run backwards by one warp of
+//                        the same 32-column blocks.
 #include <limits.h>
 #include "kernels.cuh"
 #include "relax.cuh"
