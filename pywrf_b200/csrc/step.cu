@@ -5,6 +5,7 @@
 // allocates nothing and never synchronises (a probe callback may).  The
 // boundary time of the step is derived on the device from the step counter
 // STATUS[WRF_ST_STEP], so one captured CUDA graph replays every step.
+#include <limits.h>
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -72,6 +73,15 @@ int make_grid(const WrfGrid* in, Grid& g) {
   g.rdx = (float)g.rdxd; g.rdy = (float)g.rdyd;
   g.smdiv = in->smdiv; g.emdiv = in->emdiv; g.epssm = in->epssm;
   g.cf1 = in->cf1; g.cf2 = in->cf2; g.cf3 = in->cf3; g.cfn = in->cfn; g.cfn1 = in->cfn1;
+  return WRF_OK;
+}
+
+// for the entries whose kernels hold a point's offset in 32 bits: the step and
+// its phases, and the eddy viscosities, which share its kernels
+int make_step_grid(const WrfGrid* in, Grid& g) {
+  const int rc = make_grid(in, g);
+  if (rc) return rc;
+  if (g.n3() > INT_MAX) return fail(WRF_EINVAL, "nz * ny * nx must stay below 2^31 here");
   return WRF_OK;
 }
 
@@ -379,7 +389,7 @@ int wrf_set_kernel_form(int form) {
 
 int wrf_rk3_step(const WrfGrid* gin, const WrfState* sin, void* stream, wrf_probe_fn probe, void* user) {
   Driver d;
-  int rc = make_grid(gin, d.g);
+  int rc = make_step_grid(gin, d.g);
   if (rc) return rc;
   rc = make_state(sin, d.s);
   if (rc) return rc;
@@ -400,7 +410,7 @@ namespace {
 template <typename F>
 int run_phase(const WrfGrid* gin, const WrfState* sin, void* stream, int rk, int it, F body) {
   Driver d;
-  int rc = make_grid(gin, d.g);
+  int rc = make_step_grid(gin, d.g);
   if (rc) return rc;
   rc = make_state(sin, d.s);
   if (rc) return rc;
@@ -1120,7 +1130,7 @@ int wrf_spec_bdytend_adj(const WrfGrid* gin, float* tend_bar, char var, void* st
 
 int wrf_eddy_viscosity(const WrfGrid* gin, const WrfState* sin, void* stream) {
   Grid g;
-  int rc = make_grid(gin, g);
+  int rc = make_step_grid(gin, g);
   if (rc) return rc;
   S s;
   if ((rc = state_of(sin, kKmOperands, sizeof(kKmOperands) / sizeof(int), s))) return rc;
@@ -1132,7 +1142,7 @@ int wrf_eddy_viscosity(const WrfGrid* gin, const WrfState* sin, void* stream) {
 int wrf_eddy_viscosity_adj(const WrfGrid* gin, const WrfState* sin, const WrfState* sbar, float* work,
                            void* stream) {
   Grid g;
-  int rc = make_grid(gin, g);
+  int rc = make_step_grid(gin, g);
   if (rc) return rc;
   if (!work) return fail(WRF_EINVAL, "eddy_viscosity_adj: work (6*nz*ny*nx floats) is required");
   S s, b;
@@ -1572,7 +1582,7 @@ int wrf_rk3_step_mlp(const WrfGrid* gin, const WrfState* sin, const WrfMlpNet* n
   wd.err = work->err;
   wd.colstat = work->colstat;
   Driver d;
-  int rc = make_grid(gin, d.g);
+  int rc = make_step_grid(gin, d.g);
   if (rc) return rc;
   rc = make_state(sin, d.s);
   if (rc) return rc;
