@@ -1057,7 +1057,7 @@ def acoustic_substep(st: dict, data: dict, iteration: int, nsub: int, dts: float
     is a hand-written reverse kernel, and the chain keeps only the operators'
     inputs."""
     cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3)
-    return _run_chain(_substep_ops(data, iteration, nsub, dts), cg, st)
+    return _run_chain(_substep_ops(iteration, nsub, dts), cg, st, data)
 
 
 def _scratch_like(cg, per_point: int = 0, per_column: int = 0) -> torch.Tensor:
@@ -1135,38 +1135,40 @@ class _Bars(dict):
 class _ChainOp:
     """One operator of a chain: ``reads`` are the state names its reverse
     needs (their values on entry are kept), ``writes`` those it replaces and
-    ``const`` the constant arrays that both directions use.
+    ``const`` the names of the constant arrays that both directions use.
     ``forward(cg, st, out, const, stream)`` fills ``out`` (copies of the written
-    fields, updated in place; with ``fresh``, uninitialised) and
-    ``backward(cg, saved, bars, const, stream)`` turns the written names'
-    cotangents into those of the values on entry and adds the rest.  The chain
-    saves what the reverse uses with its other tensors (an array changed in
-    between raises, saved-tensor hooks see it, a checkpoint drops it), so
-    ``backward`` holds no tensor itself."""
+    fields, updated in place; with ``fresh``, uninitialised, shaped like
+    ``fill``) and ``backward(cg, saved, bars, const, stream)`` turns the written
+    names' cotangents into those of the values on entry and adds the rest.  The
+    chain saves what the reverse uses with its other tensors (an array changed
+    in between raises, saved-tensor hooks see it, a checkpoint drops it), so
+    ``backward`` holds no tensor itself; ``const`` maps the constants of the
+    whole chain."""
 
-    def __init__(self, reads, writes, forward, backward, const=None, fresh=False, fill=None):
+    def __init__(self, reads, writes, forward, backward, const=(), fresh=False, fill=None):
         self.reads, self.writes, self.forward, self.backward = tuple(reads), tuple(writes), forward, backward
-        self.const, self.fresh, self.fill = dict(const or {}), fresh, fill
+        self.const, self.fresh, self.fill = tuple(const), fresh, fill
 
 
 def _rc(rc, name):
     N.check(rc, name)
 
 
-def _table_chain_op(op, data: dict, held=()):
+def _table_chain_op(op, held=()):
     """A chain operator from a state-table operator (see :class:`_TableOp`);
     ``held`` names those of its constants that are fields of the chain's state
     (which receive no cotangent)."""
-    reads = op.fields + tuple(held)
+    reads, data = op.fields + tuple(held), tuple(k for k in op.data if k not in held)
 
     def fwd(cg, st, out, const, stream):
-        _rc(op.fwd(cg, _table({**const, **{k: st[k] for k in reads}, **out}), stream), op.name)
+        _rc(op.fwd(cg, _table({**{k: const[k] for k in data}, **{k: st[k] for k in reads}, **out}), stream), op.name)
 
     def bwd(cg, saved, bars, const, stream):
-        likes = {k: saved[k] for k in op.fields}
-        _rc(op.adj(cg, _table({**const, **saved}), _table(bars.need(likes)), stream), op.name + "_adj")
+        likes = {k: saved[k] for k in op.fields} if held else saved
+        _rc(op.adj(cg, _table({**{k: const[k] for k in data}, **saved}), _table(bars.need(likes)), stream),
+            op.name + "_adj")
 
-    return _ChainOp(reads, op.outputs, fwd, bwd, {k: data[k] for k in op.data if k not in held})
+    return _ChainOp(reads, op.outputs, fwd, bwd, data)
 
 
 class _CallOp:
@@ -1179,67 +1181,69 @@ class _CallOp:
 
 class _Chain(torch.autograd.Function):
     """The operators ``ops`` in order on the state fields ``names`` (each
-    with what is used of it, see :func:`_run_chain`); returns the final values
-    of ``outs``."""
+    with what is used of it, see :func:`_run_chain`) and the constants ``const``;
+    returns the final values of ``outs``."""
 
     @staticmethod
-    def forward(ctx, ops, cg, names, outs, *tensors):
+    def forward(ctx, ops, cg, names, outs, const, *tensors):
         ctx.set_materialize_grads(False)
-        for use, v in zip(names.values(), tensors):
+        st = {}
+        own = set()   # ids of this chain's tensors that nothing has kept
+        for (k, use), v in zip(names.items(), tensors):
             if use == _COPY and v.dim() == 4:  # taken slot by slot
                 _cuda_only(*v.unbind())
             elif use != _LIKE:
                 _ptr(v)
-        st = {k: v.detach() for k, v in zip(names, tensors)}
-        kept = {}     # id of a kept tensor -> its place among the saved ones
-        saved, steps = [], []
-        own = set()   # ids of this chain's tensors that nothing has kept
-
-        def places(values):
-            at = []
-            for k, v in values:
-                q = kept.get(id(v))
-                if q is None:
-                    q = kept[id(v)] = len(saved)
-                    saved.append(v.detach() if v.requires_grad else v)
-                    own.discard(id(v))
-                at.append((k, q))
-            return at
-
+            st[k] = v.detach()
+            if not v.is_contiguous():
+                st[k] = st[k].contiguous() if use == _COPY else _packed_like(v)
+                own.add(id(st[k]))
+        saved = [v.detach() if v.requires_grad else v for v in const.values()]
+        kept, steps = {}, []  # id of a kept state tensor -> its place among the saved ones
         with _on(tensors[0]):
             stream = _stream(tensors[0])
             for op in ops:
-                steps.append((op.backward, places([(k, st[k]) for k in op.reads]), places(op.const.items())))
+                at = []
+                for k in op.reads:
+                    v = st[k]
+                    q = kept.get(id(v))
+                    if q is None:
+                        q = kept[id(v)] = len(saved)
+                        saved.append(v)
+                        own.discard(id(v))
+                    at.append(q)
+                steps.append((op.backward, op.reads, at))
                 out = {}
                 for k in op.writes:
                     if op.fresh:
-                        out[k] = _packed_like(st[op.fill or k])
+                        out[k] = torch.empty_like(st[op.fill or k])
                     elif id(st[k]) in own:
                         out[k] = st[k]
                     else:
-                        out[k] = st[k].clone(memory_format=torch.contiguous_format)
-                op.forward(cg, st, out, op.const, stream)
+                        out[k] = st[k].clone()
+                op.forward(cg, st, out, const, stream)
                 for k, v in out.items():
                     st[k] = v
                     own.add(id(v))
         ctx.save_for_backward(*saved)
-        ctx.steps, ctx.cg, ctx.names, ctx.outs = steps, cg, tuple(names), outs
+        ctx.steps, ctx.cg, ctx.names, ctx.outs, ctx.const = steps, cg, tuple(names), outs, tuple(const)
         ctx.device = tensors[0].get_device()
         return tuple(st[k] for k in outs)
 
     @staticmethod
     def backward(ctx, *gouts):
         saved = ctx.saved_tensors  # read once (checkpoint unpacks each saved tensor once)
+        const = dict(zip(ctx.const, saved))
         bars = _Bars()
         for k, gk in zip(ctx.outs, gouts):
             if gk is not None:
                 bars[k] = gk.contiguous().clone()
         with torch.cuda.device(ctx.device):
             stream = torch.cuda.current_stream(ctx.device).cuda_stream
-            for backward, reads, const in reversed(ctx.steps):
-                backward(ctx.cg, {k: saved[q] for k, q in reads}, bars, {k: saved[q] for k, q in const}, stream)
-        need = ctx.needs_input_grad[4:]
-        return (None, None, None, None) + tuple(bars.get(k) if w else None for k, w in zip(ctx.names, need))
+            for backward, reads, at in reversed(ctx.steps):
+                backward(ctx.cg, {k: saved[q] for k, q in zip(reads, at)}, bars, const, stream)
+        need = ctx.needs_input_grad[5:]
+        return (None,) * 5 + tuple(bars.get(k) if w else None for k, w in zip(ctx.names, need))
 
 
 # what a chain uses of a field it is given: its shape, an updated copy of it, or
@@ -1247,24 +1251,22 @@ class _Chain(torch.autograd.Function):
 _LIKE, _COPY, _READ = range(3)
 
 
-def _run_chain(ops, cg, st: dict) -> dict:
-    """``st`` after the chain: the fields the operators write replaced."""
+def _run_chain(ops, cg, st: dict, data: dict) -> dict:
+    """``st`` after the chain, whose constants are in ``data``: the fields the
+    operators write replaced."""
     names, made = {}, set()
-
-    def uses(keys, use):
-        for k in keys:
-            if k not in made and names.get(k, -1) < use:
-                names[k] = use
-
     for op in ops:
-        uses(op.reads, _READ)
-        if op.fill:
-            uses((op.fill,), _LIKE)
-        else:
-            uses(op.writes, _READ if op.fresh else _COPY)
+        for k in op.reads:
+            if k not in made:
+                names[k] = _READ
+        use = _LIKE if op.fill else _READ if op.fresh else _COPY
+        for k in (op.fill,) if op.fill else op.writes:
+            if k not in made:
+                names[k] = max(names.get(k, use), use)
         made.update(op.writes)
     outs = tuple(k for k in dict.fromkeys(k for op in ops for k in op.writes) if not k.startswith("_"))
-    new = _Chain.apply(tuple(ops), cg, names, outs, *[st[k] for k in names])
+    const = {k: data[k] for k in dict.fromkeys(k for op in ops for k in op.const)}
+    new = _Chain.apply(tuple(ops), cg, names, outs, const, *[st[k] for k in names])
     return {**st, **dict(zip(outs, new))}
 
 
@@ -1363,7 +1365,7 @@ def _advect_work(cg, name, like):
     return torch.empty(int(n.value), dtype=torch.float32, device=like.device), n
 
 
-def _advect_momentum_op(component, field, tend, data: dict):
+def _advect_momentum_op(component, field, tend):
     msf = ("msfux", "msfvy", "msftx")[component]
     msf2 = "msfvx" if component == 1 else None
     names = (msf, msf2, "fnm", "fnp", "rdn" if component == 2 else "rdnw")
@@ -1387,13 +1389,13 @@ def _advect_momentum_op(component, field, tend, data: dict):
                                             n, stream),
             "wrf_advect_momentum_adj")
 
-    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, {k: data[k] for k in names if k})
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, [k for k in names if k])
 
 
 ADVECT_DATA = ("msftx", "fnm", "fnp", "rdnw")
 
 
-def _advect_scalar_op(field, tend, data: dict):
+def _advect_scalar_op(field, tend):
     def fwd(cg, st, out, const, stream):
         _rc(N.lib().wrf_advect_scalar(ctypes.byref(cg), _ptr(st[field]), _ptr(out[tend]), _ptr(st["ru"]),
                                       _ptr(st["rv"]), _ptr(st["ww"]), *[_ptr(const[k]) for k in ADVECT_DATA], stream),
@@ -1409,10 +1411,10 @@ def _advect_scalar_op(field, tend, data: dict):
                                           _ptr(b[field]), _ptr(b["ru"]), _ptr(b["rv"]), _ptr(b["ww"]), _ptr(work), n,
                                           stream), "wrf_advect_scalar_adj")
 
-    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, {k: data[k] for k in ADVECT_DATA})
+    return _ChainOp((field, "ru", "rv", "ww"), (tend,), fwd, bwd, ADVECT_DATA)
 
 
-def _advect_moist_op(data: dict):
+def _advect_moist_op():
     """advect_tend = the advection of qv .. qg (slots 1..6) by the averaged
     fluxes, zero outside the advected points (pywrf/wrf_dynamics.py:
     3982-4051)."""
@@ -1437,18 +1439,17 @@ def _advect_moist_op(data: dict):
                                               _ptr(b["moist"][m]), *[_ptr(b[k]) for k in fluxes], _ptr(work), n,
                                               stream), "wrf_advect_scalar_adj")
 
-    return _ChainOp(("moist",) + fluxes, ("advect_tend",), fwd, bwd, {k: data[k] for k in ADVECT_DATA},
-                    fresh=True, fill="moist")
+    return _ChainOp(("moist",) + fluxes, ("advect_tend",), fwd, bwd, ADVECT_DATA, fresh=True, fill="moist")
 
 
-def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
-    """tend += horizontal_diffusion(field); ``field`` "moist": its six
-    species into the slots of ``tend``."""
+def _diffusion_op(var, field, tend, mass, visc, base=None):
+    """tend += horizontal_diffusion(field - ``base``, a constant); ``field``
+    "moist": its six species into the slots of ``tend``."""
     def each(v):
         return [v[m] for m in range(1, 7)] if v.dim() == 4 else [v]
 
     def fwd(cg, st, out, const, stream):
-        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), _ptr(const["base"]) if "base" in const else None
+        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), None if base is None else _ptr(const[base])
         for f, o in zip(each(st[field]), each(out[tend])):
             _rc(N.lib().wrf_horizontal_diffusion(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp, _ptr(st[mass]),
                                                  _ptr(st[visc]), _ptr(o), stream), "wrf_horizontal_diffusion")
@@ -1457,18 +1458,17 @@ def _diffusion_op(var, field, tend, mass, visc, data: dict, base=None):
         if bars.get(tend) is None:
             return
         b = bars.need(saved)
-        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), _ptr(const["base"]) if "base" in const else None
+        tab, bp = _table({k: const[k] for k in HDIFF_DATA}), None if base is None else _ptr(const[base])
         for f, gk, fb in zip(each(saved[field]), each(bars[tend]), each(b[field])):
             _rc(N.lib().wrf_horizontal_diffusion_adj(ctypes.byref(cg), tab, var.encode(), _ptr(f), bp,
                                                      _ptr(saved[mass]), _ptr(saved[visc]), _ptr(gk), _ptr(fb),
                                                      _ptr(b[mass]), _ptr(b[visc]), stream),
                 "wrf_horizontal_diffusion_adj")
 
-    return _ChainOp((field, mass, visc), (tend,), fwd, bwd,
-                    {k: data[k] for k in HDIFF_DATA} | ({} if base is None else {"base": base}))
+    return _ChainOp((field, mass, visc), (tend,), fwd, bwd, HDIFF_DATA + (() if base is None else (base,)))
 
 
-def _coef_w_op(dts, data: dict):
+def _coef_w_op(dts):
     names = ("a", "alpha", "gamma")
 
     def fwd(cg, st, out, const, stream):
@@ -1487,11 +1487,10 @@ def _coef_w_op(dts, data: dict):
         for k in names:
             del bars[k]
 
-    return _ChainOp(("mut", "cqw", "c2a"), names, fwd, bwd, {k: data[k] for k in ("rdn", "rdnw")}, fresh=True,
-                    fill="cqw")
+    return _ChainOp(("mut", "cqw", "c2a"), names, fwd, bwd, ("rdn", "rdnw"), fresh=True, fill="cqw")
 
 
-def _substep_ops(data: dict, iteration: int, nsub: int, dts: float) -> list:
+def _substep_ops(iteration: int, nsub: int, dts: float) -> list:
     """The operators of one acoustic substep, in the reference's order."""
     L = N.lib()
     by = ctypes.byref
@@ -1515,20 +1514,20 @@ def _substep_ops(data: dict, iteration: int, nsub: int, dts: float) -> list:
     sp = _CallOp("wrf_spec_bdyupdate_ph", SPH_INPUTS, ("ph",), (),
                  lambda cg, tab, s: L.wrf_spec_bdyupdate_ph(by(cg), tab, dts, s),
                  lambda cg, tab, b, s: L.wrf_spec_bdyupdate_ph_adj(by(cg), tab, b, dts, s))
-    ops = [_table_chain_op(uv, data), _table_chain_op(mt, data)]
+    ops = [_table_chain_op(uv), _table_chain_op(mt)]
     ops += [_spec_update_op("t", "t_tend", dts, "t"), _spec_update_op("mu", "mu_tend", dts, "m"),
             _spec_update_op("muts", "mu_tend", dts, "m")]
-    ops += [_table_chain_op(aw, data), _table_chain_op(sf, data), _table_chain_op(sp, data), _p_rho_op(data, iteration)]
+    ops += [_table_chain_op(aw), _table_chain_op(sf), _table_chain_op(sp), _p_rho_op(iteration)]
     ops.append(_halo_op(("w", "ph", "al", "p", "muts", "mu", "mudf"), "Zwppttt"))
     return ops
 
 
-def _p_rho_op(data: dict, step: int):
+def _p_rho_op(step: int):
     ren = tuple(_PRHO_FIELD.get(k, k) for k in PRHO_INPUTS)
     return _table_chain_op(_CallOp("wrf_calc_p_rho", ren, ("al", "p", "pm1"), ("rdnw",),
                                    lambda cg, tab, s: N.lib().wrf_calc_p_rho(ctypes.byref(cg), tab, step, s),
                                    lambda cg, tab, b, s: N.lib().wrf_calc_p_rho_adj(ctypes.byref(cg), tab, b, step,
-                                                                                    s)), data)
+                                                                                    s)))
 
 
 def _chain_grid(shape, rdx, rdy, **scal):
@@ -1615,16 +1614,16 @@ def acoustic_stage(st: dict, data: dict, rk_step: int, nsub: int, dts: float, *,
     returns the state after the stage."""
     cg = _chain_grid(st["u"].shape, rdx, rdy, epssm=epssm, emdiv=emdiv, smdiv=smdiv, cf1=cf1, cf2=cf2, cf3=cf3,
                      top_lid=int(bool(top_lid)))
-    return _run_chain(_acoustic_ops(data, rk_step, nsub, dts), cg, st)
+    return _run_chain(_acoustic_ops(rk_step, nsub, dts), cg, st, data)
 
 
-def _acoustic_ops(data: dict, rk_step: int, nsub: int, dts: float) -> list:
+def _acoustic_ops(rk_step: int, nsub: int, dts: float) -> list:
     """The operators of :func:`acoustic_stage`."""
-    ops = [_table_chain_op(_SmallStepPrep(rk_step), data), _p_rho_op(data, 0), _coef_w_op(dts, data),
+    ops = [_table_chain_op(_SmallStepPrep(rk_step)), _p_rho_op(0), _coef_w_op(dts),
            _halo_op(("ru_tend", "rv_tend", "ph", "al", "p", "t_1", "t_save", "mu_1", "mu", "mudf"), "uvwppttttt")]
     for it in range(1, nsub + 1):
-        ops += _substep_ops(data, it, nsub, dts)
-    ops.append(_table_chain_op(_SmallStepFinish(dts, nsub, rk_step), data))
+        ops += _substep_ops(it, nsub, dts)
+    ops.append(_table_chain_op(_SmallStepFinish(dts, nsub, rk_step)))
     if rk_step == 3:
         ops.append(_halo_op(("ru_m", "rv_m", "ww_m", "mut", "muts"), "uvwtt"))
     return ops
@@ -1826,12 +1825,12 @@ DYN_DATA = tuple(dict.fromkeys(STAGE_DATA + PREP_DATA + FORCES_DATA + _Addtend.d
                                HDIFF_DATA + ("t_init",)))
 
 
-def _first_stage_ops(data: dict, bdy: dict, dtbc: float, nz: int) -> list:
+def _first_stage_ops(bdy: dict, dtbc: float, nz: int) -> list:
     """The first stage's horizontal diffusion of u, v, w and theta into the
     physics tendencies and the lateral relaxation into the saved fields
     (pywrf/solver.py:1112-1203)."""
-    ops = [_diffusion_op(k, k, f"r{k}_tendf", "mut", "xkmh", data) for k in ("u", "v", "w")]
-    ops.append(_diffusion_op("m", "t", "t_tendf", "mut", "xkhh", data, base=data["t_init"]))
+    ops = [_diffusion_op(k, k, f"r{k}_tendf", "mut", "xkmh") for k in ("u", "v", "w")]
+    ops.append(_diffusion_op("m", "t", "t_tendf", "mut", "xkhh", base="t_init"))
     ops += [_relax_op("ru", "u_save", bdy["u"], "u", dtbc), _relax_op("rv", "v_save", bdy["v"], "v", dtbc)]
     for k, var in (("ph", "h"), ("t", "t")):
         ops += [_mass_weight_op(k, "mut", "_mass", nz), _relax_op("_mass", f"{k}_save", bdy[var], var, dtbc)]
@@ -1862,29 +1861,29 @@ def dynamics_stage(st: dict, data: dict, bt: dict, rk_step: int, nsub: int, dts:
                      cfn=cfn, cfn1=cfn1)
     ops = [_table_chain_op(_CallOp("wrf_prep", PREP_FIELDS, PREP_OUTPUTS, PREP_DATA,
                                    lambda c, tab, s: L.wrf_prep(by(c), tab, 127, s),
-                                   lambda c, tab, b, s: L.wrf_prep_adj(by(c), tab, b, 127, s)), data),
+                                   lambda c, tab, b, s: L.wrf_prep_adj(by(c), tab, b, 127, s))),
            _halo_op(("ru", "rv", "rw", "ww", "php", "alt", "p", "muu", "muv", "mut", "al", "ph"), "uvwwwtpuvtpw")]
     zeros = ("ru_tend", "rv_tend", "rw_tend", "t_tend", "ph_tend", "u_save", "v_save", "w_save", "ph_save", "t_save",
              "mu_tend", "mu_save")
     if rk_step == 1:
         tendf = ("ru_tendf", "rv_tendf", "rw_tendf", "ph_tendf", "t_tendf", "mu_tendf", "moist_tend")
         ops += [_zero_op(k, k) for k in tendf]
-        ops += [_table_chain_op(_EddyViscosity(), data), _halo_op(("xkmh", "xkhh"), "tt")]
+        ops += [_table_chain_op(_EddyViscosity()), _halo_op(("xkmh", "xkhh"), "tt")]
     ops += [_zero_op(k, k) for k in zeros]
-    ops += [_advect_momentum_op(0, "u", "ru_tend", data), _advect_momentum_op(1, "v", "rv_tend", data),
-            _advect_momentum_op(2, "w", "rw_tend", data), _advect_scalar_op("t", "t_tend", data)]
+    ops += [_advect_momentum_op(0, "u", "ru_tend"), _advect_momentum_op(1, "v", "rv_tend"),
+            _advect_momentum_op(2, "w", "rw_tend"), _advect_scalar_op("t", "t_tend")]
     ops.append(_table_chain_op(_CallOp("wrf_forces", FORCES_INPUTS, FORCES_OUTPUTS, FORCES_DATA,
                                        lambda c, tab, s: L.wrf_forces(by(c), tab, 31, s),
-                                       lambda c, tab, b, s: L.wrf_forces_adj(by(c), tab, b, 31, s)), data))
+                                       lambda c, tab, b, s: L.wrf_forces_adj(by(c), tab, b, 31, s))))
     if rk_step == 1:
-        ops += _first_stage_ops(data, bt, dtbc, st["u"].shape[0])
-    ops.append(_table_chain_op(_Addtend(rk_step), data))
-    s = _run_chain(ops, cg, st)
+        ops += _first_stage_ops(bt, dtbc, st["u"].shape[0])
+    ops.append(_table_chain_op(_Addtend(rk_step)))
+    s = _run_chain(ops, cg, st, data)
     if theta_bias is not None:
         s["t_tend"] = s["t_tend"] + theta_bias
     ops = [_spec_tend_op(k, bt[var], var) for k, var in (("ru_tend", "u"), ("rv_tend", "v"), ("ph_tend", "h"),
                                                          ("t_tend", "t"), ("mu_tend", "m"))]
-    return _run_chain(ops + _acoustic_ops(data, rk_step, nsub, dts), cg, s)
+    return _run_chain(ops + _acoustic_ops(rk_step, nsub, dts), cg, s, data)
 
 
 class _MoistUpdate:
@@ -1920,15 +1919,15 @@ def moist_stage(st: dict, data: dict, rk_step: int, dt_rk: float, rdx, rdy, bt: 
     if rk_step == 1 and (bt is None or dtbc is None):
         raise ValueError("the first stage's qv relaxation needs its boundary arrays and dtbc")
     cg = scalar_grid(st["u"].shape, rdx, rdy)
-    ops = [_advect_moist_op(data)]
+    ops = [_advect_moist_op()]
     if rk_step == 1:
-        ops.append(_diffusion_op("m", "moist", "moist_tend", "muts", "xkhh", data))
+        ops.append(_diffusion_op("m", "moist", "moist_tend", "muts", "xkhh"))
         ops += _relax_qv_ops(st["u"].shape[0], bt["q"], dtbc)
     # (the averaged fluxes enter flow_dep_bdy by their sign alone)
-    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk), data, held=("ru_m", "rv_m")))
+    ops.append(_table_chain_op(_MoistUpdate(rk_step, dt_rk), held=("ru_m", "rv_m")))
     if rk_step < 3:
         ops.append(_halo_op(("u", "v", "w", "t", "ph", "mu", "moist"), "UVwpwtM"))
-    return _run_chain(ops, cg, st)
+    return _run_chain(ops, cg, st, data)
 
 
 def _relax_qv_ops(nz: int, bdy: dict, dtbc: float) -> list:
